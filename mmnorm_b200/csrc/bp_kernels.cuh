@@ -127,8 +127,21 @@ struct NuMeasParams {
     double ti, uq, k0c;       // 0.15 or 0; slope/c; 2pi(1/lambda + J0 slope/c)
     int32_t num_ant, n, mrow, ranges, F, J0;  // mrow = N + 16 cells
 };
-// forward in interpolation form (bp_fwd_nufft_kernel; BwdParams carries the nu fields)
-const void *fwd_nufft_kernel_ptr(int *threads, int *voxels_per_thread);
+// Interpolation form by tile-local polynomials (bp_local.cu).
+struct LocalParams {
+    FwdParams f;               // geometry, antenna records, outputs; tiles and antenna splits
+    const float2 *rows;        // [num_ant][row] antenna grids (G.re, G.im)
+    int32_t n, row;            // grid cells N = 2F, row length nufft_row_fwd(N)
+    double uq;                 // slope / c: turns per sample per metre of range
+    double k0c, t0c;           // anchor phase per metre at J0 = F/2: radians, turns
+    double t0c_fixed;          // -t0c * 2^32
+    float theta_per_m;         // pi F |slope| / c
+    int32_t bx, by, runs;      // tile: bx x by columns, runs of 4 voxels in z
+    int32_t tiles_y, tiles_z;
+};
+void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs);
+const void *fwd_local_kernel_ptr(int *threads);
+int local_chunk_antennas();
 size_t nufft_meas_smem(int mrow);
 int nufft_meas_warps();
 const void *nufft_meas_kernel_ptr();
@@ -136,11 +149,16 @@ cudaError_t launch_nufft_meas(const NuMeasParams &q, const FwdParams &p,
                               const float2 *grad_image, const float2 *grad_vote, float4 *rec,
                               cudaStream_t stream);
 const char *bwd_pos_nufft_variant_name(int variant);  // null for a bad index
-cudaError_t launch_nufft_tables(int F, int N, int J0, double *sc, double2 *tw,
-                                cudaStream_t stream);
+// box: 6 floats, the voxel coordinates' per-axis minima and maxima
+cudaError_t launch_nufft_tables(const FwdParams &p, int F, int N, int J0, double *sc, double2 *tw,
+                                float *box, cudaStream_t stream);
 cudaError_t launch_nufft_grid(const float *meas, int A, int F, int N, int J0, double k0,
-                              double kd, const double *sc, const double2 *tw, void *rows,
-                              bool fwd_only, cudaStream_t stream);
+                              double kd, const double *sc, const double2 *tw, float4 *rows,
+                              cudaStream_t stream);
+cudaError_t launch_nufft_grid_window(const float *meas, int A, int F, int N, int J0, int row,
+                                     const double *sc, const double2 *tw, const AntRec *ant,
+                                     const float *box, double ti, double uq, float2 *rows,
+                                     cudaStream_t stream);
 
 // ---------------------------------------------------------- interpolated mode
 struct InterpParams {

@@ -1,0 +1,484 @@
+// bp_local.cu -- the interpolation form by tile-local polynomials: the forward kernel of mode
+// "nufft" (mmn_backproject_nufft).
+//
+// One antenna's sample sum is e^{-2pi i d t0c} M(u), u = d slope/c, with M band-limited
+// (bp_nufft.cu).  Over a compact box of voxels u covers a short interval only, on which M is a
+// polynomial of low degree to FP32 accuracy.  So a CTA takes a box of up to 512 voxels (8 x 8 x
+// 8 on a large grid) and, for 32 antennas at a time,
+//   1. bounds each antenna's range over the box: centre d_c, half width D (FP32, widened);
+//   2. evaluates M at NN Chebyshev nodes of [d_c - D, d_c + D] by the 8-tap gather from the
+//      antenna's grid row (global memory: the few cells a box needs stay in L1/L2);
+//   3. turns the node values into polynomial coefficients in shared memory;
+//   4. runs its voxels through FP64 range, FP64-wrapped anchor, one Horner evaluation and the
+//      image + vote sums.
+// Per (voxel, antenna) that leaves NN packed FMAs on coefficients that all voxels of the thread
+// share, where a tap run per pair costs 44 FMAs of weights, 8 shared loads and the FP64 cell
+// index.  A thread owns 4 voxels in a row along z, whose lateral distance is one.
+//
+// NN follows from theta = pi F |slope| / c * D, the largest phase excursion of M over the half
+// width (local_nodes).  Up to NN = 12
+// the polynomial is evaluated in monomials by Horner (theta <= 2.6, so the coefficients' sum, and with it the FP32 rounding, stays within a few units); 16 and 24 by Clenshaw in the
+// Chebyshev basis.  An antenna whose theta is larger still (a 2 cm voxel pitch at 4 GHz of
+// bandwidth), or not a number, takes a tap run per voxel.
+//
+// Bound: instruction dispatch (68 instructions a pair, 235 dispatch slots a pair before; packed
+// FP32 and FP64 instructions take about two slots).  Measured on 96^3 voxels x 4096 antennas x
+// 200 samples: 23.5 ms for the whole forward with a tap run per pair, 9.2 ms with this kernel;
+// error against 64 bits 1.2e-6 before, 2.4e-7 now (sums over 32 antennas at a time).  96 or 80
+// registers (5 or 6 CTAs per SM) measured the same or 2 % slower than 128.  The hardware sine
+// and cosine in place of cis_half_pair: 8.1 ms, but 2.2e-7 of error on short sums, more than
+// the tap form's.
+#include <algorithm>
+#include <cmath>
+
+#include "bp_stage.cuh"
+#include "nufft_taps.cuh"
+
+namespace mmn {
+
+namespace {
+
+constexpr int kLocThreads = 128;
+constexpr int kLocRun = 4;      // voxels of a thread, consecutive in z
+constexpr int kLocAnts = 32;    // antennas per chunk
+constexpr int kLocNodes = 24;   // most nodes
+constexpr int kLocHorner = 12;  // most nodes evaluated in monomials
+
+// Monomial coefficients of the Chebyshev polynomials T_0 .. T_11.
+__constant__ float kChebMono[kLocHorner][kLocHorner] = {
+    {1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
+    {0, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
+    {-1, 0, 2, 0, 0, 0, 0, 0, 0, 0, 0, 0},
+    {0, -3, 0, 4, 0, 0, 0, 0, 0, 0, 0, 0},
+    {1, 0, -8, 0, 8, 0, 0, 0, 0, 0, 0, 0},
+    {0, 5, 0, -20, 0, 16, 0, 0, 0, 0, 0, 0},
+    {-1, 0, 18, 0, -48, 0, 32, 0, 0, 0, 0, 0},
+    {0, -7, 0, 56, 0, -112, 0, 64, 0, 0, 0, 0},
+    {1, 0, -32, 0, 160, 0, -256, 0, 128, 0, 0, 0},
+    {0, 9, 0, -120, 0, 432, 0, -576, 0, 256, 0, 0},
+    {-1, 0, 50, 0, -400, 0, 1120, 0, -1280, 0, 512, 0},
+    {0, -11, 0, 220, 0, -1232, 0, 2816, 0, -2816, 0, 1024},
+};
+
+// Nodes for a phase excursion theta: 2 (theta/2)^NN / NN! < 1.2e-7 at the band's edge, which
+// is about 3e-8 rms over its samples (the error of sample j' goes with |2 j'/F|^NN); 0: too
+// wide.
+__device__ __forceinline__ int local_nodes(float theta) {
+    if (theta <= 0.94f) return 8;
+    if (theta <= 1.72f) return 10;
+    if (theta <= 2.64f) return 12;
+    if (theta <= 4.8f) return 16;
+    if (theta <= 9.8f) return 24;
+    return 0;  // NaN lands here too
+}
+
+// One antenna of a chunk, as the voxel loop reads it.
+struct __align__(16) LocRec {
+    double tx[3], rx[3];
+    double inv, off;  // x = d * inv + off on [-1, 1]
+    float txf[3], rxf[3], u[3];
+    int nn;           // nodes; 0: a tap run per voxel
+};
+static_assert(sizeof(LocRec) % 16 == 0, "LocRec rows are read in 16-byte words");
+
+// Voxel box of a tile, by all threads of the CTA: per-axis minimum and maximum of the
+// coordinates it covers (any order of the coordinate arrays).
+__device__ __forceinline__ void tile_box(const float *locs, int first, int count, int total,
+                                         float &lo, float &hi) {
+    const int lane = threadIdx.x & 31;
+    float a = __int_as_float(0x7f800000), b = -a;
+    for (int i = lane; i < count && first + i < total; i += 32) {
+        const float v = __ldg(locs + first + i);
+        a = fminf(a, v);
+        b = fmaxf(b, v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+        b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+    }
+    lo = a;
+    hi = b;
+}
+
+// This thread's place in its tile and its voxels' coordinates (clamped into the grid, so that
+// an idle slot repeats a voxel of the box).
+struct LocSlot {
+    int ix, iy, iz;  // first voxel; the run is iz .. iz + 3
+    bool column;     // the (x, y) column is inside the grid
+};
+__device__ __forceinline__ LocSlot local_slot(const LocalParams &q, int tile, int slot) {
+    const FwdParams &p = q.f;
+    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
+    const int ty = txy % q.tiles_y, tx = txy / q.tiles_y;
+    const int used = q.bx * q.by * q.runs;
+    const int s = min(slot, used - 1);
+    const int run = s % q.runs, c = s / q.runs;
+    LocSlot o;
+    o.ix = tx * q.bx + c / q.by;
+    o.iy = ty * q.by + c % q.by;
+    o.iz = (tz * q.runs + run) * kLocRun;
+    o.column = slot < used && o.ix < p.nx && o.iy < p.ny;
+    return o;
+}
+
+// Table cos(pi m / (2 NN)), m < 4 NN, and the nodes cos(pi (i + 1/2) / NN) in FP64.
+__device__ __forceinline__ void cheb_tables(int nn, float *table, double *node) {
+    for (int m = threadIdx.x; m < 4 * nn; m += blockDim.x) {
+        const double c = cospi((double)m / (2 * nn));
+        table[m] = (float)c;
+        if ((m & 1) && m < 2 * nn) node[m >> 1] = c;
+    }
+}
+
+// h_k = sum_q cf[q] x_k^q for the thread's voxels.
+template <int NN>
+__device__ __forceinline__ void eval_mono(const float2 *cf, const float (&x)[kLocRun],
+                                          float2 (&h)[kLocRun]) {
+    const float4 *c4 = reinterpret_cast<const float4 *>(cf);
+    const float4 top = c4[NN / 2 - 1];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k)
+        h[k] = __ffma2_rn(make_float2(top.z, top.w), make_float2(x[k], x[k]),
+                          make_float2(top.x, top.y));
+#pragma unroll
+    for (int q = NN / 2 - 2; q >= 0; --q) {
+        const float4 c = c4[q];
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k) {
+            const float2 xx = make_float2(x[k], x[k]);
+            h[k] = __ffma2_rn(h[k], xx, make_float2(c.z, c.w));
+            h[k] = __ffma2_rn(h[k], xx, make_float2(c.x, c.y));
+        }
+    }
+}
+
+// The same from Chebyshev coefficients, by Clenshaw's recurrence.
+__device__ __forceinline__ void eval_cheb(const float2 *cf, int nn, const float (&x)[kLocRun],
+                                          float2 (&h)[kLocRun]) {
+    float2 b1[kLocRun], b2[kLocRun];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) b1[k] = b2[k] = make_float2(0.f, 0.f);
+    for (int q = nn - 1; q >= 1; --q) {
+        const float2 c = cf[q];
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k) {
+            const float2 dd = __fadd2_rn(c, make_float2(-b2[k].x, -b2[k].y));
+            b2[k] = b1[k];
+            b1[k] = __ffma2_rn(make_float2(2.f * x[k], 2.f * x[k]), b1[k], dd);
+        }
+    }
+    const float2 c = cf[0];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k)
+        h[k] = __ffma2_rn(make_float2(x[k], x[k]), b1[k],
+                          __fadd2_rn(c, make_float2(-b2[k].x, -b2[k].y)));
+}
+
+// M at one range by a tap run from the antenna's row in global memory.
+__device__ __forceinline__ float2 tap_run(const float2 *row, double d, double uq, int n) {
+    int ix;
+    float w[kNuW];
+    nufft_taps(d, uq, n, ix, w);
+    float2 h = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kNuW; ++i)
+        h = __ffma2_rn(make_float2(w[i], w[i]), __ldg(row + ix + i), h);
+    return h;
+}
+
+// The whole sum of one (voxel, antenna) pair by a tap run; not inlined, so that the wide-box
+// path stays out of the loops' register allocation.
+__device__ __noinline__ float2 pair_sum(const float2 *row, double d, double uq, double k0c,
+                                        int n) {
+    const float2 h = tap_run(row, d, uq, n);
+    const float2 an = cis_fp64_phase(-d * k0c);
+    return make_float2(fmaf(an.x, h.x, -an.y * h.y), fmaf(an.x, h.y, an.y * h.x));
+}
+
+// 1/sqrt of a sum of squares, subnormals flushed: one MUFU.
+__device__ __forceinline__ float rsqrt_seed(float s) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(s, 1e-30f)));
+    return r;
+}
+
+// Round-trip ranges of the thread's run in FP64.  Each leg is f = D r with r an FP32
+// reciprocal-square-root seed of the FP32 difference vector, plus one Newton correction
+// (D - f^2) r / 2 (relative error ~1e-13).
+template <bool MONO>
+__device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
+                                           const float (&vz)[kLocRun], double ti,
+                                           double (&d)[kLocRun]) {
+    const float ax = vx - a.txf[0], ay = vy - a.txf[1];
+    const float sxy = fmaf(ax, ax, ay * ay);
+    const double dx = (double)vx - a.tx[0], dy = (double)vy - a.tx[1];
+    const double Dxy = fma(dx, dx, dy * dy);
+    const float bx = vx - a.rxf[0], by = vy - a.rxf[1];
+    const float txy = fmaf(bx, bx, by * by);
+    const double ex = (double)vx - a.rx[0], ey = (double)vy - a.rx[1];
+    const double Exy = fma(ex, ex, ey * ey);
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        const float az = vz[k] - a.txf[2];
+        const double r = (double)rsqrt_seed(fmaf(az, az, sxy));
+        const double dz = (double)vz[k] - a.tx[2];
+        const double D = fma(dz, dz, Dxy);
+        const double f = D * r, e = fma(-f, f, D);
+        if (MONO) {
+            d[k] = fma(e, r, fma(2.0, f, ti));  // twice the leg
+        } else {
+            const float bz = vz[k] - a.rxf[2];
+            const double s = (double)rsqrt_seed(fmaf(bz, bz, txy));
+            const double ez = (double)vz[k] - a.rx[2];
+            const double E = fma(ez, ez, Exy);
+            const double g = E * s, h = fma(-g, g, E);
+            d[k] = fma(0.5, fma(h, s, e * r), f + (g + ti));
+        }
+    }
+}
+
+// Shared memory of one CTA.
+struct __align__(16) LocShared {
+    LocRec rec[kLocAnts];
+    float2 coef[kLocAnts][kLocNodes];
+    float2 node_val[kLocAnts][kLocNodes];
+    double centre[kLocAnts], half[kLocAnts];
+    double node[kLocNodes];
+    float table[4 * kLocNodes];
+    int nn;
+};
+
+// Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the chunk's node count (0: every
+// antenna takes tap runs).  Called by all threads; barriers inside.
+__device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, int a0, int na,
+                                           const float (&lo)[3], const float (&hi)[3],
+                                           int &table_nn) {
+    const FwdParams &p = q.f;
+    __syncthreads();  // the previous chunk's readers are done
+    if (threadIdx.x == 0) sh.nn = 0;
+    __syncthreads();
+    if (threadIdx.x < na) {
+        const AntRec ar = p.ant[a0 + threadIdx.x];
+        LocRec &r = sh.rec[threadIdx.x];
+        const float t[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
+        const float o[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
+        float c, half, dmax;
+        range_bounds(lo, hi, t, o, c, half, dmax);
+        const double centre = (double)c + p.ti;
+        const double inv = 1.0 / (double)half;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            r.tx[k] = ar.tx[k];
+            r.rx[k] = ar.rx[k];
+            r.txf[k] = t[k];
+            r.rxf[k] = o[k];
+            r.u[k] = ar.virt[k];
+        }
+        sh.centre[threadIdx.x] = centre;
+        sh.half[threadIdx.x] = (double)half;
+        r.inv = inv;
+        r.off = -centre * inv;
+        // the anchor's turn count must fit the fixed-point reduction (|turns| < 2^18)
+        const bool fits = ((double)dmax + p.ti) * fabs(q.t0c) < 262144.0;
+        r.nn = fits ? local_nodes(q.theta_per_m * half) : 0;
+        atomicMax(&sh.nn, r.nn);
+    }
+    __syncthreads();
+    const int nn = sh.nn;
+    if (nn == 0) return 0;
+    if (nn != table_nn) {
+        cheb_tables(nn, sh.table, sh.node);
+        table_nn = nn;
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
+        const int la = i / nn, j = i - la * nn;
+        const LocRec &r = sh.rec[la];
+        if (r.nn == 0) continue;
+        const double d = fma(sh.node[j], sh.half[la], sh.centre[la]);
+        sh.node_val[la][j] = tap_run(q.rows + (size_t)(a0 + la) * q.row, d, q.uq, q.n);
+    }
+    __syncthreads();
+    // Chebyshev coefficients c_p = (2 - [p = 0]) / NN sum_j M_j cos(pi p (2 j + 1) / (2 NN))
+    for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
+        const int la = i / nn, c = i - la * nn;
+        float2 s = make_float2(0.f, 0.f);
+        int m = c;
+        for (int j = 0; j < nn; ++j) {
+            const float t = sh.table[m];
+            s = __ffma2_rn(make_float2(t, t), sh.node_val[la][j], s);
+            m += 2 * c;
+            if (m >= 4 * nn) m -= 4 * nn;
+        }
+        const float sc = (c == 0 ? 1.f : 2.f) / (float)nn;
+        sh.coef[la][c] = make_float2(s.x * sc, s.y * sc);
+    }
+    __syncthreads();
+    if (nn <= kLocHorner) {
+        // monomials, through the node array (its values are used up)
+        for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
+            const int la = i / nn, c = i - la * nn;
+            float2 s = make_float2(0.f, 0.f);
+            for (int m = c; m < nn; m += 2) {
+                const float t = kChebMono[m][c];
+                s = __ffma2_rn(make_float2(t, t), sh.coef[la][m], s);
+            }
+            sh.node_val[la][c] = s;
+        }
+        __syncthreads();
+    }
+    return nn;
+}
+
+// Step 4 for one chunk.  NN: 8, 10, 12 monomials; 0: Chebyshev with nn coefficients (or tap
+// runs only, nn = 0).
+template <bool MONO, int NN>
+__device__ __forceinline__ void local_forward(const LocalParams &q, const LocShared &sh, int a0,
+                                              int na, int nn, float vx, float vy,
+                                              const float (&vz)[kLocRun],
+                                              float2 (&acc)[kLocRun][4]) {
+    const double kM = 6755399441055744.0;  // 1.5 * 2^52
+    for (int la = 0; la < na; ++la) {
+        const LocRec &a = sh.rec[la];
+        double d[kLocRun];
+        run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d);
+        float2 h[kLocRun];
+        if (a.nn > 0) {
+            float x[kLocRun];
+#pragma unroll
+            for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
+            if (NN > 0)
+                eval_mono<(NN > 0 ? NN : 8)>(sh.node_val[la], x, h);
+            else
+                eval_cheb(sh.coef[la], nn, x, h);
+            // times the anchor e^{-2 pi i d t0c}: wrapped turns in 2^-32 steps
+#pragma unroll
+            for (int k = 0; k < kLocRun; k += 2) {
+                float2 c, s;
+                cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
+                              __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), c, s);
+                h[k] = make_float2(fmaf(c.x, h[k].x, -s.x * h[k].y),
+                                   fmaf(c.x, h[k].y, s.x * h[k].x));
+                h[k + 1] = make_float2(fmaf(c.y, h[k + 1].x, -s.y * h[k + 1].y),
+                                       fmaf(c.y, h[k + 1].y, s.y * h[k + 1].x));
+            }
+        } else {
+            const float2 *row = q.rows + (size_t)(a0 + la) * q.row;
+#pragma unroll
+            for (int k = 0; k < kLocRun; ++k) h[k] = pair_sum(row, d[k], q.uq, q.k0c, q.n);
+        }
+        // the vote about the run's first voxel: the others' share is (z_0 - z_k) I at the end
+        const float ux = a.u[0] - vx, uy = a.u[1] - vy, uz = a.u[2] - vz[0];
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k) {
+            acc[k][0] = __fadd2_rn(acc[k][0], h[k]);
+            acc[k][1] = __ffma2_rn(h[k], make_float2(ux, ux), acc[k][1]);
+            acc[k][2] = __ffma2_rn(h[k], make_float2(uy, uy), acc[k][2]);
+            acc[k][3] = __ffma2_rn(h[k], make_float2(uz, uz), acc[k][3]);
+        }
+    }
+}
+
+template <bool MONO>
+__device__ __forceinline__ void local_forward_nn(const LocalParams &q, const LocShared &sh, int a0,
+                                                 int na, int nn, float vx, float vy,
+                                                 const float (&vz)[kLocRun],
+                                                 float2 (&acc)[kLocRun][4]) {
+    if (nn == 8) local_forward<MONO, 8>(q, sh, a0, na, nn, vx, vy, vz, acc);
+    else if (nn == 10) local_forward<MONO, 10>(q, sh, a0, na, nn, vx, vy, vz, acc);
+    else if (nn == 12) local_forward<MONO, 12>(q, sh, a0, na, nn, vx, vy, vz, acc);
+    else local_forward<MONO, 0>(q, sh, a0, na, nn, vx, vy, vz, acc);
+}
+
+}  // namespace
+
+// grid = tiles x antenna splits.
+__global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const LocalParams q) {
+    __shared__ LocShared sh;
+    // sums over the chunks done: a chunk's 32 antennas are summed in registers and added here,
+    // which keeps the FP32 rounding of the long antenna sum down
+    __shared__ float2 total[kLocRun][4][kLocThreads];
+    const FwdParams &p = q.f;
+    const int tile = blockIdx.x % p.num_tiles, split = blockIdx.x / p.num_tiles;
+    const int a_begin = split * p.ant_per_split;
+    const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
+    float lo[3], hi[3];
+    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
+    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
+    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
+    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    const LocSlot s = local_slot(q, tile, threadIdx.x);
+    const float vx = __ldg(p.x_locs + min(s.ix, p.nx - 1));
+    const float vy = __ldg(p.y_locs + min(s.iy, p.ny - 1));
+    float vz[kLocRun];
+    float2 acc[kLocRun][4];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        vz[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
+#pragma unroll
+        for (int c = 0; c < 4; ++c) total[k][c][threadIdx.x] = make_float2(0.f, 0.f);
+    }
+    const bool mono = *p.mono_flag != 0;
+    int table_nn = 0;
+    for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
+        const int na = min(kLocAnts, a_end - a0);
+        const int nn = local_chunk(q, sh, a0, na, lo, hi, table_nn);
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[k][c] = make_float2(0.f, 0.f);
+        if (mono) local_forward_nn<true>(q, sh, a0, na, nn, vx, vy, vz, acc);
+        else local_forward_nn<false>(q, sh, a0, na, nn, vx, vy, vz, acc);
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                total[k][c][threadIdx.x] = __fadd2_rn(total[k][c][threadIdx.x], acc[k][c]);
+    }
+    if (!s.column) return;
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        if (s.iz + k >= p.nz) continue;
+        const int64_t v = ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[k][c] = total[k][c][threadIdx.x];
+        const float dz = vz[0] - vz[k];
+        acc[k][3] = __ffma2_rn(acc[k][0], make_float2(dz, dz), acc[k][3]);
+        const float a[8] = {acc[k][0].x, acc[k][0].y, acc[k][1].x, acc[k][1].y,
+                            acc[k][2].x, acc[k][2].y, acc[k][3].x, acc[k][3].y};
+        store_voxel(p, split, v, a);
+    }
+}
+
+// Tile shape: columns bx x by and runs of 4 voxels in z, at most 128 runs, chosen for few
+// tiles (idle slots of a ragged grid cost as much as used ones) with a charge for elongated
+// boxes, whose wider range interval needs more nodes.  8 x 8 x 8 on a large grid.
+void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs) {
+    double best = 1e300;
+    const int zr = (nz + kLocRun - 1) / kLocRun;
+    for (int r = 1; r <= std::min(zr, 16); ++r)
+        for (int y = 1; y <= std::min(ny, 32) && r * y <= kLocThreads; ++y) {
+            const int x = std::min({nx, kLocThreads / (r * y), 32});
+            const double tiles = (double)((nx + x - 1) / x) * ((ny + y - 1) / y) *
+                                 ((zr + r - 1) / r);
+            const double diag2 = (double)x * x + (double)y * y +
+                                 (double)(kLocRun * r) * (kLocRun * r);
+            const double cost = tiles * (1.0 + 0.01 * std::max(0.0, std::sqrt(diag2) - 13.9));
+            if (cost < best) {
+                best = cost;
+                *bx = x;
+                *by = y;
+                *runs = r;
+            }
+        }
+}
+
+const void *fwd_local_kernel_ptr(int *threads) {
+    *threads = kLocThreads;
+    return reinterpret_cast<const void *>(&bp_fwd_local_kernel);
+}
+
+int local_chunk_antennas() { return kLocAnts; }
+
+}  // namespace mmn

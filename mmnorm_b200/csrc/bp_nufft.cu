@@ -27,16 +27,17 @@
 // the warp in lane j.  Lanes whose cells fall outside a 16-cell window wait for the next
 // round, so any spread of distances is handled.
 //
-// Kernels: nufft_tables_kernel (1/phihat by midpoint quadrature in FP64, twiddles),
-// nufft_grid_kernel (per-antenna grids by a direct FP64 transform: F x (N + W - 1) per
-// antenna, small next to the voxel work), bp_bwd_pos_nufft_kernel (the forward's tiling and
+// Kernels: nufft_tables_kernel (1/phihat by midpoint quadrature in FP64, twiddles, the voxel
+// box), nufft_grid_window_kernel (the forward's per-antenna grids, only the cells that the
+// voxel box can reach; bp_local.cu reads them), nufft_grid_kernel (per-antenna grids by a
+// direct FP64 transform: F x (N + W - 1) per antenna), bp_bwd_pos_nufft_kernel (the forward's tiling and
 // double-buffered antenna staging, rows of N + W - 1 cells so no tap wraps; per-antenna
 // sums over a CTA's voxels go to the same per-tile partials as the Horner form),
 // nufft_vox_kernel + bp_bwd_meas_nufft_kernel + nufft_meas_out_kernel (measurement pass).
 #include <algorithm>
 
 #include "bp_stage.cuh"
-#include "es_taps.cuh"
+#include "nufft_taps.cuh"
 
 namespace mmn {
 
@@ -53,85 +54,54 @@ __device__ __forceinline__ double es_kernel(double z) {
 
 }  // namespace
 
-// Per (voxel, antenna) geometry of the interpolation form.
-//   d      round-trip range in FP64.  Each leg's square root starts from an FP32 rsqrt of the
-//          FP32 difference vector and takes one FP64 Newton step (relative error ~1e-13, far
-//          below what the phase needs), which avoids the IEEE FP64 square root's slow path.
-//   e3     -(unit(v - tx) + unit(v - rx)) in FP32 (the derivative of d with respect to an
-//          antenna offset; a direction needs no more).
-//   ix, s  grid cell and fractional offset of N * (u mod 1), u = d slope/c, reduced with the
-//          1.5*2^52 rounding constant (no conversion instructions); clamped so that a NaN or a
-//          fraction that rounds up to 1 still reads inside the row.
-//   w[8]   tap weights (es_taps.cuh): P_i(t) and P_i(-t) from one even and one odd part.
-struct NuPair {
-    double d;
-    float e3[3];
-    int ix;
-    float w[kNuW];
-};
-
-__device__ __forceinline__ void nufft_pair(double vxd, double vyd, double vzd, float vx, float vy,
-                                           float vz, const AntRec &ar, const float (&txf)[3],
-                                           const float (&rxf)[3], bool mono, double ti, double uq,
-                                           int n, NuPair &o) {
-    const float ax = vx - txf[0], ay = vy - txf[1], az = vz - txf[2];
-    const float rf = rsqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-    const double dx = vxd - ar.tx[0], dy = vyd - ar.tx[1], dz = vzd - ar.tx[2];
-    const double D = fma(dx, dx, fma(dy, dy, dz * dz));
-    const double r = (double)rf;
-    double f = D * r;
-    f = fma(fma(-f, f, D), 0.5 * r, f);
-    double b = f;
-    float bx = ax, by = ay, bz = az, rb = rf;
-    if (!mono) {
-        bx = vx - rxf[0];
-        by = vy - rxf[1];
-        bz = vz - rxf[2];
-        rb = rsqrtf(fmaf(bx, bx, fmaf(by, by, bz * bz)));
-        const double ex = vxd - ar.rx[0], ey = vyd - ar.rx[1], ez = vzd - ar.rx[2];
-        const double B = fma(ex, ex, fma(ey, ey, ez * ez));
-        const double rr = (double)rb;
-        b = B * rr;
-        b = fma(fma(-b, b, B), 0.5 * rr, b);
+// Per-axis bounds of the voxel coordinates, by one block: box = (min x, y, z, max x, y, z).
+__device__ void coordinate_box(const float *xs, int nx, const float *ys, int ny, const float *zs,
+                               int nz, float *box) {
+    __shared__ float s_lo[3][32], s_hi[3][32];
+    const float *arr[3] = {xs, ys, zs};
+    const int cnt[3] = {nx, ny, nz};
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float lo = __int_as_float(0x7f800000), hi = -lo;
+        for (int i = threadIdx.x; i < cnt[k]; i += blockDim.x) {
+            const float v = arr[k][i];
+            lo = fminf(lo, v);
+            hi = fmaxf(hi, v);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) {
+            s_lo[k][warp] = lo;
+            s_hi[k][warp] = hi;
+        }
     }
-    o.d = f + b + ti;
-    o.e3[0] = -fmaf(ax, rf, bx * rb);
-    o.e3[1] = -fmaf(ay, rf, by * rb);
-    o.e3[2] = -fmaf(az, rf, bz * rb);
-
-    const double kRound = 6755399441055744.0;  // 1.5 * 2^52
-    const double u = o.d * uq;
-    double uf = u - ((u + kRound) - kRound);  // [-1/2, 1/2]
-    uf = uf < 0.0 ? uf + 1.0 : uf;            // [0, 1]
-    const double x = uf * (double)n;
-    const double xt = x + kRound;
-    int ix = __double2loint(xt);
-    double fr = x - (xt - kRound);             // [-1/2, 1/2]
-    ix = fr < 0.0 ? ix - 1 : ix;
-    fr = fr < 0.0 ? fr + 1.0 : fr;
-    float sfr = (float)fr;
-    const bool lo = !(ix >= 0), hi = ix >= n;
-    ix = lo ? 0 : (hi ? n - 1 : ix);
-    sfr = lo ? 0.f : (hi ? 1.f : sfr);
-    o.ix = ix;
-
-    const float t = sfr - 0.5f, t2 = t * t;
-#pragma unroll
-    for (int i = 0; i < kNuW / 2; ++i) {
-        float e = kEsEven[i][kEsEvenTerms - 1];
-#pragma unroll
-        for (int q = kEsEvenTerms - 2; q >= 0; --q) e = fmaf(e, t2, kEsEven[i][q]);
-        float od = kEsOdd[i][kEsOddTerms - 1];
-#pragma unroll
-        for (int q = kEsOddTerms - 2; q >= 0; --q) od = fmaf(od, t2, kEsOdd[i][q]);
-        o.w[i] = fmaf(t, od, e);
-        o.w[kNuW - 1 - i] = fmaf(-t, od, e);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        float lo = s_lo[k][0], hi = s_hi[k][0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            lo = fminf(lo, s_lo[k][w]);
+            hi = fmaxf(hi, s_hi[k][w]);
+        }
+        box[k] = lo;
+        box[3 + k] = hi;
     }
 }
 
-// sc[j] = 1 / phihat((j - J0) / N) for j < F (one warp per j), tw[k] = e^{-2pi i k/N}.
+// sc[j] = 1 / phihat((j - J0) / N) for j < F (one warp per j), tw[k] = e^{-2pi i k/N}; the
+// last block writes the voxel box.
 __global__ void nufft_tables_kernel(int F, int N, int J0, double *__restrict__ sc,
-                                    double2 *__restrict__ tw) {
+                                    double2 *__restrict__ tw, const float *xs, int nx,
+                                    const float *ys, int ny, const float *zs, int nz,
+                                    float *__restrict__ box) {
+    if (blockIdx.x == gridDim.x - 1) {
+        coordinate_box(xs, nx, ys, ny, zs, nz, box);
+        return;
+    }
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t gw = gid >> 5;
     const int lane = threadIdx.x & 31;
@@ -154,15 +124,67 @@ __global__ void nufft_tables_kernel(int F, int N, int J0, double *__restrict__ s
     }
 }
 
+// The cells an antenna's tap runs can touch while its range stays inside the voxel box:
+// first cell (any integer, to be taken mod N) and count; all N when the window is not shorter
+// or not a number.
+__device__ __forceinline__ void cell_window(const float *box, const AntRec &ar, double ti,
+                                            double uq, int N, int &first, int &count) {
+    const float lo[3] = {box[0], box[1], box[2]}, hi[3] = {box[3], box[4], box[5]};
+    const float t[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
+    const float r[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
+    float c, half, dmax;
+    range_bounds(lo, hi, t, r, c, half, dmax);
+    const double a = ((double)c - half + ti) * uq * N, b = ((double)c + half + ti) * uq * N;
+    const double k0 = floor(fmin(a, b)) - kNuW / 2, k1 = floor(fmax(a, b)) + kNuW / 2 + 1;
+    first = 0;
+    count = N;
+    if (k1 - k0 + 1.0 < (double)N && fabs(k0) < 1e9) {
+        first = (int)k0;
+        count = (int)(k1 - k0) + 1;
+    }
+}
+
+// Forward rows: rows[a][jj] = (G_k.re, G_k.im) for cell k = (jj - (W/2 - 1)) mod N, jj < row.
+// One warp per antenna, one lane per cell, over the cells of the antenna's window only: a
+// 0.19 m grid at 4 GHz touches about 30 of the 400 cells of 200 samples (592 us for all cells
+// of 4096 antennas).  Cells outside the window are left unwritten and are never read.
+constexpr int kGridWarps = 4;
+__global__ void __launch_bounds__(kGridWarps * 32)
+    nufft_grid_window_kernel(const float2 *__restrict__ meas, int A, int F, int N, int J0, int row,
+                             const double *__restrict__ sc, const double2 *__restrict__ tw,
+                             const AntRec *__restrict__ ant, const float *__restrict__ box,
+                             double ti, double uq, float2 *__restrict__ rows) {
+    const int a = blockIdx.x * kGridWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (a >= A) return;
+    int first, count;
+    cell_window(box, ant[a], ti, uq, N, first, count);
+    const float2 *m = meas + (size_t)a * F;
+    float2 *out = rows + (size_t)a * row;
+    for (int c = lane; c < count; c += 32) {
+        const int k = (int)((((int64_t)first + c) % N + N) % N);
+        int idx = (int)((((int64_t)(-J0) * k) % N + N) % N);  // (j - J0) k mod N at j = 0
+        double gr = 0.0, gi = 0.0;
+#pragma unroll 4
+        for (int j = 0; j < F; ++j) {
+            const float2 mv = __ldg(m + j);
+            const double s = __ldg(sc + j);
+            const double2 t = __ldg(tw + idx);
+            const double ar = s * (double)mv.x, ai = s * (double)mv.y;
+            gr += fma(ar, t.x, -ai * t.y);
+            gi += fma(ar, t.y, ai * t.x);
+            idx += k;
+            if (idx >= N) idx -= N;
+        }
+        for (int jj = (k + kNuW / 2 - 1) % N; jj < row; jj += N)
+            out[jj] = make_float2((float)gr, (float)gi);
+    }
+}
+
 // rows[a][jj] = (G'_k.re, G_k.re, G'_k.im, G_k.im) for cell k = (jj - (W/2 - 1)) mod N,
-// jj < N + W - 1: a tap run starting at any cell reads W consecutive entries.  FWD_ONLY:
-// the forward reads only G, so its rows are (G_k.re, G_k.im) -- 8 bytes a cell -- and the
-// G' sums are not formed; those rows carry one more cell (never read) to an even length,
-// which keeps them multiples of 16 bytes for the bulk copies.
-template <bool FWD_ONLY>
+// jj < N + W - 1: a tap run starting at any cell reads W consecutive entries.
 __global__ void nufft_grid_kernel(const float2 *__restrict__ meas, int F, int N, int J0, int row,
                                   double k0, double kd, const double *__restrict__ sc,
-                                  const double2 *__restrict__ tw, void *__restrict__ rows,
+                                  const double2 *__restrict__ tw, float4 *__restrict__ rows,
                                   int blocks_per_row) {
     const int a = blockIdx.x / blocks_per_row;
     const int jj = (blockIdx.x - a * blocks_per_row) * blockDim.x + threadIdx.x;
@@ -179,19 +201,13 @@ __global__ void nufft_grid_kernel(const float2 *__restrict__ meas, int F, int N,
         const double pr = fma(ar, t.x, -ai * t.y), pi = fma(ar, t.y, ai * t.x);
         gr += pr;
         gi += pi;
-        if (!FWD_ONLY) {
-            const double kap = fma((double)j, kd, k0);
-            hr = fma(kap, pr, hr);
-            hi = fma(kap, pi, hi);
-        }
+        const double kap = fma((double)j, kd, k0);
+        hr = fma(kap, pr, hr);
+        hi = fma(kap, pi, hi);
         idx += k;
         if (idx >= N) idx -= N;
     }
-    if (FWD_ONLY)
-        static_cast<float2 *>(rows)[(size_t)a * row + jj] = make_float2((float)gr, (float)gi);
-    else
-        static_cast<float4 *>(rows)[(size_t)a * row + jj] =
-            make_float4((float)hr, (float)gr, (float)hi, (float)gi);
+    rows[(size_t)a * row + jj] = make_float4((float)hr, (float)gr, (float)hi, (float)gi);
 }
 
 // Position pass, interpolation form.  VOTE: the loss has a vote term (grad_vote set).
@@ -354,115 +370,6 @@ const NuVariant kNuVariants[] = {
     MMN_NU_VARIANT(1, 128, 16),
 };
 #undef MMN_NU_VARIANT
-
-// ---------------------------------------------------------------- forward pass
-// The forward's per-(voxel, antenna) sum c = sum_j m_j p_j by the same 8-tap gather as the
-// position pass (the rows' G cells), accumulated as I += c, W += c (virt - v) per voxel
-// over the CTA's antennas; results go through store_voxel (direct or per-split partials).
-template <int T, int NT>
-__global__ void __launch_bounds__(NT) bp_fwd_nufft_kernel(const BwdParams bp) {
-    const FwdParams &p = bp.f;
-    extern __shared__ __align__(128) unsigned char smem[];
-    Stage st;
-    st.bars = reinterpret_cast<uint64_t *>(smem);
-    st.base = smem + 128;
-    st.nas = p.ant_per_stage;
-    st.esz = 8;    // (G.re, G.im) cells
-    st.fp = p.fp;  // grid row length N + W - 1
-    st.stage_bytes = (size_t)st.nas * sizeof(AntRec) + (size_t)st.nas * st.fp * st.esz;
-    const int row_len = p.fp;
-    const int n = bp.nu_n;
-    const double uq = bp.nu_u, k0c = bp.nu_k0c;
-    const int tile = blockIdx.x % p.num_tiles;
-    const int split = blockIdx.x / p.num_tiles;
-    const int a_begin = split * p.ant_per_split;
-    const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
-    const int n_chunks = a_end > a_begin ? (a_end - a_begin + st.nas - 1) / st.nas : 0;
-
-    if (threadIdx.x == 0) {
-        mbar_init(&st.bars[0], 1);
-        mbar_init(&st.bars[1], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (n_chunks > 0) st.issue(p, 0, a_begin, a_end);
-        if (n_chunks > 1) st.issue(p, 1, a_begin, a_end);
-    }
-
-    const int64_t rbase = (int64_t)tile * (NT * T) + threadIdx.x;
-    float vx[T], vy[T], vz[T];
-    double vxd[T], vyd[T], vzd[T];
-    float acc[T][8];
-#pragma unroll
-    for (int k = 0; k < T; ++k) {
-        decode_voxel(p, rbase + (int64_t)k * NT, vx[k], vy[k], vz[k]);
-        vxd[k] = vx[k];
-        vyd[k] = vy[k];
-        vzd[k] = vz[k];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) acc[k][q] = 0.f;
-    }
-    const bool mono = *p.mono_flag != 0;
-
-    int c_failed = -1;  // chunk whose wait gave up; the drain runs after the loop
-    for (int c = 0; c < n_chunks; ++c) {
-        const int s = c & 1;
-        bool ok = mbar_wait_bounded(&st.bars[s], (uint32_t)((c >> 1) & 1), p.status);
-        if (!__syncthreads_and(ok)) {
-            c_failed = c;
-            break;
-        }
-        const AntRec *ants = st.ants(s);
-        const float2 *mstage = reinterpret_cast<const float2 *>(st.meas(s));
-        const int a0 = a_begin + c * st.nas;
-        const int na = min(st.nas, a_end - a0);
-        for (int a = 0; a < na; ++a) {
-            const AntRec &ar = ants[a];
-            const float2 *row = mstage + (size_t)a * row_len;
-            const float txf[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
-            const float rxf[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
-#pragma unroll
-            for (int k = 0; k < T; ++k) {
-                NuPair g;
-                nufft_pair(vxd[k], vyd[k], vzd[k], vx[k], vy[k], vz[k], ar, txf, rxf, mono, p.ti,
-                           uq, n, g);
-                float2 h = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < kNuW; ++i)
-                    h = __ffma2_rn(make_float2(g.w[i], g.w[i]), row[g.ix + i], h);
-                const float2 an = cis_fp64_phase(-g.d * k0c);
-                const float cr = fmaf(an.x, h.x, -an.y * h.y), ci = fmaf(an.x, h.y, an.y * h.x);
-                const float u0 = ar.virt[0] - vx[k], u1 = ar.virt[1] - vy[k],
-                            u2 = ar.virt[2] - vz[k];
-                acc[k][0] += cr;
-                acc[k][1] += ci;
-                acc[k][2] = fmaf(cr, u0, acc[k][2]);
-                acc[k][3] = fmaf(ci, u0, acc[k][3]);
-                acc[k][4] = fmaf(cr, u1, acc[k][4]);
-                acc[k][5] = fmaf(ci, u1, acc[k][5]);
-                acc[k][6] = fmaf(cr, u2, acc[k][6]);
-                acc[k][7] = fmaf(ci, u2, acc[k][7]);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0 && c + 2 < n_chunks) st.issue(p, c + 2, a_begin, a_end);
-    }
-    if (c_failed >= 0) {
-        st.drain_after_timeout((uint32_t)c_failed, c_failed + 1 < n_chunks, p.status);
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < T; ++k) store_voxel(p, split, rbase + (int64_t)k * NT, acc[k]);
-}
-
-constexpr int kNuFwdT = 2, kNuFwdNT = 128;
-
-const void *fwd_nufft_kernel_ptr(int *threads, int *voxels_per_thread) {
-    *threads = kNuFwdNT;
-    *voxels_per_thread = kNuFwdT;
-    return reinterpret_cast<const void *>(&bp_fwd_nufft_kernel<kNuFwdT, kNuFwdNT>);
-}
 
 // ------------------------------------------------------------- measurement pass
 
@@ -665,29 +572,32 @@ const void *bwd_pos_nufft_kernel_ptr(int variant, bool vote, int *threads, int *
     return vote ? v.fn_vote : v.fn_img;
 }
 
-cudaError_t launch_nufft_tables(int F, int N, int J0, double *sc, double2 *tw,
-                                cudaStream_t stream) {
+cudaError_t launch_nufft_tables(const FwdParams &p, int F, int N, int J0, double *sc, double2 *tw,
+                                float *box, cudaStream_t stream) {
     const int nt = 256;
     const int64_t tthreads = std::max<int64_t>((int64_t)F * 32, N);
-    nufft_tables_kernel<<<(unsigned)((tthreads + nt - 1) / nt), nt, 0, stream>>>(F, N, J0, sc,
-                                                                                 tw);
+    nufft_tables_kernel<<<(unsigned)((tthreads + nt - 1) / nt) + 1, nt, 0, stream>>>(
+        F, N, J0, sc, tw, p.x_locs, p.nx, p.y_locs, p.ny, p.z_locs, p.nz, box);
     return cudaGetLastError();
 }
 
 cudaError_t launch_nufft_grid(const float *meas, int A, int F, int N, int J0, double k0,
-                              double kd, const double *sc, const double2 *tw, void *rows,
-                              bool fwd_only, cudaStream_t stream) {
+                              double kd, const double *sc, const double2 *tw, float4 *rows,
+                              cudaStream_t stream) {
     const int nt = 256;
-    const int row = fwd_only ? nufft_row_fwd(N) : nufft_row(N);
+    const int row = nufft_row(N);
     const int bpr = (row + nt - 1) / nt;
-    const unsigned grid = (unsigned)((int64_t)A * bpr);
-    const float2 *m = reinterpret_cast<const float2 *>(meas);
-    if (fwd_only)
-        nufft_grid_kernel<true><<<grid, nt, 0, stream>>>(m, F, N, J0, row, k0, kd, sc, tw, rows,
-                                                         bpr);
-    else
-        nufft_grid_kernel<false><<<grid, nt, 0, stream>>>(m, F, N, J0, row, k0, kd, sc, tw, rows,
-                                                          bpr);
+    nufft_grid_kernel<<<(unsigned)((int64_t)A * bpr), nt, 0, stream>>>(
+        reinterpret_cast<const float2 *>(meas), F, N, J0, row, k0, kd, sc, tw, rows, bpr);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nufft_grid_window(const float *meas, int A, int F, int N, int J0, int row,
+                                     const double *sc, const double2 *tw, const AntRec *ant,
+                                     const float *box, double ti, double uq, float2 *rows,
+                                     cudaStream_t stream) {
+    nufft_grid_window_kernel<<<(A + kGridWarps - 1) / kGridWarps, kGridWarps * 32, 0, stream>>>(
+        reinterpret_cast<const float2 *>(meas), A, F, N, J0, row, sc, tw, ant, box, ti, uq, rows);
     return cudaGetLastError();
 }
 

@@ -807,7 +807,7 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
     pl->off_nutab = off;  // interpolation form: twiddles [N] double2, then 1/phihat [F] doubles
     if (pl->nufft || pl->meas_nufft)
         off = align_up(off + (size_t)p->num_samples * sizeof(double) +
-                       (size_t)pl->nu_n * sizeof(double2));
+                       (size_t)pl->nu_n * sizeof(double2) + 32);
     pl->off_nvox = pl->off_npart = off;
     if (pl->meas_nufft) {
         // voxel ranges: enough (antenna group, range) CTAs for two waves
@@ -870,9 +870,22 @@ extern "C" size_t mmn_backward_workspace_bytes(const mmn_problem *p) {
 // ---------------------------------------------------------------------------------
 namespace {
 
+void set_local_fields(LocalParams &q, const mmn_problem *p, int n, int row, const float2 *rows) {
+    const int F = p->num_samples, J0 = F / 2;
+    q.rows = rows;
+    q.n = n;
+    q.row = row;
+    q.uq = p->slope / kC;
+    q.t0c = 1.0 / p->wavelength + (double)J0 * p->slope / kC;
+    q.k0c = 2.0 * kPi * q.t0c;
+    q.t0c_fixed = -q.t0c * 4294967296.0;
+    q.theta_per_m = (float)(kPi * F * std::fabs(p->slope) / kC);
+}
+
 struct NuFwdPlan {
-    int n, row, threads, vpt, ant_per_stage, tiles, splits, ant_per_split;
-    size_t smem, off_ant, off_rows, off_tab, off_part, total;
+    int n, row, threads, tiles, splits, ant_per_split;
+    int bx, by, runs, tiles_y, tiles_z;
+    size_t off_ant, off_rows, off_tab, off_part, total;
     const void *fn;
 };
 
@@ -880,30 +893,28 @@ int plan_nufft_forward(const mmn_problem *p, NuFwdPlan *pl) {
     const int A = p->num_antennas, F = p->num_samples;
     const int64_t nvox = (int64_t)p->num_x * p->num_y * p->num_z;
     pl->n = 2 * F;
-    pl->row = nufft_row_fwd(pl->n);  // even: rows of 16-byte multiples
-    const int rec = (int)sizeof(AntRec) + pl->row * 8;  // (G.re, G.im) cells
-    if (rec > kMaxStageBytes) return MMN_ERR_TOO_LARGE;
-    if ((pl->row * 8) % 16 != 0) return MMN_ERR_UNSUPPORTED;  // bulk copies need 16 B rows
-    pl->fn = fwd_nufft_kernel_ptr(&pl->threads, &pl->vpt);
-    pl->ant_per_stage = std::max(1, std::min(16, 24 * 1024 / rec));
-    pl->smem = 128 + 2 * (size_t)pl->ant_per_stage * rec;
-    const int64_t per_tile = (int64_t)pl->threads * pl->vpt;
-    const int64_t tiles = (nvox + per_tile - 1) / per_tile;
+    pl->row = nufft_row_fwd(pl->n);
+    // the longest row: (G.re, G.im) cells and the antenna record within 48 KB
+    if ((int)sizeof(AntRec) + pl->row * 8 > kMaxStageBytes) return MMN_ERR_TOO_LARGE;
+    pl->fn = fwd_local_kernel_ptr(&pl->threads);
+    plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
+    pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
+    pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
+    const int64_t tiles = (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
-    pl->tiles = (int)std::max<int64_t>(1, tiles);
+    pl->tiles = (int)tiles;
+    const int chunk = local_chunk_antennas();
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (pl->smem > 48 * 1024)
-        cudaFuncSetAttribute(pl->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl->smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pl->fn, pl->threads, pl->smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pl->fn, pl->threads, 0) !=
             cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
     const int64_t slots = (int64_t)sms * per_sm;
     int best_s = 1;
     double best_cost = 1e300;
-    const int max_s = std::max(1, std::min(64, (A + pl->ant_per_stage - 1) / pl->ant_per_stage));
+    const int max_s = std::max(1, std::min(64, (A + chunk - 1) / chunk));
     for (int s = 1; s <= max_s; ++s) {
         const int64_t ctas = (int64_t)pl->tiles * s;
         const double waves = (double)((ctas + slots - 1) / slots);
@@ -915,7 +926,7 @@ int plan_nufft_forward(const mmn_problem *p, NuFwdPlan *pl) {
         if (ctas >= 8 * slots) break;
     }
     int aps = (A + best_s - 1) / best_s;
-    aps = (aps + pl->ant_per_stage - 1) / pl->ant_per_stage * pl->ant_per_stage;
+    aps = (aps + chunk - 1) / chunk * chunk;
     pl->ant_per_split = std::max(aps, 1);
     pl->splits = std::max(1, (A + pl->ant_per_split - 1) / pl->ant_per_split);
     size_t off = kStatusBytes;
@@ -923,8 +934,8 @@ int plan_nufft_forward(const mmn_problem *p, NuFwdPlan *pl) {
     off = align_up(off + (size_t)A * sizeof(AntRec));
     pl->off_rows = off;
     off = align_up(off + (size_t)A * pl->row * 8);
-    pl->off_tab = off;
-    off = align_up(off + (size_t)pl->n * sizeof(double2) + (size_t)F * sizeof(double));
+    pl->off_tab = off;  // twiddles, 1/phihat, voxel box
+    off = align_up(off + (size_t)pl->n * sizeof(double2) + (size_t)F * sizeof(double) + 32);
     pl->off_part = off;
     if (pl->splits > 1) off = align_up(off + (size_t)pl->splits * nvox * 2 * sizeof(float4));
     pl->total = off;
@@ -970,14 +981,10 @@ extern "C" int mmn_backproject_nufft(const mmn_problem *p, float *image, float *
     const int J0 = F / 2;
     double2 *tw = reinterpret_cast<double2 *>(ws + pl.off_tab);
     double *sc = reinterpret_cast<double *>(tw + pl.n);
-    const double k0 = 2.0 * kPi / p->wavelength, kd = 2.0 * kPi * p->slope / kC;
-    if (launch_nufft_tables(F, pl.n, J0, sc, tw, stream) != cudaSuccess) return MMN_ERR_CUDA;
-    if (launch_nufft_grid(p->meas, A, F, pl.n, J0, k0, kd, sc, tw, ws + pl.off_rows, true,
-                          stream) != cudaSuccess)
-        return MMN_ERR_CUDA;
-    BwdParams bq;
-    std::memset(&bq, 0, sizeof(bq));
-    FwdParams &f = bq.f;
+    float *box = reinterpret_cast<float *>(sc + F);
+    LocalParams q;
+    std::memset(&q, 0, sizeof(q));
+    FwdParams &f = q.f;
     f.x_locs = p->x_locs;
     f.y_locs = p->y_locs;
     f.z_locs = p->z_locs;
@@ -988,10 +995,7 @@ extern "C" int mmn_backproject_nufft(const mmn_problem *p, float *image, float *
     f.vox_start = 0;
     f.vox_count = nvox;
     f.ant = ant;
-    f.meas = ws + pl.off_rows;
     f.num_ant = A;
-    f.fp = pl.row;
-    f.ant_per_stage = pl.ant_per_stage;
     f.mono_flag = hdr + 1;
     f.ti = p->is_ti_radar ? 0.15 : 0.0;
     f.num_tiles = pl.tiles;
@@ -1001,14 +1005,21 @@ extern "C" int mmn_backproject_nufft(const mmn_problem *p, float *image, float *
     f.vote = reinterpret_cast<float2 *>(vote);
     f.partial = reinterpret_cast<float4 *>(ws + pl.off_part);
     f.status = hdr;
-    bq.nu_n = pl.n;
-    bq.nu_u = p->slope / kC;
-    bq.nu_k0c = 2.0 * kPi * (1.0 / p->wavelength + (double)J0 * p->slope / kC);
-    if (pl.smem > 48 * 1024)
-        cudaFuncSetAttribute(pl.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-    void *args[] = {&bq};
-    if (cudaLaunchKernel(pl.fn, dim3(pl.tiles * pl.splits), dim3(pl.threads), args, pl.smem,
-                         stream) != cudaSuccess)
+    float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_rows);
+    set_local_fields(q, p, pl.n, pl.row, rows);
+    q.bx = pl.bx;
+    q.by = pl.by;
+    q.runs = pl.runs;
+    q.tiles_y = pl.tiles_y;
+    q.tiles_z = pl.tiles_z;
+    if (launch_nufft_tables(f, F, pl.n, J0, sc, tw, box, stream) != cudaSuccess)
+        return MMN_ERR_CUDA;
+    if (launch_nufft_grid_window(p->meas, A, F, pl.n, J0, pl.row, sc, tw, ant, box, f.ti, q.uq,
+                                 rows, stream) != cudaSuccess)
+        return MMN_ERR_CUDA;
+    void *args[] = {&q};
+    if (cudaLaunchKernel(pl.fn, dim3(pl.tiles * pl.splits), dim3(pl.threads), args, 0, stream) !=
+        cudaSuccess)
         return MMN_ERR_CUDA;
     if (pl.splits > 1 && launch_reduce(f, stream) != cudaSuccess) return MMN_ERR_CUDA;
     return MMN_OK;
@@ -1118,11 +1129,13 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     double2 *tw = reinterpret_cast<double2 *>(ws + pl.off_nutab);  // 256-aligned
     double *sc = reinterpret_cast<double *>(tw + pl.nu_n);
     if (((grad_pos && pl.nufft) || (grad_meas && pl.meas_nufft)) &&
-        launch_nufft_tables(F, pl.nu_n, J0, sc, tw, stream) != cudaSuccess)
+        launch_nufft_tables(f, F, pl.nu_n, J0, sc, tw, reinterpret_cast<float *>(sc + F),
+                            stream) != cudaSuccess)
         return MMN_ERR_CUDA;
     if (grad_pos && pl.nufft) {
-        if (launch_nufft_grid(p->meas, A, F, pl.nu_n, J0, f.k0, f.kd, sc, tw, ws + pl.off_meas,
-                              false, stream) != cudaSuccess)
+        if (launch_nufft_grid(p->meas, A, F, pl.nu_n, J0, f.k0, f.kd, sc, tw,
+                              reinterpret_cast<float4 *>(ws + pl.off_meas), stream) !=
+            cudaSuccess)
             return MMN_ERR_CUDA;
         BwdParams bq = bp;
         bq.f.fp = pl.row;

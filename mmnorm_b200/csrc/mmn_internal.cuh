@@ -212,6 +212,38 @@ __device__ __forceinline__ void cis_turns_pair(int32_t a0, int32_t a1, float2 &c
     ns = make_float2(-s0, -s1);
 }
 
+// (cos, sin) of two angles given as wrapped 2^-32-turn integers, by one reduction to half a
+// turn: the remainder r in [-2^30, 2^30) (an angle in [-pi/2, pi/2)) differs from the input in
+// its top bit only, and that bit is the sign of both results -- no quarter-turn exchange.
+// Minimax polynomials on [-pi/2, pi/2] (fitted by Remez exchange: sine 3.3e-9, cosine 2.2e-10);
+// evaluated in FP32 4e-8 rms, 1.7e-7 at most (the hardware sine: 2e-7 rms).  In the local
+// forward, packed polynomials measured 3 % faster than scalar ones with immediates.
+__device__ __forceinline__ void cis_half_pair(int32_t a0, int32_t a1, float2 &c, float2 &s) {
+    const uint32_t m0 = ((uint32_t)a0 + 0x40000000u) & 0x80000000u;
+    const uint32_t m1 = ((uint32_t)a1 + 0x40000000u) & 0x80000000u;
+    const float k = 9.31322574615478515625e-10f;  // 2^-30: quarter turns
+    const float2 x = __fmul2_rn(make_float2((float)(int32_t)((uint32_t)a0 ^ m0),
+                                            (float)(int32_t)((uint32_t)a1 ^ m1)),
+                                make_float2(k, k));
+    const float2 y = __fmul2_rn(x, x);
+    float2 p = make_float2(1.508226387e-04f, 1.508226387e-04f);
+    p = __ffma2_rn(p, y, make_float2(-4.672232919e-03f, -4.672232919e-03f));
+    p = __ffma2_rn(p, y, make_float2(7.968848467e-02f, 7.968848467e-02f));
+    p = __ffma2_rn(p, y, make_float2(-6.459633612e-01f, -6.459633612e-01f));
+    p = __ffma2_rn(p, y, make_float2(1.570796290f, 1.570796290f));
+    p = __fmul2_rn(p, x);
+    float2 g = make_float2(-2.382491854e-05f, -2.382491854e-05f);
+    g = __ffma2_rn(g, y, make_float2(9.177248396e-04f, 9.177248396e-04f));
+    g = __ffma2_rn(g, y, make_float2(-2.086268839e-02f, -2.086268839e-02f));
+    g = __ffma2_rn(g, y, make_float2(2.536693228e-01f, 2.536693228e-01f));
+    g = __ffma2_rn(g, y, make_float2(-1.233700534f, -1.233700534f));
+    g = __ffma2_rn(g, y, make_float2(1.f, 1.f));
+    s = make_float2(__uint_as_float(__float_as_uint(p.x) ^ m0),
+                    __uint_as_float(__float_as_uint(p.y) ^ m1));
+    c = make_float2(__uint_as_float(__float_as_uint(g.x) ^ m0),
+                    __uint_as_float(__float_as_uint(g.y) ^ m1));
+}
+
 // ---------------------------------------------------------------- status / errors
 __device__ __forceinline__ void set_status(int32_t *status, int32_t code) {
     if (status) atomicCAS(status, 0, code);
