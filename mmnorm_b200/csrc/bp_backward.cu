@@ -231,13 +231,24 @@ __global__ void __launch_bounds__(NT) bp_bwd_pos_kernel(const BwdParams bp) {
     }
 }
 
+// grad_pos = sum over tiles of the per-tile partials: 32 outputs per block, 16 warps taking
+// every 16th tile, their sums added in order (one thread per output walked the 512 tiles of
+// the 64^3 adjoint workload alone: 48 us).
+constexpr int kPosReduceWarps = 16;
 __global__ void bwd_pos_reduce_kernel(const BwdParams bp) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= bp.num_ant_real * 3) return;
+    __shared__ float part[kPosReduceWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int idx = blockIdx.x * 32 + lane, n = bp.num_ant_real * 3;
     float s = 0.f;
-    for (int t = 0; t < bp.f.num_tiles; ++t)
-        s += bp.pos_partial[(size_t)t * bp.f.num_ant * 3 + idx];
-    bp.grad_pos[idx] = s;
+    if (idx < n)
+        for (int t = warp; t < bp.f.num_tiles; t += kPosReduceWarps)
+            s += bp.pos_partial[(size_t)t * bp.f.num_ant * 3 + idx];
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && idx < n) {
+        for (int w = 1; w < kPosReduceWarps; ++w) s += part[w][lane];
+        bp.grad_pos[idx] = s;
+    }
 }
 
 // Position pass when the loss has no vote term (dL/dW = 0): only c' = sum kappa m p is
@@ -792,9 +803,8 @@ cudaError_t launch_bwd_pos(const BwdParams &bp, int variant, size_t smem, cudaSt
 }
 
 cudaError_t launch_bwd_pos_reduce(const BwdParams &bp, cudaStream_t stream) {
-    const int nt = 256;
     const int n = bp.num_ant_real * 3;
-    bwd_pos_reduce_kernel<<<(n + nt - 1) / nt, nt, 0, stream>>>(bp);
+    bwd_pos_reduce_kernel<<<(n + 31) / 32, kPosReduceWarps * 32, 0, stream>>>(bp);
     return cudaGetLastError();
 }
 

@@ -136,11 +136,18 @@ struct LocalParams {
     double k0c, t0c;           // anchor phase per metre at J0 = F/2: radians, turns
     double t0c_fixed;          // -t0c * 2^32
     float theta_per_m;         // pi F |slope| / c
+    float half_min;            // least half width of a box's range interval: theta = 0.5, a
+                               // third of a grid cell.  The derivative's FP32 noise goes with
+                               // its inverse: on a box of one voxel 2e-5 of c' without it
     int32_t bx, by, runs;      // tile: bx x by columns, runs of 4 voxels in z
     int32_t tiles_y, tiles_z;
+    const float2 *grad_image;  // position pass: upstream gradients (either may be null)
+    const float2 *grad_vote;
+    float *pos_partial;        // [num_tiles, num_ant, 3]
 };
 void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs);
 const void *fwd_local_kernel_ptr(int *threads);
+const void *bwd_pos_local_kernel_ptr(bool vote, int *threads);
 int local_chunk_antennas();
 size_t nufft_meas_smem(int mrow);
 int nufft_meas_warps();

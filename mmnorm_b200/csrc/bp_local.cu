@@ -175,6 +175,31 @@ __device__ __forceinline__ void eval_cheb(const float2 *cf, int nn, const float 
                           __fadd2_rn(c, make_float2(-b2[k].x, -b2[k].y)));
 }
 
+// h_k and its derivative g_k in x.
+template <int NN>
+__device__ __forceinline__ void eval_mono_d(const float2 *cf, const float (&x)[kLocRun],
+                                            float2 (&h)[kLocRun], float2 (&g)[kLocRun]) {
+    const float4 *c4 = reinterpret_cast<const float4 *>(cf);
+    const float4 top = c4[NN / 2 - 1];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        g[k] = make_float2(top.z, top.w);
+        h[k] = __ffma2_rn(g[k], make_float2(x[k], x[k]), make_float2(top.x, top.y));
+    }
+#pragma unroll
+    for (int q = NN / 2 - 2; q >= 0; --q) {
+        const float4 c = c4[q];
+#pragma unroll
+        for (int k = 0; k < kLocRun; ++k) {
+            const float2 xx = make_float2(x[k], x[k]);
+            g[k] = __ffma2_rn(g[k], xx, h[k]);
+            h[k] = __ffma2_rn(h[k], xx, make_float2(c.z, c.w));
+            g[k] = __ffma2_rn(g[k], xx, h[k]);
+            h[k] = __ffma2_rn(h[k], xx, make_float2(c.x, c.y));
+        }
+    }
+}
+
 // M at one range by a tap run from the antenna's row in global memory.
 __device__ __forceinline__ float2 tap_run(const float2 *row, double d, double uq, int n) {
     int ix;
@@ -206,10 +231,12 @@ __device__ __forceinline__ float rsqrt_seed(float s) {
 // Round-trip ranges of the thread's run in FP64.  Each leg is f = D r with r an FP32
 // reciprocal-square-root seed of the FP32 difference vector, plus one Newton correction
 // (D - f^2) r / 2 (relative error ~1e-13).
+// rf, rb: the FP32 reciprocal legs.
 template <bool MONO>
 __device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
                                            const float (&vz)[kLocRun], double ti,
-                                           double (&d)[kLocRun]) {
+                                           double (&d)[kLocRun], float (&rf)[kLocRun],
+                                           float (&rb)[kLocRun]) {
     const float ax = vx - a.txf[0], ay = vy - a.txf[1];
     const float sxy = fmaf(ax, ax, ay * ay);
     const double dx = (double)vx - a.tx[0], dy = (double)vy - a.tx[1];
@@ -221,7 +248,8 @@ __device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k) {
         const float az = vz[k] - a.txf[2];
-        const double r = (double)rsqrt_seed(fmaf(az, az, sxy));
+        rf[k] = rsqrt_seed(fmaf(az, az, sxy));
+        const double r = (double)rf[k];
         const double dz = (double)vz[k] - a.tx[2];
         const double D = fma(dz, dz, Dxy);
         const double f = D * r, e = fma(-f, f, D);
@@ -229,7 +257,8 @@ __device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
             d[k] = fma(e, r, fma(2.0, f, ti));  // twice the leg
         } else {
             const float bz = vz[k] - a.rxf[2];
-            const double s = (double)rsqrt_seed(fmaf(bz, bz, txy));
+            rb[k] = rsqrt_seed(fmaf(bz, bz, txy));
+            const double s = (double)rb[k];
             const double ez = (double)vz[k] - a.rx[2];
             const double E = fma(ez, ez, Exy);
             const double g = E * s, h = fma(-g, g, E);
@@ -251,6 +280,9 @@ struct __align__(16) LocShared {
 
 // Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the chunk's node count (0: every
 // antenna takes tap runs).  Called by all threads; barriers inside.
+// With DERIV and more than kLocHorner nodes, node_val receives the Chebyshev coefficients of
+// the derivative.
+template <bool DERIV>
 __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, int a0, int na,
                                            const float (&lo)[3], const float (&hi)[3],
                                            int &table_nn) {
@@ -265,6 +297,7 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
         const float o[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
         float c, half, dmax;
         range_bounds(lo, hi, t, o, c, half, dmax);
+        half = fmaxf(half, q.half_min);
         const double centre = (double)c + p.ti;
         const double inv = 1.0 / (double)half;
 #pragma unroll
@@ -327,6 +360,17 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
             sh.node_val[la][c] = s;
         }
         __syncthreads();
+    } else if (DERIV) {
+        // d_p = (2 - [p = 0]) sum_{m > p, m - p odd} m c_m
+        for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
+            const int la = i / nn, c = i - la * nn;
+            float2 s = make_float2(0.f, 0.f);
+            for (int m = c + 1; m < nn; m += 2)
+                s = __ffma2_rn(make_float2((float)m, (float)m), sh.coef[la][m], s);
+            const float f = c == 0 ? 1.f : 2.f;
+            sh.node_val[la][c] = make_float2(f * s.x, f * s.y);
+        }
+        __syncthreads();
     }
     return nn;
 }
@@ -342,7 +386,8 @@ __device__ __forceinline__ void local_forward(const LocalParams &q, const LocSha
     for (int la = 0; la < na; ++la) {
         const LocRec &a = sh.rec[la];
         double d[kLocRun];
-        run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d);
+        float rf[kLocRun], rb[kLocRun];
+        run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d, rf, rb);
         float2 h[kLocRun];
         if (a.nn > 0) {
             float x[kLocRun];
@@ -423,7 +468,7 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
     int table_nn = 0;
     for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
         const int na = min(kLocAnts, a_end - a0);
-        const int nn = local_chunk(q, sh, a0, na, lo, hi, table_nn);
+        const int nn = local_chunk<false>(q, sh, a0, na, lo, hi, table_nn);
 #pragma unroll
         for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
@@ -449,6 +494,210 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
                             acc[k][2].x, acc[k][2].y, acc[k][3].x, acc[k][3].y};
         store_voxel(p, split, v, a);
     }
+}
+
+// ---------------------------------------------------------------- position pass
+// dL/ddelta_a = sum_v Im(conj(G) c') (-(e_tx + e_rx)) + Re(conj(gW) c) (bp_backward.cu) with c'
+// = sum_j kappa_j m_j p_j = i dc/dd: the derivative of the same polynomial, so the pass needs
+// no second grid (M' enters scaled by bandwidth / carrier, a few per cent of c').  The four
+// voxels of a thread share their lateral legs; a warp's three sums per antenna go through one
+// transposed reduction (6 shuffles) and the CTA's to the per-tile partials.
+namespace {
+
+// M and dM/dd of a pair by a tap run (wide boxes).
+__device__ __noinline__ float4 tap_run_d(const float2 *row, double d, double uq, int n) {
+    int ix;
+    float w[kNuW], t;
+    nufft_taps(d, uq, n, ix, w, &t);
+    const float t2 = t * t;
+    float2 h = make_float2(0.f, 0.f), g = h;
+#pragma unroll
+    for (int i = 0; i < kNuW; ++i) {
+        // P_i'(t) = sum 2q e_q t^(2q-1) + (2q+1) o_q t^(2q); mirror taps: -P_i'(-t)
+        const int m = i < kNuW / 2 ? i : kNuW - 1 - i;
+        float e = (2.f * (kEsEvenTerms - 1)) * kEsEven[m][kEsEvenTerms - 1];
+#pragma unroll
+        for (int q = kEsEvenTerms - 2; q >= 1; --q) e = fmaf(e, t2, 2.f * q * kEsEven[m][q]);
+        float o = (2.f * kEsOddTerms - 1.f) * kEsOdd[m][kEsOddTerms - 1];
+#pragma unroll
+        for (int q = kEsOddTerms - 2; q >= 0; --q) o = fmaf(o, t2, (2.f * q + 1.f) * kEsOdd[m][q]);
+        const float wd = i < kNuW / 2 ? fmaf(t, e, o) : fmaf(t, e, -o);
+        const float2 c = __ldg(row + ix + i);
+        h = __ffma2_rn(make_float2(w[i], w[i]), c, h);
+        g = __ffma2_rn(make_float2(wd, wd), c, g);
+    }
+    const float s = (float)(uq * n);
+    return make_float4(h.x, h.y, g.x * s, g.y * s);
+}
+
+// Sums of v0, v1, v2 over the warp: in lanes 0-7, 8-15 and 16-23.
+__device__ __forceinline__ float warp_sum3(float v0, float v1, float v2) {
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 16, mid = lane & 8;
+    float a = (hi ? v2 : v0) + __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 16);
+    float b = v1 + __shfl_xor_sync(0xffffffffu, v1, 16);
+    a = (mid ? b : a) + __shfl_xor_sync(0xffffffffu, mid ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+template <bool VOTE, bool MONO, int NN>
+__device__ __forceinline__ void local_position(const LocalParams &q, const LocShared &sh, int a0,
+                                               int na, int nn, float vx, float vy,
+                                               const float (&vz)[kLocRun],
+                                               const float2 (&gi)[kLocRun],
+                                               const float2 (&gw)[kLocRun][3], float *wsum) {
+    const double kM = 6755399441055744.0;  // 1.5 * 2^52
+    const int lane = threadIdx.x & 31;
+    const float k0c = (float)q.k0c;
+    for (int la = 0; la < na; ++la) {
+        const LocRec &a = sh.rec[la];
+        double d[kLocRun];
+        float rf[kLocRun], rb[kLocRun];
+        run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d, rf, rb);
+        float2 h[kLocRun], g[kLocRun];  // M, dM/dd
+        if (a.nn > 0) {
+            float x[kLocRun];
+#pragma unroll
+            for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
+            if (NN > 0) {
+                eval_mono_d<(NN > 0 ? NN : 8)>(sh.node_val[la], x, h, g);
+            } else {
+                eval_cheb(sh.coef[la], nn, x, h);
+                eval_cheb(sh.node_val[la], nn, x, g);
+            }
+            const float inv = (float)a.inv;
+#pragma unroll
+            for (int k = 0; k < kLocRun; ++k) g[k] = __fmul2_rn(g[k], make_float2(inv, inv));
+        } else {
+            const float2 *row = q.rows + (size_t)(a0 + la) * q.row;
+#pragma unroll
+            for (int k = 0; k < kLocRun; ++k) {
+                const float4 t = tap_run_d(row, d[k], q.uq, q.n);
+                h[k] = make_float2(t.x, t.y);
+                g[k] = make_float2(t.z, t.w);
+            }
+        }
+        const float ax = vx - a.txf[0], ay = vy - a.txf[1];
+        const float bx = vx - a.rxf[0], by = vy - a.rxf[1];
+        const float ux = a.u[0] - vx, uy = a.u[1] - vy;
+        float sf = 0.f, sb = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < kLocRun; k += 2) {
+            float2 ac, as;
+            cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
+                          __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), ac, as);
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const int j = k + l;
+                const float c = l ? ac.y : ac.x, s = l ? as.y : as.x;
+                // c' = anchor (k0c M + i M')
+                const float tr = fmaf(k0c, h[j].x, -g[j].y), ti = fmaf(k0c, h[j].y, g[j].x);
+                float Gr = gi[j].x, Gi = gi[j].y;
+                if (VOTE) {
+                    const float uz = a.u[2] - vz[j];
+                    Gr = fmaf(gw[j][0].x, ux, fmaf(gw[j][1].x, uy, fmaf(gw[j][2].x, uz, Gr)));
+                    Gi = fmaf(gw[j][0].y, ux, fmaf(gw[j][1].y, uy, fmaf(gw[j][2].y, uz, Gi)));
+                }
+                // Im(conj(G) anchor T) = Im(B T), B = conj(G) anchor
+                const float Br = fmaf(Gr, c, Gi * s), Bi = fmaf(Gr, s, -Gi * c);
+                const float s1 = fmaf(Br, ti, Bi * tr);
+                const float tf = s1 * rf[j];
+                sf += tf;
+                g2 = fmaf(-tf, vz[j] - a.txf[2], g2);
+                const float tb = MONO ? tf : s1 * rb[j];
+                if (!MONO) sb += tb;
+                if (!MONO) g2 = fmaf(-tb, vz[j] - a.rxf[2], g2);
+                if (VOTE) {
+                    const float cr = fmaf(c, h[j].x, -s * h[j].y), ci = fmaf(c, h[j].y, s * h[j].x);
+                    g0 = fmaf(gw[j][0].x, cr, fmaf(gw[j][0].y, ci, g0));
+                    g1 = fmaf(gw[j][1].x, cr, fmaf(gw[j][1].y, ci, g1));
+                    if (MONO)  // g2 is doubled below
+                        g2 = fmaf(0.5f * gw[j][2].x, cr, fmaf(0.5f * gw[j][2].y, ci, g2));
+                    else
+                        g2 = fmaf(gw[j][2].x, cr, fmaf(gw[j][2].y, ci, g2));
+                }
+            }
+        }
+        if (MONO) {
+            g0 = fmaf(-2.f * ax, sf, g0);
+            g1 = fmaf(-2.f * ay, sf, g1);
+            g2 += g2;
+        } else {
+            g0 = fmaf(-ax, sf, fmaf(-bx, sb, g0));
+            g1 = fmaf(-ay, sf, fmaf(-by, sb, g1));
+        }
+        const float s = warp_sum3(g0, g1, g2);
+        if ((lane & 7) == 0 && lane < 24) wsum[la * 3 + (lane >> 3)] = s;
+    }
+}
+
+template <bool VOTE, bool MONO>
+__device__ __forceinline__ void local_position_nn(const LocalParams &q, const LocShared &sh,
+                                                  int a0, int na, int nn, float vx, float vy,
+                                                  const float (&vz)[kLocRun],
+                                                  const float2 (&gi)[kLocRun],
+                                                  const float2 (&gw)[kLocRun][3], float *wsum) {
+    if (nn == 8) local_position<VOTE, MONO, 8>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
+    else if (nn == 10) local_position<VOTE, MONO, 10>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
+    else if (nn == 12) local_position<VOTE, MONO, 12>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
+    else local_position<VOTE, MONO, 0>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
+}
+
+}  // namespace
+
+// grid = tiles x antenna splits.  VOTE: the loss has a vote term.
+template <bool VOTE>
+__global__ void __launch_bounds__(kLocThreads, 4) bp_bwd_pos_local_kernel(const LocalParams q) {
+    __shared__ LocShared sh;
+    __shared__ float wsum[kLocThreads / 32][kLocAnts * 3];
+    const FwdParams &p = q.f;
+    const int tile = blockIdx.x % p.num_tiles, split = blockIdx.x / p.num_tiles;
+    const int a_begin = split * p.ant_per_split;
+    const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
+    float lo[3], hi[3];
+    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
+    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
+    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
+    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    const LocSlot s = local_slot(q, tile, threadIdx.x);
+    const float vx = __ldg(p.x_locs + min(s.ix, p.nx - 1));
+    const float vy = __ldg(p.y_locs + min(s.iy, p.ny - 1));
+    float vz[kLocRun];
+    float2 gi[kLocRun], gw[kLocRun][3];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        vz[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
+        const bool ok = s.column && s.iz + k < p.nz;
+        const int64_t v = ok ? ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k : 0;
+        gi[k] = ok && q.grad_image ? q.grad_image[v] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            gw[k][c] = VOTE && ok ? q.grad_vote[c * p.nvox + v] : make_float2(0.f, 0.f);
+    }
+    const bool mono = *p.mono_flag != 0;
+    float *mine = wsum[threadIdx.x >> 5];
+    int table_nn = 0;
+    for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
+        const int na = min(kLocAnts, a_end - a0);
+        const int nn = local_chunk<true>(q, sh, a0, na, lo, hi, table_nn);
+        if (mono) local_position_nn<VOTE, true>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, mine);
+        else local_position_nn<VOTE, false>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, mine);
+        __syncthreads();
+        for (int i = threadIdx.x; i < na * 3; i += kLocThreads) {
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLocThreads / 32; ++w) t += wsum[w][i];
+            q.pos_partial[((size_t)tile * p.num_ant + a0) * 3 + i] = t;
+        }
+    }
+}
+
+const void *bwd_pos_local_kernel_ptr(bool vote, int *threads) {
+    *threads = kLocThreads;
+    return vote ? reinterpret_cast<const void *>(&bp_bwd_pos_local_kernel<true>)
+                : reinterpret_cast<const void *>(&bp_bwd_pos_local_kernel<false>);
 }
 
 // Tile shape: columns bx x by and runs of 4 voxels in z, at most 128 runs, chosen for few

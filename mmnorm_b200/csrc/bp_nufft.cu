@@ -134,6 +134,7 @@ __device__ __forceinline__ void cell_window(const float *box, const AntRec &ar, 
     const float r[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
     float c, half, dmax;
     range_bounds(lo, hi, t, r, c, half, dmax);
+    // (the local kernels may widen a box by a third of a cell: one cell of slack either side)
     const double a = ((double)c - half + ti) * uq * N, b = ((double)c + half + ti) * uq * N;
     const double k0 = floor(fmin(a, b)) - kNuW / 2, k1 = floor(fmax(a, b)) + kNuW / 2 + 1;
     first = 0;
@@ -360,11 +361,12 @@ struct NuVariant {
      reinterpret_cast<const void *>(&bp_bwd_pos_nufft_kernel<T, NT, false>),               \
      "interp_t" #T "_n" #NT "_s" #CAP}
 
-// At 64^3 voxels, 4096 antennas, 128 samples (position pass alone; with vote term / image
-// loss only): 9.00/8.43, 9.64/8.16, 11.1/11.8, 10.7/9.85 ms in this order; the first is the
-// default.
+// Variant 0, the default, is the tile-local form (bp_local.cu; its pointers are filled in by
+// bwd_pos_nufft_kernel_ptr).  The others are launch shapes of this file's tap-run kernel: at
+// 64^3 voxels, 4096 antennas, 128 samples (position pass alone; with vote term / image loss
+// only) 9.64/8.16, 11.1/11.8, 10.7/9.85 ms in this order.
 const NuVariant kNuVariants[] = {
-    MMN_NU_VARIANT(2, 128, 24),
+    {4, 128, 0, nullptr, nullptr, "interp_local_t4_n128"},
     MMN_NU_VARIANT(2, 256, 24),
     MMN_NU_VARIANT(1, 256, 48),
     MMN_NU_VARIANT(1, 128, 16),
@@ -569,6 +571,7 @@ const void *bwd_pos_nufft_kernel_ptr(int variant, bool vote, int *threads, int *
     *threads = v.nt;
     *voxels_per_thread = v.t;
     *stage_cap_bytes = v.stage_cap * 1024;
+    if (!v.fn_vote) return bwd_pos_local_kernel_ptr(vote, threads);
     return vote ? v.fn_vote : v.fn_img;
 }
 

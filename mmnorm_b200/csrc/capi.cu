@@ -734,6 +734,8 @@ struct BwdPlan {
     int64_t vox_per_split;
     const void *fn;
     bool nufft;       // position pass in interpolation form
+    bool local;       // ... by tile-local polynomials
+    int bx, by, runs, tiles_y, tiles_z;
     bool meas_nufft;  // measurement pass in interpolation form
     int nu_n, row;
     int mrow, mranges;
@@ -758,8 +760,10 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
     if (pl->nufft) {
         pl->fn = bwd_pos_nufft_kernel_ptr(g_pos_variant.load(), !image_only, &pl->threads,
                                           &pl->vpt, &cap);
-        pl->row = nufft_row(pl->nu_n);
+        pl->local = cap == 0;
+        pl->row = pl->local ? nufft_row_fwd(pl->nu_n) : nufft_row(pl->nu_n);
     } else {
+        pl->local = false;
         pl->fn = image_only ? bwd_pos_img_kernel_ptr(&pl->threads, &pl->vpt)
                             : bwd_pos_kernel_ptr(g_bwd_variant.load(), &pl->threads, &pl->vpt);
         pl->row = pl->fp;
@@ -769,7 +773,15 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
     pl->smem = 128 + 2 * (size_t)pl->ant_per_stage * rec +
                (size_t)(pl->threads / 32) * pl->ant_per_stage * 3 * sizeof(float);
     const int64_t per_tile = (int64_t)pl->threads * pl->vpt;
-    const int64_t tiles = (nvox + per_tile - 1) / per_tile;
+    int64_t tiles = (nvox + per_tile - 1) / per_tile;
+    if (pl->local) {
+        pl->ant_per_stage = local_chunk_antennas();
+        pl->smem = 0;
+        plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
+        pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
+        pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
+        tiles = (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
+    }
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
     pl->tiles = (int)std::max<int64_t>(1, tiles);
     int dev = 0, sms = 148, per_sm = 1;
@@ -803,7 +815,7 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
     pl->off_ant = off;
     off = align_up(off + (size_t)A * sizeof(AntRec));
     pl->off_meas = off;
-    off = align_up(off + (size_t)A * pl->row * 16);
+    off = align_up(off + (size_t)A * pl->row * (pl->local ? 8 : 16));
     pl->off_nutab = off;  // interpolation form: twiddles [N] double2, then 1/phihat [F] doubles
     if (pl->nufft || pl->meas_nufft)
         off = align_up(off + (size_t)p->num_samples * sizeof(double) +
@@ -880,6 +892,7 @@ void set_local_fields(LocalParams &q, const mmn_problem *p, int n, int row, cons
     q.k0c = 2.0 * kPi * q.t0c;
     q.t0c_fixed = -q.t0c * 4294967296.0;
     q.theta_per_m = (float)(kPi * F * std::fabs(p->slope) / kC);
+    q.half_min = q.theta_per_m > 0.5f ? 0.5f / q.theta_per_m : 1.f;
 }
 
 struct NuFwdPlan {
@@ -1132,7 +1145,30 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
         launch_nufft_tables(f, F, pl.nu_n, J0, sc, tw, reinterpret_cast<float *>(sc + F),
                             stream) != cudaSuccess)
         return MMN_ERR_CUDA;
-    if (grad_pos && pl.nufft) {
+    if (grad_pos && pl.local) {
+        LocalParams q;
+        std::memset(&q, 0, sizeof(q));
+        float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_meas);
+        set_local_fields(q, p, pl.nu_n, pl.row, rows);
+        q.f = f;
+        q.bx = pl.bx;
+        q.by = pl.by;
+        q.runs = pl.runs;
+        q.tiles_y = pl.tiles_y;
+        q.tiles_z = pl.tiles_z;
+        q.grad_image = bp.grad_image;
+        q.grad_vote = bp.grad_vote;
+        q.pos_partial = bp.pos_partial;
+        if (launch_nufft_grid_window(p->meas, A, F, pl.nu_n, J0, pl.row, sc, tw, ant,
+                                     reinterpret_cast<float *>(sc + F), f.ti, q.uq, rows,
+                                     stream) != cudaSuccess)
+            return MMN_ERR_CUDA;
+        void *args[] = {&q};
+        if (cudaLaunchKernel(pl.fn, dim3(pl.tiles * pl.splits), dim3(pl.threads), args, 0,
+                             stream) != cudaSuccess)
+            return MMN_ERR_CUDA;
+        if (launch_bwd_pos_reduce(bp, stream) != cudaSuccess) return MMN_ERR_CUDA;
+    } else if (grad_pos && pl.nufft) {
         if (launch_nufft_grid(p->meas, A, F, pl.nu_n, J0, f.k0, f.kd, sc, tw,
                               reinterpret_cast<float4 *>(ws + pl.off_meas), stream) !=
             cudaSuccess)

@@ -10,8 +10,9 @@ namespace mmn {
 // fractional offset by the 1.5*2^52 rounding constant (no conversion instructions), clamped
 // so that a NaN or a fraction that rounds up to 1 still reads inside the row; the weights
 // from es_taps.cuh, P_i(t) and P_i(-t) from one even and one odd part.
+// offset: if not null, receives the fractional offset less 1/2.
 __device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell,
-                                           float (&w)[kNuW]) {
+                                           float (&w)[kNuW], float *offset = nullptr) {
     const double kRound = 6755399441055744.0;  // 1.5 * 2^52
     const double u = d * uq;
     double uf = u - ((u + kRound) - kRound);  // [-1/2, 1/2]
@@ -29,6 +30,7 @@ __device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell
     cell = ix;
 
     const float t = sfr - 0.5f, t2 = t * t;
+    if (offset) *offset = t;
 #pragma unroll
     for (int i = 0; i < kNuW / 2; ++i) {
         float e = kEsEven[i][kEsEvenTerms - 1];
