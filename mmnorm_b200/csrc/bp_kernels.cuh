@@ -114,19 +114,15 @@ const void *bwd_pos_img_kernel_ptr(int *threads, int *voxels_per_thread);
 const void *bwd_pos_nufft_kernel_ptr(int variant, bool vote, int *threads, int *voxels_per_thread,
                                      int *stage_cap_bytes);
 int bwd_pos_nufft_num_variants();
-// Interpolation-form measurement pass.
+// Output transform of the interpolation-form measurement pass.
 struct NuMeasParams {
-    const AntRec *ant;
-    const float4 *vox;        // [nvox][5] records (nufft_vox_kernel)
-    const int32_t *mono_flag;
-    float2 *part;             // [ranges][num_ant][mrow] per-range antenna grids
+    const float2 *part;       // [ranges][num_ant][mrow] per-range antenna grids
     const double *sc;         // [F] 1/phihat((j - J0)/N)
     const double2 *tw;        // [N] e^{-2pi i k/N}
     float2 *grad_meas;        // [num_ant][F]
-    int64_t nvox, vox_per_range;
-    double ti, uq, k0c;       // 0.15 or 0; slope/c; 2pi(1/lambda + J0 slope/c)
     int32_t num_ant, n, mrow, ranges, F, J0;  // mrow = N + 16 cells
 };
+cudaError_t launch_nufft_meas_out(const NuMeasParams &q, cudaStream_t stream);
 // Interpolation form by tile-local polynomials (bp_local.cu).
 struct LocalParams {
     FwdParams f;               // geometry, antenna records, outputs; tiles and antenna splits
@@ -144,17 +140,20 @@ struct LocalParams {
     const float2 *grad_image;  // position pass: upstream gradients (either may be null)
     const float2 *grad_vote;
     float *pos_partial;        // [num_tiles, num_ant, 3]
+    float4 *vox;               // measurement pass: voxel records in box order
 };
 void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs);
+// measurement pass: bytes of the voxel records, shared memory of the antenna rows (mrow cells
+// each), warps (antennas) per CTA
+size_t local_meas_vox_bytes(int64_t tiles);
+size_t local_meas_smem(int mrow);
+int local_meas_warps();
+const void *local_meas_kernel_ptr(bool vote);
+cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int ranges,
+                              int tiles_per_range, cudaStream_t stream);
 const void *fwd_local_kernel_ptr(int *threads);
 const void *bwd_pos_local_kernel_ptr(bool vote, int *threads);
 int local_chunk_antennas();
-size_t nufft_meas_smem(int mrow);
-int nufft_meas_warps();
-const void *nufft_meas_kernel_ptr();
-cudaError_t launch_nufft_meas(const NuMeasParams &q, const FwdParams &p,
-                              const float2 *grad_image, const float2 *grad_vote, float4 *rec,
-                              cudaStream_t stream);
 const char *bwd_pos_nufft_variant_name(int variant);  // null for a bad index
 // box: 6 floats, the voxel coordinates' per-axis minima and maxima
 cudaError_t launch_nufft_tables(const FwdParams &p, int F, int N, int J0, double *sc, double2 *tw,

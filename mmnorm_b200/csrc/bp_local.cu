@@ -700,6 +700,350 @@ const void *bwd_pos_local_kernel_ptr(bool vote, int *threads) {
                 : reinterpret_cast<const void *>(&bp_bwd_pos_local_kernel<false>);
 }
 
+// ------------------------------------------------------------- measurement pass
+// dL/dm[a, J0+j'] = sum_v h_v e^{2 pi i j' u_v}, h_v = G_a(v) conj(anchor): the transpose of the
+// forward's evaluation.  Per (box, antenna) the voxels' h are reduced to NN Chebyshev moments
+// sum_v h_v T_q(x_v) in registers (two packed instructions each); the transposed interpolation
+// turns the moments into NN node values, and only those are spread onto the antenna's grid row
+// (8 cells each).  A warp owns one antenna and its row and walks a range of boxes, 32 voxel
+// runs at a time; everything is summed in a fixed order.  Boxes too wide for the nodes spread
+// every voxel.
+namespace {
+
+constexpr int kLocMeasWarps = 4;
+constexpr int kLocMeasSlots = 128;  // voxel runs of a box
+
+// Voxel records in box order: per box kLocMeasSlots x (x, y, -, -), (z_0 .. z_3), then per run
+// position k (gI) or (gI, gW_x), (gW_y, gW_z); and the boxes' bounds.
+struct LocVox {
+    float4 *xy, *z, *box;  // [tiles][slots], [tiles][slots], [tiles][2]
+    float4 *g;             // vote: [tiles][4][2][slots] float4; image only: [tiles][4][slots] float2
+};
+__device__ __forceinline__ LocVox loc_vox(const LocalParams &q) {
+    LocVox r;
+    const size_t n = (size_t)q.f.num_tiles * kLocMeasSlots;
+    r.box = q.vox;
+    r.xy = r.box + 2 * (size_t)q.f.num_tiles;
+    r.z = r.xy + n;
+    r.g = r.z + n;
+    return r;
+}
+
+__global__ void __launch_bounds__(kLocMeasSlots) local_vox_kernel(const LocalParams q) {
+    const FwdParams &p = q.f;
+    const int tile = blockIdx.x, slot = threadIdx.x;
+    const LocVox r = loc_vox(q);
+    float lo[3], hi[3];
+    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
+    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
+    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
+    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    if (slot == 0) {
+        r.box[2 * tile] = make_float4(lo[0], lo[1], lo[2], 0.f);
+        r.box[2 * tile + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    }
+    const LocSlot s = local_slot(q, tile, slot);
+    const size_t at = (size_t)tile * kLocMeasSlots + slot;
+    r.xy[at] = make_float4(__ldg(p.x_locs + min(s.ix, p.nx - 1)),
+                           __ldg(p.y_locs + min(s.iy, p.ny - 1)), 0.f, 0.f);
+    float z[kLocRun];
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) {
+        z[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
+        const bool ok = s.column && s.iz + k < p.nz;
+        const int64_t v = ok ? ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k : 0;
+        const float2 zero = make_float2(0.f, 0.f);
+        const float2 gi = ok && q.grad_image ? q.grad_image[v] : zero;
+        const size_t gk = (size_t)tile * kLocRun + k;
+        if (q.grad_vote) {
+            const float2 a = ok ? q.grad_vote[v] : zero, b = ok ? q.grad_vote[p.nvox + v] : zero,
+                         c = ok ? q.grad_vote[2 * p.nvox + v] : zero;
+            r.g[(2 * gk) * kLocMeasSlots + slot] = make_float4(gi.x, gi.y, a.x, a.y);
+            r.g[(2 * gk + 1) * kLocMeasSlots + slot] = make_float4(b.x, b.y, c.x, c.y);
+        } else {
+            reinterpret_cast<float2 *>(r.g)[gk * kLocMeasSlots + slot] = gi;
+        }
+    }
+    r.z[at] = make_float4(z[0], z[1], z[2], z[3]);
+}
+
+// Tables of every node count, back to back: cos(pi m / (2 NN)), m < 4 NN, and the nodes.
+constexpr int kNodeTotal = 8 + 10 + 12 + 16 + 24;
+__device__ __forceinline__ int node_offset(int nn) {  // sum of the smaller counts
+    return nn == 8 ? 0 : nn == 10 ? 8 : nn == 12 ? 18 : nn == 16 ? 30 : 46;
+}
+
+// Per-warp scratch of the spread.
+struct LocSpread {
+    float2 w[32][kNuW];
+    int ix[32];
+    float mom[2 * kLocNodes];
+};
+
+// Adds value * (tap weights at range d) of every active lane to the warp's grid row, in lane
+// order per cell.
+__device__ __noinline__ void spread_row(LocSpread &sp, float2 *row, int mrow, double d,
+                                        float2 value, bool active, double uq, int n) {
+    const int lane = threadIdx.x & 31;
+    int ix;
+    float w[kNuW];
+    nufft_taps(d, uq, n, ix, w);
+#pragma unroll
+    for (int i = 0; i < kNuW; ++i) sp.w[lane][i] = make_float2(value.x * w[i], value.y * w[i]);
+    sp.ix[lane] = ix;
+    __syncwarp();
+    unsigned pending = __ballot_sync(0xffffffffu, active);
+    while (pending) {
+        const bool mine_p = (pending >> lane) & 1u;
+        const int base = __reduce_min_sync(0xffffffffu, mine_p ? ix : 0x7fffffff);
+        const unsigned mine = __ballot_sync(0xffffffffu, mine_p && ix - base <= 32 - kNuW);
+        float2 s = make_float2(0.f, 0.f);
+        for (unsigned m = mine; m; m &= m - 1) {
+            const int i = __ffs(m) - 1;
+            const unsigned o = (unsigned)(base + lane - sp.ix[i]);
+            if (o < (unsigned)kNuW) s = __fadd2_rn(s, sp.w[i][o]);
+        }
+        if (base + lane < mrow) row[base + lane] = __fadd2_rn(row[base + lane], s);
+        pending &= ~mine;
+    }
+    __syncwarp();
+}
+
+// Transposed warp sum of N (a power of two) values: out[i] = sum over lanes of v[i].
+template <int N>
+__device__ __forceinline__ void warp_sums(float *v, float *out) {
+    const int lane = threadIdx.x & 31;
+    int at = 0;  // index of v[0] in the original order
+    int bit = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, bit >>= 1) {
+        const bool up = lane & bit;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+        at += up ? h : 0;
+    }
+#pragma unroll
+    for (; bit >= 1; bit >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+    out[at] = v[0];  // the lanes of a group write the same value
+}
+
+// One box against the warp's antenna: the moments into sp.mom (NN > 0), or every voxel's
+// spread (NN = 0).
+template <bool VOTE, bool MONO, int NN>
+__device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &vx, int tile,
+                                            const LocRec &a, LocSpread &sp, float2 *row,
+                                            int mrow) {
+    const double kM = 6755399441055744.0;  // 1.5 * 2^52
+    const int lane = threadIdx.x & 31;
+    constexpr int NV = NN > 0 ? NN : 1;
+    float2 mom[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) mom[i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int slot = lane; slot < kLocMeasSlots; slot += 32) {
+        const size_t at = (size_t)tile * kLocMeasSlots + slot;
+        const float4 xy = __ldg(vx.xy + at), z4 = __ldg(vx.z + at);
+        const float vz[kLocRun] = {z4.x, z4.y, z4.z, z4.w};
+        double d[kLocRun];
+        float rf[kLocRun], rb[kLocRun];
+        run_ranges<MONO>(a, xy.x, xy.y, vz, q.f.ti, d, rf, rb);
+        const float ux = a.u[0] - xy.x, uy = a.u[1] - xy.y;
+#pragma unroll
+        for (int k = 0; k < kLocRun; k += 2) {
+            float2 ac, as;
+            if (NN > 0)
+                cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
+                              __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), ac, as);
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const int j = k + l;
+                const size_t gk = (size_t)tile * kLocRun + j;
+                float Gr, Gi;
+                if (VOTE) {
+                    const float4 g0 = __ldg(vx.g + (2 * gk) * kLocMeasSlots + slot);
+                    const float4 g1 = __ldg(vx.g + (2 * gk + 1) * kLocMeasSlots + slot);
+                    const float uz = a.u[2] - vz[j];
+                    Gr = fmaf(g1.z, uz, fmaf(g1.x, uy, fmaf(g0.z, ux, g0.x)));
+                    Gi = fmaf(g1.w, uz, fmaf(g1.y, uy, fmaf(g0.w, ux, g0.y)));
+                } else {
+                    const float2 g = __ldg(reinterpret_cast<const float2 *>(vx.g) +
+                                           gk * kLocMeasSlots + slot);
+                    Gr = g.x;
+                    Gi = g.y;
+                }
+                if (NN > 0) {
+                    const float c = l ? ac.y : ac.x, s = l ? as.y : as.x;
+                    float2 t0 = make_float2(fmaf(Gr, c, Gi * s), fmaf(Gi, c, -Gr * s));
+                    const float x = (float)fma(d[j], a.inv, a.off);
+                    const float2 x2 = make_float2(x + x, x + x);
+                    float2 t1 = __fmul2_rn(make_float2(x, x), t0);
+                    mom[0] = __fadd2_rn(mom[0], t0);
+                    if (NN > 1) mom[1 % NV] = __fadd2_rn(mom[1 % NV], t1);
+#pragma unroll
+                    for (int i = 2; i < NN; ++i) {
+                        const float2 t2 =
+                            __ffma2_rn(x2, t1, make_float2(-t0.x, -t0.y));
+                        mom[i % NV] = __fadd2_rn(mom[i % NV], t2);
+                        t0 = t1;
+                        t1 = t2;
+                    }
+                } else {
+                    const float2 an = cis_fp64_phase(-d[j] * q.k0c);
+                    spread_row(sp, row, mrow, d[j],
+                               make_float2(fmaf(Gr, an.x, Gi * an.y), fmaf(Gi, an.x, -Gr * an.y)),
+                               true, q.uq, q.n);
+                }
+            }
+        }
+    }
+    if (NN > 0) {
+        float *v = reinterpret_cast<float *>(mom);
+        if (NN == 8) warp_sums<16>(v, sp.mom);
+        if (NN == 10) {
+            warp_sums<16>(v, sp.mom);
+            warp_sums<4>(v + 16, sp.mom + 16);
+        }
+        if (NN == 12) {
+            warp_sums<16>(v, sp.mom);
+            warp_sums<8>(v + 16, sp.mom + 16);
+        }
+        if (NN == 16) warp_sums<32>(v, sp.mom);
+        if (NN == 24) {
+            warp_sums<32>(v, sp.mom);
+            warp_sums<16>(v + 32, sp.mom + 32);
+        }
+        __syncwarp();
+    }
+}
+
+template <bool VOTE, bool MONO>
+__device__ __forceinline__ void box_moments_nn(const LocalParams &q, const LocVox &vx, int tile,
+                                               const LocRec &a, LocSpread &sp, float2 *row,
+                                               int mrow) {
+    switch (a.nn) {
+        case 8: box_moments<VOTE, MONO, 8>(q, vx, tile, a, sp, row, mrow); break;
+        case 10: box_moments<VOTE, MONO, 10>(q, vx, tile, a, sp, row, mrow); break;
+        case 12: box_moments<VOTE, MONO, 12>(q, vx, tile, a, sp, row, mrow); break;
+        case 16: box_moments<VOTE, MONO, 16>(q, vx, tile, a, sp, row, mrow); break;
+        case 24: box_moments<VOTE, MONO, 24>(q, vx, tile, a, sp, row, mrow); break;
+        default: box_moments<VOTE, MONO, 0>(q, vx, tile, a, sp, row, mrow);
+    }
+}
+
+}  // namespace
+
+// blockIdx.x = antenna group (one antenna per warp) + groups * box range.
+template <bool VOTE>
+__global__ void __launch_bounds__(kLocMeasWarps * 32)
+    bp_bwd_meas_local_kernel(const LocalParams q, float2 *part, int mrow, int tiles_per_range) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ LocRec s_rec[kLocMeasWarps];
+    __shared__ LocSpread s_spread[kLocMeasWarps];
+    __shared__ double s_node[kNodeTotal];
+    __shared__ float s_table[4 * kNodeTotal];
+    const FwdParams &p = q.f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int groups = (p.num_ant + kLocMeasWarps - 1) / kLocMeasWarps;
+    const int a = blockIdx.x % groups * kLocMeasWarps + warp, range = blockIdx.x / groups;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+        const int nn = c < 3 ? 8 + 2 * c : 8 * (c - 1);
+        cheb_tables(nn, s_table + 4 * node_offset(nn), s_node + node_offset(nn));
+    }
+    __syncthreads();
+    if (a >= p.num_ant) return;  // warps are independent from here on
+    float2 *row = reinterpret_cast<float2 *>(dyn) + (size_t)warp * mrow;
+    for (int c = lane; c < mrow; c += 32) row[c] = make_float2(0.f, 0.f);
+    LocRec &rec = s_rec[warp];
+    LocSpread &sp = s_spread[warp];
+    const AntRec ar = p.ant[a];
+    const float t[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
+    const float r[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            rec.tx[k] = ar.tx[k];
+            rec.rx[k] = ar.rx[k];
+            rec.txf[k] = t[k];
+            rec.rxf[k] = r[k];
+            rec.u[k] = ar.virt[k];
+        }
+    }
+    const bool mono = *p.mono_flag != 0;
+    const LocVox vx = loc_vox(q);
+    const int t0 = range * tiles_per_range, t1 = min(p.num_tiles, t0 + tiles_per_range);
+    for (int tile = t0; tile < t1; ++tile) {
+        const float4 l4 = __ldg(vx.box + 2 * tile), h4 = __ldg(vx.box + 2 * tile + 1);
+        const float lo[3] = {l4.x, l4.y, l4.z}, hi[3] = {h4.x, h4.y, h4.z};
+        float c, half, dmax;
+        range_bounds(lo, hi, t, r, c, half, dmax);
+        half = fmaxf(half, q.half_min);
+        const double centre = (double)c + p.ti;
+        const bool fits = ((double)dmax + p.ti) * fabs(q.t0c) < 262144.0;
+        const int nn = fits ? local_nodes(q.theta_per_m * half) : 0;
+        __syncwarp();
+        if (lane == 0) {
+            const double inv = 1.0 / (double)half;
+            rec.inv = inv;
+            rec.off = -centre * inv;
+            rec.nn = nn;
+        }
+        __syncwarp();
+        if (mono) box_moments_nn<VOTE, true>(q, vx, tile, rec, sp, row, mrow);
+        else box_moments_nn<VOTE, false>(q, vx, tile, rec, sp, row, mrow);
+        if (nn > 0) {
+            // node values: sum_q (2 - [q = 0]) / NN cos(pi q (2 i + 1) / (2 NN)) moment_q
+            const int no = node_offset(nn), i = min(lane, nn - 1);
+            const float *table = s_table + 4 * no;
+            const float2 *mom = reinterpret_cast<const float2 *>(sp.mom);
+            float2 s = make_float2(0.5f * mom[0].x, 0.5f * mom[0].y);
+            int m = 2 * i + 1;
+            for (int k = 1; k < nn; ++k) {
+                const float w = table[m];
+                s = __ffma2_rn(make_float2(w, w), mom[k], s);
+                m += 2 * i + 1;
+                if (m >= 4 * nn) m -= 4 * nn;
+            }
+            const float sc = 2.f / (float)nn;
+            spread_row(sp, row, mrow, fma(s_node[no + i], (double)half, centre),
+                       make_float2(s.x * sc, s.y * sc), lane < nn, q.uq, q.n);
+        }
+    }
+    __syncwarp();
+    float2 *dst = part + ((size_t)range * p.num_ant + a) * mrow;
+    for (int c = lane; c < mrow; c += 32) dst[c] = row[c];
+}
+
+size_t local_meas_vox_bytes(int64_t tiles) {
+    return (size_t)tiles * (2 * sizeof(float4) +
+                            kLocMeasSlots * (2 + 2 * kLocRun) * sizeof(float4));
+}
+
+size_t local_meas_smem(int mrow) { return (size_t)kLocMeasWarps * mrow * sizeof(float2); }
+
+int local_meas_warps() { return kLocMeasWarps; }
+
+const void *local_meas_kernel_ptr(bool vote) {
+    return vote ? reinterpret_cast<const void *>(&bp_bwd_meas_local_kernel<true>)
+                : reinterpret_cast<const void *>(&bp_bwd_meas_local_kernel<false>);
+}
+
+cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int ranges,
+                              int tiles_per_range, cudaStream_t stream) {
+    local_vox_kernel<<<q.f.num_tiles, kLocMeasSlots, 0, stream>>>(q);
+    const void *fn = local_meas_kernel_ptr(q.grad_vote != nullptr);
+    const size_t smem = local_meas_smem(mrow);
+    if (smem > 32 * 1024)
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int groups = (q.f.num_ant + kLocMeasWarps - 1) / kLocMeasWarps;
+    void *args[] = {const_cast<LocalParams *>(&q), &part, &mrow, &tiles_per_range};
+    return cudaLaunchKernel(fn, dim3((unsigned)((int64_t)groups * ranges)),
+                            dim3(kLocMeasWarps * 32), args, smem, stream);
+}
+
 // Tile shape: columns bx x by and runs of 4 voxels in z, at most 128 runs, chosen for few
 // tiles (idle slots of a ragged grid cost as much as used ones) with a charge for elongated
 // boxes, whose wider range interval needs more nodes.  8 x 8 x 8 on a large grid.

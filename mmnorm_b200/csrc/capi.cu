@@ -735,11 +735,11 @@ struct BwdPlan {
     const void *fn;
     bool nufft;       // position pass in interpolation form
     bool local;       // ... by tile-local polynomials
-    int bx, by, runs, tiles_y, tiles_z;
+    int bx, by, runs, tiles_y, tiles_z, ltiles;  // voxel boxes of the local passes
     bool meas_nufft;  // measurement pass in interpolation form
     int nu_n, row;
     int mrow, mranges;
-    int64_t mvox_per_range;
+    int mtiles_per_range;
 };
 
 // image_only: the loss has no vote term (grad_vote NULL): the Horner form needs one chain
@@ -774,13 +774,17 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
                (size_t)(pl->threads / 32) * pl->ant_per_stage * 3 * sizeof(float);
     const int64_t per_tile = (int64_t)pl->threads * pl->vpt;
     int64_t tiles = (nvox + per_tile - 1) / per_tile;
+    plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
+    pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
+    pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
+    const int64_t ltiles =
+        (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
+    if (ltiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
+    pl->ltiles = (int)ltiles;
     if (pl->local) {
         pl->ant_per_stage = local_chunk_antennas();
         pl->smem = 0;
-        plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
-        pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
-        pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
-        tiles = (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
+        tiles = ltiles;
     }
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
     pl->tiles = (int)std::max<int64_t>(1, tiles);
@@ -822,26 +826,23 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
                        (size_t)pl->nu_n * sizeof(double2) + 32);
     pl->off_nvox = pl->off_npart = off;
     if (pl->meas_nufft) {
-        // voxel ranges: enough (antenna group, range) CTAs for two waves
+        // box ranges: enough (antenna group, range) CTAs for two waves
         pl->mrow = pl->nu_n + 16;
-        const size_t msmem = nufft_meas_smem(pl->mrow);
-        const void *mfn = nufft_meas_kernel_ptr();
-        if (msmem > 48 * 1024)
+        const size_t msmem = local_meas_smem(pl->mrow);
+        const void *mfn = local_meas_kernel_ptr(!image_only);
+        if (msmem > 32 * 1024)
             cudaFuncSetAttribute(mfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
-        int dev = 0, sms = 148, per_sm = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mfn, nufft_meas_warps() * 32,
+        int per_sm = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mfn, local_meas_warps() * 32,
                                                           msmem) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
-        const int64_t groups = (A + nufft_meas_warps() - 1) / nufft_meas_warps();
+        const int64_t groups = (A + local_meas_warps() - 1) / local_meas_warps();
         const int64_t want = (2 * (int64_t)sms * per_sm + groups - 1) / std::max<int64_t>(groups, 1);
-        const int64_t chunks = std::max<int64_t>(1, (nvox + 31) / 32);
-        const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>({want, 64, chunks}));
-        pl->mvox_per_range = (chunks + ranges - 1) / ranges * 32;
-        pl->mranges = (int)std::max<int64_t>(1, (nvox + pl->mvox_per_range - 1) / pl->mvox_per_range);
-        off = align_up(off + (size_t)nvox * 5 * sizeof(float4));
+        const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>({want, 64, ltiles}));
+        pl->mtiles_per_range = (int)((ltiles + ranges - 1) / ranges);
+        pl->mranges = (pl->ltiles + pl->mtiles_per_range - 1) / pl->mtiles_per_range;
+        off = align_up(off + local_meas_vox_bytes(ltiles));
         pl->off_npart = off;
         off = align_up(off + (size_t)pl->mranges * A * pl->mrow * sizeof(float2));
     }
@@ -1145,19 +1146,22 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
         launch_nufft_tables(f, F, pl.nu_n, J0, sc, tw, reinterpret_cast<float *>(sc + F),
                             stream) != cudaSuccess)
         return MMN_ERR_CUDA;
+    // the local passes' common parameters
+    LocalParams lq;
+    std::memset(&lq, 0, sizeof(lq));
+    set_local_fields(lq, p, pl.nu_n, pl.row, nullptr);
+    lq.f = f;
+    lq.bx = pl.bx;
+    lq.by = pl.by;
+    lq.runs = pl.runs;
+    lq.tiles_y = pl.tiles_y;
+    lq.tiles_z = pl.tiles_z;
+    lq.grad_image = bp.grad_image;
+    lq.grad_vote = bp.grad_vote;
     if (grad_pos && pl.local) {
-        LocalParams q;
-        std::memset(&q, 0, sizeof(q));
+        LocalParams q = lq;
         float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_meas);
-        set_local_fields(q, p, pl.nu_n, pl.row, rows);
-        q.f = f;
-        q.bx = pl.bx;
-        q.by = pl.by;
-        q.runs = pl.runs;
-        q.tiles_y = pl.tiles_y;
-        q.tiles_z = pl.tiles_z;
-        q.grad_image = bp.grad_image;
-        q.grad_vote = bp.grad_vote;
+        q.rows = rows;
         q.pos_partial = bp.pos_partial;
         if (launch_nufft_grid_window(p->meas, A, F, pl.nu_n, J0, pl.row, sc, tw, ant,
                                      reinterpret_cast<float *>(sc + F), f.ti, q.uq, rows,
@@ -1197,29 +1201,24 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
         if (launch_bwd_pos_reduce(bp, stream) != cudaSuccess) return MMN_ERR_CUDA;
     }
     if (grad_meas && pl.meas_nufft) {
-        NuMeasParams q;
-        std::memset(&q, 0, sizeof(q));
-        q.ant = ant;
-        q.vox = reinterpret_cast<const float4 *>(ws + pl.off_nvox);
-        q.mono_flag = hdr + 1;
-        q.part = reinterpret_cast<float2 *>(ws + pl.off_npart);
-        q.sc = sc;
-        q.tw = tw;
-        q.grad_meas = reinterpret_cast<float2 *>(grad_meas);
-        q.nvox = f.nvox;
-        q.vox_per_range = pl.mvox_per_range;
-        q.ti = f.ti;
-        q.uq = p->slope / kC;
-        q.k0c = 2.0 * kPi * (1.0 / p->wavelength + (double)J0 * p->slope / kC);
-        q.num_ant = A;
-        q.n = pl.nu_n;
-        q.mrow = pl.mrow;
-        q.ranges = pl.mranges;
-        q.F = F;
-        q.J0 = J0;
-        if (launch_nufft_meas(q, f, reinterpret_cast<const float2 *>(grad_image),
-                              reinterpret_cast<const float2 *>(grad_vote),
-                              reinterpret_cast<float4 *>(ws + pl.off_nvox), stream) != cudaSuccess)
+        LocalParams q = lq;
+        q.f.num_tiles = pl.ltiles;
+        q.vox = reinterpret_cast<float4 *>(ws + pl.off_nvox);
+        NuMeasParams o;
+        std::memset(&o, 0, sizeof(o));
+        o.part = reinterpret_cast<const float2 *>(ws + pl.off_npart);
+        o.sc = sc;
+        o.tw = tw;
+        o.grad_meas = reinterpret_cast<float2 *>(grad_meas);
+        o.num_ant = A;
+        o.n = pl.nu_n;
+        o.mrow = pl.mrow;
+        o.ranges = pl.mranges;
+        o.F = F;
+        o.J0 = J0;
+        if (launch_local_meas(q, reinterpret_cast<float2 *>(ws + pl.off_npart), pl.mrow,
+                              pl.mranges, pl.mtiles_per_range, stream) != cudaSuccess ||
+            launch_nufft_meas_out(o, stream) != cudaSuccess)
             return MMN_ERR_CUDA;
     } else if (grad_meas) {
         if (launch_bwd_vox_rec(bp, reinterpret_cast<float4 *>(ws + pl.off_vox), stream) !=

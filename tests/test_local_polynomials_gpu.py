@@ -55,7 +55,7 @@ def test_forward_edges(cuda_dev, oracle, shape, ants, spacing, rx):
 
 @SHAPES
 @pytest.mark.parametrize("rx,vote", [(1, True), (1, False), (3, True), (3, False)])
-def test_position_gradient_edges(cuda_dev, oracle, shape, ants, spacing, rx, vote):
+def test_gradient_edges(cuda_dev, oracle, shape, ants, spacing, rx, vote):
     from mmnorm_b200 import ops
     sc = _scene(shape, ants, 50, spacing, 200 + ants)
     rng = np.random.default_rng(ants)
@@ -66,13 +66,13 @@ def test_position_gradient_edges(cuda_dev, oracle, shape, ants, spacing, rx, vot
     gW = gW if vote else np.zeros_like(gW)
     args = [_t(a, cuda_dev) for a in (sc.x_locs, sc.y_locs, sc.z_locs, sc.antenna_locs, rxo,
                                       sc.meas)]
-    gp = ops.backproject_backward(*args, sc.wavelength, sc.slope, _t(gI, cuda_dev),
-                                  _t(gW, cuda_dev) if vote else None, is_ti_radar=rx == 3,
-                                  want_meas=False)[1]
-    _, gp_o = oracle.full_backward(sc.voxel_centres(), sc.antenna_locs, rxo, sc.meas,
+    gm, gp = ops.backproject_backward(*args, sc.wavelength, sc.slope, _t(gI, cuda_dev),
+                                      _t(gW, cuda_dev) if vote else None, is_ti_radar=rx == 3)
+    gm_o, gp_o = oracle.full_backward(sc.voxel_centres(), sc.antenna_locs, rxo, sc.meas,
                                    sc.wavelength, sc.slope, gI.astype(np.complex128),
                                    gW.T.astype(np.complex128), is_ti=rx == 3)
     assert oracle.rel_l2(gp.cpu().numpy().astype(np.float64), gp_o) < 1e-5
+    assert oracle.rel_l2(gm.cpu().numpy().astype(np.complex128), gm_o) < TOL
 
 
 def test_forward_unordered_axes(cuda_dev, oracle):
