@@ -141,11 +141,13 @@ struct LocalParams {
     const float2 *grad_vote;
     float *pos_partial;        // [num_tiles, num_ant, 3]
     float4 *vox;               // measurement pass: voxel records in box order
+    int32_t slots;             // ... voxel runs per box, a multiple of 32
 };
-void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs);
+// most: voxel runs of a tile
+void plan_local_tiles(int nx, int ny, int nz, int most, int *bx, int *by, int *runs);
 // measurement pass: bytes of the voxel records, shared memory of the antenna rows (mrow cells
 // each), warps (antennas) per CTA
-size_t local_meas_vox_bytes(int64_t tiles);
+size_t local_meas_vox_bytes(int64_t tiles, int slots);
 size_t local_meas_smem(int mrow);
 int local_meas_warps();
 const void *local_meas_kernel_ptr(bool vote);

@@ -708,12 +708,16 @@ const void *bwd_pos_local_kernel_ptr(bool vote, int *threads) {
 // (8 cells each).  A warp owns one antenna and its row and walks a range of boxes, 32 voxel
 // runs at a time; everything is summed in a fixed order.  Boxes too wide for the nodes spread
 // every voxel.
+//
+// A box costs some 500 instructions besides its voxels' 85 each (bounds, the warp sums, the
+// spread), so boxes are larger than the forward's where enough of them remain to fill the GPU:
+// 2048, else 1024, else 512 voxels.  64^3 voxels x 4096 antennas x 128 samples (this pass):
+// 16.3 ms with a spread per voxel, 6.2 / 5.1 / 4.5 ms with boxes of 512 / 1024 / 2048.
 namespace {
 
 constexpr int kLocMeasWarps = 4;
-constexpr int kLocMeasSlots = 128;  // voxel runs of a box
 
-// Voxel records in box order: per box kLocMeasSlots x (x, y, -, -), (z_0 .. z_3), then per run
+// Voxel records in box order: per box q.slots x (x, y, -, -), (z_0 .. z_3), then per run
 // position k (gI) or (gI, gW_x), (gW_y, gW_z); and the boxes' bounds.
 struct LocVox {
     float4 *xy, *z, *box;  // [tiles][slots], [tiles][slots], [tiles][2]
@@ -721,7 +725,7 @@ struct LocVox {
 };
 __device__ __forceinline__ LocVox loc_vox(const LocalParams &q) {
     LocVox r;
-    const size_t n = (size_t)q.f.num_tiles * kLocMeasSlots;
+    const size_t n = (size_t)q.f.num_tiles * q.slots;
     r.box = q.vox;
     r.xy = r.box + 2 * (size_t)q.f.num_tiles;
     r.z = r.xy + n;
@@ -729,7 +733,7 @@ __device__ __forceinline__ LocVox loc_vox(const LocalParams &q) {
     return r;
 }
 
-__global__ void __launch_bounds__(kLocMeasSlots) local_vox_kernel(const LocalParams q) {
+__global__ void __launch_bounds__(512) local_vox_kernel(const LocalParams q) {
     const FwdParams &p = q.f;
     const int tile = blockIdx.x, slot = threadIdx.x;
     const LocVox r = loc_vox(q);
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(kLocMeasSlots) local_vox_kernel(const LocalPar
         r.box[2 * tile + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
     const LocSlot s = local_slot(q, tile, slot);
-    const size_t at = (size_t)tile * kLocMeasSlots + slot;
+    const size_t at = (size_t)tile * q.slots + slot;
     r.xy[at] = make_float4(__ldg(p.x_locs + min(s.ix, p.nx - 1)),
                            __ldg(p.y_locs + min(s.iy, p.ny - 1)), 0.f, 0.f);
     float z[kLocRun];
@@ -758,10 +762,10 @@ __global__ void __launch_bounds__(kLocMeasSlots) local_vox_kernel(const LocalPar
         if (q.grad_vote) {
             const float2 a = ok ? q.grad_vote[v] : zero, b = ok ? q.grad_vote[p.nvox + v] : zero,
                          c = ok ? q.grad_vote[2 * p.nvox + v] : zero;
-            r.g[(2 * gk) * kLocMeasSlots + slot] = make_float4(gi.x, gi.y, a.x, a.y);
-            r.g[(2 * gk + 1) * kLocMeasSlots + slot] = make_float4(b.x, b.y, c.x, c.y);
+            r.g[(2 * gk) * q.slots + slot] = make_float4(gi.x, gi.y, a.x, a.y);
+            r.g[(2 * gk + 1) * q.slots + slot] = make_float4(b.x, b.y, c.x, c.y);
         } else {
-            reinterpret_cast<float2 *>(r.g)[gk * kLocMeasSlots + slot] = gi;
+            reinterpret_cast<float2 *>(r.g)[gk * q.slots + slot] = gi;
         }
     }
     r.z[at] = make_float4(z[0], z[1], z[2], z[3]);
@@ -843,8 +847,8 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
 #pragma unroll
     for (int i = 0; i < NV; ++i) mom[i] = make_float2(0.f, 0.f);
 #pragma unroll 1
-    for (int slot = lane; slot < kLocMeasSlots; slot += 32) {
-        const size_t at = (size_t)tile * kLocMeasSlots + slot;
+    for (int slot = lane; slot < q.slots; slot += 32) {
+        const size_t at = (size_t)tile * q.slots + slot;
         const float4 xy = __ldg(vx.xy + at), z4 = __ldg(vx.z + at);
         const float vz[kLocRun] = {z4.x, z4.y, z4.z, z4.w};
         double d[kLocRun];
@@ -863,14 +867,14 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
                 const size_t gk = (size_t)tile * kLocRun + j;
                 float Gr, Gi;
                 if (VOTE) {
-                    const float4 g0 = __ldg(vx.g + (2 * gk) * kLocMeasSlots + slot);
-                    const float4 g1 = __ldg(vx.g + (2 * gk + 1) * kLocMeasSlots + slot);
+                    const float4 g0 = __ldg(vx.g + (2 * gk) * q.slots + slot);
+                    const float4 g1 = __ldg(vx.g + (2 * gk + 1) * q.slots + slot);
                     const float uz = a.u[2] - vz[j];
                     Gr = fmaf(g1.z, uz, fmaf(g1.x, uy, fmaf(g0.z, ux, g0.x)));
                     Gi = fmaf(g1.w, uz, fmaf(g1.y, uy, fmaf(g0.w, ux, g0.y)));
                 } else {
                     const float2 g = __ldg(reinterpret_cast<const float2 *>(vx.g) +
-                                           gk * kLocMeasSlots + slot);
+                                           gk * q.slots + slot);
                     Gr = g.x;
                     Gi = g.y;
                 }
@@ -937,7 +941,7 @@ __device__ __forceinline__ void box_moments_nn(const LocalParams &q, const LocVo
 
 // blockIdx.x = antenna group (one antenna per warp) + groups * box range.
 template <bool VOTE>
-__global__ void __launch_bounds__(kLocMeasWarps * 32)
+__global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
     bp_bwd_meas_local_kernel(const LocalParams q, float2 *part, int mrow, int tiles_per_range) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ LocRec s_rec[kLocMeasWarps];
@@ -1017,9 +1021,8 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32)
     for (int c = lane; c < mrow; c += 32) dst[c] = row[c];
 }
 
-size_t local_meas_vox_bytes(int64_t tiles) {
-    return (size_t)tiles * (2 * sizeof(float4) +
-                            kLocMeasSlots * (2 + 2 * kLocRun) * sizeof(float4));
+size_t local_meas_vox_bytes(int64_t tiles, int slots) {
+    return (size_t)tiles * (2 + (size_t)slots * (2 + 2 * kLocRun)) * sizeof(float4);
 }
 
 size_t local_meas_smem(int mrow) { return (size_t)kLocMeasWarps * mrow * sizeof(float2); }
@@ -1033,7 +1036,7 @@ const void *local_meas_kernel_ptr(bool vote) {
 
 cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int ranges,
                               int tiles_per_range, cudaStream_t stream) {
-    local_vox_kernel<<<q.f.num_tiles, kLocMeasSlots, 0, stream>>>(q);
+    local_vox_kernel<<<q.f.num_tiles, q.slots, 0, stream>>>(q);
     const void *fn = local_meas_kernel_ptr(q.grad_vote != nullptr);
     const size_t smem = local_meas_smem(mrow);
     if (smem > 32 * 1024)
@@ -1044,20 +1047,21 @@ cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int 
                             dim3(kLocMeasWarps * 32), args, smem, stream);
 }
 
-// Tile shape: columns bx x by and runs of 4 voxels in z, at most 128 runs, chosen for few
+// Tile shape: columns bx x by and runs of 4 voxels in z, at most `most` runs, chosen for few
 // tiles (idle slots of a ragged grid cost as much as used ones) with a charge for elongated
 // boxes, whose wider range interval needs more nodes.  8 x 8 x 8 on a large grid.
-void plan_local_tiles(int nx, int ny, int nz, int *bx, int *by, int *runs) {
+void plan_local_tiles(int nx, int ny, int nz, int most, int *bx, int *by, int *runs) {
     double best = 1e300;
     const int zr = (nz + kLocRun - 1) / kLocRun;
+    const double cube = std::sqrt(3.0) * std::cbrt((double)most * kLocRun);
     for (int r = 1; r <= std::min(zr, 16); ++r)
-        for (int y = 1; y <= std::min(ny, 32) && r * y <= kLocThreads; ++y) {
-            const int x = std::min({nx, kLocThreads / (r * y), 32});
+        for (int y = 1; y <= std::min(ny, 32) && r * y <= most; ++y) {
+            const int x = std::min({nx, most / (r * y), 32});
             const double tiles = (double)((nx + x - 1) / x) * ((ny + y - 1) / y) *
                                  ((zr + r - 1) / r);
             const double diag2 = (double)x * x + (double)y * y +
                                  (double)(kLocRun * r) * (kLocRun * r);
-            const double cost = tiles * (1.0 + 0.01 * std::max(0.0, std::sqrt(diag2) - 13.9));
+            const double cost = tiles * (1.0 + 0.01 * std::max(0.0, std::sqrt(diag2) - cube));
             if (cost < best) {
                 best = cost;
                 *bx = x;

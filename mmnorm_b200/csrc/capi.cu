@@ -726,6 +726,26 @@ std::atomic<int> g_pos_form{MMN_PASS_INTERP};
 std::atomic<int> g_pos_variant{0};
 std::atomic<int> g_meas_form{MMN_PASS_INTERP};
 
+// Voxel boxes of a local pass.
+struct LocalTiles {
+    int bx, by, runs, tiles_y, tiles_z;
+    int64_t tiles;
+    void plan(const mmn_problem *p, int most) {
+        plan_local_tiles(p->num_x, p->num_y, p->num_z, most, &bx, &by, &runs);
+        tiles_y = (p->num_y + by - 1) / by;
+        tiles_z = (p->num_z + 4 * runs - 1) / (4 * runs);
+        tiles = (int64_t)((p->num_x + bx - 1) / bx) * tiles_y * tiles_z;
+    }
+    void set(LocalParams &q) const {
+        q.bx = bx;
+        q.by = by;
+        q.runs = runs;
+        q.tiles_y = tiles_y;
+        q.tiles_z = tiles_z;
+        q.f.num_tiles = (int)tiles;
+    }
+};
+
 struct BwdPlan {
     int fp, ant_per_stage, tiles, splits, ant_per_split, threads, vpt;
     size_t smem;
@@ -735,11 +755,11 @@ struct BwdPlan {
     const void *fn;
     bool nufft;       // position pass in interpolation form
     bool local;       // ... by tile-local polynomials
-    int bx, by, runs, tiles_y, tiles_z, ltiles;  // voxel boxes of the local passes
+    LocalTiles pos, meas;  // voxel boxes of the local passes
     bool meas_nufft;  // measurement pass in interpolation form
     int nu_n, row;
     int mrow, mranges;
-    int mtiles_per_range;
+    int mtiles_per_range, mslots;
 };
 
 // image_only: the loss has no vote term (grad_vote NULL): the Horner form needs one chain
@@ -774,17 +794,11 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
                (size_t)(pl->threads / 32) * pl->ant_per_stage * 3 * sizeof(float);
     const int64_t per_tile = (int64_t)pl->threads * pl->vpt;
     int64_t tiles = (nvox + per_tile - 1) / per_tile;
-    plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
-    pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
-    pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
-    const int64_t ltiles =
-        (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
-    if (ltiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
-    pl->ltiles = (int)ltiles;
     if (pl->local) {
         pl->ant_per_stage = local_chunk_antennas();
         pl->smem = 0;
-        tiles = ltiles;
+        pl->pos.plan(p, pl->threads);
+        tiles = pl->pos.tiles;
     }
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
     pl->tiles = (int)std::max<int64_t>(1, tiles);
@@ -839,10 +853,16 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
             per_sm = 1;
         const int64_t groups = (A + local_meas_warps() - 1) / local_meas_warps();
         const int64_t want = (2 * (int64_t)sms * per_sm + groups - 1) / std::max<int64_t>(groups, 1);
-        const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>({want, 64, ltiles}));
-        pl->mtiles_per_range = (int)((ltiles + ranges - 1) / ranges);
-        pl->mranges = (pl->ltiles + pl->mtiles_per_range - 1) / pl->mtiles_per_range;
-        off = align_up(off + local_meas_vox_bytes(ltiles));
+        // the largest boxes (fewest reductions and spreads) that still make that many ranges
+        for (pl->mslots = 512;; pl->mslots /= 2) {
+            pl->meas.plan(p, pl->mslots);
+            if (pl->mslots == 128 || pl->meas.tiles >= want) break;
+        }
+        if (pl->meas.tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
+        const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>({want, 64, pl->meas.tiles}));
+        pl->mtiles_per_range = (int)((pl->meas.tiles + ranges - 1) / ranges);
+        pl->mranges = (int)((pl->meas.tiles + pl->mtiles_per_range - 1) / pl->mtiles_per_range);
+        off = align_up(off + local_meas_vox_bytes(pl->meas.tiles, pl->mslots));
         pl->off_npart = off;
         off = align_up(off + (size_t)pl->mranges * A * pl->mrow * sizeof(float2));
     }
@@ -911,7 +931,7 @@ int plan_nufft_forward(const mmn_problem *p, NuFwdPlan *pl) {
     // the longest row: (G.re, G.im) cells and the antenna record within 48 KB
     if ((int)sizeof(AntRec) + pl->row * 8 > kMaxStageBytes) return MMN_ERR_TOO_LARGE;
     pl->fn = fwd_local_kernel_ptr(&pl->threads);
-    plan_local_tiles(p->num_x, p->num_y, p->num_z, &pl->bx, &pl->by, &pl->runs);
+    plan_local_tiles(p->num_x, p->num_y, p->num_z, pl->threads, &pl->bx, &pl->by, &pl->runs);
     pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
     pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
     const int64_t tiles = (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
@@ -1151,16 +1171,12 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     std::memset(&lq, 0, sizeof(lq));
     set_local_fields(lq, p, pl.nu_n, pl.row, nullptr);
     lq.f = f;
-    lq.bx = pl.bx;
-    lq.by = pl.by;
-    lq.runs = pl.runs;
-    lq.tiles_y = pl.tiles_y;
-    lq.tiles_z = pl.tiles_z;
     lq.grad_image = bp.grad_image;
     lq.grad_vote = bp.grad_vote;
     if (grad_pos && pl.local) {
         LocalParams q = lq;
         float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_meas);
+        pl.pos.set(q);
         q.rows = rows;
         q.pos_partial = bp.pos_partial;
         if (launch_nufft_grid_window(p->meas, A, F, pl.nu_n, J0, pl.row, sc, tw, ant,
@@ -1202,7 +1218,8 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     }
     if (grad_meas && pl.meas_nufft) {
         LocalParams q = lq;
-        q.f.num_tiles = pl.ltiles;
+        pl.meas.set(q);
+        q.slots = pl.mslots;
         q.vox = reinterpret_cast<float4 *>(ws + pl.off_nvox);
         NuMeasParams o;
         std::memset(&o, 0, sizeof(o));
