@@ -3,13 +3,14 @@
 //
 // Per (voxel, virtual antenna) the reference takes ONE sample -- the range-FFT bin
 // floor(d/fft_spacing/2) -- and ONE phasor exp(-j*2*pi*d/lambda) evaluated in FP64
-// (imaging_gpu.cu:90-105; surface_normal_est.cu:99-124).  These kernels keep that
-// arithmetic expression for expression (FP32 distance, FP64 phase and cos/sin, FP32
-// accumulation in antenna order), so their outputs reproduce the reference's
-// kernels; what changes is the structure around it: the antenna geometry streams
-// through shared memory in chunks instead of being re-read from global memory by
-// every thread, the measurement gather is a single 8-byte load of the complex bin,
-// and the image pass can fuse the vote vector W = sum_i c_i (tx_i + o_i/2 - v).
+// (imaging_gpu.cu:90-105; surface_normal_est.cu:99-124).  The exact form gives that
+// arithmetic's bits (FP32 distance, the FP32 roundings of the FP64 cos and sin, FP32
+// accumulation in antenna order), so its outputs reproduce the reference's kernels; what
+// changes is the structure around it: the antenna geometry streams through shared memory in
+// chunks, each thread's two voxels ride in the halves of packed FP32 instructions, the
+// measurement gather is a single 8-byte load of the complex bin, the phasor comes from a short
+// FP64 evaluation that proves its own FP32 rounding (phasor2_exact), and the image pass can
+// fuse the vote vector W = sum_i c_i (tx_i + o_i/2 - v).
 #include <atomic>
 
 #include "bp_kernels.cuh"
@@ -21,186 +22,10 @@ std::atomic<int> g_interp_fast_form{0};
 
 namespace {
 constexpr int kInterpThreads = 256;
+// antennas per loop pass (exact: 1 measured 13.80 ms, 2 13.54; fast: 1 7.06, 2 6.91, 4 6.78)
+constexpr int kExactUnroll = 2, kFastUnroll = 4;
 constexpr int kInterpChunk = 256;  // antennas staged per shared-memory chunk
-
-struct Contrib {
-    float re, im;
-    bool valid;
-};
-
-__device__ __forceinline__ void load_meas(const InterpParams &p, unsigned idx, float &mr,
-                                          float &mi) {
-    if (p.meas) {
-        const float2 m = __ldg(p.meas + idx);
-        mr = m.x;
-        mi = m.y;
-    } else {
-        mr = __ldg(p.meas_r + idx);
-        mi = __ldg(p.meas_i + idx);
-    }
-}
-
-// One (voxel, virtual antenna) term of imaging_gpu.cu:70-105 with the same floating-point
-// operations in the same order (FP32 legs and path, FP64 phase and cos/sin, FP32 complex
-// product), so the sums reproduce the reference kernel's bits.
-__device__ __forceinline__ Contrib pair_contrib(const InterpParams &p, unsigned i, float vx,
-                                                float vy, float vz, float tx, float ty,
-                                                float tz, float ox, float oy, float oz) {
-    Contrib r;
-    r.valid = false;
-    float dx = vx - tx;
-    float dy = vy - ty;
-    float dz = vz - tz;
-    float leg_out = sqrtf(dx * dx +
-                          dy * dy +
-                          dz * dz);
-    float leg_back = sqrtf((dx - ox) * (dx - ox) +
-                           (dy - oy) * (dy - oy) +
-                           (dz - oz) * (dz - oz));
-    float path = leg_out + leg_back;
-    if (p.is_ti != 0) {
-        path += 0.15;
-    }
-    if (path < 0 || path > p.fft_spacing * p.nbins) {
-        return r;
-    }
-    int bin = floorf(path / p.fft_spacing / 2);
-    float m_re, m_im;
-    load_meas(p, i * p.nbins + bin, m_re, m_im);
-    float ph_re = cos(-2 * kPi * path / p.wavelength);
-    float ph_im = sin(-2 * kPi * path / p.wavelength);
-    r.re = (m_re * ph_re - m_im * ph_im);
-    r.im = (m_re * ph_im + m_im * ph_re);
-    r.valid = true;
-    return r;
-}
-
-__device__ __forceinline__ void stage_chunk(const InterpParams &p, int a0, int n, float *sh) {
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const int i = a0 + j;
-        const int rx = i % p.num_rx;
-        sh[6 * j + 0] = p.ant[3 * i + 0];
-        sh[6 * j + 1] = p.ant[3 * i + 1];
-        sh[6 * j + 2] = p.ant[3 * i + 2];
-        sh[6 * j + 3] = p.rxo[3 * rx + 0];
-        sh[6 * j + 4] = p.rxo[3 * rx + 1];
-        sh[6 * j + 5] = p.rxo[3 * rx + 2];
-    }
-}
 }  // namespace
-
-// Image pass (cuda_image, interpolated branch), optionally fusing the vote vector.
-__global__ void __launch_bounds__(kInterpThreads) interp_image_kernel(const InterpParams p) {
-    __shared__ float sh[6 * kInterpChunk];
-    const int64_t rel = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t ind = rel + p.start;
-    const bool active = rel < p.count && ind < p.nvox;
-    const int64_t v = active ? ind : 0;
-    const int64_t nyz = (int64_t)p.ny * p.nz;
-    const int x = (int)(v / nyz);
-    const int y = (int)((v - (int64_t)x * nyz) / p.nz);
-    const int z = (int)(v - (int64_t)x * nyz - (int64_t)y * p.nz);
-    const float vx = p.x_locs[x];
-    const float vy = p.y_locs[y];
-    const float vz = p.z_locs[z];
-    float acc_re = 0;
-    float acc_im = 0;
-    float w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int a0 = 0; a0 < p.num_ant; a0 += kInterpChunk) {
-        const int n = min(kInterpChunk, p.num_ant - a0);
-        __syncthreads();
-        stage_chunk(p, a0, n, sh);
-        __syncthreads();
-        if (!active) continue;
-        for (int j = 0; j < n; ++j) {
-            const float *g = sh + 6 * j;
-            const Contrib c = pair_contrib(p, (unsigned)(a0 + j), vx, vy, vz, g[0], g[1], g[2],
-                                           g[3], g[4], g[5]);
-            if (!c.valid) continue;
-            acc_re += c.re;
-            acc_im += c.im;
-            if (p.vote) {
-                const float ex = (g[0] + g[3] / 2) - vx;
-                const float ey = (g[1] + g[4] / 2) - vy;
-                const float ez = (g[2] + g[5] / 2) - vz;
-                w[0] = fmaf(c.re, ex, w[0]);
-                w[1] = fmaf(c.im, ex, w[1]);
-                w[2] = fmaf(c.re, ey, w[2]);
-                w[3] = fmaf(c.im, ey, w[3]);
-                w[4] = fmaf(c.re, ez, w[4]);
-                w[5] = fmaf(c.im, ez, w[5]);
-            }
-        }
-    }
-    if (!active) return;
-    if (p.out_r) {
-        p.out_r[v] = acc_re;
-        p.out_i[v] = acc_im;
-    }
-    if (p.image) p.image[v] = make_float2(acc_re, acc_im);
-    if (p.vote) {
-        p.vote[v] = make_float2(w[0], w[1]);
-        p.vote[p.nvox + v] = make_float2(w[2], w[3]);
-        p.vote[2 * p.nvox + v] = make_float2(w[4], w[5]);
-    }
-}
-
-// Normal pass (cuda_sn_est, surface_normal_est.cu:63-149) over a valid-voxel list; the
-// weight and the virtual-antenna direction use the reference's operations in order.
-__global__ void __launch_bounds__(kInterpThreads) interp_normals_kernel(const InterpParams p) {
-    __shared__ float sh[6 * kInterpChunk];
-    const int64_t rel = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t ind64 = rel + p.start;
-    const bool active = rel < p.count && ind64 < p.num_valid && ind64 >= 0;
-    const int ind = active ? (int)ind64 : 0;
-    int x = 0, y = 0, z = 0;
-    if (active) {
-        x = p.vidx_x[ind];
-        y = p.vidx_y[ind];
-        z = p.vidx_z[ind];
-    }
-    const float vx = p.x_locs[x];
-    const float vy = p.y_locs[y];
-    const float vz = p.z_locs[z];
-    const float i_re = active ? p.img_r[x * p.ny * p.nz + y * p.nz + z] : 1.f;
-    const float i_im = active ? p.img_i[x * p.ny * p.nz + y * p.nz + z] : 0.f;
-    const float mag = sqrtf(i_re * i_re + i_im * i_im);
-    float acc_x = 0;
-    float acc_y = 0;
-    float acc_z = 0;
-    for (int a0 = 0; a0 < p.num_ant; a0 += kInterpChunk) {
-        const int n = min(kInterpChunk, p.num_ant - a0);
-        __syncthreads();
-        stage_chunk(p, a0, n, sh);
-        __syncthreads();
-        if (!active) continue;
-        for (int j = 0; j < n; ++j) {
-            const float *g = sh + 6 * j;
-            const float tx = g[0], ty = g[1], tz = g[2];
-            const float ox = g[3], oy = g[4], oz = g[5];
-            const Contrib c = pair_contrib(p, (unsigned)(a0 + j), vx, vy, vz, tx, ty, tz, ox,
-                                           oy, oz);
-            if (!c.valid) continue;
-            float c_re = c.re;
-            float c_im = c.im;
-            float ux = tx + ox / 2;
-            float uy = ty + oy / 2;
-            float uz = tz + oz / 2;
-            float ex = ux - vx;
-            float ey = uy - vy;
-            float ez = uz - vz;
-            float wgt = (c_re * i_re) + (c_im * i_im);
-            wgt /= mag;
-            acc_x += (ex * wgt);
-            acc_y += (ey * wgt);
-            acc_z += (ez * wgt);
-        }
-    }
-    if (!active) return;
-    p.n_x[ind] = acc_x;
-    p.n_y[ind] = acc_y;
-    p.n_z[ind] = acc_z;
-}
 
 // ---------------------------------------------------------------------------------
 // Fast form.  The path length and the range bin are the reference's (same FP32
@@ -443,7 +268,7 @@ __global__ void __launch_bounds__(kInterpThreads) interp_normals_fast_kernel(con
 }
 
 // ---------------------------------------------------------------------------------
-// Fast form, packed: each thread's two voxels ride in the two halves of Blackwell's packed
+// Packed kernels (both forms): each thread's two voxels ride in the two halves of Blackwell's packed
 // FP32 instructions (FADD2 / FMUL2 / FFMA2; each half rounds exactly like the scalar
 // instruction), so the per-pair arithmetic -- differences, squared range, range bin,
 // turn count, complex product, vote -- issues once per voxel pair.  The square roots, the
@@ -494,6 +319,24 @@ __device__ __forceinline__ bool pack_chunk_has_offsets(const PackAnt *sh, int n)
     return __syncthreads_or(any) != 0;
 }
 
+// Correctly rounded square roots of two values: s = x y from the hardware reciprocal square root
+// y, then Heron's step s + (x - s^2) y / 2 with the residual exact in one FMA (Markstein, IBM J.
+// Res. Dev. 34, 1990).  That rounds like sqrtf for every mantissa and exponent parity (checked
+// exhaustively over [1, 4), 2^24 inputs); outside [2^-100, 2^100], and for NaN, sqrtf itself.
+__device__ __forceinline__ float2 sqrt2(float2 x) {
+    float2 y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(x.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(x.y));
+    const float2 s = __fmul2_rn(x, y);
+    const float2 h = __fmul2_rn(y, dup(0.5f));
+    const float2 e = __ffma2_rn(make_float2(-s.x, -s.y), s, x);
+    float2 r = __ffma2_rn(e, h, s);
+    if (!(fminf(x.x, x.y) >= 7.888609052210118e-31f && fmaxf(x.x, x.y) <= 1.2676506002282294e30f) ||
+        !(x.x == x.x && x.y == x.y))
+        r = make_float2(sqrtf(x.x), sqrtf(x.y));
+    return r;
+}
+
 __device__ __forceinline__ float2 sumsq2(float2 dx, float2 dy, float2 dz) {
     return __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
 }
@@ -506,7 +349,7 @@ __device__ __forceinline__ float2 path2(float2 vx, float2 vy, float2 vz, const P
     const float2 dy = __fadd2_rn(vy, a.nty);
     const float2 dz = __fadd2_rn(vz, a.ntz);
     const float2 s = sumsq2(dx, dy, dz);
-    const float2 leg = make_float2(sqrtf(s.x), sqrtf(s.y));
+    const float2 leg = sqrt2(s);
     float2 path;
     if (MONO) {
         path = __fadd2_rn(leg, leg);
@@ -515,7 +358,7 @@ __device__ __forceinline__ float2 path2(float2 vx, float2 vy, float2 vz, const P
         const float2 by = __fadd2_rn(dy, a.noy);
         const float2 bz = __fadd2_rn(dz, a.noz);
         const float2 sb = sumsq2(bx, by, bz);
-        path = __fadd2_rn(leg, make_float2(sqrtf(sb.x), sqrtf(sb.y)));
+        path = __fadd2_rn(leg, sqrt2(sb));
     }
     if (ti) {  // float += double, as the reference adds its 0.15 m
         path.x += 0.15;
@@ -524,19 +367,24 @@ __device__ __forceinline__ float2 path2(float2 vx, float2 vy, float2 vz, const P
     return path;
 }
 
-// fast_bin for two paths (the arithmetic packed, the rare division fallback per voxel).
-__device__ __forceinline__ int2 bin2(float2 path, float fsp, float half_inv) {
+// The reference's range bin floor(RN(path / fsp) / 2) (imaging_gpu.cu:100) of two paths, plus
+// kBinBias and clamped to bin nbins - 1 (an in-range path's bin is at most nbins / 2; anything
+// else, a NaN's too, must only stay inside the row).  h = path * (1/(2 fsp)) is within 2e-7 h of
+// the rounded quotient's half, so floor(h) -- one addition rounded down -- is that bin unless h
+// lies within 1.2e-6 (h + 1) of an integer; then, and for a NaN (a path's, or half_inv's, which
+// sends every path here), the reference's own division decides.
+constexpr uint32_t kBinBias = 0x4B000000u;  // bits of 2^23
+__device__ __forceinline__ uint2 bin2(float2 path, float fsp, float half_inv, uint32_t nbins) {
     const float2 h = __fmul2_rn(path, dup(half_inv));
-    const float2 hm = __fadd2_rn(h, dup(kRoundMagic));
-    const float2 r = __fadd2_rn(hm, dup(-kRoundMagic));
-    const bool ax = r.x > h.x, ay = r.y > h.y;
-    const float2 fr = __fadd2_rn(__fadd2_rn(h, make_float2(-r.x, -r.y)),
-                                 make_float2(ax ? 1.f : 0.f, ay ? 1.f : 0.f));
-    const float2 tol = __fmul2_rn(make_float2(fmaxf(h.x, 1.f), fmaxf(h.y, 1.f)), dup(1.2e-6f));
-    int2 b = make_int2(__float_as_int(hm.x) - __float_as_int(kRoundMagic) - (ax ? 1 : 0),
-                       __float_as_int(hm.y) - __float_as_int(kRoundMagic) - (ay ? 1 : 0));
-    if (fr.x < tol.x || fr.x > 1.f - tol.x) b.x = (int)floorf(path.x / fsp / 2);
-    if (fr.y < tol.y || fr.y > 1.f - tol.y) b.y = (int)floorf(path.y / fsp / 2);
+    const float2 hm = make_float2(__fadd_rd(h.x, 8388608.f), __fadd_rd(h.y, 8388608.f));
+    const float2 fr = __fadd2_rn(h, __fadd2_rn(dup(8388608.f), make_float2(-hm.x, -hm.y)));
+    const float2 mid = __fadd2_rn(fr, dup(-0.5f));
+    const float2 lim = __ffma2_rn(h, dup(-1.2e-6f), dup(0.5f - 1.2e-6f));
+    uint2 b = make_uint2(__float_as_uint(hm.x), __float_as_uint(hm.y));
+    if (!(fabsf(mid.x) < lim.x)) b.x = (uint32_t)(int)floorf(path.x / fsp / 2) + kBinBias;
+    if (!(fabsf(mid.y) < lim.y)) b.y = (uint32_t)(int)floorf(path.y / fsp / 2) + kBinBias;
+    b.x = min(b.x, nbins - 1u + kBinBias);
+    b.y = min(b.y, nbins - 1u + kBinBias);
     return b;
 }
 
@@ -554,42 +402,126 @@ __device__ __forceinline__ void phasor2(float2 path, float hi, float lo, float2 
     __sincosf(ang.y, &s.y, &c.y);
 }
 
-template <bool MONO, bool VOTE, bool SOA>
+// The reference's own phasor (FP64 phase, cos, sin, rounded to FP32): the fallback of
+// phasor2_exact.
+__device__ __noinline__ float2 phasor_library(float path, float wavelength) {
+    float ph_re = cos(-2 * kPi * path / wavelength);
+    float ph_im = sin(-2 * kPi * path / wavelength);
+    return make_float2(ph_re, ph_im);
+}
+
+// FP64 (cos, sin) of -2 pi path / lambda as bounds: the turns path * (-1/lambda), reduced to
+// half a turn in one FMA, then polynomials in r^2 (fitted at Chebyshev nodes on |r| <= 1/4: sine
+// 7.8e-14, cosine 1.9e-15).  The reference's rounded phase and this one differ by less than
+// 3.8e-16 relative (two roundings and the rounded pi there, the rounded 1/lambda here), i.e. by
+// less than 2.4e-15 path / lambda radians; with 1.5e-13 for the fits, the evaluation and the
+// library functions' ulps,
+//     delta = 2.5e-15 path / lambda + 1.5e-13
+// bounds the distance of both components.  lo and hi are the FP32 roundings of the bounds'
+// ends: where they agree, every value between them, the reference's among them, rounds to that.
+__device__ __forceinline__ bool phasor_exact(float path, double ninv, float &c, float &s) {
+    const double kM = 3377699720527872.0;  // 1.5 * 2^51: the sum rounds to half turns
+    const double P = (double)path;
+    const double t = fma(P, ninv, kM);
+    const uint32_t flip = (uint32_t)__double2loint(t) << 31;  // odd half turns negate both
+    const double r = fma(P, ninv, kM - t);
+    const double y = r * r;
+    double p = fma(3.6658551595639612, y, -15.081483206893);
+    p = fma(p, y, 42.058134871372054);
+    p = fma(p, y, -76.70584754377326);
+    p = fma(p, y, 81.60524914901583);
+    p = fma(p, y, -41.341702239903675);
+    p = fma(p, y, 6.28318530717927);
+    const double sn = p * r;
+    double g = fma(-1.6452233497893094, y, 7.896555735851554);
+    g = fma(g, y, -26.42588874334368);
+    g = fma(g, y, 60.24463060817376);
+    g = fma(g, y, -85.45681703563287);
+    g = fma(g, y, 64.93939402133272);
+    g = fma(g, y, -19.739208802174744);
+    g = fma(g, y, 0.9999999999999981);
+    const double delta = fma(P, -2.5e-15 * ninv, 1.5e-13);
+    const float c_lo = (float)(g - delta), c_hi = (float)(g + delta);
+    const float s_lo = (float)(sn - delta), s_hi = (float)(sn + delta);
+    c = __uint_as_float(__float_as_uint(c_lo) ^ flip);
+    s = __uint_as_float(__float_as_uint(s_lo) ^ flip);
+    return c_lo == c_hi && s_lo == s_hi;
+}
+
+// The reference's FP32 phasors of two paths, bit for bit: about one evaluation in 4000 cannot
+// decide its rounding and takes the library functions.  Bound: instruction dispatch (the FP64
+// and packed instructions take about two slots).  90 x 100 x 70 voxels x 4096 antennas, four
+// receivers, TI offset: 20.3 ms with the two library calls per pair, 13.5 ms.
+__device__ __forceinline__ void phasor2_exact(float2 path, float wavelength, double ninv,
+                                              float2 &c, float2 &s) {
+    if (!phasor_exact(path.x, ninv, c.x, s.x)) {
+        const float2 a = phasor_library(path.x, wavelength);
+        c.x = a.x;
+        s.x = a.y;
+    }
+    if (!phasor_exact(path.y, ninv, c.y, s.y)) {
+        const float2 a = phasor_library(path.y, wavelength);
+        c.y = a.x;
+        s.y = a.y;
+    }
+}
+
+// c_i of two voxels against one antenna, as imaging_gpu.cu:90-105; v0, v1: the path lies in
+// the measured range (the reference skips the others).
+template <bool MONO, bool SOA, bool EXACT>
+__device__ __forceinline__ void pack_pair(const InterpParams &p, const PackAnt &a, ptrdiff_t row,
+                                          float range_max, bool ti, float2 vx, float2 vy,
+                                          float2 vz, float2 &re, float2 &im, bool &v0, bool &v1) {
+    const float2 path = path2<MONO>(vx, vy, vz, a, ti);
+    v0 = !(path.x > range_max);  // a path is never negative
+    v1 = !(path.y > range_max);
+    const uint2 b = bin2(path, p.fft_spacing, p.half_inv_fsp, (uint32_t)p.nbins);
+    float2 mre, mim;
+    if (SOA) {
+        const float *mr = p.meas_r + row - kBinBias, *mi = p.meas_i + row - kBinBias;
+        mre = make_float2(__ldg(mr + b.x), __ldg(mr + b.y));
+        mim = make_float2(__ldg(mi + b.x), __ldg(mi + b.y));
+    } else {
+        const float2 *m = p.meas + row - kBinBias;
+        const float2 m0 = __ldg(m + b.x), m1 = __ldg(m + b.y);
+        mre = make_float2(m0.x, m1.x);
+        mim = make_float2(m0.y, m1.y);
+    }
+    float2 c, s;
+    if (EXACT) phasor2_exact(path, p.wavelength, p.neg_inv_lambda, c, s);
+    else phasor2(path, p.inv_lambda_hi, p.inv_lambda_lo, c, s);
+    // the reference kernel's products as they are contracted: fma(m_re, c, -(m_im s)) and
+    // fma(m_im, c, m_re s)
+    re = __ffma2_rn(mre, c, __fmul2_rn(mim, make_float2(-s.x, -s.y)));
+    im = __ffma2_rn(mim, c, __fmul2_rn(mre, s));
+}
+
+template <bool MONO, bool VOTE, bool SOA, bool EXACT>
 __device__ __forceinline__ void pack_image_chunk(const InterpParams &p, const PackAnt *sh,
                                                  int a0, int n, float range_max, bool ti,
                                                  float2 vx, float2 vy, float2 vz, float2 nvx,
                                                  float2 nvy, float2 nvz, float2 (&acc)[8]) {
-#pragma unroll 2
+    constexpr int kUnroll = EXACT ? kExactUnroll : kFastUnroll;
+#pragma unroll kUnroll
     for (int j = 0; j < n; ++j) {
         const PackAnt &a = sh[j];
-        const size_t row = (size_t)(a0 + j) * (size_t)p.nbins;
-        const float2 path = path2<MONO>(vx, vy, vz, a, ti);
-        const bool v0 = !(path.x < 0 || path.x > range_max);
-        const bool v1 = !(path.y < 0 || path.y > range_max);
-        int2 b = bin2(path, p.fft_spacing, p.half_inv_fsp);
-        b.x = v0 ? b.x : 0;
-        b.y = v1 ? b.y : 0;
-        float2 mre, mim;
-        if (SOA) {
-            mre = make_float2(__ldg(p.meas_r + row + b.x), __ldg(p.meas_r + row + b.y));
-            mim = make_float2(__ldg(p.meas_i + row + b.x), __ldg(p.meas_i + row + b.y));
-        } else {
-            const float2 m0 = __ldg(p.meas + row + b.x), m1 = __ldg(p.meas + row + b.y);
-            mre = make_float2(m0.x, m1.x);
-            mim = make_float2(m0.y, m1.y);
+        const ptrdiff_t row = (ptrdiff_t)(a0 + j) * p.nbins;
+        float2 re, im;
+        bool v0, v1;
+        pack_pair<MONO, SOA, EXACT>(p, a, row, range_max, ti, vx, vy, vz, re, im, v0, v1);
+        float2 ex = __fadd2_rn(a.ux, nvx);
+        float2 ey = __fadd2_rn(a.uy, nvy);
+        float2 ez = __fadd2_rn(a.uz, nvz);
+        if (!(v0 && v1)) {  // a skipped pair adds nothing, whatever its vector is
+            re = make_float2(v0 ? re.x : 0.f, v1 ? re.y : 0.f);
+            im = make_float2(v0 ? im.x : 0.f, v1 ? im.y : 0.f);
+            ex = make_float2(v0 ? ex.x : 0.f, v1 ? ex.y : 0.f);
+            ey = make_float2(v0 ? ey.x : 0.f, v1 ? ey.y : 0.f);
+            ez = make_float2(v0 ? ez.x : 0.f, v1 ? ez.y : 0.f);
         }
-        float2 c, s;
-        phasor2(path, p.inv_lambda_hi, p.inv_lambda_lo, c, s);
-        float2 re = __ffma2_rn(mre, c, __fmul2_rn(mim, make_float2(-s.x, -s.y)));
-        float2 im = __ffma2_rn(mre, s, __fmul2_rn(mim, c));
-        re = make_float2(v0 ? re.x : 0.f, v1 ? re.y : 0.f);
-        im = make_float2(v0 ? im.x : 0.f, v1 ? im.y : 0.f);
         acc[0] = __fadd2_rn(acc[0], re);
         acc[1] = __fadd2_rn(acc[1], im);
         if (VOTE) {
-            const float2 ex = __fadd2_rn(a.ux, nvx);
-            const float2 ey = __fadd2_rn(a.uy, nvy);
-            const float2 ez = __fadd2_rn(a.uz, nvz);
             acc[2] = __ffma2_rn(re, ex, acc[2]);
             acc[3] = __ffma2_rn(im, ex, acc[3]);
             acc[4] = __ffma2_rn(re, ey, acc[4]);
@@ -600,23 +532,24 @@ __device__ __forceinline__ void pack_image_chunk(const InterpParams &p, const Pa
     }
 }
 
-template <bool VOTE, bool SOA>
+template <bool VOTE, bool SOA, bool EXACT>
 __device__ __forceinline__ void pack_image_dispatch(const InterpParams &p, const PackAnt *sh,
                                                     int a0, int n, float range_max, bool ti,
                                                     bool offsets, float2 vx, float2 vy,
                                                     float2 vz, float2 nvx, float2 nvy,
                                                     float2 nvz, float2 (&acc)[8]) {
     if (offsets)
-        pack_image_chunk<false, VOTE, SOA>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
+        pack_image_chunk<false, VOTE, SOA, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
                                                   nvy, nvz, acc);
     else
-        pack_image_chunk<true, VOTE, SOA>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
+        pack_image_chunk<true, VOTE, SOA, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
                                                  nvy, nvz, acc);
 }
 }  // namespace
 
-// Image pass in packed fast form: voxels rel and rel + blockDim of each 2*blockDim tile
-// (coalesced stores), optionally fusing the vote vector.
+// Image pass: voxels rel and rel + blockDim of each 2*blockDim tile (coalesced stores),
+// optionally fusing the vote vector.
+template <bool EXACT>
 __global__ void __launch_bounds__(kInterpThreads) interp_image_pack_kernel(const InterpParams p) {
     __shared__ PackAnt sh[kInterpChunk];
     const int64_t nyz = (int64_t)p.ny * p.nz;
@@ -653,15 +586,15 @@ __global__ void __launch_bounds__(kInterpThreads) interp_image_pack_kernel(const
         __syncthreads();
         const bool offsets = pack_chunk_has_offsets(sh, n);
         if (p.vote) {
-            if (soa) pack_image_dispatch<true, true>(p, sh, a0, n, range_max, ti, offsets,
+            if (soa) pack_image_dispatch<true, true, EXACT>(p, sh, a0, n, range_max, ti, offsets,
                                                             vx, vy, vz, nvx, nvy, nvz, acc);
-            else pack_image_dispatch<true, false>(p, sh, a0, n, range_max, ti, offsets,
+            else pack_image_dispatch<true, false, EXACT>(p, sh, a0, n, range_max, ti, offsets,
                                                          vx, vy, vz, nvx, nvy, nvz, acc);
         } else {
-            if (soa) pack_image_dispatch<false, true>(p, sh, a0, n, range_max, ti,
+            if (soa) pack_image_dispatch<false, true, EXACT>(p, sh, a0, n, range_max, ti,
                                                              offsets, vx, vy, vz, nvx, nvy, nvz,
                                                              acc);
-            else pack_image_dispatch<false, false>(p, sh, a0, n, range_max, ti, offsets,
+            else pack_image_dispatch<false, false, EXACT>(p, sh, a0, n, range_max, ti, offsets,
                                                           vx, vy, vz, nvx, nvy, nvz, acc);
         }
     }
@@ -685,48 +618,44 @@ __global__ void __launch_bounds__(kInterpThreads) interp_image_pack_kernel(const
 }
 
 namespace {
-template <bool MONO, bool SOA>
+// mag: |I| of the two voxels (exact form, the reference's quotient) or 1/|I| (fast form).
+template <bool MONO, bool SOA, bool EXACT>
 __device__ __forceinline__ void pack_normals_chunk(const InterpParams &p, const PackAnt *sh,
                                                    int a0, int n, float range_max, bool ti,
                                                    float2 vx, float2 vy, float2 vz, float2 nvx,
                                                    float2 nvy, float2 nvz, float2 ire,
-                                                   float2 iim, float2 inv_mag,
-                                                   float2 (&acc)[3]) {
-#pragma unroll 2
+                                                   float2 iim, float2 mag, float2 (&acc)[3]) {
+    constexpr int kUnroll = EXACT ? kExactUnroll : kFastUnroll;
+#pragma unroll kUnroll
     for (int j = 0; j < n; ++j) {
         const PackAnt &a = sh[j];
-        const size_t row = (size_t)(a0 + j) * (size_t)p.nbins;
-        const float2 path = path2<MONO>(vx, vy, vz, a, ti);
-        const bool v0 = !(path.x < 0 || path.x > range_max);
-        const bool v1 = !(path.y < 0 || path.y > range_max);
-        int2 b = bin2(path, p.fft_spacing, p.half_inv_fsp);
-        b.x = v0 ? b.x : 0;
-        b.y = v1 ? b.y : 0;
-        float2 mre, mim;
-        if (SOA) {
-            mre = make_float2(__ldg(p.meas_r + row + b.x), __ldg(p.meas_r + row + b.y));
-            mim = make_float2(__ldg(p.meas_i + row + b.x), __ldg(p.meas_i + row + b.y));
-        } else {
-            const float2 m0 = __ldg(p.meas + row + b.x), m1 = __ldg(p.meas + row + b.y);
-            mre = make_float2(m0.x, m1.x);
-            mim = make_float2(m0.y, m1.y);
+        const ptrdiff_t row = (ptrdiff_t)(a0 + j) * p.nbins;
+        float2 re, im;
+        bool v0, v1;
+        pack_pair<MONO, SOA, EXACT>(p, a, row, range_max, ti, vx, vy, vz, re, im, v0, v1);
+        // weight Re(c conj(I)) / |I| (surface_normal_est.cu:138-139)
+        float2 w = __ffma2_rn(re, ire, __fmul2_rn(im, iim));
+        if (EXACT) w = make_float2(w.x / mag.x, w.y / mag.y);
+        else w = __fmul2_rn(w, mag);
+        float2 ex = __fadd2_rn(a.ux, nvx);
+        float2 ey = __fadd2_rn(a.uy, nvy);
+        float2 ez = __fadd2_rn(a.uz, nvz);
+        if (!(v0 && v1)) {  // a skipped pair adds nothing, whatever its vector is
+            w = make_float2(v0 ? w.x : 0.f, v1 ? w.y : 0.f);
+            ex = make_float2(v0 ? ex.x : 0.f, v1 ? ex.y : 0.f);
+            ey = make_float2(v0 ? ey.x : 0.f, v1 ? ey.y : 0.f);
+            ez = make_float2(v0 ? ez.x : 0.f, v1 ? ez.y : 0.f);
         }
-        float2 c, s;
-        phasor2(path, p.inv_lambda_hi, p.inv_lambda_lo, c, s);
-        const float2 re = __ffma2_rn(mre, c, __fmul2_rn(mim, make_float2(-s.x, -s.y)));
-        const float2 im = __ffma2_rn(mre, s, __fmul2_rn(mim, c));
-        // weight Re(c conj(I)) / |I| (surface_normal_est.cu:138-139); zero for a skipped pair
-        float2 w = __fmul2_rn(__ffma2_rn(re, ire, __fmul2_rn(im, iim)), inv_mag);
-        w = make_float2(v0 ? w.x : 0.f, v1 ? w.y : 0.f);
-        acc[0] = __ffma2_rn(__fadd2_rn(a.ux, nvx), w, acc[0]);
-        acc[1] = __ffma2_rn(__fadd2_rn(a.uy, nvy), w, acc[1]);
-        acc[2] = __ffma2_rn(__fadd2_rn(a.uz, nvz), w, acc[2]);
+        acc[0] = __ffma2_rn(ex, w, acc[0]);
+        acc[1] = __ffma2_rn(ey, w, acc[1]);
+        acc[2] = __ffma2_rn(ez, w, acc[2]);
     }
 }
 }  // namespace
 
-// Normal pass in packed fast form over a valid-voxel list: entries ind and ind + blockDim
-// of each 2*blockDim tile per thread.
+// Normal pass (cuda_sn_est, surface_normal_est.cu:63-149) over a valid-voxel list: entries ind
+// and ind + blockDim of each 2*blockDim tile per thread.
+template <bool EXACT>
 __global__ void __launch_bounds__(kInterpThreads) interp_normals_pack_kernel(const InterpParams p) {
     __shared__ PackAnt sh[kInterpChunk];
     const float range_max = p.fft_spacing * p.nbins;
@@ -752,14 +681,15 @@ __global__ void __launch_bounds__(kInterpThreads) interp_normals_pack_kernel(con
         const int64_t v = ((int64_t)x * p.ny + y) * p.nz + z;
         pr[k] = active[k] ? p.img_r[v] : 1.f;
         pi[k] = active[k] ? p.img_i[v] : 0.f;
-        pm[k] = 1.f / sqrtf(pr[k] * pr[k] + pi[k] * pi[k]);
+        pm[k] = sqrtf(fmaf(pr[k], pr[k], pi[k] * pi[k]));
+        if (!EXACT) pm[k] = 1.f / pm[k];
     }
     const float2 vx = make_float2(px[0], px[1]), vy = make_float2(py[0], py[1]),
                  vz = make_float2(pz[0], pz[1]);
     const float2 nvx = make_float2(-px[0], -px[1]), nvy = make_float2(-py[0], -py[1]),
                  nvz = make_float2(-pz[0], -pz[1]);
     const float2 ire = make_float2(pr[0], pr[1]), iim = make_float2(pi[0], pi[1]),
-                 inv_mag = make_float2(pm[0], pm[1]);
+                 mag = make_float2(pm[0], pm[1]);
     float2 acc[3] = {dup(0.f), dup(0.f), dup(0.f)};
     const bool soa = p.meas == nullptr;
     for (int a0 = 0; a0 < p.num_ant; a0 += kInterpChunk) {
@@ -770,15 +700,15 @@ __global__ void __launch_bounds__(kInterpThreads) interp_normals_pack_kernel(con
         const bool offsets = pack_chunk_has_offsets(sh, n);
         if (!active[0] && !active[1]) continue;
         if (offsets) {
-            if (soa) pack_normals_chunk<false, true>(p, sh, a0, n, range_max, ti, vx, vy, vz,
-                                                     nvx, nvy, nvz, ire, iim, inv_mag, acc);
-            else pack_normals_chunk<false, false>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
-                                                  nvy, nvz, ire, iim, inv_mag, acc);
+            if (soa) pack_normals_chunk<false, true, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz,
+                                                     nvx, nvy, nvz, ire, iim, mag, acc);
+            else pack_normals_chunk<false, false, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
+                                                  nvy, nvz, ire, iim, mag, acc);
         } else {
-            if (soa) pack_normals_chunk<true, true>(p, sh, a0, n, range_max, ti, vx, vy, vz,
-                                                    nvx, nvy, nvz, ire, iim, inv_mag, acc);
-            else pack_normals_chunk<true, false>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
-                                                 nvy, nvz, ire, iim, inv_mag, acc);
+            if (soa) pack_normals_chunk<true, true, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz,
+                                                    nvx, nvy, nvz, ire, iim, mag, acc);
+            else pack_normals_chunk<true, false, EXACT>(p, sh, a0, n, range_max, ti, vx, vy, vz, nvx,
+                                                 nvy, nvz, ire, iim, mag, acc);
         }
     }
 #pragma unroll
@@ -790,28 +720,32 @@ __global__ void __launch_bounds__(kInterpThreads) interp_normals_pack_kernel(con
     }
 }
 
+namespace {
+unsigned pack_blocks(int64_t count) {
+    const int64_t per = (int64_t)kInterpThreads * 2;
+    return (unsigned)((count + per - 1) / per);
+}
+}  // namespace
+
 cudaError_t launch_interp_image(const InterpParams &p, cudaStream_t stream) {
     if (p.count <= 0) return cudaSuccess;
-    const int64_t blocks = (p.count + kInterpThreads - 1) / kInterpThreads;
-    interp_image_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
+    interp_image_pack_kernel<true><<<pack_blocks(p.count), kInterpThreads, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
 cudaError_t launch_interp_normals(const InterpParams &p, cudaStream_t stream) {
     if (p.count <= 0) return cudaSuccess;
-    const int64_t blocks = (p.count + kInterpThreads - 1) / kInterpThreads;
-    interp_normals_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
+    interp_normals_pack_kernel<true><<<pack_blocks(p.count), kInterpThreads, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
 cudaError_t launch_interp_image_fast(const InterpParams &p, cudaStream_t stream) {
     if (p.count <= 0) return cudaSuccess;
-    const int64_t per = (int64_t)kInterpThreads * 2;  // kFastT == 2 in every form
-    const int64_t blocks = (p.count + per - 1) / per;
+    const unsigned blocks = pack_blocks(p.count);  // kFastT == 2 in every form
     if (g_interp_fast_form.load() == 1)
-        interp_image_fast_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
+        interp_image_fast_kernel<<<blocks, kInterpThreads, 0, stream>>>(p);
     else
-        interp_image_pack_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
+        interp_image_pack_kernel<false><<<blocks, kInterpThreads, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
@@ -821,9 +755,8 @@ cudaError_t launch_interp_normals_fast(const InterpParams &p, cudaStream_t strea
         const int64_t blocks = (p.count + kInterpThreads - 1) / kInterpThreads;
         interp_normals_fast_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
     } else {
-        const int64_t per = (int64_t)kInterpThreads * 2;
-        const int64_t blocks = (p.count + per - 1) / per;
-        interp_normals_pack_kernel<<<(unsigned)blocks, kInterpThreads, 0, stream>>>(p);
+        interp_normals_pack_kernel<false>
+            <<<pack_blocks(p.count), kInterpThreads, 0, stream>>>(p);
     }
     return cudaGetLastError();
 }

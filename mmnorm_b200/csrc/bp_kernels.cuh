@@ -193,7 +193,8 @@ struct InterpParams {
     float *n_x, *n_y, *n_z;
     int32_t num_valid;
     int32_t pad1;
-    // fast form only: 1/lambda split into two floats (hi + lo) and 1/(2 fft_spacing)
+    double neg_inv_lambda;   // -1/lambda (exact form)
+    // 1/lambda split into two floats (hi + lo; fast form) and 1/(2 fft_spacing)
     float inv_lambda_hi, inv_lambda_lo, half_inv_fsp;
     int32_t mono;            // 1 when every RX offset is zero (fast form)
 };

@@ -228,14 +228,18 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 bool is_interp(int mode) { return mode == MMN_MODE_INTERP || mode == MMN_MODE_INTERP_FAST; }
 
-// Constants of the interpolated mode's fast form: 1/lambda as the sum of two floats (the
-// reference forms its phase from the FP32 wavelength promoted to FP64) and 1/(2 fft_spacing)
-// from the correctly rounded FP32 reciprocal.
-void set_fast_fields(InterpParams &ip) {
+// Constants of the interpolated mode's kernels: 1/lambda as the sum of two floats (fast form;
+// the reference forms its phase from the FP32 wavelength promoted to FP64) and in FP64 (exact
+// form), and 1/(2 fft_spacing) from the correctly rounded FP32 reciprocal.  A NaN sends the
+// exact form's every evaluation to the reference's own expression: more turns than its
+// reduction takes, more bins than the rounding constant holds (the fast form refuses those).
+void set_interp_fields(InterpParams &ip) {
     const double inv = 1.0 / (double)ip.wavelength;
     ip.inv_lambda_hi = (float)inv;
     ip.inv_lambda_lo = (float)(inv - (double)ip.inv_lambda_hi);
-    ip.half_inv_fsp = 0.5f * (1.0f / ip.fft_spacing);
+    ip.half_inv_fsp = ip.nbins > kMaxFastBins ? std::nanf("") : 0.5f * (1.0f / ip.fft_spacing);
+    const double turns = (double)ip.fft_spacing * ip.nbins * inv;
+    ip.neg_inv_lambda = turns < 1099511627776.0 ? -inv : std::nan("");  // 2^40
 }
 
 }  // namespace
@@ -404,8 +408,8 @@ int mmn_backproject(const mmn_problem *p, int32_t mode, float *image, float *vot
         ip.image = reinterpret_cast<float2 *>(image);
         ip.vote = reinterpret_cast<float2 *>(vote);
         if (p->pos_offsets) return MMN_ERR_UNSUPPORTED;
+        set_interp_fields(ip);
         if (mode == MMN_MODE_INTERP_FAST) {
-            set_fast_fields(ip);
             return launch_interp_image_fast(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
         }
         return launch_interp_image(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
@@ -561,9 +565,9 @@ int mmn_cuda_image(float *p_xyz_r, float *p_xyz_i, const float *x_locs, const fl
         ip.nvox = nvox;
         ip.out_r = p_xyz_r;
         ip.out_i = p_xyz_i;
+        set_interp_fields(ip);
         if (use_interpolated_processing == 2) {
             if (samples_per_meas > kMaxFastBins) return MMN_ERR_TOO_LARGE;
-            set_fast_fields(ip);
             return launch_interp_image_fast(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
         }
         return launch_interp_image(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
@@ -658,9 +662,9 @@ int cuda_sn_est_impl(bool fast, float *normals_x, float *normals_y, float *norma
     ip.n_y = normals_y;
     ip.n_z = normals_z;
     ip.num_valid = num_valid_idx;
+    set_interp_fields(ip);
     if (fast) {
         if (samples_per_meas > kMaxFastBins) return MMN_ERR_TOO_LARGE;
-        set_fast_fields(ip);
         return launch_interp_normals_fast(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
     }
     return launch_interp_normals(ip, stream) == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
