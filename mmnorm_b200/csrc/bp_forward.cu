@@ -29,6 +29,14 @@
 //    antenna pairs in the halves of FFMA2 (the sample duplicated into (re, re, im, im)
 //    or antenna-pair records), or scalar FFMA.
 //
+// Bound of the second-order forms: instruction dispatch, where a packed instruction takes about
+// two slots: per pair of the default variant 8 a step of its two chains, 1/2 a shared load, some
+// 110 for range, rotation and vote and 32 a block (128^3 voxels x 4096 antennas x 256 samples:
+// 1300 of the 1316 slots that pass).  Integer turn counts by one FP64 FMA each and the range's
+// shared Newton factor took 48^3 x 1024 x 64 from 1418 to 1340 us; running a row's last partial
+// block on the same chains instead of a scalar first-order loop took a 75 x 61 x 53 grid x 1236
+// antennas x 100 samples from 6.85 to 5.56 ms.
+//
 // PLAIN form.  FP32 distance and FP32 phase -d*kappa_j with one sincosf per sample,
 // then a complex multiply-add -- the straightforward FP32 kernel.
 //
@@ -157,40 +165,59 @@ __device__ __forceinline__ void clen_block(const float4 *mb, bool clen, const fl
     }
 }
 
-// A 64-sample block of the split second-order form (kFormMixedClenEO): the even and the
+// A block of 2 n samples of the split second-order form (kFormMixedClenEO): the even and the
 // odd samples as two chains in w = z^2, E = sum_k m_{2k} w^k and O = sum_k m_{2k+1} w^k,
 // each by Clenshaw's recurrence with the real multiplier c2w = 2 cos(2 phi), and
 // h = E + z O.  One 16-byte load (samples 2k, 2k+1) feeds one step of both chains; the
 // chains are half as long and their modes e^{+-2 i phi} twice as far from 0, which keeps
 // the growth of b and the effect of the FP32 multiplier's rounding several times smaller
-// than one chain over the whole block.
-template <int T>
-__device__ __forceinline__ void clen_block_eo(const float4 *mb, const float (&zr)[T],
+// than one chain over the whole block.  N: 32 (a whole block), or 0 for a row's last n >= 1
+// sample pairs (the sample above an odd count is one of the row's padded zeros).
+template <int T, int N>
+__device__ __forceinline__ void clen_block_eo(const float4 *mb, int n, const float (&zr)[T],
                                               const float (&zi)[T], const float (&wr)[T],
                                               const float (&wi)[T], float (&sr)[T],
                                               float (&si)[T]) {
-    const float4 top = mb[31];  // samples 62 (even k = 31), 63 (odd k = 31)
+    const float4 top = mb[(N > 0 ? N : n) - 1];
     float2 be1[T], be2[T], bo1[T], bo2[T], c2[T];
 #pragma unroll
     for (int k = 0; k < T; ++k) {
         c2[k] = make_float2(2.f * wr[k], 2.f * wr[k]);
-        be1[k] = make_float2(top.x, top.y);  // b_31 of each chain
+        be1[k] = make_float2(top.x, top.y);  // b_{n-1} of each chain
         bo1[k] = make_float2(top.z, top.w);
         be2[k] = bo2[k] = make_float2(0.f, 0.f);
     }
+    if constexpr (N > 0) {
 #pragma unroll
-    for (int q = 30; q >= 0; --q) {
-        const float4 mm = mb[q];
+        for (int q = N - 2; q >= 0; --q) {
+            const float4 mm = mb[q];
 #pragma unroll
-        for (int k = 0; k < T; ++k) {
-            const float2 de = __fadd2_rn(make_float2(mm.x, mm.y),
-                                         make_float2(-be2[k].x, -be2[k].y));
-            const float2 dd = __fadd2_rn(make_float2(mm.z, mm.w),
-                                         make_float2(-bo2[k].x, -bo2[k].y));
-            be2[k] = be1[k];
-            bo2[k] = bo1[k];
-            be1[k] = __ffma2_rn(c2[k], be1[k], de);
-            bo1[k] = __ffma2_rn(c2[k], bo1[k], dd);
+            for (int k = 0; k < T; ++k) {
+                const float2 de = __fadd2_rn(make_float2(mm.x, mm.y),
+                                             make_float2(-be2[k].x, -be2[k].y));
+                const float2 dd = __fadd2_rn(make_float2(mm.z, mm.w),
+                                             make_float2(-bo2[k].x, -bo2[k].y));
+                be2[k] = be1[k];
+                bo2[k] = bo1[k];
+                be1[k] = __ffma2_rn(c2[k], be1[k], de);
+                bo1[k] = __ffma2_rn(c2[k], bo1[k], dd);
+            }
+        }
+    } else {
+#pragma unroll 4
+        for (int q = n - 2; q >= 0; --q) {
+            const float4 mm = mb[q];
+#pragma unroll
+            for (int k = 0; k < T; ++k) {
+                const float2 de = __fadd2_rn(make_float2(mm.x, mm.y),
+                                             make_float2(-be2[k].x, -be2[k].y));
+                const float2 dd = __fadd2_rn(make_float2(mm.z, mm.w),
+                                             make_float2(-bo2[k].x, -bo2[k].y));
+                be2[k] = be1[k];
+                bo2[k] = bo1[k];
+                be1[k] = __ffma2_rn(c2[k], be1[k], de);
+                bo1[k] = __ffma2_rn(c2[k], bo1[k], dd);
+            }
         }
     }
 #pragma unroll
@@ -642,26 +669,27 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                 }
             } else if constexpr (FORM == kFormMixedClenEO) {
                 // 64-sample blocks, each as even and odd chains in w = z^2 (clen_block_eo),
-                // used for a warp's antenna when every lane has |cos 2 phi| <= kClenMaxCos;
-                // otherwise, and for a row's last partial block, first-order Horner.
+                // used for a warp's antenna when every lane has |cos 2 phi| <= kClenMaxCos,
+                // otherwise first-order Horner; a row's last partial block by the same chains
+                // at its own length.  Start phase, block step and rotation are 2^-32-turn
+                // integers of one FP64 FMA each: the step's rounding (2^-33 turns) is 7e-10
+                // rad a block.
                 static_assert(T % 2 == 0, "the second-order form takes voxels in pairs");
                 const int ns = p.nsmp > 0 ? min(p.nsmp, fp) : fp;
                 const int nblk_c = ns / 64;
                 const float4 *m4 = reinterpret_cast<const float4 *>(mstage) + (size_t)a * (fp / 2);
-                unsigned long long ph[T], stp[T];
+                int32_t ph[T], stp[T];
                 float zr[T], zi[T], wr[T], wi[T];
                 bool eo = true;
                 {
-                    int32_t za[T], wa[T];
+                    int32_t za[T];
 #pragma unroll
                     for (int k = 0; k < T; ++k) {
                         const double d = range_fp64_newton((double)vx[k], (double)vy[k],
                                                            (double)vz[k], ar, mono, p.ti);
-                        const unsigned long long u = turns_fixed64(-d * p.tsmp);
-                        za[k] = (int32_t)(u >> 32);
-                        wa[k] = (int32_t)((u << 1) >> 32);  // 2 phi, exact in fixed point
-                        stp[k] = u << 6;
-                        ph[k] = turns_fixed_top(-d * p.t0);
+                        za[k] = turns_fixed32(d, p.fx_smp);
+                        stp[k] = turns_fixed32(d, p.fx_blk);
+                        ph[k] = turns_fixed32(d, p.fx_t0);
                         cr[k] = ci[k] = 0.f;
                     }
 #pragma unroll
@@ -672,7 +700,8 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                         zr[2 * q + 1] = c.y;
                         zi[2 * q] = s.x;
                         zi[2 * q + 1] = s.y;
-                        cis_turns_pair(wa[2 * q], wa[2 * q + 1], c, s, nsn);
+                        cis_turns_pair((int32_t)((uint32_t)za[2 * q] << 1),
+                                       (int32_t)((uint32_t)za[2 * q + 1] << 1), c, s, nsn);
                         wr[2 * q] = c.x;
                         wr[2 * q + 1] = c.y;
                         wi[2 * q] = s.x;
@@ -687,8 +716,8 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
 #pragma unroll
                     for (int k = 0; k < T; ++k) {
                         float anr, ani;
-                        fixed_cis(ph[k], anr, ani);
-                        ph[k] += stp[k];
+                        __sincosf((float)ph[k] * 1.46291807926715968e-9f, &ani, &anr);  // 2 pi / 2^32
+                        ph[k] = (int32_t)((uint32_t)ph[k] + (uint32_t)stp[k]);
                         cr[k] = fmaf(anr, sr[k], fmaf(-ani, si[k], cr[k]));
                         ci[k] = fmaf(anr, si[k], fmaf(ani, sr[k], ci[k]));
                     }
@@ -696,7 +725,7 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                 for (int b = 0; b < nblk_c; ++b) {
                     float sr[T], si[T];
                     if (eo)
-                        clen_block_eo<T>(m4 + b * 32, zr, zi, wr, wi, sr, si);
+                        clen_block_eo<T, 32>(m4 + b * 32, 32, zr, zi, wr, wi, sr, si);
                     else
                         clen_block<T, 64>(m4 + b * 32, false, none, zr, zi, sr, si);
                     anchor(sr, si);
@@ -704,8 +733,12 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                 const int rem = ns - nblk_c * 64;
                 if (rem > 0) {
                     float sr[T], si[T];
-                    clen_partial<T>(reinterpret_cast<const float2 *>(m4 + nblk_c * 32), rem,
-                                    false, none, zr, zi, sr, si);
+                    if (eo)
+                        clen_block_eo<T, 0>(m4 + nblk_c * 32, (rem + 1) >> 1, zr, zi, wr, wi, sr,
+                                            si);
+                    else
+                        clen_partial<T>(reinterpret_cast<const float2 *>(m4 + nblk_c * 32), rem,
+                                        false, none, zr, zi, sr, si);
                     anchor(sr, si);
                 }
             } else if constexpr (FORM == kFormMixedScalar) {
@@ -829,8 +862,8 @@ __device__ __forceinline__ void init_stage_barriers(unsigned char *smem) {
 }
 
 // One launch, grid = tiles x splits (one work item per CTA).
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly>
-__global__ void __launch_bounds__(NT) bp_fwd_kernel(const FwdParams p) {
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+__global__ void __launch_bounds__(NT, MINB) bp_fwd_kernel(const FwdParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t gchunk = 0;
     const int failed = fwd_item<T, NT, FORM, ANCHOR, false>(p, blockIdx.x % p.num_tiles,
@@ -844,8 +877,8 @@ __global__ void __launch_bounds__(NT) bp_fwd_kernel(const FwdParams p) {
 // Persistent launch over a work list of (object, voxel tile, antenna split) items: every
 // CTA pops the next item from a global counter until the list is exhausted.  Items are
 // sorted by cost, largest first, so the tail is made of the smallest items.
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly>
-__global__ void __launch_bounds__(NT) bp_fwd_persistent(const BatchParams bp) {
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+__global__ void __launch_bounds__(NT, MINB) bp_fwd_persistent(const BatchParams bp) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_item;
     init_stage_barriers(smem);
@@ -966,13 +999,13 @@ __global__ void stage_meas(const float *__restrict__ src, const float *__restric
 }
 
 // ------------------------------------------------------------------ instantiations
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
 static const void *fwd_ptr() {
-    return reinterpret_cast<const void *>(&bp_fwd_kernel<T, NT, FORM, ANCHOR>);
+    return reinterpret_cast<const void *>(&bp_fwd_kernel<T, NT, FORM, ANCHOR, MINB>);
 }
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
 static const void *pers_ptr() {
-    return reinterpret_cast<const void *>(&bp_fwd_persistent<T, NT, FORM, ANCHOR>);
+    return reinterpret_cast<const void *>(&bp_fwd_persistent<T, NT, FORM, ANCHOR, MINB>);
 }
 
 const FwdVariant *fwd_variants(int *count) {
@@ -980,7 +1013,7 @@ const FwdVariant *fwd_variants(int *count) {
     static const FwdVariant v[] = {
         // default: 64-sample blocks as two second-order chains in z^2 (near the Horner
         // form's accuracy at close to the fastest form's speed)
-        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2>()},
+        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>()},
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), "mixed_clen_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
         {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed>(), "mixed_ffma2_fx_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed>()},
         // each block as two 16-step chains joined by z^16 (kFormMixedPairSplit)

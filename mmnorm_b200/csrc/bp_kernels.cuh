@@ -26,6 +26,7 @@ struct FwdParams {
     double t0, tblk;       // 1/lambda and 32*slope/c: turns per metre of range
     double tsmp;           // slope/c: turns per metre of range per sample
     double ti;             // 0.15 or 0
+    double fx_t0, fx_smp, fx_blk;  // -2^32 times t0, tsmp and 64 tsmp (turns_fixed32)
     int32_t num_tiles;
     int32_t num_splits;
     int32_t ant_per_split;

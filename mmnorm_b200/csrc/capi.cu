@@ -158,6 +158,12 @@ int plan_forward(int64_t nvox, int64_t vox_start, int64_t vox_count, int A, int 
     return MMN_OK;
 }
 
+void set_fixed_fields(FwdParams &f) {
+    f.fx_t0 = -4294967296.0 * f.t0;
+    f.fx_smp = -4294967296.0 * f.tsmp;
+    f.fx_blk = 64.0 * f.fx_smp;
+}
+
 int run_forward(const FwdPlan &pl, const mmn_problem *p, const float *meas_r,
                 const float *meas_i, float2 *image, float2 *vote, float *out_r, float *out_i,
                 unsigned char *ws, cudaStream_t stream) {
@@ -202,6 +208,7 @@ int run_forward(const FwdPlan &pl, const mmn_problem *p, const float *meas_r,
     fp.t0 = 1.0 / p->wavelength;
     fp.tblk = (double)kBlockF * p->slope / kC;
     fp.tsmp = p->slope / kC;
+    set_fixed_fields(fp);
     fp.ti = p->is_ti_radar ? 0.15 : 0.0;
     fp.num_tiles = pl.tiles;
     fp.num_splits = pl.splits;
@@ -1549,6 +1556,7 @@ extern "C" int mmn_batch_upload(mmn_batch *b, void *workspace, size_t workspace_
         f.t0 = 1.0 / p.wavelength;
         f.tblk = (double)kBlockF * p.slope / kC;
         f.tsmp = p.slope / kC;
+        set_fixed_fields(f);
         f.ti = p.is_ti_radar ? 0.15 : 0.0;
         f.num_tiles = ob.tiles;
         f.num_splits = std::max(1, ob.splits);

@@ -133,28 +133,35 @@ __device__ __forceinline__ double range_fp64(double vx, double vy, double vz,
 // Cheaper forms of the per-(voxel, antenna) prologue (the "fx2" anchor family).
 // ---------------------------------------------------------------------------------
 
-// sqrt(r2) in FP64 from an FP32 reciprocal-square-root seed and one Newton step
-// s' = s + (r2 - s^2) / (2 s), s = r2 * y: the seed's ~2^-22 relative error squares to
-// ~1e-13 (a femtometre at a metre of range).  r2 below 1e-30 (a voxel on the antenna)
-// gives a value below 2e-15 instead of 0.
-__device__ __forceinline__ double sqrt_newton(double r2) {
-    const double y = (double)rsqrtf(fmaxf((float)r2, 1e-30f));
-    const double s = r2 * y;
-    return fma(fma(-s, s, r2), 0.5 * y, s);
+// FP32 reciprocal square root of an FP64 square: the seed of the ranges below.  Squares below
+// 1e-30 (a voxel on the antenna) are raised to it, so no subnormal reaches the MUFU.
+__device__ __forceinline__ double rsqrt_seed64(double r2) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf((float)r2, 1e-30f)));
+    return (double)y;
 }
 
+// FP64 round-trip distance TX -> v -> RX (+ ti).  Each leg is s = r2 y with the FP32 seed y and
+// one Newton correction (r2 - s^2) y / 2: the seed's ~2^-22 relative error squares to ~1e-13 (a
+// femtometre at a metre of range).
 __device__ __forceinline__ double range_fp64_newton(double vx, double vy, double vz,
                                                     const AntRec &a, bool mono, double ti) {
     const double dx = vx - a.tx[0], dy = vy - a.tx[1], dz = vz - a.tx[2];
-    const double f = sqrt_newton(fma(dx, dx, fma(dy, dy, dz * dz)));
-    double d;
-    if (mono) {
-        d = f + f;
-    } else {
-        const double bx = vx - a.rx[0], by = vy - a.rx[1], bz = vz - a.rx[2];
-        d = f + sqrt_newton(fma(bx, bx, fma(by, by, bz * bz)));
-    }
-    return d + ti;
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double y = rsqrt_seed64(r2);
+    const double s = r2 * y, e = fma(-s, s, r2);
+    if (mono) return fma(e, y, fma(2.0, s, ti));  // twice the leg
+    const double bx = vx - a.rx[0], by = vy - a.rx[1], bz = vz - a.rx[2];
+    const double q2 = fma(bx, bx, fma(by, by, bz * bz));
+    const double w = rsqrt_seed64(q2);
+    const double t = q2 * w, g = fma(-t, t, q2);
+    return fma(0.5, fma(g, w, e * y), s + (t + ti));
+}
+
+// The wrapped turn count of d * k as a 2^-32-turn integer, from the 1.5*2^52 rounding constant:
+// k holds turns per metre times 2^32.  Valid for |d k| < 2^51 (2^19 turns).
+__device__ __forceinline__ int32_t turns_fixed32(double d, double k) {
+    return __double2loint(fma(d, k, 6755399441055744.0));
 }
 
 // w turns as 32.32 fixed point (the top word = the wrapped turn count in 2^-32 steps),
