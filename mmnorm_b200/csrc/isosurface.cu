@@ -344,20 +344,35 @@ __global__ void __launch_bounds__(kIsoThreads) iso_channel_kernel(const IsoParam
     if (threadIdx.x == 0) p.block_hits[bslot] = total;
 }
 
-// channel[item][k] = sum over the item's blocks (in block order) of their partials
-__global__ void iso_reduce_kernel(const IsoParams p, float2 *__restrict__ channel) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)p.num_items * p.num_wl) return;
-    const int item = (int)(idx / p.num_wl), k = (int)(idx % p.num_wl);
+// channel[item][k] = sum over the item's blocks of their partials in FP64: 32 wavelengths per
+// block, kIsoReduceWarps warps taking every kIsoReduceWarps-th ray block that hit anything, their
+// sums added in warp order (one thread per wavelength walked the 1184 ray blocks alone: 95 us for
+// 30 items of 512 wavelengths).
+constexpr int kIsoReduceWarps = 16;
+__global__ void __launch_bounds__(kIsoReduceWarps * 32)
+    iso_reduce_kernel(const IsoParams p, float2 *__restrict__ channel) {
+    __shared__ double2 part[kIsoReduceWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int item = blockIdx.y, k = blockIdx.x * 32 + lane;
     double sr = 0.0, si = 0.0;
-    for (int b = 0; b < p.blocks_per_item; ++b) {
-        const int64_t bslot = (int64_t)item * p.blocks_per_item + b;
-        if (p.block_hits[bslot] == 0) continue;
-        const float2 v = p.partial[bslot * p.num_wl + k];
-        sr += v.x;
-        si += v.y;
+    if (k < p.num_wl) {
+#pragma unroll 4
+        for (int b = warp; b < p.blocks_per_item; b += kIsoReduceWarps) {
+            const int64_t bslot = (int64_t)item * p.blocks_per_item + b;
+            if (p.block_hits[bslot] == 0) continue;
+            const float2 v = p.partial[bslot * p.num_wl + k];
+            sr += v.x;
+            si += v.y;
+        }
     }
-    channel[idx] = make_float2((float)sr, (float)si);
+    part[warp][lane] = make_double2(sr, si);
+    __syncthreads();
+    if (warp != 0 || k >= p.num_wl) return;
+    for (int w = 1; w < kIsoReduceWarps; ++w) {
+        sr += part[w][lane].x;
+        si += part[w][lane].y;
+    }
+    channel[(int64_t)item * p.num_wl + k] = make_float2((float)sr, (float)si);
 }
 
 // rough hits of one antenna's rays (for tests against the reference extension): per pixel
@@ -486,8 +501,8 @@ extern "C" int mmn_iso_channels(const mmn_iso_scene *s, const float *taus, int32
                                            iso_up((size_t)items * blocks * sizeof(int32_t)));
     if (cudaMemsetAsync(w, 0, kIsoStatus, stream) != cudaSuccess) return MMN_ERR_CUDA;
     mmn::iso_channel_kernel<<<dim3(blocks, (unsigned)items), mmn::kIsoThreads, 0, stream>>>(p);
-    const int64_t n = items * s->num_wl;
-    mmn::iso_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
+    mmn::iso_reduce_kernel<<<dim3((unsigned)((s->num_wl + 31) / 32), (unsigned)items),
+                             mmn::kIsoReduceWarps * 32, 0, stream>>>(
         p, reinterpret_cast<float2 *>(channels));
     return cudaGetLastError() == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
 }
