@@ -65,7 +65,7 @@ cudaError_t launch_fwd(const FwdVariant &var, const FwdParams &p, size_t smem,
 cudaError_t launch_reduce(const FwdParams &p, cudaStream_t stream);
 cudaError_t launch_prep_antennas(const float *ant, const float *rxo, int R, const float *pos_off,
                                  int A, int A_pad, AntRec *out, int32_t *mono_flag,
-                                 cudaStream_t stream);
+                                 int32_t *header, cudaStream_t stream);
 cudaError_t launch_stage_meas(const float *src, const float *im, int A, int F, int Fp,
                               int layout, void *dst, cudaStream_t stream);
 

@@ -85,7 +85,7 @@ int check_problem(const mmn_problem *p, int mode) {
 }
 
 int plan_forward(int64_t nvox, int64_t vox_start, int64_t vox_count, int A, int F, int mode,
-                 bool meas_aligned, bool want_partial_space, FwdPlan *pl) {
+                 bool meas_aligned, bool may_split, FwdPlan *pl) {
     int nvar = 0;
     const FwdVariant *vars = fwd_variants(&nvar);
     int vi = variant_index_for(mode);
@@ -123,6 +123,16 @@ int plan_forward(int64_t nvox, int64_t vox_start, int64_t vox_count, int A, int 
         per_sm < 1)
         per_sm = 1;
     const int64_t slots = (int64_t)sms * per_sm;
+    // A problem whose tiles times whole-stage splits leave CTA slots empty takes shorter stages
+    // of one split each: 16^3 voxels x 256 antennas x 64 samples ran 128 CTAs of 16 antennas in
+    // 21 us, 296 CTAs of 7 take 18 (the arithmetic alone is 12).
+    const int64_t fill = std::min<int64_t>(64, slots / pl->tiles);
+    if (may_split && fill > (A + pl->ant_per_stage - 1) / pl->ant_per_stage && A > 0) {
+        int nas = (int)((A + fill - 1) / fill);
+        if (pairs) nas = (nas + 1) & ~1;
+        pl->ant_per_stage = std::min(pl->ant_per_stage, std::max(nas, 4));
+        pl->smem = 128 + 2 * (size_t)pl->ant_per_stage * rec + (pl->var->plain ? pl->fp * 4 : 0);
+    }
     // split count: minimise waves * antennas-per-CTA, with a 2 % charge per extra split
     int best_s = 1;
     double best_cost = 1e300;
@@ -152,7 +162,7 @@ int plan_forward(int64_t nvox, int64_t vox_start, int64_t vox_count, int A, int 
     pl->off_meas = off;
     if (pl->copy_meas) off = align_up(off + (size_t)A * pl->fp * esz);
     pl->off_partial = off;
-    if (pl->splits > 1 || want_partial_space)
+    if (pl->splits > 1)
         off = align_up(off + (size_t)pl->splits * (size_t)vox_count * 8 * sizeof(float));
     pl->total = off;
     return MMN_OK;
@@ -169,12 +179,10 @@ int run_forward(const FwdPlan &pl, const mmn_problem *p, const float *meas_r,
                 unsigned char *ws, cudaStream_t stream) {
     const int A = p->num_antennas;
     const int F = p->num_samples;
-    cudaError_t e = cudaMemsetAsync(ws, 0, 16, stream);
-    if (e != cudaSuccess) return MMN_ERR_CUDA;
     AntRec *ant = reinterpret_cast<AntRec *>(ws + pl.off_ant);
     int32_t *hdr = reinterpret_cast<int32_t *>(ws);
-    e = launch_prep_antennas(p->antenna_locs, p->rx_offsets, p->num_rx, p->pos_offsets, A,
-                             pl.a_pad, ant, hdr + 1, stream);
+    cudaError_t e = launch_prep_antennas(p->antenna_locs, p->rx_offsets, p->num_rx,
+                                         p->pos_offsets, A, pl.a_pad, ant, hdr + 1, hdr, stream);
     if (e != cudaSuccess) return MMN_ERR_CUDA;
     const void *meas = p->meas;
     if (meas_r || pl.copy_meas) {
@@ -334,7 +342,7 @@ size_t mmn_workspace_bytes(const mmn_problem *p, int32_t mode, int32_t want_vote
     const int64_t nvox = (int64_t)p->num_x * p->num_y * p->num_z;
     FwdPlan pl;
     if (plan_forward(nvox, 0, nvox, p->num_antennas, p->num_samples, mode, aligned16(p->meas),
-                     false, &pl) != MMN_OK)
+                     true, &pl) != MMN_OK)
         return 0;
     return pl.total;
 }
@@ -347,7 +355,7 @@ int mmn_plan_info(const mmn_problem *p, int32_t mode, int32_t *tiles, int32_t *s
     const int64_t nvox = (int64_t)p->num_x * p->num_y * p->num_z;
     FwdPlan pl;
     rc = plan_forward(nvox, 0, nvox, p->num_antennas, p->num_samples, mode, aligned16(p->meas),
-                      false, &pl);
+                      true, &pl);
     if (rc != MMN_OK) return rc;
     if (tiles) *tiles = pl.tiles;
     if (splits) *splits = pl.splits;
@@ -365,7 +373,7 @@ int mmn_plan_launches(const mmn_problem *p, int32_t mode, int32_t *launches) {
     const int64_t nvox = (int64_t)p->num_x * p->num_y * p->num_z;
     FwdPlan pl;
     rc = plan_forward(nvox, 0, nvox, p->num_antennas, p->num_samples, mode, aligned16(p->meas),
-                      false, &pl);
+                      true, &pl);
     if (rc != MMN_OK) return rc;
     // antenna records, the staging copy (a layout other than the caller's rows, padding,
     // or misaligned rows), the forward kernel, the split reduction
@@ -423,7 +431,7 @@ int mmn_backproject(const mmn_problem *p, int32_t mode, float *image, float *vot
     }
     FwdPlan pl;
     rc = plan_forward(nvox, 0, nvox, p->num_antennas, p->num_samples, mode, aligned16(p->meas),
-                      false, &pl);
+                      true, &pl);
     if (rc != MMN_OK) return rc;
     if (workspace_bytes < pl.total) return MMN_ERR_WORKSPACE;
     return run_forward(pl, p, nullptr, nullptr, reinterpret_cast<float2 *>(image),
@@ -451,6 +459,7 @@ int mmn_normals(int64_t num_voxels, const float *image, const float *vote, float
         return MMN_ERR_INVALID_ARGUMENT;
     unsigned int *max_bits = reinterpret_cast<unsigned int *>(
         static_cast<unsigned char *>(workspace) + 8);
+    // (a small image in one launch, without the workspace)
     cudaError_t e = launch_normals(num_voxels, reinterpret_cast<const float2 *>(image),
                                    reinterpret_cast<const float2 *>(vote), filter_percent,
                                    normals, mask, raw, max_bits, stream);
@@ -510,7 +519,7 @@ size_t mmn_cuda_image_workspace_bytes_for(int num_x, int num_y, int num_z, int n
     if (count < 1) return kStatusBytes;
     FwdPlan pl;
     if (plan_forward(nvox, start_ind, count, num_antennas, samples_per_meas, MMN_MODE_MIXED,
-                     false, false, &pl) != MMN_OK)
+                     false, true, &pl) != MMN_OK)
         return 0;
     return pl.total;  // SoA input: plan_forward with meas_aligned=false always stages
 }
@@ -597,7 +606,7 @@ int mmn_cuda_image(float *p_xyz_r, float *p_xyz_i, const float *x_locs, const fl
     p.is_ti_radar = is_ti_radar;
     FwdPlan pl;
     int rc = plan_forward(nvox, start_ind, count, num_antennas, samples_per_meas, MMN_MODE_MIXED,
-                          false, false, &pl);
+                          false, true, &pl);
     if (rc != MMN_OK) return rc;
     if (workspace_bytes < pl.total) return MMN_ERR_WORKSPACE;
     return run_forward(pl, &p, meas_r, meas_i, nullptr, nullptr, p_xyz_r, p_xyz_i, ws, stream);
@@ -1017,11 +1026,10 @@ extern "C" int mmn_backproject_nufft(const mmn_problem *p, float *image, float *
     if (rc != MMN_OK) return rc;
     if (workspace_bytes < pl.total) return MMN_ERR_WORKSPACE;
     unsigned char *ws = static_cast<unsigned char *>(workspace);
-    if (cudaMemsetAsync(ws, 0, 16, stream) != cudaSuccess) return MMN_ERR_CUDA;
     int32_t *hdr = reinterpret_cast<int32_t *>(ws);
     AntRec *ant = reinterpret_cast<AntRec *>(ws + pl.off_ant);
     if (launch_prep_antennas(p->antenna_locs, p->rx_offsets, p->num_rx, p->pos_offsets, A, A, ant,
-                             hdr + 1, stream) != cudaSuccess)
+                             hdr + 1, hdr, stream) != cudaSuccess)
         return MMN_ERR_CUDA;
     const int J0 = F / 2;
     double2 *tw = reinterpret_cast<double2 *>(ws + pl.off_tab);
@@ -1124,11 +1132,10 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     if (rc != MMN_OK) return rc;
     if (workspace_bytes < pl.total) return MMN_ERR_WORKSPACE;
     unsigned char *ws = static_cast<unsigned char *>(workspace);
-    if (cudaMemsetAsync(ws, 0, 16, stream) != cudaSuccess) return MMN_ERR_CUDA;
     AntRec *ant = reinterpret_cast<AntRec *>(ws + pl.off_ant);
     int32_t *hdr = reinterpret_cast<int32_t *>(ws);
     if (launch_prep_antennas(p->antenna_locs, p->rx_offsets, p->num_rx, p->pos_offsets, A, A, ant,
-                             hdr + 1, stream) != cudaSuccess)
+                             hdr + 1, hdr, stream) != cudaSuccess)
         return MMN_ERR_CUDA;
     BwdParams bp;
     std::memset(&bp, 0, sizeof(bp));
@@ -1598,7 +1605,7 @@ extern "C" int mmn_batch_run(mmn_batch *b, void *workspace, cudaStream_t stream)
         if (launch_prep_antennas(p.antenna_locs, p.rx_offsets, p.num_rx, p.pos_offsets,
                                  p.num_antennas, ob.a_pad,
                                  reinterpret_cast<AntRec *>(ws + ob.off_ant),
-                                 reinterpret_cast<int32_t *>(ws + b->off_flags) + o,
+                                 reinterpret_cast<int32_t *>(ws + b->off_flags) + o, nullptr,
                                  stream) != cudaSuccess)
             return MMN_ERR_CUDA;
         if (launch_stage_meas(p.meas, nullptr, p.num_antennas, p.num_samples, ob.fp,

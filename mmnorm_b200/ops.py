@@ -23,7 +23,8 @@ def _vp(t):
 
 
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(index))
 
 
 def _plain(t):
@@ -123,9 +124,8 @@ def backproject(x_locs, y_locs, z_locs, antenna_locs, rx_offsets, meas, waveleng
                      slope, fft_spacing, is_ti_radar, pos_offsets)
     dev = meas.device
     nx, ny, nz = p.num_x, p.num_y, p.num_z
-    V = nx * ny * nz
-    image = torch.empty(V, dtype=torch.complex64, device=dev)
-    vote = torch.empty((3, V), dtype=torch.complex64, device=dev) if want_vote else None
+    image = torch.empty((nx, ny, nz), dtype=torch.complex64, device=dev)
+    vote = torch.empty((3, nx, ny, nz), dtype=torch.complex64, device=dev) if want_vote else None
     lib = _lib.load()
     if mode == "nufft":
         nbytes = lib.mmn_backproject_nufft_workspace_bytes(ctypes.byref(p))
@@ -136,14 +136,14 @@ def backproject(x_locs, y_locs, z_locs, antenna_locs, rx_offsets, meas, waveleng
         rc = lib.mmn_backproject_nufft(ctypes.byref(p), _vp(image), _vp(vote), _vp(workspace),
                                        workspace.numel(), _stream(dev))
         _lib.check(rc, "mmn_backproject_nufft")
-        return image.view(nx, ny, nz), (vote.view(3, nx, ny, nz) if vote is not None else None)
+        return image, vote
     nbytes = workspace_bytes(p, mode)
     if workspace is None or workspace.numel() < nbytes:
         workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     rc = lib.mmn_backproject(ctypes.byref(p), _lib.MODES[mode], _vp(image), _vp(vote),
                              _vp(workspace), workspace.numel(), _stream(dev))
     _lib.check(rc, "mmn_backproject")
-    return image.view(nx, ny, nz), (vote.view(3, nx, ny, nz) if vote is not None else None)
+    return image, vote
 
 
 def surface_normals(image, vote, filter_percent=0.05, want_raw=False):
@@ -157,7 +157,7 @@ def surface_normals(image, vote, filter_percent=0.05, want_raw=False):
     _need(img, "image", torch.complex64, dev)
     _need(w, "vote", torch.complex64, dev)
     normals = torch.empty((V, 3), dtype=torch.float32, device=dev)
-    mask = torch.empty(V, dtype=torch.uint8, device=dev)
+    mask = torch.empty(V, dtype=torch.bool, device=dev)   # the kernel writes bytes 0 / 1
     raw = torch.empty((V, 3), dtype=torch.float32, device=dev) if want_raw else None
     lib = _lib.load()
     nbytes = lib.mmn_normals_workspace_bytes(V)
@@ -165,7 +165,7 @@ def surface_normals(image, vote, filter_percent=0.05, want_raw=False):
     rc = lib.mmn_normals(V, _vp(img), _vp(w), float(filter_percent), _vp(normals), _vp(mask),
                          _vp(raw), _vp(ws), nbytes, _stream(dev))
     _lib.check(rc, "mmn_normals")
-    out = (normals.view(*shape, 3), mask.view(shape).bool())
+    out = (normals.view(*shape, 3), mask.view(shape))
     if want_raw:
         out = out + (raw.view(*shape, 3),)
     return out
@@ -195,13 +195,13 @@ def surface_normals_from_max(image, vote, max_abs, filter_percent=0.05, want_raw
     _need(w, "vote", torch.complex64, dev)
     _need(max_abs, "max_abs", torch.float32, dev, (1,))
     normals = torch.empty((V, 3), dtype=torch.float32, device=dev)
-    mask = torch.empty(V, dtype=torch.uint8, device=dev)
+    mask = torch.empty(V, dtype=torch.bool, device=dev)   # the kernel writes bytes 0 / 1
     raw = torch.empty((V, 3), dtype=torch.float32, device=dev) if want_raw else None
     rc = _lib.load().mmn_normals_from_max(V, _vp(img), _vp(w), _vp(max_abs),
                                           float(filter_percent), _vp(normals), _vp(mask),
                                           _vp(raw), _stream(dev))
     _lib.check(rc, "mmn_normals_from_max")
-    out = (normals.view(*shape, 3), mask.view(shape).bool())
+    out = (normals.view(*shape, 3), mask.view(shape))
     if want_raw:
         out = out + (raw.view(*shape, 3),)
     return out
