@@ -20,9 +20,10 @@
 // hardware sincos on the wrapped angle (f_k uniform, f_k = c / lambda_k).
 //
 // Work item = (offset set t, antenna a); grid = (ray blocks, items).  A block takes every
-// blocks-per-item-th tile of 256 rays, marches them through every component, collects the
-// hits in ray order and adds them to its partial channel [K]; a second kernel adds the
-// blocks' partials in block order (FP64) -- deterministic run to run.
+// blocks-per-item-th tile of 256 rays, gathers the rays that can reach the box into batches,
+// marches them through every component, collects the hits in ray order and adds them to its
+// partial channel [K]; a second kernel adds the blocks' partials in a fixed order (FP64) --
+// deterministic run to run.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -57,6 +58,8 @@ struct IsoParams {
     int32_t *block_hits;       // [items][blocks]
     int blocks_per_item;
     int32_t *status;
+    float *plane;              // [width + height] view-plane coordinates of columns and rows
+    float *basis;              // [A][12] RayBasis of each antenna
 };
 
 __device__ __forceinline__ float deg_to_rad(const float &deg) { return (deg * (kPiF / 180.f)); }
@@ -91,15 +94,16 @@ __device__ RayBasis ray_basis(const IsoParams &p, float rdx, float rdy, float rd
     return b;
 }
 
-// ray direction of pixel (px, py)
-__device__ void ray_direction(const IsoParams &p, const RayBasis &b, int px, int py, float &dx,
-                              float &dy, float &dz) {
-    const float horiz_fov = b.horiz_fov, vert_fov = b.vert_fov;
-    // the angle is formed in double (a float plus 0.5) and narrowed, as the reference does
-    const float horiz_angle = -horiz_fov + (horiz_fov*2) * (__int2float_rd(px) + 0.5)/ __int2float_rd(p.width);
-    const float vert_angle = -vert_fov + (vert_fov*2) * (__int2float_rd(py) + 0.5)/ __int2float_rd(p.height);
-    const float view_plane_x = tan(horiz_angle);
-    const float view_plane_y = tan(vert_angle);
+// view-plane coordinate of column (or row) i of n: the angle is formed in double (a float plus
+// 0.5) and narrowed, as the reference does
+__device__ float view_plane(float fov, int i, int n) {
+    const float angle = -fov + (fov*2) * (__int2float_rd(i) + 0.5)/ __int2float_rd(n);
+    return tan(angle);
+}
+
+// ray direction through a point of the view plane
+__device__ void ray_direction(const RayBasis &b, float view_plane_x, float view_plane_y,
+                              float &dx, float &dy, float &dz) {
     const float s_x = view_plane_x * b.u_x + view_plane_y * b.v_x - b.w_x;
     const float s_y = view_plane_x * b.u_y + view_plane_y * b.v_y - b.w_y;
     const float s_z = view_plane_x * b.u_z + view_plane_y * b.v_z - b.w_z;
@@ -154,34 +158,95 @@ __device__ __forceinline__ float grid_at(const float *g, float tau, int idx, int
     return __fsub_rn(g[idx], tau);
 }
 
+// Constants of the march, the same at every step.
+struct MarchGrid {
+    float voxel_size, inv;             // and its reciprocal
+    float edge_x, edge_y, edge_z;      // (max - min) / voxel_size
+    bool exact;                        // flat indices are exact in FP32
+};
+__device__ __forceinline__ MarchGrid march_grid(const IsoParams &p) {
+    MarchGrid m;
+    m.voxel_size = (p.bb_max_y - p.bb_min_y) / (p.res_y - 1);
+    m.inv = 1.f / m.voxel_size;
+    m.edge_x = (p.bb_max_x - p.bb_min_x) / m.voxel_size;
+    m.edge_y = (p.bb_max_y - p.bb_min_y) / m.voxel_size;
+    m.edge_z = (p.bb_max_z - p.bb_min_z) / m.voxel_size;
+    m.exact = ((int64_t)p.res_x + 2) * (p.res_y + 2) * (p.res_z + 2) < (1 << 24);
+    return m;
+}
+
+// floorf(a / voxel_size) for a >= 0: a * inv is within 3e-7 of the rounded quotient, relative, so
+// its floor -- one addition rounded down -- is the quotient's unless it lies within 1.2e-6 (h + 1)
+// of an integer (or the quotient is beyond 2^22, or NaN); then the division decides.
+__device__ __forceinline__ float floor_cell(float a, const MarchGrid &m) {
+    const float h = a * m.inv;
+    const float r = __fadd_rd(h, 8388608.f) - 8388608.f;
+    if (fabsf((h - r) - 0.5f) < fmaf(h, -1.2e-6f, 0.5f - 1.2e-6f) && h < 4194304.f) return r;
+    return floorf(a / m.voxel_size);
+}
+
 // signed distance at a point (the reference's ValueAt); ok=false if an index left the grid
-__device__ float value_at(const IsoParams &p, const float *g, float tau, float px, float py, float pz,
-                          float dx, float dy, float dz, bool first_time, bool &ok) {
+__device__ __forceinline__ float value_at(const IsoParams &p, const MarchGrid &mg, const float *g,
+                                          float tau, float px, float py, float pz, float dx,
+                                          float dy, float dz, bool first_time, bool &ok) {
     if (!inside_box(p, px, py, pz)) {
         if (first_time)
             return box_distance(p, px, py, pz, dx, dy, dz) + 0.00001f;
         return -1;
     }
     const int n = p.res_x * p.res_y * p.res_z;
-    const float voxel_size = (p.bb_max_y - p.bb_min_y) / (p.res_y - 1);
-    float mx = floorf((px - p.bb_min_x) / voxel_size);
-    float my = floorf((py - p.bb_min_y) / voxel_size);
-    float mz = floorf((pz - p.bb_min_z) / voxel_size);
-    if (mx == (p.bb_max_x - p.bb_min_x) / voxel_size) mx = (p.bb_max_x - p.bb_min_x) / voxel_size - 1;
-    if (my == (p.bb_max_y - p.bb_min_y) / voxel_size) my = (p.bb_max_y - p.bb_min_y) / voxel_size - 1;
-    if (mz == (p.bb_max_z - p.bb_min_z) / voxel_size) mz = (p.bb_max_z - p.bb_min_z) / voxel_size - 1;
+    const float voxel_size = mg.voxel_size;
+    float mx = floor_cell(px - p.bb_min_x, mg);
+    float my = floor_cell(py - p.bb_min_y, mg);
+    float mz = floor_cell(pz - p.bb_min_z, mg);
+    if (mx == mg.edge_x) mx = mg.edge_x - 1;
+    if (my == mg.edge_y) my = mg.edge_y - 1;
+    if (mz == mg.edge_z) mz = mg.edge_z - 1;
     const int rx = p.res_x, ry = p.res_y, rz = p.res_z;
-    const float g000 = grid_at(g, tau, flat_index(mx, my, mz, rx, ry, rz), n, ok);
-    const float g010 = grid_at(g, tau, flat_index(mx, my + 1, mz, rx, ry, rz), n, ok);
-    const float g001 = grid_at(g, tau, flat_index(mx, my, mz + 1, rx, ry, rz), n, ok);
-    const float g011 = grid_at(g, tau, flat_index(mx, my + 1, mz + 1, rx, ry, rz), n, ok);
-    const float g100 = grid_at(g, tau, flat_index(mx + 1, my, mz, rx, ry, rz), n, ok);
-    const float g110 = grid_at(g, tau, flat_index(mx + 1, my + 1, mz, rx, ry, rz), n, ok);
-    const float g101 = grid_at(g, tau, flat_index(mx + 1, my, mz + 1, rx, ry, rz), n, ok);
-    const float g111 = grid_at(g, tau, flat_index(mx + 1, my + 1, mz + 1, rx, ry, rz), n, ok);
-    if (g000 < kUndef + 10 || g010 < kUndef + 10 || g001 < kUndef + 10 || g011 < kUndef + 10 ||
-        g100 < kUndef + 10 || g110 < kUndef + 10 || g101 < kUndef + 10 || g111 < kUndef + 10)
-        return kMinStep;
+    float g000, g010, g001, g011, g100, g110, g101, g111;
+    if (mg.exact) {
+        // every index the reference forms in FP32 is exact: one base and integer strides
+        const int base = ((int)mx * ry + (int)my) * rz + (int)mz;
+        const int sx = ry * rz;
+        if (base < 0 || base + sx + rz + 1 >= n) {
+            ok = false;
+            return 0.f;
+        }
+        const float *q = g + base;
+        g000 = __ldg(q);
+        g001 = __ldg(q + 1);
+        g010 = __ldg(q + rz);
+        g011 = __ldg(q + rz + 1);
+        g100 = __ldg(q + sx);
+        g101 = __ldg(q + sx + 1);
+        g110 = __ldg(q + sx + rz);
+        g111 = __ldg(q + sx + rz + 1);
+        // the subtraction of tau keeps the order, so the least corner decides for all (a NaN
+        // corner compares false in the reference too, and fminf passes it over)
+        const float least = fminf(fminf(fminf(g000, g001), fminf(g010, g011)),
+                                  fminf(fminf(g100, g101), fminf(g110, g111)));
+        if (__fsub_rn(least, tau) < kUndef + 10) return kMinStep;
+        g000 = __fsub_rn(g000, tau);
+        g001 = __fsub_rn(g001, tau);
+        g010 = __fsub_rn(g010, tau);
+        g011 = __fsub_rn(g011, tau);
+        g100 = __fsub_rn(g100, tau);
+        g101 = __fsub_rn(g101, tau);
+        g110 = __fsub_rn(g110, tau);
+        g111 = __fsub_rn(g111, tau);
+    } else {
+        g000 = grid_at(g, tau, flat_index(mx, my, mz, rx, ry, rz), n, ok);
+        g010 = grid_at(g, tau, flat_index(mx, my + 1, mz, rx, ry, rz), n, ok);
+        g001 = grid_at(g, tau, flat_index(mx, my, mz + 1, rx, ry, rz), n, ok);
+        g011 = grid_at(g, tau, flat_index(mx, my + 1, mz + 1, rx, ry, rz), n, ok);
+        g100 = grid_at(g, tau, flat_index(mx + 1, my, mz, rx, ry, rz), n, ok);
+        g110 = grid_at(g, tau, flat_index(mx + 1, my + 1, mz, rx, ry, rz), n, ok);
+        g101 = grid_at(g, tau, flat_index(mx + 1, my, mz + 1, rx, ry, rz), n, ok);
+        g111 = grid_at(g, tau, flat_index(mx + 1, my + 1, mz + 1, rx, ry, rz), n, ok);
+        if (g000 < kUndef + 10 || g010 < kUndef + 10 || g001 < kUndef + 10 || g011 < kUndef + 10 ||
+            g100 < kUndef + 10 || g110 < kUndef + 10 || g101 < kUndef + 10 || g111 < kUndef + 10)
+            return kMinStep;
+    }
     const float tx = (px - (p.bb_min_x + mx * voxel_size)) / voxel_size;
     const float ex_y0z0 = (1.f - tx) * g000 + tx * g100;
     const float ex_y1z0 = (1.f - tx) * g010 + tx * g110;
@@ -198,7 +263,8 @@ __device__ float value_at(const IsoParams &p, const float *g, float tau, float p
 __device__ bool march(const IsoParams &p, const float *g, float tau, float ox, float oy, float oz,
                       float dx, float dy, float dz, float &hx, float &hy, float &hz, float &vx,
                       float &vy, float &vz) {
-    const float voxel_size = (p.bb_max_y - p.bb_min_y) / (p.res_y - 1);
+    const MarchGrid mg = march_grid(p);
+    const float voxel_size = mg.voxel_size;
     bool first_time = true;
     float depth = 0;
     for (int steps = 0; steps < kMaxSteps; steps++) {
@@ -206,7 +272,7 @@ __device__ bool march(const IsoParams &p, const float *g, float tau, float ox, f
         const float ry = oy + depth * dy;
         const float rz = oz + depth * dz;
         bool ok = true;
-        const float distance = value_at(p, g, tau, rx, ry, rz, dx, dy, dz, first_time, ok);
+        const float distance = value_at(p, mg, g, tau, rx, ry, rz, dx, dy, dz, first_time, ok);
         if (!ok) return false;
         first_time = false;
         if (distance == -1) return false;
@@ -262,33 +328,146 @@ __device__ bool refine(const IsoParams &p, const float *g, float tau, float hx, 
     return true;
 }
 
+// Whether the line through the eye and a point of the view plane misses the bounding box grown
+// by `margin`.  A ray can only hit where its first step from the eye -- to the box's entry, or,
+// for a ray that no face of the box receives, the step of -1 + 1e-5 that the reference's sentinel
+// turns into -- lands inside the box, and both points lie on that line.  The slab test's FP32
+// rounding (about 1e-6 of the distance) is far inside the margin; NaN rejects nothing.  (A first
+// step shorter than a voxel, the sentinel's among them, is a hit at the eye itself: it counts only
+// if the eye's cell is in the grid, so an eye within two voxels of the box keeps every ray.)
+__device__ __forceinline__ bool line_misses(const IsoParams &p, const RayBasis &b, float margin,
+                                            float ex, float ey, float ez, float vx, float vy) {
+    const float s[3] = {vx * b.u_x + vy * b.v_x - b.w_x, vx * b.u_y + vy * b.v_y - b.w_y,
+                        vx * b.u_z + vy * b.v_z - b.w_z};
+    const float o[3] = {ex, ey, ez};
+    const float lo[3] = {p.bb_min_x, p.bb_min_y, p.bb_min_z};
+    const float hi[3] = {p.bb_max_x, p.bb_max_y, p.bb_max_z};
+    float t0 = -__int_as_float(0x7f800000), t1 = -t0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float inv = __fdividef(1.f, copysignf(fmaxf(fabsf(s[k]), 1e-12f), s[k]));
+        const float a = (lo[k] - margin - o[k]) * inv, c = (hi[k] + margin - o[k]) * inv;
+        t0 = fmaxf(t0, fminf(a, c));
+        t1 = fminf(t1, fmaxf(a, c));
+    }
+    return t0 > t1;
+}
+
+// The tables that every block of an antenna shares: view-plane coordinates and view frames (the
+// frame alone is 27 powf calls, which each thread of each block formed for itself before).
+__global__ void iso_prep_kernel(const IsoParams p) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.width) {
+        p.plane[i] = view_plane(deg_to_rad(p.width_fov), i, p.width);
+    } else if (i < p.width + p.height) {
+        p.plane[i] = view_plane(deg_to_rad(p.height_fov), i - p.width, p.height);
+    } else if (i - p.width - p.height < p.num_ant) {
+        const int a = i - p.width - p.height;
+        const RayBasis b = ray_basis(p, p.rx_dirs[3 * a], p.rx_dirs[3 * a + 1], p.rx_dirs[3 * a + 2]);
+        float *o = p.basis + 12 * a;
+        o[0] = b.w_x;
+        o[1] = b.w_y;
+        o[2] = b.w_z;
+        o[3] = b.u_x;
+        o[4] = b.u_y;
+        o[5] = b.u_z;
+        o[6] = b.v_x;
+        o[7] = b.v_y;
+        o[8] = b.v_z;
+    }
+}
+
+// Rays whose line misses the box (99 % of them at +-80 degrees over a 0.2 m object at 0.45 m) are
+// dropped before the exact direction and march, whose 12 powf calls, divisions and two steps they
+// spent on finding that out; the rest are gathered into batches of 256, so that the warps that
+// march are full.  30 items of 1024 x 1024 rays: 1520 us, 860 without the misses, 716 with the batches,
+// 490 with integer cell indices and one comparison for a cell's eight corners.
 __global__ void __launch_bounds__(kIsoThreads) iso_channel_kernel(const IsoParams p) {
     __shared__ unsigned long long s_ph0[kIsoThreads], s_stp[kIsoThreads];
     __shared__ int s_warp[kIsoThreads / 32 + 1];
+    __shared__ int s_ray[2 * kIsoThreads];  // a batch and what one more tile can add
     const int item = blockIdx.y;
     const int t = item / p.num_ant, a = item % p.num_ant;
     const int npix = p.width * p.height;
     const int ntiles = (npix + kIsoThreads - 1) / kIsoThreads;
     const float eye_x = (float)p.rx_locs[3 * a], eye_y = (float)p.rx_locs[3 * a + 1],
                 eye_z = (float)p.rx_locs[3 * a + 2];
-    const RayBasis basis = ray_basis(p, p.rx_dirs[3 * a], p.rx_dirs[3 * a + 1], p.rx_dirs[3 * a + 2]);
+    RayBasis basis;
+    {
+        const float *o = p.basis + 12 * a;
+        basis.w_x = o[0];
+        basis.w_y = o[1];
+        basis.w_z = o[2];
+        basis.u_x = o[3];
+        basis.u_y = o[4];
+        basis.u_z = o[5];
+        basis.v_x = o[6];
+        basis.v_y = o[7];
+        basis.v_z = o[8];
+    }
+    // 1e-4 of the farthest box point's distance, and more than the first step's 1e-5
+    const float margin =
+        2e-5f + 1e-4f * (fmaxf(fabsf(p.bb_min_x - eye_x), fabsf(p.bb_max_x - eye_x)) +
+                         fmaxf(fabsf(p.bb_min_y - eye_y), fabsf(p.bb_max_y - eye_y)) +
+                         fmaxf(fabsf(p.bb_min_z - eye_z), fabsf(p.bb_max_z - eye_z)));
+    const float skin = 2.f * fmaxf(p.voxel_size_ref, (p.bb_max_y - p.bb_min_y) / (p.res_y - 1));
+    const bool beside = !(eye_x < p.bb_min_x - skin || eye_x > p.bb_max_x + skin ||
+                          eye_y < p.bb_min_y - skin || eye_y > p.bb_max_y + skin ||
+                          eye_z < p.bb_min_z - skin || eye_z > p.bb_max_z + skin);
     const int64_t ncell = (int64_t)p.res_x * p.res_y * p.res_z;
     const int64_t bslot = (int64_t)item * p.blocks_per_item + blockIdx.x;
     float2 *dst = p.partial + bslot * p.num_wl;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int total = 0;  // block-uniform: hits added to dst so far
-    // this block's tiles of 256 rays, in order; every component's isosurface in turn (the
-    // reference sums the components' channels)
-    for (int tile = blockIdx.x; tile < ntiles; tile += p.blocks_per_item) {
-        const int pixel = tile * kIsoThreads + threadIdx.x;
+    int count = 0;  // block-uniform: rays waiting in s_ray
+    int tile = blockIdx.x;
+    for (;;) {
+        // this block's tiles of 256 rays, in order, until a full batch of rays can reach the box
+        while (count < kIsoThreads && tile < ntiles) {
+            const int pixel = tile * kIsoThreads + threadIdx.x;
+            const int py = min(pixel, npix - 1) / p.width;
+            const float plane_x = __ldg(p.plane + (min(pixel, npix - 1) - py * p.width));
+            const float plane_y = __ldg(p.plane + p.width + py);
+            const bool reach = pixel < npix &&
+                               (beside || !line_misses(p, basis, margin, eye_x, eye_y, eye_z,
+                                                       plane_x, plane_y));
+            tile += p.blocks_per_item;
+            if (!__syncthreads_or(reach)) continue;
+            const unsigned ball = __ballot_sync(0xffffffffu, reach);
+            if (lane == 0) s_warp[warp] = __popc(ball);
+            __syncthreads();
+            int at = count + __popc(ball & ((1u << lane) - 1u)), sum = 0;
+#pragma unroll
+            for (int w = 0; w < kIsoThreads / 32; ++w) {
+                const int cnt = s_warp[w];
+                at += w < warp ? cnt : 0;
+                sum += cnt;
+            }
+            if (reach) s_ray[at] = pixel;
+            count += sum;
+            __syncthreads();  // the counts are rewritten by the next tile
+        }
+        if (count == 0) break;
+        const bool mine = threadIdx.x < count;
         float dx = 0.f, dy = 0.f, dz = 0.f;
-        if (pixel < npix) ray_direction(p, basis, pixel % p.width, pixel / p.width, dx, dy, dz);
+        if (mine) {
+            const int pixel = s_ray[threadIdx.x], py = pixel / p.width;
+            ray_direction(basis, __ldg(p.plane + (pixel - py * p.width)),
+                          __ldg(p.plane + p.width + py), dx, dy, dz);
+        }
+        // the rest of the list moves to its front (barriers of the loop below order the writes)
+        const int left = max(count - kIsoThreads, 0);
+        const int later = threadIdx.x < left ? s_ray[kIsoThreads + threadIdx.x] : 0;
+        __syncthreads();
+        if (threadIdx.x < left) s_ray[threadIdx.x] = later;
+        count = left;
+        // every component's isosurface in turn (the reference sums the components' channels)
         for (int c = 0; c < p.num_comp; ++c) {
             const float *g = p.grids + (int64_t)c * ncell;
             const float tau = p.taus[(int64_t)t * p.num_comp + c];
             bool hit = false;
             double d = 0.0;
-            if (pixel < npix) {
+            if (mine) {
                 float hx, hy, hz, vx, vy, vz, ix, iy, iz;
                 if (march(p, g, tau, eye_x, eye_y, eye_z, dx, dy, dz, hx, hy, hz, vx, vy, vz) &&
                     refine(p, g, tau, hx, hy, hz, vx, vy, vz, dx, dy, dz, ix, iy, iz)) {
@@ -299,7 +478,7 @@ __global__ void __launch_bounds__(kIsoThreads) iso_channel_kernel(const IsoParam
                     hit = true;
                 }
             }
-            // the hits of this tile and component, compacted in ray order
+            // the hits of this batch and component, compacted in ray order
             const unsigned ball = __ballot_sync(0xffffffffu, hit);
             if (lane == 0) s_warp[warp] = __popc(ball);
             __syncthreads();
@@ -384,7 +563,8 @@ __global__ void iso_march_debug_kernel(const IsoParams p, int comp, float tau, i
     float dx, dy, dz;
     const RayBasis basis =
         ray_basis(p, p.rx_dirs[3 * ant], p.rx_dirs[3 * ant + 1], p.rx_dirs[3 * ant + 2]);
-    ray_direction(p, basis, pixel % p.width, pixel / p.width, dx, dy, dz);
+    ray_direction(basis, view_plane(basis.horiz_fov, pixel % p.width, p.width),
+                  view_plane(basis.vert_fov, pixel / p.width, p.height), dx, dy, dz);
     const int64_t ncell = (int64_t)p.res_x * p.res_y * p.res_z;
     float hx = -1, hy = -1, hz = -1, vx = -1, vy = -1, vz = -1;
     if (!march(p, p.grids + comp * ncell, tau, (float)p.rx_locs[3 * ant],
@@ -424,14 +604,30 @@ int iso_check(const mmn_iso_scene *s) {
     return MMN_OK;
 }
 
-// ray-tile blocks per work item: at most 8 per SM (each loops over its share of the tiles)
-int64_t iso_blocks(const mmn_iso_scene *s) {
+// Ray-tile blocks per work item: some 24 per SM over all items, at most 8 per SM for one (each
+// loops over its share of the tiles), and an odd number, so that the stride from tile to tile
+// does not keep a block in one column of the view (4 tiles to a row of 1024 rays: half the blocks
+// never saw the object).
+int64_t iso_blocks(const mmn_iso_scene *s, int64_t items) {
     const int64_t npix = (int64_t)s->width * s->height;
     const int64_t tiles = (npix + mmn::kIsoThreads - 1) / mmn::kIsoThreads;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return std::min<int64_t>(tiles, (int64_t)sms * 8);
+    const int64_t want = std::max<int64_t>(16, (int64_t)sms * 24 / std::max<int64_t>(items, 1));
+    return std::min<int64_t>(tiles, std::min<int64_t>(want, (int64_t)sms * 8) | 1);
+}
+
+// Partial slots (items x blocks) that a workspace for `items` holds: enough for any smaller count
+// too, whose blocks per item are more.
+int64_t iso_slots(const mmn_iso_scene *s, int64_t items) {
+    int64_t slots = items * iso_blocks(s, items);
+    for (int64_t i = 1; i <= items && i <= 512; ++i) {
+        const int64_t b = iso_blocks(s, i);
+        slots = std::max(slots, i * b);
+        if (b <= 17) break;  // the least: constant from here on
+    }
+    return slots;
 }
 
 mmn::IsoParams iso_params(const mmn_iso_scene *s) {
@@ -467,10 +663,11 @@ mmn::IsoParams iso_params(const mmn_iso_scene *s) {
 extern "C" size_t mmn_iso_channels_workspace_bytes(const mmn_iso_scene *s, int32_t num_sets,
                                                    int32_t num_antennas) {
     if (iso_check(s) != MMN_OK || num_sets < 1 || num_antennas < 1) return 0;
-    const int64_t blocks = iso_blocks(s);
     const int64_t items = (int64_t)num_sets * num_antennas;
-    return kIsoStatus + iso_up((size_t)items * blocks * sizeof(int32_t)) +
-           iso_up((size_t)items * blocks * s->num_wl * sizeof(float2));
+    const int64_t slots = iso_slots(s, items);
+    return kIsoStatus + iso_up((size_t)slots * sizeof(int32_t)) +
+           iso_up((size_t)slots * s->num_wl * sizeof(float2)) +
+           iso_up(((size_t)s->width + s->height + 12 * (size_t)num_antennas) * sizeof(float));
 }
 
 extern "C" int mmn_iso_channels(const mmn_iso_scene *s, const float *taus, int32_t num_sets,
@@ -486,7 +683,7 @@ extern "C" int mmn_iso_channels(const mmn_iso_scene *s, const float *taus, int32
     const size_t need = mmn_iso_channels_workspace_bytes(s, num_sets, num_antennas);
     if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))
         return MMN_ERR_WORKSPACE;
-    const int blocks = (int)iso_blocks(s);
+    const int blocks = (int)iso_blocks(s, items);
     unsigned char *w = static_cast<unsigned char *>(workspace);
     mmn::IsoParams p = iso_params(s);
     p.taus = taus;
@@ -499,7 +696,14 @@ extern "C" int mmn_iso_channels(const mmn_iso_scene *s, const float *taus, int32
     p.block_hits = reinterpret_cast<int32_t *>(w + kIsoStatus);
     p.partial = reinterpret_cast<float2 *>(w + kIsoStatus +
                                            iso_up((size_t)items * blocks * sizeof(int32_t)));
+    p.plane = reinterpret_cast<float *>(w + kIsoStatus +
+                                        iso_up((size_t)items * blocks * sizeof(int32_t)) +
+                                        iso_up((size_t)items * blocks * s->num_wl *
+                                               sizeof(float2)));
+    p.basis = p.plane + s->width + s->height;
     if (cudaMemsetAsync(w, 0, kIsoStatus, stream) != cudaSuccess) return MMN_ERR_CUDA;
+    const int64_t prep = (int64_t)s->width + s->height + num_antennas;
+    mmn::iso_prep_kernel<<<(unsigned)((prep + 127) / 128), 128, 0, stream>>>(p);
     mmn::iso_channel_kernel<<<dim3(blocks, (unsigned)items), mmn::kIsoThreads, 0, stream>>>(p);
     mmn::iso_reduce_kernel<<<dim3((unsigned)((s->num_wl + 31) / 32), (unsigned)items),
                              mmn::kIsoReduceWarps * 32, 0, stream>>>(
