@@ -11,7 +11,7 @@
 // exactly:
 //   * the frontier of level k is stored in queue order;
 //   * every (frontier position i, direction d) that reaches an unvisited voxel of the
-//     component bids key 6*i + d for it (64-bit atomicMin): the smallest key is the cell
+//     component bids key 6*i + d for it (atomicMin): the smallest key is the cell
 //     that dequeues first, which is the cell that enqueues the voxel sequentially;
 //   * the winning bids, read in key order (an exclusive scan over the 6*|frontier| slots),
 //     are the next level's queue order -- the order in which the sequential search appends
@@ -66,91 +66,136 @@ __device__ void uf_union(int32_t *parent, int32_t a, int32_t b, int32_t *status)
     set_status(status, MMN_ERR_TIMEOUT);
 }
 
-__global__ void cc_init_kernel(const uint8_t *__restrict__ mask, int64_t n,
+// parent = the first voxel of the run along z as far back as this warp's 32 voxels reach (a run
+// that enters the warp links to the voxel before it), so the z direction needs no unions; -1
+// outside the mask.
+__global__ void cc_init_kernel(const uint8_t *__restrict__ mask, int64_t n, int nz,
                                int32_t *__restrict__ parent, int32_t *__restrict__ count) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool in = v < n && mask[v];
+    const int iz = v < n ? (int)((uint32_t)v % (uint32_t)nz) : 0;
+    // lanes that continue the run of the lane before them
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    const unsigned cont = __ballot_sync(
+        0xffffffffu, in && iz > 0 && (lane > 0 ? (m >> (lane - 1)) & 1u : mask[v - 1] != 0));
     if (v >= n) return;
-    parent[v] = mask[v] ? (int32_t)v : -1;
     count[v] = 0;
+    if (!in) {
+        parent[v] = -1;
+        return;
+    }
+    // the nearest lane at or below this one that does not continue a run
+    const unsigned stops = ~cont & (lane == 31 ? 0xffffffffu : (1u << (lane + 1)) - 1u);
+    const int first = stops ? 31 - __clz(stops) : -1;
+    parent[v] = (int32_t)(v - lane + first);  // first = -1: the voxel before the warp's
 }
 
+// Unions with the +x and +y neighbours, only where two runs begin to touch: if the voxels before
+// both along z are in the mask too, those two are already being joined.
 __global__ void cc_union_kernel(const uint8_t *__restrict__ mask, int nx, int ny, int nz,
                                 int32_t *parent, int32_t *status) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n = (uint32_t)nx * ny * nz;
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n || !mask[v]) return;
-    const int64_t nyz = (int64_t)ny * nz;
+    const uint32_t nyz = (uint32_t)ny * nz;
     const int ix = (int)(v / nyz);
-    const int iy = (int)((v / nz) % ny);
-    const int iz = (int)(v % nz);
-    if (ix + 1 < nx && mask[v + nyz]) uf_union(parent, (int32_t)v, (int32_t)(v + nyz), status);
-    if (iy + 1 < ny && mask[v + nz]) uf_union(parent, (int32_t)v, (int32_t)(v + nz), status);
-    if (iz + 1 < nz && mask[v + 1]) uf_union(parent, (int32_t)v, (int32_t)(v + 1), status);
+    const int iz = (int)(v % (uint32_t)nz), iy = (int)(v / (uint32_t)nz % (uint32_t)ny);
+    const bool before = iz > 0 && mask[v - 1];
+    if (ix + 1 < nx && mask[v + nyz] && !(before && mask[v + nyz - 1]))
+        uf_union(parent, (int32_t)v, (int32_t)(v + nyz), status);
+    if (iy + 1 < ny && mask[v + nz] && !(before && mask[v + nz - 1]))
+        uf_union(parent, (int32_t)v, (int32_t)(v + nz), status);
 }
 
+// Roots, and the components' sizes (one atomic per warp and root: a component's voxels all add to
+// one word).
 __global__ void cc_flatten_kernel(int64_t n, int32_t *parent, int32_t *__restrict__ count,
                                   int32_t *status) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n || parent[v] < 0) return;
+    const bool in = v < n && parent[v] >= 0;
+    const unsigned active = __ballot_sync(0xffffffffu, in);
+    if (!in) return;
     const int32_t r = uf_find(parent, (int32_t)v, status);
     parent[v] = r;
-    atomicAdd(&count[r], 1);
+    const unsigned same = __match_any_sync(active, r);
+    if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&count[r], __popc(same));
 }
 
 // ------------------------------------------------------------------ breadth-first search
 struct BfsArgs {
     int nx, ny, nz;
-    int32_t comp_root;
     const double *normals;   // [V, 3]
-    const int32_t *root;     // [V] component root or -1
-    uint8_t *visited;        // [V]
-    unsigned long long *bid; // [V] smallest key bid this level (all-ones: none)
+    uint32_t *state;         // [V] all-ones: open; 0: closed (visited, NaN or another component);
+                             // during a level an open voxel holds its smallest bid (key + 1)
     double *rsdf;            // [V]
     double dx;
 };
 
-// direction d: (-x, +y, +x, -y, +z, -z), sdf.py's dX/dY/dZ order
-__device__ __forceinline__ bool neighbour(const BfsArgs &a, int32_t v, int d, int32_t &out) {
-    const int64_t nyz = (int64_t)a.ny * a.nz;
-    const int ix = (int)(v / nyz);
-    const int iy = (int)((v / a.nz) % a.ny);
-    const int iz = (int)(v % a.nz);
-    int jx = ix, jy = iy, jz = iz;
-    switch (d) {
-        case 0: jx = ix - 1; break;
-        case 1: jy = iy + 1; break;
-        case 2: jx = ix + 1; break;
-        case 3: jy = iy - 1; break;
-        case 4: jz = iz + 1; break;
-        default: jz = iz - 1; break;
-    }
-    if (jx < 0 || jy < 0 || jz < 0 || jx >= a.nx || jy >= a.ny || jz >= a.nz) return false;
-    out = (int32_t)(((int64_t)jx * a.ny + jy) * a.nz + jz);
-    return true;
+// One word per voxel says whether it can still be reached: a bid is one atomicMin whatever it
+// meets (0 stays the least), and a voxel is won by the key it then holds.
+__global__ void bfs_state_kernel(const double *__restrict__ normals,
+                                 const int32_t *__restrict__ root, int32_t comp_root, int64_t n,
+                                 uint32_t *__restrict__ state) {
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    state[v] = root[v] == comp_root && !isnan(normals[3 * v]) ? 0xffffffffu : 0u;
 }
 
-__device__ __forceinline__ bool open_voxel(const BfsArgs &a, int32_t n) {
-    return !a.visited[n] && !isnan(a.normals[3 * (int64_t)n]) && a.root[n] == a.comp_root;
+struct Cell {
+    int ix, iy, iz;
+};
+__device__ __forceinline__ Cell cell_of(const BfsArgs &a, int32_t v) {
+    const uint32_t t = (uint32_t)v / (uint32_t)a.nz;
+    Cell c;
+    c.iz = (int)((uint32_t)v - t * (uint32_t)a.nz);
+    c.ix = (int)(t / (uint32_t)a.ny);
+    c.iy = (int)(t - (uint32_t)c.ix * (uint32_t)a.ny);
+    return c;
+}
+
+// neighbour in direction d: (-x, +y, +x, -y, +z, -z), sdf.py's dX/dY/dZ order
+__device__ __forceinline__ bool neighbour(const BfsArgs &a, int32_t v, const Cell &c, int d,
+                                          int32_t &out) {
+    switch (d) {
+        case 0: out = v - a.ny * a.nz; return c.ix > 0;
+        case 1: out = v + a.nz; return c.iy + 1 < a.ny;
+        case 2: out = v + a.ny * a.nz; return c.ix + 1 < a.nx;
+        case 3: out = v - a.nz; return c.iy > 0;
+        case 4: out = v + 1; return c.iz + 1 < a.nz;
+        default: out = v - 1; return c.iz > 0;
+    }
+}
+
+// value of voxel n reached in direction d from a cell of value `from`: step * dx as numpy forms
+// it, then dot(): 0 + s0*n0 + s1*n1 + s2*n2 in FP64, in order
+__device__ __forceinline__ double step_value(const BfsArgs &a, int32_t n, int d, double from) {
+    const double sx = d == 0 ? -1.0 : (d == 2 ? 1.0 : 0.0);
+    const double sy = d == 1 ? 1.0 : (d == 3 ? -1.0 : 0.0);
+    const double sz = d == 4 ? 1.0 : (d == 5 ? -1.0 : 0.0);
+    const double *nv = a.normals + 3 * (int64_t)n;
+    double acc = 0.0;
+    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sx, a.dx), __ldg(nv)));
+    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sy, a.dx), __ldg(nv + 1)));
+    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sz, a.dx), __ldg(nv + 2)));
+    return __dadd_rn(from, acc);
 }
 
 __global__ void bfs_bid_kernel(const BfsArgs a, const int32_t *__restrict__ frontier, int64_t nf) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nf * 6) return;
+    const int32_t v = frontier[k / 6];
     int32_t n;
-    if (!neighbour(a, frontier[k / 6], (int)(k % 6), n) || !open_voxel(a, n)) return;
-    atomicMin(&a.bid[n], (unsigned long long)k);
+    if (neighbour(a, v, cell_of(a, v), (int)(k % 6), n)) atomicMin(&a.state[n], (uint32_t)k + 1u);
 }
 
 __global__ void bfs_flag_kernel(const BfsArgs a, const int32_t *__restrict__ frontier, int64_t nf,
                                 int32_t *__restrict__ flag) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nf * 6) return;
+    const int32_t v = frontier[k / 6];
     int32_t n;
-    int32_t f = 0;
-    if (neighbour(a, frontier[k / 6], (int)(k % 6), n) && open_voxel(a, n) &&
-        a.bid[n] == (unsigned long long)k)
-        f = 1;
-    flag[k] = f;
+    flag[k] = neighbour(a, v, cell_of(a, v), (int)(k % 6), n) && a.state[n] == (uint32_t)k + 1u;
 }
 
 // after the exclusive scan pos[k] is the winner's place in the next frontier
@@ -161,28 +206,19 @@ __global__ void bfs_emit_kernel(const BfsArgs a, const int32_t *__restrict__ fro
     const int32_t v = frontier[k / 6];
     const int d = (int)(k % 6);
     int32_t n;
-    if (!neighbour(a, v, d, n) || !open_voxel(a, n) || a.bid[n] != (unsigned long long)k) return;
-    // step * dx as numpy forms it, then dot(): 0 + s0*n0 + s1*n1 + s2*n2 in FP64, in order
-    const double sx = d == 0 ? -1.0 : (d == 2 ? 1.0 : 0.0);
-    const double sy = d == 1 ? 1.0 : (d == 3 ? -1.0 : 0.0);
-    const double sz = d == 4 ? 1.0 : (d == 5 ? -1.0 : 0.0);
-    const double *nv = a.normals + 3 * (int64_t)n;
-    double acc = 0.0;
-    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sx, a.dx), nv[0]));
-    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sy, a.dx), nv[1]));
-    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sz, a.dx), nv[2]));
-    a.rsdf[n] = __dadd_rn(a.rsdf[v], acc);
+    if (!neighbour(a, v, cell_of(a, v), d, n) || a.state[n] != (uint32_t)k + 1u) return;
+    a.rsdf[n] = step_value(a, n, d, a.rsdf[v]);
     next[pos[k]] = n;
 }
 
-__global__ void bfs_mark_kernel(const int32_t *__restrict__ next, int64_t n, uint8_t *visited) {
+__global__ void bfs_mark_kernel(const int32_t *__restrict__ next, int64_t n, uint32_t *state) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) visited[next[k]] = 1;
+    if (k < n) state[next[k]] = 0;
 }
 
-__global__ void bfs_seed_kernel(int32_t seed, int32_t *frontier, uint8_t *visited, double *rsdf) {
+__global__ void bfs_seed_kernel(int32_t seed, int32_t *frontier, uint32_t *state, double *rsdf) {
     frontier[0] = seed;
-    visited[seed] = 1;
+    state[seed] = 0;
     rsdf[seed] = 0.0;
 }
 
@@ -190,11 +226,19 @@ __global__ void bfs_seed_kernel(int32_t seed, int32_t *frontier, uint8_t *visite
 // and rsdf values as the per-level kernels above, with __syncthreads between the phases
 // instead of kernel boundaries and a host read-back -- until the frontier empties or grows
 // past kSmallFrontier entries (then the per-level kernels take over from the frontier it
-// leaves in global memory).  Each thread owns a run of consecutive slots k = 6 i + d, so
-// a block-wide exclusive scan of the threads' winner counts gives the queue order.  The
+// leaves in global memory).  The frontier stays in shared memory; a thread owns consecutive
+// entries, all six directions of one at a time, so that a level's latency is one round of
+// reductions, one of loads and one of normals.  What bounds it then is one SM's scattered traffic
+// (a 32-byte sector a bid), so a bit per open voxel is kept in shared memory too, where it fits
+// (MASK), and only open neighbours cost a bid and a load.  100 x 96 x 72 cap: 2.85 ms when each
+// slot walked frontier, visited, normal, root and bid in turn; 1.21 ms; 0.89 ms with the bits (86 levels).
+// A block-wide exclusive scan of the threads' winner counts gives the queue order.  The
 // loop ends: every level marks at least one new voxel of a finite component.
 constexpr int kSmallThreads = 1024;
-constexpr int kSmallFrontier = 4096;  // 24576 slots: at most 24 per thread (one bit each)
+constexpr int kSmallFrontier = 4096;
+constexpr int kSmallPer = kSmallFrontier / kSmallThreads;  // entries per thread, at most
+constexpr size_t kSmallBytes = 2 * kSmallFrontier * sizeof(int32_t);
+constexpr size_t kSmallMost = 224 * 1024;  // shared memory of one CTA, less the static part
 
 struct SmallState {
     int64_t nf;       // frontier size on exit (0: the search is complete)
@@ -203,40 +247,68 @@ struct SmallState {
     int32_t pad;
 };
 
+template <bool MASK>
 __global__ void __launch_bounds__(kSmallThreads) bfs_small_kernel(const BfsArgs a, int32_t *fa,
                                                                   int32_t *fb, int64_t nf0,
                                                                   SmallState *state) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    int32_t *cell = reinterpret_cast<int32_t *>(dyn);                      // [2][kSmallFrontier]
+    uint32_t *open = reinterpret_cast<uint32_t *>(cell + 2 * kSmallFrontier);  // MASK: [V / 32]
     __shared__ int32_t warp_tot[kSmallThreads / 32];
-    __shared__ int32_t s_total;
-    int32_t *cur = fa, *nxt = fb;
-    int64_t nf = nf0, marked = 0;
-    int32_t parity = 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    while (nf > 0 && nf <= kSmallFrontier) {
-        const int slots = (int)nf * 6;
-        const int per = (slots + kSmallThreads - 1) / kSmallThreads;
-        const int k0 = tid * per;
-        const int k1 = min(k0 + per, slots);
-        // bids
-        for (int k = k0; k < k1; ++k) {
-            int32_t n;
-            if (neighbour(a, cur[k / 6], k % 6, n) && open_voxel(a, n))
-                atomicMin(&a.bid[n], (unsigned long long)k);
+    int nf = (int)nf0, cur = 0;
+    int64_t marked = 0;
+    for (int i = tid; i < nf; i += kSmallThreads) cell[i] = fa[i];
+    if (MASK) {
+        const int nvox = a.nx * a.ny * a.nz;
+        for (int v0 = 0; v0 < nvox; v0 += kSmallThreads) {
+            const int v = v0 + tid;
+            const unsigned b = __ballot_sync(0xffffffffu, v < nvox && __ldcg(&a.state[v]) != 0u);
+            if (lane == 0 && v < nvox) open[v >> 5] = b;
         }
-        __syncthreads();
-        // winners of this thread's slots
-        uint32_t won = 0;
-        int32_t cnt = 0;
-        for (int k = k0; k < k1; ++k) {
-            int32_t n;
-            // the bids came from atomics at L2 this level: read them past L1
-            if (neighbour(a, cur[k / 6], k % 6, n) && open_voxel(a, n) &&
-                __ldcg(&a.bid[n]) == (unsigned long long)k) {
-                won |= 1u << (k - k0);
-                ++cnt;
+    }
+    __syncthreads();
+    bool spilled = false;  // the next frontier went to global memory
+    while (nf > 0 && !spilled) {
+        const int32_t *cc = cell + cur * kSmallFrontier;
+        int32_t *nc = cell + (cur ^ 1) * kSmallFrontier;
+        const int per = (nf + kSmallThreads - 1) / kSmallThreads;
+        const int i0 = tid * per, i1 = min(i0 + per, nf);
+        // bids
+        uint32_t bid = 0;
+        for (int i = i0; i < i1; ++i) {
+            const int32_t v = cc[i];
+            const Cell c = cell_of(a, v);
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                int32_t n;
+                if (neighbour(a, v, c, d, n) && (!MASK || open[n >> 5] >> (n & 31) & 1u)) {
+                    atomicMin(&a.state[n], (uint32_t)(6 * i + d) + 1u);
+                    bid |= 1u << (6 * (i - i0) + d);
+                }
             }
         }
+        __syncthreads();
+        // winners of this thread's slots; the bids came from atomics at L2: read them past L1
+        uint32_t won = 0;
+        for (int i = i0; i < i1; ++i) {
+            const uint32_t mine = bid >> (6 * (i - i0)) & 63u;
+            if (!mine) continue;
+            const int32_t v = cc[i];
+            const Cell c = cell_of(a, v);
+            uint32_t got[6];
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                int32_t n;
+                neighbour(a, v, c, d, n);
+                got[d] = mine >> d & 1u ? __ldcg(&a.state[n]) : 0u;
+            }
+#pragma unroll
+            for (int d = 0; d < 6; ++d)
+                if (got[d] == (uint32_t)(6 * i + d) + 1u) won |= 1u << (6 * (i - i0) + d);
+        }
         // exclusive scan of the counts over the block, in thread (= slot) order
+        const int32_t cnt = __popc(won);
         int32_t incl = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -245,53 +317,47 @@ __global__ void __launch_bounds__(kSmallThreads) bfs_small_kernel(const BfsArgs 
         }
         if (lane == 31) warp_tot[warp] = incl;
         __syncthreads();
-        if (warp == 0) {
-            int32_t w = warp_tot[lane];
+        int32_t w = warp_tot[lane];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        const int32_t total = __shfl_sync(0xffffffffu, w, 31);
+        const int32_t before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+        int32_t pos = incl - cnt + (warp > 0 ? before : 0);
+        spilled = total > kSmallFrontier;
+        // emit in queue order
+        for (int i = i0; i < i1; ++i) {
+            const uint32_t mine = won >> (6 * (i - i0)) & 63u;
+            if (!mine) continue;
+            const int32_t v = cc[i];
+            const Cell c = cell_of(a, v);
+            const double from = a.rsdf[v];
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                if (!(mine >> d & 1u)) continue;
+                int32_t n;
+                neighbour(a, v, c, d, n);
+                const double x = step_value(a, n, d, from);
+                a.rsdf[n] = x;
+                a.state[n] = 0;
+                if (MASK) atomicAnd(&open[n >> 5], ~(1u << (n & 31)));
+                (spilled ? fb : nc)[pos++] = n;
             }
-            warp_tot[lane] = w;  // inclusive over warps
-            if (lane == 31) s_total = w;
         }
-        __syncthreads();
-        int32_t pos = incl - cnt + (warp > 0 ? warp_tot[warp - 1] : 0);
-        // emit in queue order (the per-level emit kernel's arithmetic)
-        for (int k = k0; k < k1; ++k) {
-            if (!(won >> (k - k0) & 1u)) continue;
-            const int32_t v = cur[k / 6];
-            const int d = k % 6;
-            int32_t n;
-            neighbour(a, v, d, n);
-            const double sx = d == 0 ? -1.0 : (d == 2 ? 1.0 : 0.0);
-            const double sy = d == 1 ? 1.0 : (d == 3 ? -1.0 : 0.0);
-            const double sz = d == 4 ? 1.0 : (d == 5 ? -1.0 : 0.0);
-            const double *nv = a.normals + 3 * (int64_t)n;
-            double acc = 0.0;
-            acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sx, a.dx), nv[0]));
-            acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sy, a.dx), nv[1]));
-            acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(sz, a.dx), nv[2]));
-            a.rsdf[n] = __dadd_rn(a.rsdf[v], acc);
-            nxt[pos++] = n;
-        }
-        __syncthreads();
-        const int32_t total = s_total;
-        for (int i = tid; i < total; i += kSmallThreads) a.visited[nxt[i]] = 1;
         __syncthreads();
         marked += total;
         nf = total;
-        int32_t *t = cur;
-        cur = nxt;
-        nxt = t;
-        parity ^= 1;
+        cur ^= 1;
     }
     if (tid == 0) {
         state->nf = nf;
         state->visited = marked;
-        state->parity = parity;
+        state->parity = spilled ? 1 : 0;
     }
 }
+static_assert(6 * kSmallPer <= 32, "a thread's winners are bits of one word");
 
 // ---------------------------------------------------------------- exclusive int32 scan
 constexpr int kScanThreads = 256;
@@ -404,7 +470,7 @@ extern "C" int mmn_components(int32_t nx, int32_t ny, int32_t nz, const uint8_t 
     const int64_t n = (int64_t)nx * ny * nz;
     int32_t *status = static_cast<int32_t *>(workspace);
     if (cudaMemsetAsync(status, 0, kStatus, stream) != cudaSuccess) return MMN_ERR_CUDA;
-    cc_init_kernel<<<grid_for(n, 256), 256, 0, stream>>>(mask, n, root, count);
+    cc_init_kernel<<<grid_for(n, 256), 256, 0, stream>>>(mask, n, nz, root, count);
     cc_union_kernel<<<grid_for(n, 256), 256, 0, stream>>>(mask, nx, ny, nz, root, status);
     cc_flatten_kernel<<<grid_for(n, 256), 256, 0, stream>>>(n, root, count, status);
     return cudaGetLastError() == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
@@ -413,7 +479,7 @@ extern "C" int mmn_components(int32_t nx, int32_t ny, int32_t nz, const uint8_t 
 extern "C" size_t mmn_rsdf_workspace_bytes(int32_t nx, int32_t ny, int32_t nz) {
     if (bad_dims(nx, ny, nz)) return 0;
     const int64_t n = (int64_t)nx * ny * nz;
-    return kStatus + up256((size_t)n) + up256((size_t)n * 8) + 2 * up256((size_t)n * 4) +
+    return kStatus + up256((size_t)n * 4) + 2 * up256((size_t)n * 4) +
            up256(((size_t)6 * n + 1) * 4) + up256(scan_temp_elems(6 * n) * 4) + 256;
 }
 
@@ -432,10 +498,8 @@ extern "C" int mmn_rsdf_component(int32_t nx, int32_t ny, int32_t nz, const doub
         return MMN_ERR_WORKSPACE;
     unsigned char *w = static_cast<unsigned char *>(workspace);
     size_t off = kStatus;
-    uint8_t *visited = w + off;
-    off += up256((size_t)n);
-    unsigned long long *bid = reinterpret_cast<unsigned long long *>(w + off);
-    off += up256((size_t)n * 8);
+    uint32_t *state = reinterpret_cast<uint32_t *>(w + off);
+    off += up256((size_t)n * 4);
     int32_t *fa = reinterpret_cast<int32_t *>(w + off);
     off += up256((size_t)n * 4);
     int32_t *fb = reinterpret_cast<int32_t *>(w + off);
@@ -444,22 +508,25 @@ extern "C" int mmn_rsdf_component(int32_t nx, int32_t ny, int32_t nz, const doub
     off += up256(((size_t)6 * n + 1) * 4);
     int32_t *temp = reinterpret_cast<int32_t *>(w + off);
 
-    if (cudaMemsetAsync(w, 0, kStatus, stream) != cudaSuccess ||
-        cudaMemsetAsync(visited, 0, (size_t)n, stream) != cudaSuccess ||
-        cudaMemsetAsync(bid, 0xff, (size_t)n * 8, stream) != cudaSuccess)
-        return MMN_ERR_CUDA;
+    if (cudaMemsetAsync(w, 0, kStatus, stream) != cudaSuccess) return MMN_ERR_CUDA;
     BfsArgs a;
     a.nx = nx;
     a.ny = ny;
     a.nz = nz;
-    a.comp_root = comp_root;
     a.normals = normals;
-    a.root = root;
-    a.visited = visited;
-    a.bid = bid;
+    a.state = state;
     a.rsdf = rsdf;
     a.dx = dx;
-    bfs_seed_kernel<<<1, 1, 0, stream>>>(seed, fa, visited, rsdf);
+    bfs_state_kernel<<<grid_for(n, 256), 256, 0, stream>>>(normals, root, comp_root, n, state);
+    bfs_seed_kernel<<<1, 1, 0, stream>>>(seed, fa, state, rsdf);
+    const size_t with_bits = kSmallBytes + ((size_t)n + 31) / 32 * 4;
+    const bool bits = with_bits <= kSmallMost;
+    const size_t small_bytes = bits ? with_bits : kSmallBytes;
+    const void *small_fn = bits ? reinterpret_cast<const void *>(&bfs_small_kernel<true>)
+                                : reinterpret_cast<const void *>(&bfs_small_kernel<false>);
+    if (cudaFuncSetAttribute(small_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)small_bytes) != cudaSuccess)
+        return MMN_ERR_CUDA;
     int64_t nf = 1, total = 1;
     // the single-CTA search's exit state, in the workspace header after the status word
     SmallState *small = reinterpret_cast<SmallState *>(w + 64);
@@ -467,7 +534,10 @@ extern "C" int mmn_rsdf_component(int32_t nx, int32_t ny, int32_t nz, const doub
     // the search
     for (int64_t level = 0; nf > 0 && level <= n; ++level) {
         if (nf <= kSmallFrontier) {
-            bfs_small_kernel<<<1, kSmallThreads, 0, stream>>>(a, fa, fb, nf, small);
+            void *args[] = {&a, &fa, &fb, &nf, &small};
+            if (cudaLaunchKernel(small_fn, dim3(1), dim3(kSmallThreads), args, small_bytes,
+                                 stream) != cudaSuccess)
+                return MMN_ERR_CUDA;
             SmallState hs;
             if (cudaGetLastError() != cudaSuccess ||
                 cudaMemcpyAsync(&hs, small, sizeof(hs), cudaMemcpyDeviceToHost, stream) !=
@@ -494,7 +564,7 @@ extern "C" int mmn_rsdf_component(int32_t nx, int32_t ny, int32_t nz, const doub
             cudaStreamSynchronize(stream) != cudaSuccess)
             return MMN_ERR_CUDA;
         if (next_n > 0)
-            bfs_mark_kernel<<<grid_for(next_n, 256), 256, 0, stream>>>(fb, next_n, visited);
+            bfs_mark_kernel<<<grid_for(next_n, 256), 256, 0, stream>>>(fb, next_n, state);
         if (cudaGetLastError() != cudaSuccess) return MMN_ERR_CUDA;
         nf = next_n;
         total += next_n;
