@@ -280,6 +280,14 @@ int mmn_components(int32_t num_x, int32_t num_y, int32_t num_z, const uint8_t *m
                    cudaStream_t stream);
 
 /*
+ * Start voxel of a component's search (sdf.py:187-193), on the host: of the `count` voxels with
+ * flat indices flat[] in a grid of num_y x num_z columns, the one nearest the mean of their
+ * coordinates (x, y, z: the axes), the first among ties, with numpy's order of operations.
+ */
+int mmn_rsdf_seed(const int64_t *flat, int64_t count, int32_t num_y, int32_t num_z,
+                  const double *x, const double *y, const double *z, int64_t *seed);
+
+/*
  * Relative signed distance field of one component by breadth-first integration of the
  * normals (_construct_rsdf_components, src/data_processing/sdf.py:122-224): from voxel
  * `seed` (rsdf 0), every voxel of the component with root `comp_root` receives

@@ -122,6 +122,7 @@ SIGNATURES = [
     ("mmn_components_workspace_bytes", _SZ, [ctypes.c_int64]),
     ("mmn_components", _I, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _P, _P, _P, _P,
                             _SZ, _P]),
+    ("mmn_rsdf_seed", _I, [_P, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, _P, _P, _P, _P]),
     ("mmn_rsdf_workspace_bytes", _SZ, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
     ("mmn_rsdf_component", _I, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _P, _P,
                                 ctypes.c_int32, ctypes.c_int32, ctypes.c_double, _P, _P, _P,

@@ -17,6 +17,7 @@ the RSDF and the set of valid components do not depend on it.
 from __future__ import annotations
 
 import ctypes
+from concurrent import futures
 
 import numpy as np
 import torch
@@ -95,8 +96,17 @@ def _seed(all_normals, coords_full, labeled, component_num):
 def _seed_from_voxels(flat, shape, axes):
     """_seed for a component given its voxels' flat indices in ascending (C) order: the same
     coordinate rows, in the same order and dtype, as coords_full[labeled == component], so
-    numpy's mean, norms and argmin -- and the chosen voxel -- are the same."""
+    numpy's mean, norms and argmin -- and the chosen voxel -- are the same.  FP64 axes take
+    the library's native form of the same sums (mmn_rsdf_seed)."""
     ny, nz = shape[1], shape[2]
+    if len(flat) and all(a.dtype == np.float64 and a.shape == (n,) for a, n in zip(axes, shape)):
+        flat = np.ascontiguousarray(flat, dtype=np.int64)
+        keep = [np.ascontiguousarray(a) for a in axes]
+        out = ctypes.c_int64(0)
+        _lib.check(_lib.load().mmn_rsdf_seed(flat.ctypes.data, len(flat), ny, nz,
+                                             *[a.ctypes.data for a in keep], ctypes.byref(out)),
+                   "mmn_rsdf_seed")
+        return out.value
     ii, rem = np.divmod(flat, ny * nz)
     jj, kk = np.divmod(rem, nz)
     x, y, z = axes
@@ -164,12 +174,19 @@ def construct_rsdf_components(all_normals, coords_full, labeled, valid_labels, x
 def compute_rsdf(all_normals, x_locs, y_locs, z_locs):
     """Steps 2-3 of compute_rsdf (sdf.py:285-289) on normals already masked by the binary
     image and normalised: (rsdf, labeled, valid_labels, coords_full)."""
-    coords_full = coordinate_grid(x_locs, y_locs, z_locs)
     dev = _device()
+    # the coordinate grid is host memory only: filled beside the copies and the search
+    with futures.ThreadPoolExecutor(max_workers=1) as pool:
+        grid = pool.submit(coordinate_grid, x_locs, y_locs, z_locs)
+        rsdf, labeled, valid = _compute_rsdf(all_normals, x_locs, y_locs, z_locs, dev)
+        return rsdf, labeled, valid, grid.result()
+
+
+def _compute_rsdf(all_normals, x_locs, y_locs, z_locs, dev):
     normals = torch.as_tensor(np.ascontiguousarray(all_normals, dtype=np.float64), device=dev)
     roots = component_roots(~torch.isnan(normals[..., 0]))
     labeled, valid = find_connected_components(all_normals, x_locs, _roots=roots)
     axes = (np.asarray(x_locs), np.asarray(y_locs), np.asarray(z_locs))
-    rsdf = construct_rsdf_components(all_normals, coords_full, labeled, valid, x_locs,
-                                     _roots=roots, _normals=normals, _axes=axes)
-    return rsdf, labeled, valid, coords_full
+    rsdf = construct_rsdf_components(all_normals, None, labeled, valid, x_locs, _roots=roots,
+                                     _normals=normals, _axes=axes)
+    return rsdf, labeled, valid

@@ -59,3 +59,21 @@ def test_seed_ties_resolve_to_the_first_voxel():
     ref = tuple(int(v) for v in rsdf._seed(normals, coords, labeled, 2))
     got = np.unravel_index(rsdf._seed_from_voxels(np.flatnonzero(mask), shape, (x, y, z)), shape)
     assert tuple(int(v) for v in got) == ref
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 1, 40), (7, 1, 3), (30, 41, 52)])
+@pytest.mark.parametrize("special", [None, "ties", "nan"])
+def test_native_seed_is_numpys_choice(shape, special):
+    """mmn_rsdf_seed (FP64 axes) against numpy's own mean, norms and argmin on the same rows:
+    unordered axes, ties, a NaN coordinate, lists of one voxel and of the whole grid."""
+    rng = np.random.default_rng(sum(shape))
+    axes = [np.arange(n) * 0.002 if special == "ties" else rng.standard_normal(n) for n in shape]
+    if special == "nan":
+        axes[2][-1] = np.nan
+    V = int(np.prod(shape))
+    for m in sorted({1, min(V, 2), (V + 1) // 2, V}):
+        flat = np.sort(rng.choice(V, m, replace=False))
+        ii, jj, kk = np.unravel_index(flat, shape)
+        rows = np.stack([axes[0][ii], axes[1][jj], axes[2][kk]], axis=1)
+        ref = flat[np.argmin(np.linalg.norm(rows - np.mean(rows, axis=0)[None], axis=1))]
+        assert rsdf._seed_from_voxels(flat, shape, axes) == ref
