@@ -64,6 +64,8 @@ def _restated(x, y, z, ant, rxo, meas, fsp, lam, ti, image=None):
     ((8, 8, 8), 257, 4, True, 256, False),
     ((5, 16, 13), 300, 1, True, 1024, True),
     ((16, 11, 3), 24, 4, False, 2048, True),
+    ((3, 5, 9), 20, 4, True, 512, False),    # columns of an odd length in pairs along z
+    ((4, 1, 64), 70, 1, True, 512, True),
 ])
 def test_bits(cuda_dev, shape, ants, rx, ti, bins, far):
     import torch
