@@ -862,7 +862,7 @@ __device__ __forceinline__ void init_stage_barriers(unsigned char *smem) {
 }
 
 // One launch, grid = tiles x splits (one work item per CTA).
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 0>
 __global__ void __launch_bounds__(NT, MINB) bp_fwd_kernel(const FwdParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t gchunk = 0;
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(NT, MINB) bp_fwd_kernel(const FwdParams p) {
 // Persistent launch over a work list of (object, voxel tile, antenna split) items: every
 // CTA pops the next item from a global counter until the list is exhausted.  Items are
 // sorted by cost, largest first, so the tail is made of the smallest items.
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 0>
 __global__ void __launch_bounds__(NT, MINB) bp_fwd_persistent(const BatchParams bp) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_item;
@@ -1025,36 +1025,44 @@ __global__ void stage_meas(const float *__restrict__ src, const float *__restric
 }
 
 // ------------------------------------------------------------------ instantiations
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 0>
 static const void *fwd_ptr() {
     return reinterpret_cast<const void *>(&bp_fwd_kernel<T, NT, FORM, ANCHOR, MINB>);
 }
-template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 1>
+template <int T, int NT, int FORM, int ANCHOR = kAnchorPoly, int MINB = 0>
 static const void *pers_ptr() {
     return reinterpret_cast<const void *>(&bp_fwd_persistent<T, NT, FORM, ANCHOR, MINB>);
 }
 
 const FwdVariant *fwd_variants(int *count) {
-    // index order: the MIXED variants first (default first), then the PLAIN ones
+    // index order: the MIXED variants first (default first), then the PLAIN ones.  The last
+    // template argument is the launch bound's CTAs per SM: without one the compiler settles on
+    // fewer registers than the two stages' shared memory leaves room for.  1 is given where it
+    // measured faster at 256 and 64 samples (mixed_ffma2_fx2_t2_n256 90.5 -> 84.7 ms,
+    // mixed_clen_fx2_t2_n128_s24 84.3 -> 79.2, mixed_clen64_fx2_t2_n256 77.9 -> 75.8,
+    // mixed_clen_fx2_t4_n128 78.5 -> 77.0 on 128^3 voxels x 1024 antennas x 256 samples;
+    // plain_t2_n256 9.88 -> 9.39 s at 16384 antennas); it cost
+    // mixed_clen64_fx2_t4_n128 75.0 -> 80.4, mixed_antpair_fx2_t1_n256 86.5 -> 89.2 and
+    // mixed_ffma_t4_n128 105 -> 117.
     static const FwdVariant v[] = {
         // default: 64-sample blocks as two second-order chains in z^2 (near the Horner
         // form's accuracy at close to the fastest form's speed)
         {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>()},
-        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), "mixed_clen_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
+        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2, 1>(), "mixed_clen_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
         {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed>(), "mixed_ffma2_fx_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed>()},
         // each block as two 16-step chains joined by z^16 (kFormMixedPairSplit)
         {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPairSplit, kAnchorFixed2>(), "mixed_split_fx2_t2_n128_s24", 1, pers_ptr<2, 128, kFormMixedPairSplit, kAnchorFixed2>(), 24 * 1024},
-        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPairSplit, kAnchorFixed2>(), "mixed_split_fx2_t2_n256", 1, pers_ptr<2, 256, kFormMixedPairSplit, kAnchorFixed2>()},
+        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPairSplit, kAnchorFixed2, 1>(), "mixed_split_fx2_t2_n256", 1, pers_ptr<2, 256, kFormMixedPairSplit, kAnchorFixed2>()},
         {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPairSplit, kAnchorFixed2>(), "mixed_split_fx2_t2_n128_s16", 1, pers_ptr<2, 128, kFormMixedPairSplit, kAnchorFixed2>(), 16 * 1024},
         // the cheaper prologue (kAnchorFixed2)
-        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), "mixed_ffma2_fx2_t2_n128_s24", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 24 * 1024},
-        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed2>(), "mixed_ffma2_fx2_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed2>()},
-        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed2>(), "mixed_ffma2_fx2_t2_n256_s24", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed2>(), 24 * 1024},
+        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2, 1>(), "mixed_ffma2_fx2_t2_n128_s24", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 24 * 1024},
+        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed2, 1>(), "mixed_ffma2_fx2_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed2>()},
+        {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed2, 1>(), "mixed_ffma2_fx2_t2_n256_s24", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed2>(), 24 * 1024},
         {1, 256, false, 8, fwd_ptr<1, 256, kFormMixedAntPair, kAnchorFixed2>(), "mixed_antpair_fx2_t1_n256", 2, pers_ptr<1, 256, kFormMixedAntPair, kAnchorFixed2>()},
         {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedAntPair, kAnchorFixed2>(), "mixed_antpair_fx2_t2_n256", 2, pers_ptr<2, 256, kFormMixedAntPair, kAnchorFixed2>()},
         // smaller stages: more resident CTAs (shared memory limits occupancy otherwise)
-        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), "mixed_ffma2_fx2_t2_n128_s16", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 16 * 1024},
-        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), "mixed_ffma2_fx2_t2_n128_s12", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 12 * 1024},
+        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2, 1>(), "mixed_ffma2_fx2_t2_n128_s16", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 16 * 1024},
+        {2, 128, false, 16, fwd_ptr<2, 128, kFormMixedPair, kAnchorFixed2, 1>(), "mixed_ffma2_fx2_t2_n128_s12", 1, pers_ptr<2, 128, kFormMixedPair, kAnchorFixed2>(), 12 * 1024},
         {1, 256, false, 8, fwd_ptr<1, 256, kFormMixedAntPair, kAnchorFixed2>(), "mixed_antpair_fx2_t1_n256_s24", 2, pers_ptr<1, 256, kFormMixedAntPair, kAnchorFixed2>(), 24 * 1024},
         {1, 128, false, 8, fwd_ptr<1, 128, kFormMixedAntPair, kAnchorFixed2>(), "mixed_antpair_fx2_t1_n128_s24", 2, pers_ptr<1, 128, kFormMixedAntPair, kAnchorFixed2>(), 24 * 1024},
         {1, 128, false, 8, fwd_ptr<1, 128, kFormMixedAntPair, kAnchorFixed2>(), "mixed_antpair_fx2_t1_n128_s16", 2, pers_ptr<1, 128, kFormMixedAntPair, kAnchorFixed2>(), 16 * 1024},
@@ -1079,14 +1087,14 @@ const FwdVariant *fwd_variants(int *count) {
         // second-order (Clenshaw) block sums over (re, im) samples, one FADD2 + FFMA2 per
         // sample and chain
         {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClen, kAnchorFixed2>(), "mixed_clen_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClen, kAnchorFixed2>()},
-        {2, 128, false, 8, fwd_ptr<2, 128, kFormMixedClen, kAnchorFixed2>(), "mixed_clen_fx2_t2_n128_s24", 0, pers_ptr<2, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
-        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), "mixed_clen_fx2_t4_n128", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>()},
+        {2, 128, false, 8, fwd_ptr<2, 128, kFormMixedClen, kAnchorFixed2, 1>(), "mixed_clen_fx2_t2_n128_s24", 0, pers_ptr<2, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
+        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2, 1>(), "mixed_clen_fx2_t4_n128", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>()},
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>(), "mixed_clen64_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>(), 24 * 1024},
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>(), "mixed_clen64_fx2_t4_n128", 0, pers_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>()},
-        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClen64, kAnchorFixed2>(), "mixed_clen64_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClen64, kAnchorFixed2>()},
+        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClen64, kAnchorFixed2, 1>(), "mixed_clen64_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClen64, kAnchorFixed2>()},
         // 64-sample blocks as two chains in z^2: closer to the Horner form's accuracy
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), "mixed_clen64eo_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), 24 * 1024},
-        {2, 256, true, 8, fwd_ptr<2, 256, kFormPlain>(), "plain_t2_n256", 0, nullptr},
+        {2, 256, true, 8, fwd_ptr<2, 256, kFormPlain, kAnchorPoly, 1>(), "plain_t2_n256", 0, nullptr},
         {2, 128, true, 8, fwd_ptr<2, 128, kFormPlain>(), "plain_t2_n128", 0, nullptr},
         {1, 128, true, 8, fwd_ptr<1, 128, kFormPlain>(), "plain_t1_n128", 0, nullptr},
     };
