@@ -846,10 +846,21 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
     float2 mom[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) mom[i] = make_float2(0.f, 0.f);
+    // The coordinates lead the FP64 chain and come from L2: a run ahead (64^3 voxels x 4096 antennas x
+    // 128 samples, forward and backward: 12.56 -> 12.36 ms).
+    const float4 *pxy = vx.xy + (size_t)tile * q.slots, *pz = vx.z + (size_t)tile * q.slots;
+    float4 nxy = make_float4(0.f, 0.f, 0.f, 0.f), nz = nxy;
+    if (lane < q.slots) {
+        nxy = __ldg(pxy + lane);
+        nz = __ldg(pz + lane);
+    }
 #pragma unroll 1
     for (int slot = lane; slot < q.slots; slot += 32) {
-        const size_t at = (size_t)tile * q.slots + slot;
-        const float4 xy = __ldg(vx.xy + at), z4 = __ldg(vx.z + at);
+        const float4 xy = nxy, z4 = nz;
+        if (slot + 32 < q.slots) {
+            nxy = __ldg(pxy + slot + 32);
+            nz = __ldg(pz + slot + 32);
+        }
         const float vz[kLocRun] = {z4.x, z4.y, z4.z, z4.w};
         double d[kLocRun];
         float rf[kLocRun], rb[kLocRun];
