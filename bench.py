@@ -385,7 +385,7 @@ def ours_arm(args):
                         "variant": ops.variants("plain")[ptuned["best"]]["name"]}
 
     if rank == 0 and world == 1 and args.nufft_steps > 0:
-        # the same sums by 8-tap interpolation from per-antenna oversampled grids (a type-2
+        # the same sums by polynomials per voxel box from per-antenna grids (a type-2
         # non-uniform FFT): not the mixed recurrence, so reported beside it, with its
         # distance from the mixed form's outputs on this workload
         img_m, vote_m, _, _ = step()

@@ -135,9 +135,9 @@ int mmn_backproject_backward(const mmn_problem *p, const float *grad_image,
 /*
  * How the backward evaluates the two per-(voxel, antenna) sample sums the position
  * gradient needs (no reference counterpart).  MMN_POS_INTERP (the default): interpolation
- * with an 8-cell exponential-of-semicircle kernel from each antenna's spectrum on a 2x
- * oversampled grid (a type-2 non-uniform FFT; ~1e-7 relative, the FP32 chains' level),
- * used when F <= ~1500; MMN_POS_HORNER: two FP32 Horner chains over all F samples, as the
+ * from each antenna's spectrum on a 2x oversampled grid (a type-2 non-uniform FFT, 8-cell
+ * exponential-of-semicircle kernel) at the nodes of a polynomial per voxel box (~1e-7
+ * relative, the FP32 chains' level), used when F <= ~1500; MMN_POS_HORNER: two FP32 Horner chains over all F samples, as the
  * forward evaluates its sum.  Process-wide; the measurement gradient is the same in both.
  */
 #define MMN_PASS_INTERP 0
@@ -147,9 +147,9 @@ int mmn_backproject_backward(const mmn_problem *p, const float *grad_image,
 int mmn_set_position_pass(int32_t form);
 /*
  * The same choice for the measurement gradient dL/dm[a,j] = sum_v G conj(p) (no reference
- * counterpart): MMN_PASS_INTERP (the default) spreads each voxel onto 8 cells of the
- * antenna's oversampled grid and transforms each grid back to the F samples (type-1
- * non-uniform FFT, deterministic warp reductions; F up to ~1500); MMN_PASS_HORNER sums
+ * counterpart): MMN_PASS_INTERP (the default) reduces each voxel box to its polynomial
+ * moments, spreads those onto the antenna's oversampled grid and transforms each grid back
+ * to the F samples (type-1 non-uniform FFT, fixed summation order; F up to ~1500); MMN_PASS_HORNER sums
  * over voxels for every sample.  Process-wide.
  */
 int mmn_set_measurement_pass(int32_t form);
@@ -164,9 +164,10 @@ int mmn_get_position_variant(void); /* the selected index */
  * Fused backprojection + vote with the per-(voxel, antenna) sample sum evaluated by
  * interpolation (no counterpart in the reference; not its "interpolated mode", which reads
  * one range bin): each antenna's samples go once onto a 2x oversampled grid, and each
- * (voxel, antenna) gathers 8 cells with exponential-of-semicircle weights -- a type-2
- * non-uniform FFT, O(8) per pair instead of O(F).  Same outputs and problem fields as
- * mmn_backproject in MMN_MODE_MIXED, ~1e-7 relative from it; F up to ~1500
+ * (voxel, antenna) evaluates a polynomial of 8-24 terms that its voxel box took from the
+ * grid (8 cells a node, exponential-of-semicircle weights) -- a type-2 non-uniform FFT whose
+ * cost per pair does not grow with F.  Same outputs and problem fields as
+ * mmn_backproject in MMN_MODE_MIXED, ~1e-7 relative from it; F up to ~3000
  * (MMN_ERR_TOO_LARGE above).  Needs mmn_backproject_nufft_workspace_bytes() of workspace.
  */
 size_t mmn_backproject_nufft_workspace_bytes(const mmn_problem *p);

@@ -918,7 +918,7 @@ extern "C" size_t mmn_backward_workspace_bytes(const mmn_problem *p) {
 }
 
 // ---------------------------------------------------------------------------------
-// Forward in interpolation form: the per-(voxel, antenna) sample sum by an 8-tap gather
+// Forward in interpolation form: the per-(voxel, antenna) sample sum by local polynomials
 // from each antenna's 2x oversampled grid (the position pass's machinery).
 // ---------------------------------------------------------------------------------
 namespace {

@@ -116,8 +116,9 @@ def backproject(x_locs, y_locs, z_locs, antenna_locs, rx_offsets, meas, waveleng
     not normalised) and ``vote`` complex64 [3, NX, NY, NZ] (or None).
     ``mode``: 'mixed' (FP64 range/wrap + FP32 recurrence), 'plain' (FP32 sincos per
     sample), 'interp' (reference interpolated mode; ``meas`` holds range-FFT bins) or
-    'nufft' (the mixed form's sum by an 8-tap gather from each antenna's 2x oversampled
-    grid, ~1e-7 from 'mixed', O(8) instead of O(F) per voxel and antenna; F <= ~1500).
+    'nufft' (the mixed form's sum by polynomials over voxel boxes, taken from each antenna's
+    2x oversampled grid; ~1e-7 from the exact sum, 8-24 terms instead of F per voxel and
+    antenna; F <= ~3000).
     """
     meas = _plain(meas)
     p = make_problem(x_locs, y_locs, z_locs, antenna_locs, rx_offsets, meas, wavelength,
@@ -244,7 +245,8 @@ POSITION_PASSES = {"interp": 0, "horner": 1}
 
 def set_position_pass(form):
     """How the backward evaluates the position gradient's per-(voxel, antenna) sample sums:
-    "interp" (default; interpolation from a 2x oversampled per-antenna spectrum, F <= ~1500)
+    "interp" (default; polynomials over voxel boxes from a 2x oversampled per-antenna
+    spectrum, F <= ~1500)
     or "horner" (two FP32 Horner chains over all samples).  Process-wide."""
     _lib.check(_lib.load().mmn_set_position_pass(POSITION_PASSES[form]), "mmn_set_position_pass")
 
@@ -260,8 +262,9 @@ def set_interp_fast_form(form):
 
 
 def set_measurement_pass(form):
-    """How the backward evaluates the measurement gradient: "interp" (default; spread onto
-    each antenna's 2x oversampled grid, then one transform per antenna; F <= ~1500) or
+    """How the backward evaluates the measurement gradient: "interp" (default; moments per
+    voxel box, spread onto each antenna's 2x oversampled grid, then one transform per
+    antenna; F <= ~1500) or
     "horner" (a sum over voxels for every sample).  Process-wide."""
     _lib.check(_lib.load().mmn_set_measurement_pass(POSITION_PASSES[form]),
                "mmn_set_measurement_pass")
