@@ -809,8 +809,10 @@ __device__ __noinline__ void spread_row(LocSpread &sp, float2 *row, int mrow, do
         }
         if (base + lane < mrow) row[base + lane] = __fadd2_rn(row[base + lane], s);
         pending &= ~mine;
+        // the next window, 25 cells on or less where the row wraps, reads cells that other lanes
+        // wrote here (the ballot orders no memory); it also frees the scratch for the next call
+        __syncwarp();
     }
-    __syncwarp();
 }
 
 // Transposed warp sum of N (a power of two) values: out[i] = sum over lanes of v[i].

@@ -1,0 +1,41 @@
+"""The tile-local kernels of the interpolation form at the limits of their approximations, against
+the FP64 oracle: short antenna grids (32 to 64 cells) on which a box's cells wrap past the row's
+end, with boxes narrow enough for the nodes and too wide for them.
+
+Tolerance 2e-6 relative L2, as for these kernels at ordinary sizes (test_local_polynomials_gpu)."""
+import numpy as np
+import pytest
+
+from test_local_polynomials_gpu import TOL, _scene
+from test_forward_gpu import _t
+
+pytestmark = pytest.mark.gpu
+
+
+def _gradients(dev, oracle, sc, rxo, ti, seed):
+    """(measurement, position) gradients twice, and the oracle's."""
+    from mmnorm_b200 import ops
+    rng = np.random.default_rng(seed)
+    V = sc.num_voxels
+    gI = (rng.standard_normal(V) + 1j * rng.standard_normal(V)).astype(np.complex64)
+    gW = (rng.standard_normal((3, V)) + 1j * rng.standard_normal((3, V))).astype(np.complex64)
+    args = [_t(a, dev) for a in (sc.x_locs, sc.y_locs, sc.z_locs, sc.antenna_locs, rxo, sc.meas)]
+    runs = [[g.cpu().numpy() for g in ops.backproject_backward(
+        *args, sc.wavelength, sc.slope, _t(gI, dev), _t(gW, dev), is_ti_radar=ti)]
+        for _ in range(2)]
+    ref = oracle.full_backward(sc.voxel_centres(), sc.antenna_locs, rxo, sc.meas, sc.wavelength,
+                               sc.slope, gI.astype(np.complex128), gW.T.astype(np.complex128),
+                               is_ti=ti)
+    return runs, ref
+
+
+@pytest.mark.parametrize("nf", [16, 21, 32])
+@pytest.mark.parametrize("shape,spacing", [((9, 8, 7), 0.004), ((10, 9, 10), 0.012),
+                                           ((8, 9, 8), 0.05), ((3, 2, 13), 0.11)])
+def test_short_grids_that_wrap(cuda_dev, oracle, nf, shape, spacing):
+    sc = _scene(shape, 37, nf, spacing, 300 + nf)
+    # the grid's period of c / slope ends inside the scene (round-trip ranges near 1.2 m)
+    sc.f_hi = sc.f_lo + (nf - 1) * 2.99792458e8 / 1.2
+    runs, (gm_o, _) = _gradients(cuda_dev, oracle, sc, np.zeros((1, 3), np.float32), False, nf)
+    assert np.array_equal(runs[0][0], runs[1][0])
+    assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < TOL
