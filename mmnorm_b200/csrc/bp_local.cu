@@ -530,6 +530,13 @@ __device__ __noinline__ float4 tap_run_d(const float2 *row, double d, double uq,
     return make_float4(h.x, h.y, g.x * s, g.y * s);
 }
 
+// The anchors of two pairs from FP64 phases (wide boxes and ranges beyond the fixed-point turns):
+// (cos, cos, sin, sin)
+__device__ __noinline__ float4 cis_wide_pair(double d0, double d1, double k0c) {
+    const float2 a = cis_fp64_phase(-d0 * k0c), b = cis_fp64_phase(-d1 * k0c);
+    return make_float4(a.x, b.x, a.y, b.y);
+}
+
 // Sums of v0, v1, v2 over the warp: in lanes 0-7, 8-15 and 16-23.
 __device__ __forceinline__ float warp_sum3(float v0, float v1, float v2) {
     const int lane = threadIdx.x & 31;
@@ -586,8 +593,14 @@ __device__ __forceinline__ void local_position(const LocalParams &q, const LocSh
 #pragma unroll
         for (int k = 0; k < kLocRun; k += 2) {
             float2 ac, as;
-            cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
-                          __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), ac, as);
+            if (a.nn > 0) {
+                cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
+                              __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), ac, as);
+            } else {  // the fixed-point turns may not hold the anchor's (local_chunk)
+                const float4 w = cis_wide_pair(d[k], d[k + 1], q.k0c);
+                ac = make_float2(w.x, w.y);
+                as = make_float2(w.z, w.w);
+            }
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
                 const int j = k + l;

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from test_local_polynomials_gpu import TOL, _scene
-from test_forward_gpu import _t
+from test_forward_gpu import _t, run_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,22 @@ def test_short_grids_that_wrap(cuda_dev, oracle, nf, shape, spacing):
     runs, (gm_o, _) = _gradients(cuda_dev, oracle, sc, np.zeros((1, 3), np.float32), False, nf)
     assert np.array_equal(runs[0][0], runs[1][0])
     assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < TOL
+
+
+@pytest.mark.parametrize("wavelength", [2.1e-6, 0.9e-6])
+@pytest.mark.parametrize("rx", [1, 3])
+def test_anchors_beyond_the_fixed_point_range(cuda_dev, oracle, wavelength, rx):
+    """Ranges of 5.7e5 and 1.3e6 wavelengths, past the 2^18 turns that the 2^-32-turn anchors
+    hold.  The ranges' FP64 Newton step (1.5e-13 relative) is up to 1.3e-6 rad of anchor phase
+    here: 3e-6 for the sums and, with the 1e-5 of the position gradient's FP32 directions, 1.2e-5
+    for that."""
+    sc = _scene((6, 7, 9), 35, 40, 0.004, 400)
+    sc.f_lo, sc.f_hi = 2.99792458e8 / wavelength, 2.99792458e8 / wavelength + 4e9
+    rxo = np.array([[0, 0, 0], [0.004, -0.01, 0], [0.02, 0.003, 0.001]], np.float32)[-rx:]
+    I, W = run_ops(cuda_dev, sc, "nufft", rxo=rxo, ti=rx == 3)
+    Io, Wo = oracle.full(sc.voxel_centres(), sc.antenna_locs, rxo, sc.meas, sc.wavelength,
+                         sc.slope, is_ti=rx == 3)
+    assert oracle.rel_l2(I, Io) < 3e-6 and oracle.rel_l2(W, Wo) < 3e-6
+    runs, (gm_o, gp_o) = _gradients(cuda_dev, oracle, sc, rxo, rx == 3, rx)
+    assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < 3e-6
+    assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1.2e-5
