@@ -374,7 +374,8 @@ __global__ void __launch_bounds__(256) iso_defined_kernel(const IsoParams p) {
 // turns into -- lands inside the box, and both points lie on that line.  The slab test's FP32
 // rounding (about 1e-6 of the distance) is far inside the margin; NaN rejects nothing.  (A first
 // step shorter than a voxel, the sentinel's among them, is a hit at the eye itself: it counts only
-// if the eye's cell is in the grid, so an eye within two voxels of the box keeps every ray.)
+// if the eye's cell is in the grid, so an eye within two voxels of the box, or of the grid's cells
+// where these reach past it, keeps every ray.)
 __device__ __forceinline__ bool line_misses(const float (&lo)[3], const float (&hi)[3],
                                             const RayBasis &b, float margin, float ex, float ey,
                                             float ez, float vx, float vy) {
@@ -450,18 +451,23 @@ __global__ void __launch_bounds__(kIsoThreads, 5) iso_channel_kernel(const IsoPa
         2e-5f + 1e-4f * (fmaxf(fabsf(p.bb_min_x - eye_x), fabsf(p.bb_max_x - eye_x)) +
                          fmaxf(fabsf(p.bb_min_y - eye_y), fabsf(p.bb_max_y - eye_y)) +
                          fmaxf(fabsf(p.bb_min_z - eye_z), fabsf(p.bb_max_z - eye_z)));
-    const float skin = 2.f * fmaxf(p.voxel_size_ref, (p.bb_max_y - p.bb_min_y) / (p.res_y - 1));
-    const bool beside = !(eye_x < p.bb_min_x - skin || eye_x > p.bb_max_x + skin ||
-                          eye_y < p.bb_min_y - skin || eye_y > p.bb_max_y + skin ||
-                          eye_z < p.bb_min_z - skin || eye_z > p.bb_max_z + skin);
+    const float vs = (p.bb_max_y - p.bb_min_y) / (p.res_y - 1);
+    const float skin = 2.f * fmaxf(p.voxel_size_ref, vs);
+    // a cell is vs wide on every axis, whatever the box's own spacing there
+    const bool beside =
+        !(eye_x < p.bb_min_x - skin || eye_x > fmaxf(p.bb_max_x, p.bb_min_x + p.res_x * vs) + skin ||
+          eye_y < p.bb_min_y - skin || eye_y > fmaxf(p.bb_max_y, p.bb_min_y + p.res_y * vs) + skin ||
+          eye_z < p.bb_min_z - skin || eye_z > fmaxf(p.bb_max_z, p.bb_min_z + p.res_z * vs) + skin);
     // the box that rays have to reach: the whole grid's, or, where it is known and every undefined
     // cell is one to the march too (its step longer than a voxel, tau within the bounds' slack),
-    // the defined voxels'
+    // the defined voxels'.  Past its last layer of voxels a box has cells whose corners are the
+    // next row's voxels: no narrowing then (a hundredth of a cell is rounding: added below).
     float box_lo[3] = {p.bb_min_x, p.bb_min_y, p.bb_min_z};
     float box_hi[3] = {p.bb_max_x, p.bb_max_y, p.bb_max_z};
     {
-        const float vs = (p.bb_max_y - p.bb_min_y) / (p.res_y - 1);
-        bool narrow = p.defined != nullptr && vs <= kMinStep;
+        bool narrow = p.defined != nullptr && vs <= kMinStep &&
+                      p.bb_max_x - p.bb_min_x <= (p.res_x - 0.99f) * vs &&
+                      p.bb_max_z - p.bb_min_z <= (p.res_z - 0.99f) * vs;
         for (int c = 0; c < p.num_comp; ++c)
             narrow = narrow && p.taus[(int64_t)t * p.num_comp + c] > -4.9f;
         if (narrow) {
@@ -470,7 +476,7 @@ __global__ void __launch_bounds__(kIsoThreads, 5) iso_channel_kernel(const IsoPa
             for (int k = 0; k < 3; ++k) {
                 const float low = box_lo[k];
                 box_lo[k] = low + (res[k] - p.defined[3 + k]) * vs;
-                box_hi[k] = low + (p.defined[k] - 1) * vs;
+                box_hi[k] = low + (p.defined[k] - 0.99f) * vs;
             }
         }
     }
