@@ -122,11 +122,11 @@ __device__ __forceinline__ LocSlot local_slot(const LocalParams &q, int tile, in
     return o;
 }
 
-// Table cos(pi m / (2 NN)), m < 4 NN, and the nodes cos(pi (i + 1/2) / NN) in FP64.
-__device__ __forceinline__ void cheb_tables(int nn, float *table, double *node) {
+// Table cos(pi m / (2 NN)), m < 4 NN, and the nodes cos(pi (i + 1/2) / NN).
+__device__ __forceinline__ void cheb_tables(int nn, double *table, double *node) {
     for (int m = threadIdx.x; m < 4 * nn; m += blockDim.x) {
         const double c = cospi((double)m / (2 * nn));
-        table[m] = (float)c;
+        table[m] = c;
         if ((m & 1) && m < 2 * nn) node[m >> 1] = c;
     }
 }
@@ -200,7 +200,22 @@ __device__ __forceinline__ void eval_mono_d(const float2 *cf, const float (&x)[k
     }
 }
 
-// M at one range by a tap run from the antenna's row in global memory.
+// M at one node by a tap run from the antenna's row in global memory, in FP64.
+__device__ __forceinline__ double2 tap_run64(const float2 *row, double d, double uq, int n) {
+    int ix;
+    double w[kNuW];
+    nufft_taps64(d, uq, n, ix, w);
+    double2 h = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < kNuW; ++i) {
+        const float2 g = __ldg(row + ix + i);
+        h.x = fma(w[i], (double)g.x, h.x);
+        h.y = fma(w[i], (double)g.y, h.y);
+    }
+    return h;
+}
+
+// M at one range by a tap run.
 __device__ __forceinline__ float2 tap_run(const float2 *row, double d, double uq, int n) {
     int ix;
     float w[kNuW];
@@ -270,18 +285,24 @@ __device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
 // Shared memory of one CTA.
 struct __align__(16) LocShared {
     LocRec rec[kLocAnts];
-    float2 coef[kLocAnts][kLocNodes];
-    float2 node_val[kLocAnts][kLocNodes];
+    double2 node_val[kLocAnts][kLocNodes];
+    float2 coef[kLocAnts][kLocNodes];   // monomials, or Chebyshev coefficients
+    float2 deriv[kLocAnts][kLocNodes];  // Chebyshev coefficients of the derivative
     double centre[kLocAnts], half[kLocAnts];
     double node[kLocNodes];
-    float table[4 * kLocNodes];
+    double table[4 * kLocNodes];
+    double basis[kLocHorner * kLocHorner];  // monomials from node values
     int nn;
 };
 
 // Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the chunk's node count (0: every
 // antenna takes tap runs).  Called by all threads; barriers inside.
-// With DERIV and more than kLocHorner nodes, node_val receives the Chebyshev coefficients of
-// the derivative.
+// Node values and coefficients are formed in FP64: their rounding is shared by all voxels of a
+// box, and in FP32 it put the sums of 256 antennas 2.06e-7 from 64 bits (position gradient
+// 2.27e-7), where tap runs per pair were 1.75e-7 (2.05e-7) and this is 1.78e-7 (1.98e-7).  The
+// products with one basis matrix in place of two transforms pay for it: 96^3 x 4096 x 200 went
+// from 9.17 to 9.02 ms.
+// With DERIV and more than kLocHorner nodes, the derivative's coefficients too.
 template <bool DERIV>
 __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, int a0, int na,
                                            const float (&lo)[3], const float (&hi)[3],
@@ -324,43 +345,60 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
         cheb_tables(nn, sh.table, sh.node);
         table_nn = nn;
         __syncthreads();
+        if (nn <= kLocHorner) {
+            // monomial c of the interpolant: sum_j basis[c][j] M_j
+            for (int i = threadIdx.x; i < nn * nn; i += kLocThreads) {
+                const int c = i / nn, j = i - c * nn;
+                double s = 0.0;
+                for (int m = c; m < nn; m += 2)
+                    s = fma((double)kChebMono[m][c] * (m == 0 ? 1.0 : 2.0),
+                            sh.table[m * (2 * j + 1) % (4 * nn)], s);
+                sh.basis[i] = s / nn;
+            }
+            __syncthreads();
+        }
     }
     for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
         const int la = i / nn, j = i - la * nn;
         const LocRec &r = sh.rec[la];
         if (r.nn == 0) continue;
         const double d = fma(sh.node[j], sh.half[la], sh.centre[la]);
-        sh.node_val[la][j] = tap_run(q.rows + (size_t)(a0 + la) * q.row, d, q.uq, q.n);
-    }
-    __syncthreads();
-    // Chebyshev coefficients c_p = (2 - [p = 0]) / NN sum_j M_j cos(pi p (2 j + 1) / (2 NN))
-    for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
-        const int la = i / nn, c = i - la * nn;
-        float2 s = make_float2(0.f, 0.f);
-        int m = c;
-        for (int j = 0; j < nn; ++j) {
-            const float t = sh.table[m];
-            s = __ffma2_rn(make_float2(t, t), sh.node_val[la][j], s);
-            m += 2 * c;
-            if (m >= 4 * nn) m -= 4 * nn;
-        }
-        const float sc = (c == 0 ? 1.f : 2.f) / (float)nn;
-        sh.coef[la][c] = make_float2(s.x * sc, s.y * sc);
+        sh.node_val[la][j] = tap_run64(q.rows + (size_t)(a0 + la) * q.row, d, q.uq, q.n);
     }
     __syncthreads();
     if (nn <= kLocHorner) {
-        // monomials, through the node array (its values are used up)
         for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
             const int la = i / nn, c = i - la * nn;
-            float2 s = make_float2(0.f, 0.f);
-            for (int m = c; m < nn; m += 2) {
-                const float t = kChebMono[m][c];
-                s = __ffma2_rn(make_float2(t, t), sh.coef[la][m], s);
+            const double *b = sh.basis + c * nn;
+            double2 s = make_double2(0.0, 0.0);
+            for (int j = 0; j < nn; ++j) {
+                const double2 v = sh.node_val[la][j];
+                s.x = fma(b[j], v.x, s.x);
+                s.y = fma(b[j], v.y, s.y);
             }
-            sh.node_val[la][c] = s;
+            sh.coef[la][c] = make_float2((float)s.x, (float)s.y);
         }
         __syncthreads();
-    } else if (DERIV) {
+        return nn;
+    }
+    // Chebyshev coefficients c_p = (2 - [p = 0]) / NN sum_j M_j cos(pi p (2 j + 1) / (2 NN))
+    for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
+        const int la = i / nn, c = i - la * nn;
+        double2 s = make_double2(0.0, 0.0);
+        int m = c;
+        for (int j = 0; j < nn; ++j) {
+            const double t = sh.table[m];
+            const double2 v = sh.node_val[la][j];
+            s.x = fma(t, v.x, s.x);
+            s.y = fma(t, v.y, s.y);
+            m += 2 * c;
+            if (m >= 4 * nn) m -= 4 * nn;
+        }
+        const double sc = (c == 0 ? 1.0 : 2.0) / nn;
+        sh.coef[la][c] = make_float2((float)(s.x * sc), (float)(s.y * sc));
+    }
+    __syncthreads();
+    if (DERIV) {
         // d_p = (2 - [p = 0]) sum_{m > p, m - p odd} m c_m
         for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
             const int la = i / nn, c = i - la * nn;
@@ -368,7 +406,7 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
             for (int m = c + 1; m < nn; m += 2)
                 s = __ffma2_rn(make_float2((float)m, (float)m), sh.coef[la][m], s);
             const float f = c == 0 ? 1.f : 2.f;
-            sh.node_val[la][c] = make_float2(f * s.x, f * s.y);
+            sh.deriv[la][c] = make_float2(f * s.x, f * s.y);
         }
         __syncthreads();
     }
@@ -394,7 +432,7 @@ __device__ __forceinline__ void local_forward(const LocalParams &q, const LocSha
 #pragma unroll
             for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
             if (NN > 0)
-                eval_mono<(NN > 0 ? NN : 8)>(sh.node_val[la], x, h);
+                eval_mono<(NN > 0 ? NN : 8)>(sh.coef[la], x, h);
             else
                 eval_cheb(sh.coef[la], nn, x, h);
             // times the anchor e^{-2 pi i d t0c}: wrapped turns in 2^-32 steps
@@ -569,10 +607,10 @@ __device__ __forceinline__ void local_position(const LocalParams &q, const LocSh
 #pragma unroll
             for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
             if (NN > 0) {
-                eval_mono_d<(NN > 0 ? NN : 8)>(sh.node_val[la], x, h, g);
+                eval_mono_d<(NN > 0 ? NN : 8)>(sh.coef[la], x, h, g);
             } else {
                 eval_cheb(sh.coef[la], nn, x, h);
-                eval_cheb(sh.node_val[la], nn, x, g);
+                eval_cheb(sh.deriv[la], nn, x, g);
             }
             const float inv = (float)a.inv;
 #pragma unroll
@@ -973,7 +1011,7 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
     __shared__ LocRec s_rec[kLocMeasWarps];
     __shared__ LocSpread s_spread[kLocMeasWarps];
     __shared__ double s_node[kNodeTotal];
-    __shared__ float s_table[4 * kNodeTotal];
+    __shared__ double s_table[4 * kNodeTotal];
     const FwdParams &p = q.f;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = (p.num_ant + kLocMeasWarps - 1) / kLocMeasWarps;
@@ -1027,12 +1065,12 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
         if (nn > 0) {
             // node values: sum_q (2 - [q = 0]) / NN cos(pi q (2 i + 1) / (2 NN)) moment_q
             const int no = node_offset(nn), i = min(lane, nn - 1);
-            const float *table = s_table + 4 * no;
+            const double *table = s_table + 4 * no;
             const float2 *mom = reinterpret_cast<const float2 *>(sp.mom);
             float2 s = make_float2(0.5f * mom[0].x, 0.5f * mom[0].y);
             int m = 2 * i + 1;
             for (int k = 1; k < nn; ++k) {
-                const float w = table[m];
+                const float w = (float)table[m];
                 s = __ffma2_rn(make_float2(w, w), mom[k], s);
                 m += 2 * i + 1;
                 if (m >= 4 * nn) m -= 4 * nn;

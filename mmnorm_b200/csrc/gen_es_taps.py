@@ -9,7 +9,8 @@ t = s - 1/2, tap i is P_i(t) = phi(t + W/2 - 1/2 - i) and, phi being even, tap W
 P_i(-t).  So only P_0..P_3 are fitted (degree 8, least squares on 4001 points of
 [-1/2, 1/2]) and stored as even and odd parts:  P_i(t) = E_i(t^2) + t O_i(t^2), which gives
 both taps of a mirror pair from one E and one O.  Fit error below 2e-8 (phi(0) = 1); the
-FP32 evaluation's rounding is about 1e-7.  Run:  python mmnorm_b200/csrc/gen_es_taps.py
+FP32 evaluation's rounding is about 1e-7.  The same coefficients in FP64 follow (kEsEven64,
+kEsOdd64), for the few tap runs whose values many voxels share.  Run:  python mmnorm_b200/csrc/gen_es_taps.py
 """
 import os
 
@@ -26,7 +27,7 @@ def es(z):
     return np.where(q > 0, np.exp(BETA * (np.sqrt(np.clip(q, 0.0, None)) - 1.0)), 0.0)
 
 
-def fit():
+def fit64():
     t = np.linspace(-0.5, 0.5, 4001)
     even, odd, worst = [], [], 0.0
     for i in range(W // 2):
@@ -37,9 +38,14 @@ def fit():
             y = es(sign * t + W / 2 - 0.5 - i) if sign > 0 else es(t + W / 2 - 0.5 - tap)
             worst = max(worst, float(np.abs(np.polynomial.polynomial.polyval(sign * t, c)
                                             - y).max()))
-        even.append(c[0::2].astype(np.float32))
-        odd.append(c[1::2].astype(np.float32))
+        even.append(c[0::2])
+        odd.append(c[1::2])
     return even, odd, worst
+
+
+def fit():
+    even, odd, worst = fit64()
+    return [c.astype(np.float32) for c in even], [c.astype(np.float32) for c in odd], worst
 
 
 def main():
@@ -61,6 +67,11 @@ def main():
     lines += ["    {" + ", ".join("%.9ef" % float(v) for v in c) + "}," for c in even]
     lines += ["};", "__constant__ float kEsOdd[%d][%d] = {" % (W // 2, no)]
     lines += ["    {" + ", ".join("%.9ef" % float(v) for v in c) + "}," for c in odd]
+    even, odd, _ = fit64()
+    lines += ["};", "__constant__ double kEsEven64[%d][%d] = {" % (W // 2, ne)]
+    lines += ["    {" + ", ".join("%.16e" % v for v in c) + "}," for c in even]
+    lines += ["};", "__constant__ double kEsOdd64[%d][%d] = {" % (W // 2, no)]
+    lines += ["    {" + ", ".join("%.16e" % v for v in c) + "}," for c in odd]
     lines += ["};", "", "}  // namespace mmn", ""]
     with open(out, "w") as f:
         f.write("\n".join(lines))

@@ -6,13 +6,11 @@
 
 namespace mmn {
 
-// First grid cell and the 8 tap weights of N * (u mod 1), u = d slope/c: the cell and the
-// fractional offset by the 1.5*2^52 rounding constant (no conversion instructions), clamped
-// so that a NaN or a fraction that rounds up to 1 still reads inside the row; the weights
-// from es_taps.cuh, P_i(t) and P_i(-t) from one even and one odd part.
-// offset: if not null, receives the fractional offset less 1/2.
-__device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell,
-                                           float (&w)[kNuW], float *offset = nullptr) {
+// First grid cell of N * (u mod 1), u = d slope/c, and the fractional offset less 1/2: both by
+// the 1.5*2^52 rounding constant (no conversion instructions), clamped so that a NaN or a
+// fraction that rounds up to 1 still reads inside the row.  T: the offset's type.
+template <class T>
+__device__ __forceinline__ void nufft_cell(double d, double uq, int n, int &cell, T &offset) {
     const double kRound = 6755399441055744.0;  // 1.5 * 2^52
     const double u = d * uq;
     double uf = u - ((u + kRound) - kRound);  // [-1/2, 1/2]
@@ -23,13 +21,19 @@ __device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell
     double fr = x - (xt - kRound);             // [-1/2, 1/2]
     ix = fr < 0.0 ? ix - 1 : ix;
     fr = fr < 0.0 ? fr + 1.0 : fr;
-    float sfr = (float)fr;
     const bool lo = !(ix >= 0), hi = ix >= n;
-    ix = lo ? 0 : (hi ? n - 1 : ix);
-    sfr = lo ? 0.f : (hi ? 1.f : sfr);
-    cell = ix;
+    cell = lo ? 0 : (hi ? n - 1 : ix);
+    offset = lo ? (T)-0.5 : (hi ? (T)0.5 : (T)(fr - 0.5));
+}
 
-    const float t = sfr - 0.5f, t2 = t * t;
+// First grid cell and the 8 tap weights: the weights from es_taps.cuh, P_i(t) and P_i(-t) from
+// one even and one odd part.
+// offset: if not null, receives the fractional offset less 1/2.
+__device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell,
+                                           float (&w)[kNuW], float *offset = nullptr) {
+    float t;
+    nufft_cell(d, uq, n, cell, t);
+    const float t2 = t * t;
     if (offset) *offset = t;
 #pragma unroll
     for (int i = 0; i < kNuW / 2; ++i) {
@@ -41,6 +45,25 @@ __device__ __forceinline__ void nufft_taps(double d, double uq, int n, int &cell
         for (int q = kEsOddTerms - 2; q >= 0; --q) od = fmaf(od, t2, kEsOdd[i][q]);
         w[i] = fmaf(t, od, e);
         w[kNuW - 1 - i] = fmaf(-t, od, e);
+    }
+}
+
+// The same weights in FP64.
+__device__ __forceinline__ void nufft_taps64(double d, double uq, int n, int &cell,
+                                             double (&w)[kNuW]) {
+    double t;
+    nufft_cell(d, uq, n, cell, t);
+    const double t2 = t * t;
+#pragma unroll
+    for (int i = 0; i < kNuW / 2; ++i) {
+        double e = kEsEven64[i][kEsEvenTerms - 1];
+#pragma unroll
+        for (int q = kEsEvenTerms - 2; q >= 0; --q) e = fma(e, t2, kEsEven64[i][q]);
+        double od = kEsOdd64[i][kEsOddTerms - 1];
+#pragma unroll
+        for (int q = kEsOddTerms - 2; q >= 0; --q) od = fma(od, t2, kEsOdd64[i][q]);
+        w[i] = fma(t, od, e);
+        w[kNuW - 1 - i] = fma(-t, od, e);
     }
 }
 
