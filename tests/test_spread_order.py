@@ -75,6 +75,10 @@ static void nufft_taps(double, double, int, int &cell, float (&w)[kNuW]) {
     cell = g_cell[threadIdx.x];
     for (int i = 0; i < kNuW; ++i) w[i] = 1.f + i;
 }
+static void nufft_taps64(double, double, int, int &cell, double (&w)[kNuW]) {
+    cell = g_cell[threadIdx.x];
+    for (int i = 0; i < kNuW; ++i) w[i] = 1.0 + i;
+}
 #define __device__
 #define __noinline__
 #define __forceinline__
@@ -91,7 +95,10 @@ extern "C" int spread(const int *cells, const int *active, int calls, int mrow, 
         for (int l = 0; l < 32; ++l)
             t.emplace_back([&, l, c] {
                 threadIdx.x = l; t_epoch = 1000 * c;
-                spread_row(sh.sp, sh.row, mrow, 0.0, make_float2(1.f + l, -2.f * l), active[32 * c + l] != 0, 0.0, 0);
+                const float2 v = make_float2(1.f + l, -2.f * l);
+                const bool on = active[32 * c + l] != 0;
+                if (c & 1) spread_row<false>(sh.sp, sh.row, mrow, 0.0, v, on, 0.0, 0);
+                else spread_row<true>(sh.sp, sh.row, mrow, 0.0, v, on, 0.0, 0);
             });
         for (auto &x : t) x.join();
     }
@@ -105,7 +112,7 @@ extern "C" int spread(const int *cells, const int *active, int calls, int mrow, 
 def lib(tmp_path_factory):
     with open(SOURCE) as f:
         text = f.read()
-    body = re.search(r"__device__ [^\n]*void spread_row\(.*?\n}\n", text, re.S)
+    body = re.search(r"template [^\n]*\n__device__ [^\n]*void spread_row\(.*?\n}\n", text, re.S)
     assert body, "spread_row not found"
     d = tmp_path_factory.mktemp("spread")
     src, out = str(d / "spread.cpp"), str(d / "spread.so")
