@@ -46,6 +46,8 @@
 // thread with bulk TMA copies (cp.async.bulk) completing on an mbarrier.  With one
 // split per tile the CTA writes the final image/vote; otherwise it writes an 8-float
 // partial per voxel that bp_reduce_partials sums in split order (deterministic).
+#include <type_traits>
+
 #include "bp_stage.cuh"
 
 namespace mmn {
@@ -64,6 +66,7 @@ constexpr int kFormMixedClen = 5;
 constexpr int kFormMixedClen64 = 6;  // the same with 64-sample blocks
 // 64-sample blocks as two interleaved second-order chains in z^2 (clen_block_eo)
 constexpr int kFormMixedClenEO = 7;
+constexpr int kFormMixedClenEOWide = 8;  // the same with 64-bit block phases (wide_steps)
 // The second-order form is used for a warp's (voxels, antenna) pairs when every lane's
 // per-sample rotation z = e^{-i theta} has |cos theta| <= kClenMaxCos (theta in
 // [0.2, pi - 0.2]); otherwise that antenna's blocks run the first-order Horner form.
@@ -667,18 +670,22 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                                     sr, si);
                     anchor(sr, si, 0);
                 }
-            } else if constexpr (FORM == kFormMixedClenEO) {
+            } else if constexpr (FORM == kFormMixedClenEO || FORM == kFormMixedClenEOWide) {
                 // 64-sample blocks, each as even and odd chains in w = z^2 (clen_block_eo),
                 // used for a warp's antenna when every lane has |cos 2 phi| <= kClenMaxCos,
                 // otherwise first-order Horner; a row's last partial block by the same chains
                 // at its own length.  Start phase, block step and rotation are 2^-32-turn
                 // integers of one FP64 FMA each: the step's rounding (2^-33 turns) is 7e-10
-                // rad a block.
+                // rad a block.  w's angle is twice z's integer: w = z^2, as the chains need it,
+                // within 2^-32 turns.  Wide: the step with 32 bits more and any range that the
+                // rotation has, every block's phase one exact modular addition.
+                constexpr bool kWide = FORM == kFormMixedClenEOWide;
+                using Phase = std::conditional_t<kWide, unsigned long long, uint32_t>;
                 static_assert(T % 2 == 0, "the second-order form takes voxels in pairs");
                 const int ns = p.nsmp > 0 ? min(p.nsmp, fp) : fp;
                 const int nblk_c = ns / 64;
                 const float4 *m4 = reinterpret_cast<const float4 *>(mstage) + (size_t)a * (fp / 2);
-                int32_t ph[T], stp[T];
+                Phase ph[T], stp[T];
                 float zr[T], zi[T], wr[T], wi[T];
                 bool eo = true;
                 {
@@ -688,8 +695,13 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
                         const double d = range_fp64_newton((double)vx[k], (double)vy[k],
                                                            (double)vz[k], ar, mono, p.ti);
                         za[k] = turns_fixed32(d, p.fx_smp);
-                        stp[k] = turns_fixed32(d, p.fx_blk);
-                        ph[k] = turns_fixed32(d, p.fx_t0);
+                        ph[k] = (uint32_t)turns_fixed32(d, p.fx_t0);
+                        if constexpr (kWide) {
+                            ph[k] <<= 32;
+                            stp[k] = turns_fixed64(-d * p.tsmp) << 6;
+                        } else {
+                            stp[k] = (uint32_t)turns_fixed32(d, p.fx_blk);
+                        }
                         cr[k] = ci[k] = 0.f;
                     }
 #pragma unroll
@@ -716,8 +728,9 @@ __device__ __forceinline__ int fwd_item(const FwdParams &p, int tile, int split,
 #pragma unroll
                     for (int k = 0; k < T; ++k) {
                         float anr, ani;
-                        __sincosf((float)ph[k] * 1.46291807926715968e-9f, &ani, &anr);  // 2 pi / 2^32
-                        ph[k] = (int32_t)((uint32_t)ph[k] + (uint32_t)stp[k]);
+                        const int32_t top = (int32_t)(kWide ? ph[k] >> (kWide ? 32 : 0) : ph[k]);
+                        __sincosf((float)top * 1.46291807926715968e-9f, &ani, &anr);  // 2 pi / 2^32
+                        ph[k] += stp[k];
                         cr[k] = fmaf(anr, sr[k], fmaf(-ani, si[k], cr[k]));
                         ci[k] = fmaf(anr, si[k], fmaf(ani, sr[k], ci[k]));
                     }
@@ -1047,7 +1060,7 @@ const FwdVariant *fwd_variants(int *count) {
     static const FwdVariant v[] = {
         // default: 64-sample blocks as two second-order chains in z^2 (near the Horner
         // form's accuracy at close to the fastest form's speed)
-        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>()},
+        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), 0, fwd_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2, 2>(), pers_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2, 2>()},
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2, 1>(), "mixed_clen_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
         {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed>(), "mixed_ffma2_fx_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed>()},
         // each block as two 16-step chains joined by z^16 (kFormMixedPairSplit)
@@ -1093,7 +1106,7 @@ const FwdVariant *fwd_variants(int *count) {
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>(), "mixed_clen64_fx2_t4_n128", 0, pers_ptr<4, 128, kFormMixedClen64, kAnchorFixed2>()},
         {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClen64, kAnchorFixed2, 1>(), "mixed_clen64_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClen64, kAnchorFixed2>()},
         // 64-sample blocks as two chains in z^2: closer to the Horner form's accuracy
-        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), "mixed_clen64eo_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), 24 * 1024},
+        {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), "mixed_clen64eo_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClenEO, kAnchorFixed2>(), 24 * 1024, fwd_ptr<4, 128, kFormMixedClenEOWide, kAnchorFixed2>(), pers_ptr<4, 128, kFormMixedClenEOWide, kAnchorFixed2>()},
         {2, 256, true, 8, fwd_ptr<2, 256, kFormPlain, kAnchorPoly, 1>(), "plain_t2_n256", 0, nullptr},
         {2, 128, true, 8, fwd_ptr<2, 128, kFormPlain>(), "plain_t2_n128", 0, nullptr},
         {1, 128, true, 8, fwd_ptr<1, 128, kFormPlain>(), "plain_t1_n128", 0, nullptr},
@@ -1102,11 +1115,11 @@ const FwdVariant *fwd_variants(int *count) {
     return v;
 }
 
-cudaError_t launch_fwd(const FwdVariant &var, const FwdParams &p, size_t smem,
+cudaError_t launch_fwd(const FwdVariant &var, const void *fn, const FwdParams &p, size_t smem,
                        cudaStream_t stream) {
     void *args[] = {const_cast<FwdParams *>(&p)};
     const int grid = p.num_tiles * p.num_splits;
-    return cudaLaunchKernel(var.fn, dim3(grid), dim3(var.nt), args, smem, stream);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(var.nt), args, smem, stream);
 }
 
 cudaError_t launch_reduce(const FwdParams &p, cudaStream_t stream) {

@@ -48,6 +48,7 @@ struct FwdVariant {
     int layout; // staged sample layout (stage_meas): 0 (re,im), 1 (re,re,im,im), 2 antenna pairs
     const void *persistent_fn;  // bp_fwd_persistent instantiation of the same form, or null
     int max_stage_bytes;        // cap on one shared-memory stage; 0: the library default
+    const void *wide_fn, *wide_persistent_fn;  // 64-bit block phases (wide_steps), or null
 };
 
 // Batched (persistent) forward: per-object FwdParams and a cost-sorted work list.
@@ -60,7 +61,8 @@ struct BatchParams {
 };
 
 const FwdVariant *fwd_variants(int *count);
-cudaError_t launch_fwd(const FwdVariant &var, const FwdParams &p, size_t smem,
+// fn: the variant's kernel, or its wide one
+cudaError_t launch_fwd(const FwdVariant &var, const void *fn, const FwdParams &p, size_t smem,
                        cudaStream_t stream);
 cudaError_t launch_reduce(const FwdParams &p, cudaStream_t stream);
 cudaError_t launch_prep_antennas(const float *ant, const float *rxo, int R, const float *pos_off,

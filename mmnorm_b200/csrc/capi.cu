@@ -168,6 +168,15 @@ int plan_forward(int64_t nvox, int64_t vox_start, int64_t vox_count, int A, int 
     return MMN_OK;
 }
 
+// Whether a row's block steps take 64 bits.  32-bit steps of 64 samples are right while 64 d
+// slope/c < 2^19 turns; the start phase needs d / wavelength < 2^19 already, so that holds wherever
+// 64 slope/c <= 1/wavelength (a 4 GHz sweep of 256 samples at 77 GHz: 3.3 and 257 turns a metre).
+// Their rounding of 2^-33 turns stays under 1.1e-8 rad over 16 blocks, well under the hardware
+// sine's 4e-7; longer rows take 64-bit steps too (2.5 % more time at 100 samples).
+bool wide_steps(double slope, double wavelength, int F) {
+    return 64.0 * std::fabs(slope) / kC * wavelength > 1.0 || F > 1024;
+}
+
 void set_fixed_fields(FwdParams &f) {
     f.fx_t0 = -4294967296.0 * f.t0;
     f.fx_smp = -4294967296.0 * f.tsmp;
@@ -227,10 +236,11 @@ int run_forward(const FwdPlan &pl, const mmn_problem *p, const float *meas_r,
     fp.out_i = out_i;
     fp.partial = reinterpret_cast<float4 *>(ws + pl.off_partial);
     fp.status = hdr;
+    const void *fn = pl.var->wide_fn && wide_steps(p->slope, p->wavelength, F) ? pl.var->wide_fn
+                                                                              : pl.var->fn;
     if (pl.smem > 48 * 1024)
-        cudaFuncSetAttribute(pl.var->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pl.smem);
-    e = launch_fwd(*pl.var, fp, pl.smem, stream);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+    e = launch_fwd(*pl.var, fn, fp, pl.smem, stream);
     if (e != cudaSuccess) return MMN_ERR_CUDA;
     if (pl.splits > 1) {
         e = launch_reduce(fp, stream);
@@ -1390,6 +1400,7 @@ struct mmn_batch {
     int n = 0;
     int mode = 0;
     const FwdVariant *var = nullptr;
+    const void *fn = nullptr;  // the variant's persistent kernel, or its wide one
     size_t smem = 0;
     int ctas = 0;
     struct Obj {
@@ -1432,6 +1443,11 @@ extern "C" int mmn_batch_create(const mmn_problem *problems, int32_t num_objects
     b->n = num_objects;
     b->mode = mode;
     b->var = &vars[vi];
+    b->fn = b->var->persistent_fn;
+    for (int o = 0; o < num_objects; ++o)
+        if (b->var->wide_persistent_fn &&
+            wide_steps(problems[o].slope, problems[o].wavelength, problems[o].num_samples))
+            b->fn = b->var->wide_persistent_fn;
     b->probs.assign(problems, problems + num_objects);
     b->images.assign(images, images + num_objects);
     b->votes.assign(num_objects, nullptr);
@@ -1461,10 +1477,9 @@ extern "C" int mmn_batch_create(const mmn_problem *problems, int32_t num_objects
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (b->smem > 48 * 1024)
-        cudaFuncSetAttribute(b->var->persistent_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)b->smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->var->persistent_fn, b->var->nt,
-                                                      b->smem) != cudaSuccess ||
+        cudaFuncSetAttribute(b->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->fn, b->var->nt, b->smem) !=
+            cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
     b->ctas = sms * per_sm;
@@ -1621,8 +1636,8 @@ extern "C" int mmn_batch_run(mmn_batch *b, void *workspace, cudaStream_t stream)
         bp.counter = reinterpret_cast<int *>(ws + b->off_counter);
         void *args[] = {&bp};
         const int grid = std::min<int>(b->ctas, (int)b->items.size());
-        if (cudaLaunchKernel(b->var->persistent_fn, dim3(grid), dim3(b->var->nt), args, b->smem,
-                             stream) != cudaSuccess)
+        if (cudaLaunchKernel(b->fn, dim3(grid), dim3(b->var->nt), args, b->smem, stream) !=
+            cudaSuccess)
             return MMN_ERR_CUDA;
     }
     for (int o = 0; o < b->n; ++o)
