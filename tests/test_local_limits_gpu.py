@@ -58,3 +58,17 @@ def test_anchors_beyond_the_fixed_point_range(cuda_dev, oracle, wavelength, rx):
     runs, (gm_o, gp_o) = _gradients(cuda_dev, oracle, sc, rxo, rx == 3, rx)
     assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < 3e-6
     assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1.2e-5
+
+
+@pytest.mark.parametrize("ants,nf,spacing", [(1, 40, 0.3), (3, 300, 0.25), (4, 17, 0.3),
+                                             (5, 300, 0.004), (9, 700, 0.4)])
+def test_few_antennas_with_wide_windows(cuda_dev, oracle, ants, nf, spacing):
+    """Grid windows of up to all 2 F cells, spread over several warps an antenna.  Ranges of some
+    metres: FP32 anchors and tap offsets as at ordinary sizes (2e-6)."""
+    sc = _scene((6, 5, 9), ants, nf, spacing, 600 + nf)
+    I, W = run_ops(cuda_dev, sc, "nufft")
+    Io, Wo = oracle.full(sc.voxel_centres(), sc.antenna_locs, np.zeros((1, 3)), sc.meas,
+                         sc.wavelength, sc.slope)
+    assert oracle.rel_l2(I, Io) < TOL and oracle.rel_l2(W, Wo) < TOL
+    runs, (_, gp_o) = _gradients(cuda_dev, oracle, sc, np.zeros((1, 3), np.float32), False, nf)
+    assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1e-5
