@@ -127,6 +127,15 @@ struct NuMeasParams {
 };
 cudaError_t launch_nufft_meas_out(const NuMeasParams &q, cudaStream_t stream);
 // Interpolation form by tile-local polynomials (bp_local.cu).
+// Voxel boxes: bx x by columns of `runs` runs of 4 voxels.  The runs lie along the grid axis
+// axis[2], the columns count along axis[0] and axis[1].
+struct LocalTiles {
+    int64_t stride[3];         // flat-index strides of those axes
+    int64_t tiles;
+    int32_t axis[3], dim[3];   // grid axes and the grid's extents along them
+    int32_t bx, by, runs;
+    int32_t tiles_y, tiles_z;  // boxes along axis[1] and axis[2]
+};
 struct LocalParams {
     FwdParams f;               // geometry, antenna records, outputs; tiles and antenna splits
     const float2 *rows;        // [num_ant][row] antenna grids (G.re, G.im)
@@ -138,16 +147,16 @@ struct LocalParams {
     float half_min;            // least half width of a box's range interval: theta = 0.5, a
                                // third of a grid cell.  The derivative's FP32 noise goes with
                                // its inverse: on a box of one voxel 2e-5 of c' without it
-    int32_t bx, by, runs;      // tile: bx x by columns, runs of 4 voxels in z
-    int32_t tiles_y, tiles_z;
+    LocalTiles t;
+    const float *locs[3];      // coordinates along t.axis
     const float2 *grad_image;  // position pass: upstream gradients (either may be null)
     const float2 *grad_vote;
     float *pos_partial;        // [num_tiles, num_ant, 3]
     float4 *vox;               // measurement pass: voxel records in box order
     int32_t slots;             // ... voxel runs per box, a multiple of 32
 };
-// most: voxel runs of a tile
-void plan_local_tiles(int nx, int ny, int nz, int most, int *bx, int *by, int *runs);
+// most: voxel runs of a box
+void plan_local_tiles(int nx, int ny, int nz, int most, LocalTiles *t);
 // measurement pass: bytes of the voxel records, shared memory of the antenna rows (mrow cells
 // each), warps (antennas) per CTA
 size_t local_meas_vox_bytes(int64_t tiles, int slots);

@@ -101,27 +101,42 @@ __device__ __forceinline__ void tile_box(const float *locs, int first, int count
     hi = b;
 }
 
-// This thread's place in its tile and its voxels' coordinates (clamped into the grid, so that
-// an idle slot repeats a voxel of the box).
-struct LocSlot {
-    int ix, iy, iz;  // first voxel; the run is iz .. iz + 3
-    bool column;     // the (x, y) column is inside the grid
-};
-__device__ __forceinline__ LocSlot local_slot(const LocalParams &q, int tile, int slot) {
-    const FwdParams &p = q.f;
-    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
-    const int ty = txy % q.tiles_y, tx = txy / q.tiles_y;
-    const int used = q.bx * q.by * q.runs;
-    const int s = min(slot, used - 1);
-    const int run = s % q.runs, c = s / q.runs;
-    LocSlot o;
-    o.ix = tx * q.bx + c / q.by;
-    o.iy = ty * q.by + c % q.by;
-    o.iz = (tz * q.runs + run) * kLocRun;
-    o.column = slot < used && o.ix < p.nx && o.iy < p.ny;
-    return o;
+// ... of a tile on every axis, in the boxes' axis order.
+__device__ __forceinline__ void tile_bounds(const LocalParams &q, int tile, float (&lo)[3],
+                                            float (&hi)[3]) {
+    const LocalTiles &t = q.t;
+    const int tz = tile % t.tiles_z, txy = tile / t.tiles_z;
+    tile_box(q.locs[0], txy / t.tiles_y * t.bx, t.bx, t.dim[0], lo[0], hi[0]);
+    tile_box(q.locs[1], txy % t.tiles_y * t.by, t.by, t.dim[1], lo[1], hi[1]);
+    tile_box(q.locs[2], tz * t.runs * kLocRun, t.runs * kLocRun, t.dim[2], lo[2], hi[2]);
 }
 
+// A thread's place in its tile and its voxels' coordinates (clamped into the grid, so that
+// an idle slot repeats a voxel of the box).
+struct LocSlot {
+    float vx, vy, vz[kLocRun];  // along the boxes' axes
+    int64_t v;                  // flat index of the run's first voxel
+    int count;                  // voxels of the run inside the grid; 0: an idle slot
+};
+__device__ __forceinline__ LocSlot local_slot(const LocalParams &q, int tile, int slot) {
+    const LocalTiles &t = q.t;
+    const int tz = tile % t.tiles_z, txy = tile / t.tiles_z;
+    const int ty = txy % t.tiles_y, tx = txy / t.tiles_y;
+    const int used = t.bx * t.by * t.runs;
+    const int s = min(slot, used - 1);
+    const int run = s % t.runs, c = s / t.runs;
+    const int ix = tx * t.bx + c / t.by, iy = ty * t.by + c % t.by;
+    const int iz = (tz * t.runs + run) * kLocRun;
+    LocSlot o;
+    o.vx = __ldg(q.locs[0] + min(ix, t.dim[0] - 1));
+    o.vy = __ldg(q.locs[1] + min(iy, t.dim[1] - 1));
+#pragma unroll
+    for (int k = 0; k < kLocRun; ++k) o.vz[k] = __ldg(q.locs[2] + min(iz + k, t.dim[2] - 1));
+    o.v = ix * t.stride[0] + iy * t.stride[1] + iz * t.stride[2];
+    o.count = slot < used && ix < t.dim[0] && iy < t.dim[1]
+                  ? max(0, min(kLocRun, t.dim[2] - iz)) : 0;
+    return o;
+}
 // Table cos(pi m / (2 NN)), m < 4 NN, and the nodes cos(pi (i + 1/2) / NN).
 __device__ __forceinline__ void cheb_tables(int nn, double *table, double *node) {
     for (int m = threadIdx.x; m < 4 * nn; m += blockDim.x) {
@@ -295,6 +310,20 @@ struct __align__(16) LocShared {
     int nn;
 };
 
+// An antenna's positions in the boxes' axis order; t, o: TX and RX in FP32.
+__device__ __forceinline__ void load_antenna(const AntRec *ar, const LocalTiles &lt, LocRec &r,
+                                             float (&t)[3], float (&o)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int x = lt.axis[k];
+        r.tx[k] = ar->tx[x];
+        r.rx[k] = ar->rx[x];
+        r.u[k] = ar->virt[x];
+        r.txf[k] = t[k] = (float)r.tx[k];
+        r.rxf[k] = o[k] = (float)r.rx[k];
+    }
+}
+
 // Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the chunk's node count (0: every
 // antenna takes tap runs).  Called by all threads; barriers inside.
 // Node values and coefficients are formed in FP64: their rounding is shared by all voxels of a
@@ -312,23 +341,14 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
     if (threadIdx.x == 0) sh.nn = 0;
     __syncthreads();
     if (threadIdx.x < na) {
-        const AntRec ar = p.ant[a0 + threadIdx.x];
         LocRec &r = sh.rec[threadIdx.x];
-        const float t[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
-        const float o[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
+        float t[3], o[3];
+        load_antenna(p.ant + a0 + threadIdx.x, q.t, r, t, o);
         float c, half, dmax;
         range_bounds(lo, hi, t, o, c, half, dmax);
         half = fmaxf(half, q.half_min);
         const double centre = (double)c + p.ti;
         const double inv = 1.0 / (double)half;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            r.tx[k] = ar.tx[k];
-            r.rx[k] = ar.rx[k];
-            r.txf[k] = t[k];
-            r.rxf[k] = o[k];
-            r.u[k] = ar.virt[k];
-        }
         sh.centre[threadIdx.x] = centre;
         sh.half[threadIdx.x] = (double)half;
         r.inv = inv;
@@ -487,21 +507,13 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
     const int a_begin = split * p.ant_per_split;
     const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
     float lo[3], hi[3];
-    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
-    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
-    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
-    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    tile_bounds(q, tile, lo, hi);
     const LocSlot s = local_slot(q, tile, threadIdx.x);
-    const float vx = __ldg(p.x_locs + min(s.ix, p.nx - 1));
-    const float vy = __ldg(p.y_locs + min(s.iy, p.ny - 1));
-    float vz[kLocRun];
     float2 acc[kLocRun][4];
 #pragma unroll
-    for (int k = 0; k < kLocRun; ++k) {
-        vz[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
+    for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
         for (int c = 0; c < 4; ++c) total[k][c][threadIdx.x] = make_float2(0.f, 0.f);
-    }
     const bool mono = *p.mono_flag != 0;
     int table_nn = 0;
     for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
@@ -511,26 +523,34 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
         for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[k][c] = make_float2(0.f, 0.f);
-        if (mono) local_forward_nn<true>(q, sh, a0, na, nn, vx, vy, vz, acc);
-        else local_forward_nn<false>(q, sh, a0, na, nn, vx, vy, vz, acc);
+        if (mono) local_forward_nn<true>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, acc);
+        else local_forward_nn<false>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, acc);
 #pragma unroll
         for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
                 total[k][c][threadIdx.x] = __fadd2_rn(total[k][c][threadIdx.x], acc[k][c]);
     }
-    if (!s.column) return;
+    const LocSlot e = local_slot(q, tile, threadIdx.x);  // (again: nothing of it stays in the loop)
+    // W's components back in the grid's axis order
+    int from[3];
+#pragma unroll
+    for (int o = 0; o < 3; ++o) from[o] = q.t.axis[0] == o ? 1 : (q.t.axis[1] == o ? 2 : 3);
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k) {
-        if (s.iz + k >= p.nz) continue;
-        const int64_t v = ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k;
+        if (k >= e.count) continue;
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[k][c] = total[k][c][threadIdx.x];
-        const float dz = vz[0] - vz[k];
+        const float dz = e.vz[0] - e.vz[k];
         acc[k][3] = __ffma2_rn(acc[k][0], make_float2(dz, dz), acc[k][3]);
-        const float a[8] = {acc[k][0].x, acc[k][0].y, acc[k][1].x, acc[k][1].y,
-                            acc[k][2].x, acc[k][2].y, acc[k][3].x, acc[k][3].y};
-        store_voxel(p, split, v, a);
+        float a[8] = {acc[k][0].x, acc[k][0].y};
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            const float2 w = from[o] == 1 ? acc[k][1] : (from[o] == 2 ? acc[k][2] : acc[k][3]);
+            a[2 + 2 * o] = w.x;
+            a[3 + 2 * o] = w.y;
+        }
+        store_voxel(p, split, e.v + k * q.t.stride[2], a);
     }
 }
 
@@ -708,24 +728,17 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_bwd_pos_local_kernel(const 
     const int a_begin = split * p.ant_per_split;
     const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
     float lo[3], hi[3];
-    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
-    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
-    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
-    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    tile_bounds(q, tile, lo, hi);
     const LocSlot s = local_slot(q, tile, threadIdx.x);
-    const float vx = __ldg(p.x_locs + min(s.ix, p.nx - 1));
-    const float vy = __ldg(p.y_locs + min(s.iy, p.ny - 1));
-    float vz[kLocRun];
     float2 gi[kLocRun], gw[kLocRun][3];
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k) {
-        vz[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
-        const bool ok = s.column && s.iz + k < p.nz;
-        const int64_t v = ok ? ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k : 0;
+        const bool ok = k < s.count;
+        const int64_t v = ok ? s.v + k * q.t.stride[2] : 0;
         gi[k] = ok && q.grad_image ? q.grad_image[v] : make_float2(0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-            gw[k][c] = VOTE && ok ? q.grad_vote[c * p.nvox + v] : make_float2(0.f, 0.f);
+            gw[k][c] = VOTE && ok ? q.grad_vote[q.t.axis[c] * p.nvox + v] : make_float2(0.f, 0.f);
     }
     const bool mono = *p.mono_flag != 0;
     float *mine = wsum[threadIdx.x >> 5];
@@ -733,14 +746,15 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_bwd_pos_local_kernel(const 
     for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
         const int na = min(kLocAnts, a_end - a0);
         const int nn = local_chunk<true>(q, sh, a0, na, lo, hi, table_nn);
-        if (mono) local_position_nn<VOTE, true>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, mine);
-        else local_position_nn<VOTE, false>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, mine);
+        if (mono) local_position_nn<VOTE, true>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, gi, gw, mine);
+        else local_position_nn<VOTE, false>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, gi, gw, mine);
         __syncthreads();
         for (int i = threadIdx.x; i < na * 3; i += kLocThreads) {
             float t = 0.f;
 #pragma unroll
             for (int w = 0; w < kLocThreads / 32; ++w) t += wsum[w][i];
-            q.pos_partial[((size_t)tile * p.num_ant + a0) * 3 + i] = t;
+            const int la = i / 3, c = i - 3 * la;
+            q.pos_partial[((size_t)tile * p.num_ant + a0 + la) * 3 + q.t.axis[c]] = t;
         }
     }
 }
@@ -789,37 +803,32 @@ __global__ void __launch_bounds__(512) local_vox_kernel(const LocalParams q) {
     const int tile = blockIdx.x, slot = threadIdx.x;
     const LocVox r = loc_vox(q);
     float lo[3], hi[3];
-    const int tz = tile % q.tiles_z, txy = tile / q.tiles_z;
-    tile_box(p.x_locs, txy / q.tiles_y * q.bx, q.bx, p.nx, lo[0], hi[0]);
-    tile_box(p.y_locs, txy % q.tiles_y * q.by, q.by, p.ny, lo[1], hi[1]);
-    tile_box(p.z_locs, tz * q.runs * kLocRun, q.runs * kLocRun, p.nz, lo[2], hi[2]);
+    tile_bounds(q, tile, lo, hi);
     if (slot == 0) {
         r.box[2 * tile] = make_float4(lo[0], lo[1], lo[2], 0.f);
         r.box[2 * tile + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
     const LocSlot s = local_slot(q, tile, slot);
     const size_t at = (size_t)tile * q.slots + slot;
-    r.xy[at] = make_float4(__ldg(p.x_locs + min(s.ix, p.nx - 1)),
-                           __ldg(p.y_locs + min(s.iy, p.ny - 1)), 0.f, 0.f);
-    float z[kLocRun];
+    r.xy[at] = make_float4(s.vx, s.vy, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k) {
-        z[k] = __ldg(p.z_locs + min(s.iz + k, p.nz - 1));
-        const bool ok = s.column && s.iz + k < p.nz;
-        const int64_t v = ok ? ((int64_t)s.ix * p.ny + s.iy) * p.nz + s.iz + k : 0;
+        const bool ok = k < s.count;
+        const int64_t v = ok ? s.v + k * q.t.stride[2] : 0;
         const float2 zero = make_float2(0.f, 0.f);
         const float2 gi = ok && q.grad_image ? q.grad_image[v] : zero;
         const size_t gk = (size_t)tile * kLocRun + k;
         if (q.grad_vote) {
-            const float2 a = ok ? q.grad_vote[v] : zero, b = ok ? q.grad_vote[p.nvox + v] : zero,
-                         c = ok ? q.grad_vote[2 * p.nvox + v] : zero;
+            const float2 a = ok ? q.grad_vote[q.t.axis[0] * p.nvox + v] : zero,
+                         b = ok ? q.grad_vote[q.t.axis[1] * p.nvox + v] : zero,
+                         c = ok ? q.grad_vote[q.t.axis[2] * p.nvox + v] : zero;
             r.g[(2 * gk) * q.slots + slot] = make_float4(gi.x, gi.y, a.x, a.y);
             r.g[(2 * gk + 1) * q.slots + slot] = make_float4(b.x, b.y, c.x, c.y);
         } else {
             reinterpret_cast<float2 *>(r.g)[gk * q.slots + slot] = gi;
         }
     }
-    r.z[at] = make_float4(z[0], z[1], z[2], z[3]);
+    r.z[at] = make_float4(s.vz[0], s.vz[1], s.vz[2], s.vz[3]);
 }
 
 // Tables of every node count, back to back: cos(pi m / (2 NN)), m < 4 NN, and the nodes.
@@ -1067,18 +1076,11 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
     for (int c = lane; c < mrow; c += 32) row[c] = make_float2(0.f, 0.f);
     LocRec &rec = s_rec[warp];
     LocSpread &sp = s_spread[warp];
-    const AntRec ar = p.ant[a];
-    const float t[3] = {(float)ar.tx[0], (float)ar.tx[1], (float)ar.tx[2]};
-    const float r[3] = {(float)ar.rx[0], (float)ar.rx[1], (float)ar.rx[2]};
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            rec.tx[k] = ar.tx[k];
-            rec.rx[k] = ar.rx[k];
-            rec.txf[k] = t[k];
-            rec.rxf[k] = r[k];
-            rec.u[k] = ar.virt[k];
-        }
+    float t[3], r[3];
+    {
+        LocRec mine;
+        load_antenna(p.ant + a, q.t, mine, t, r);
+        if (lane == 0) rec = mine;
     }
     const bool mono = *p.mono_flag != 0;
     const LocVox vx = loc_vox(q);
@@ -1152,28 +1154,65 @@ cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int 
                             dim3(kLocMeasWarps * 32), args, smem, stream);
 }
 
-// Tile shape: columns bx x by and runs of 4 voxels in z, at most `most` runs, chosen for few
-// tiles (idle slots of a ragged grid cost as much as used ones) with a charge for elongated
-// boxes, whose wider range interval needs more nodes.  8 x 8 x 8 on a large grid.
-void plan_local_tiles(int nx, int ny, int nz, int most, int *bx, int *by, int *runs) {
+// Box shape for one order of the axes (the grid's extents along them, the runs' last): columns
+// bx x by and runs, at most `most` runs in all and at most `side` columns or voxels a side, chosen
+// for few boxes (idle slots of a ragged grid cost as much as used ones) with a charge for elongated
+// ones, whose wider range interval needs more nodes.  8 x 8 x 8 on a large grid.  Returns the cost.
+static double plan_order(const int (&dim)[3], int most, int side, LocalTiles *t) {
     double best = 1e300;
-    const int zr = (nz + kLocRun - 1) / kLocRun;
+    const int zr = (dim[2] + kLocRun - 1) / kLocRun;
     const double cube = std::sqrt(3.0) * std::cbrt((double)most * kLocRun);
-    for (int r = 1; r <= std::min(zr, 16); ++r)
-        for (int y = 1; y <= std::min(ny, 32) && r * y <= most; ++y) {
-            const int x = std::min({nx, most / (r * y), 32});
-            const double tiles = (double)((nx + x - 1) / x) * ((ny + y - 1) / y) *
+    for (int r = 1; r <= std::min({zr, most, std::max(side / 2, 1)}); ++r)
+        for (int y = 1; y <= std::min(dim[1], side) && r * y <= most; ++y) {
+            const int x = std::min({dim[0], most / (r * y), side});
+            const double tiles = (double)((dim[0] + x - 1) / x) * ((dim[1] + y - 1) / y) *
                                  ((zr + r - 1) / r);
             const double diag2 = (double)x * x + (double)y * y +
                                  (double)(kLocRun * r) * (kLocRun * r);
             const double cost = tiles * (1.0 + 0.01 * std::max(0.0, std::sqrt(diag2) - cube));
             if (cost < best) {
                 best = cost;
-                *bx = x;
-                *by = y;
-                *runs = r;
+                t->bx = x;
+                t->by = y;
+                t->runs = r;
             }
         }
+    return best;
+}
+
+// The runs lie along z unless that leaves over a quarter of the slots idle (a grid thin in z: a
+// plane used one voxel of a run's four, 1.9 ms for 300 x 300 x 1 voxels x 2048 antennas x 128
+// samples; along y 0.6) and another axis does at least a tenth better.  Lines and bars also get
+// longer boxes than the 32 a side that wider grids do (8192 voxels in a row x 4096 antennas: 1.6 ms
+// with 16 of 128 threads at work, 0.17 so).
+void plan_local_tiles(int nx, int ny, int nz, int most, LocalTiles *t) {
+    static const int order[3][3] = {{0, 1, 2}, {0, 2, 1}, {1, 2, 0}};
+    const int n[3] = {nx, ny, nz};
+    const int64_t stride[3] = {(int64_t)ny * nz, nz, 1};
+    const auto share = [&](double cost) {  // of the slots in use, if boxes are not elongated
+        return (double)nx * ny * nz / (cost * most * kLocRun);
+    };
+    double best = 1e300;
+    for (int side : {32, 2 * most}) {
+        for (const auto &o : order) {
+            LocalTiles c;
+            const int dim[3] = {n[o[0]], n[o[1]], n[o[2]]};
+            const double cost = plan_order(dim, most, side, &c);
+            if (cost >= 0.9 * best) continue;
+            best = cost;
+            *t = c;
+            for (int k = 0; k < 3; ++k) {
+                t->axis[k] = o[k];
+                t->dim[k] = dim[k];
+                t->stride[k] = stride[o[k]];
+            }
+            if (share(best) > 0.75) break;
+        }
+        if (share(best) > 0.5) break;
+    }
+    t->tiles_y = (t->dim[1] + t->by - 1) / t->by;
+    t->tiles_z = (t->dim[2] + kLocRun * t->runs - 1) / (kLocRun * t->runs);
+    t->tiles = (int64_t)((t->dim[0] + t->bx - 1) / t->bx) * t->tiles_y * t->tiles_z;
 }
 
 const void *fwd_local_kernel_ptr(int *threads) {

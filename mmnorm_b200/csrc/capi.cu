@@ -756,26 +756,6 @@ std::atomic<int> g_pos_form{MMN_PASS_INTERP};
 std::atomic<int> g_pos_variant{0};
 std::atomic<int> g_meas_form{MMN_PASS_INTERP};
 
-// Voxel boxes of a local pass.
-struct LocalTiles {
-    int bx, by, runs, tiles_y, tiles_z;
-    int64_t tiles;
-    void plan(const mmn_problem *p, int most) {
-        plan_local_tiles(p->num_x, p->num_y, p->num_z, most, &bx, &by, &runs);
-        tiles_y = (p->num_y + by - 1) / by;
-        tiles_z = (p->num_z + 4 * runs - 1) / (4 * runs);
-        tiles = (int64_t)((p->num_x + bx - 1) / bx) * tiles_y * tiles_z;
-    }
-    void set(LocalParams &q) const {
-        q.bx = bx;
-        q.by = by;
-        q.runs = runs;
-        q.tiles_y = tiles_y;
-        q.tiles_z = tiles_z;
-        q.f.num_tiles = (int)tiles;
-    }
-};
-
 struct BwdPlan {
     int fp, ant_per_stage, tiles, splits, ant_per_split, threads, vpt;
     size_t smem;
@@ -827,7 +807,7 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
     if (pl->local) {
         pl->ant_per_stage = local_chunk_antennas();
         pl->smem = 0;
-        pl->pos.plan(p, pl->threads);
+        plan_local_tiles(p->num_x, p->num_y, p->num_z, pl->threads, &pl->pos);
         tiles = pl->pos.tiles;
     }
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
@@ -885,10 +865,12 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
         const int64_t want = (2 * (int64_t)sms * per_sm + groups - 1) / std::max<int64_t>(groups, 1);
         // the largest boxes (fewest reductions and spreads) that still make that many ranges
         for (pl->mslots = 512;; pl->mslots /= 2) {
-            pl->meas.plan(p, pl->mslots);
+            plan_local_tiles(p->num_x, p->num_y, p->num_z, pl->mslots, &pl->meas);
             if (pl->mslots == 128 || pl->meas.tiles >= want) break;
         }
         if (pl->meas.tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
+        // (the records' slots: those in use, by whole warps)
+        pl->mslots = (pl->meas.bx * pl->meas.by * pl->meas.runs + 31) / 32 * 32;
         const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>({want, 64, pl->meas.tiles}));
         pl->mtiles_per_range = (int)((pl->meas.tiles + ranges - 1) / ranges);
         pl->mranges = (int)((pl->meas.tiles + pl->mtiles_per_range - 1) / pl->mtiles_per_range);
@@ -933,6 +915,13 @@ extern "C" size_t mmn_backward_workspace_bytes(const mmn_problem *p) {
 // ---------------------------------------------------------------------------------
 namespace {
 
+void set_local_tiles(LocalParams &q, const mmn_problem *p, const LocalTiles &t) {
+    const float *locs[3] = {p->x_locs, p->y_locs, p->z_locs};
+    q.t = t;
+    q.f.num_tiles = (int)t.tiles;
+    for (int k = 0; k < 3; ++k) q.locs[k] = locs[t.axis[k]];
+}
+
 void set_local_fields(LocalParams &q, const mmn_problem *p, int n, int row, const float2 *rows) {
     const int F = p->num_samples, J0 = F / 2;
     q.rows = rows;
@@ -948,7 +937,7 @@ void set_local_fields(LocalParams &q, const mmn_problem *p, int n, int row, cons
 
 struct NuFwdPlan {
     int n, row, threads, tiles, splits, ant_per_split;
-    int bx, by, runs, tiles_y, tiles_z;
+    LocalTiles t;
     size_t off_ant, off_rows, off_tab, off_part, total;
     const void *fn;
 };
@@ -961,10 +950,8 @@ int plan_nufft_forward(const mmn_problem *p, NuFwdPlan *pl) {
     // the longest row: (G.re, G.im) cells and the antenna record within 48 KB
     if ((int)sizeof(AntRec) + pl->row * 8 > kMaxStageBytes) return MMN_ERR_TOO_LARGE;
     pl->fn = fwd_local_kernel_ptr(&pl->threads);
-    plan_local_tiles(p->num_x, p->num_y, p->num_z, pl->threads, &pl->bx, &pl->by, &pl->runs);
-    pl->tiles_y = (p->num_y + pl->by - 1) / pl->by;
-    pl->tiles_z = (p->num_z + 4 * pl->runs - 1) / (4 * pl->runs);
-    const int64_t tiles = (int64_t)((p->num_x + pl->bx - 1) / pl->bx) * pl->tiles_y * pl->tiles_z;
+    plan_local_tiles(p->num_x, p->num_y, p->num_z, pl->threads, &pl->t);
+    const int64_t tiles = pl->t.tiles;
     if (tiles > (int64_t)1 << 30) return MMN_ERR_TOO_LARGE;
     pl->tiles = (int)tiles;
     const int chunk = local_chunk_antennas();
@@ -1070,11 +1057,7 @@ extern "C" int mmn_backproject_nufft(const mmn_problem *p, float *image, float *
     f.status = hdr;
     float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_rows);
     set_local_fields(q, p, pl.n, pl.row, rows);
-    q.bx = pl.bx;
-    q.by = pl.by;
-    q.runs = pl.runs;
-    q.tiles_y = pl.tiles_y;
-    q.tiles_z = pl.tiles_z;
+    set_local_tiles(q, p, pl.t);
     if (launch_nufft_tables(f, F, pl.n, J0, sc, tw, box, stream) != cudaSuccess)
         return MMN_ERR_CUDA;
     if (launch_nufft_grid_window(p->meas, A, F, pl.n, J0, pl.row, sc, tw, ant, box, f.ti, q.uq,
@@ -1204,7 +1187,7 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     if (grad_pos && pl.local) {
         LocalParams q = lq;
         float2 *rows = reinterpret_cast<float2 *>(ws + pl.off_meas);
-        pl.pos.set(q);
+        set_local_tiles(q, p, pl.pos);
         q.rows = rows;
         q.pos_partial = bp.pos_partial;
         if (launch_nufft_grid_window(p->meas, A, F, pl.nu_n, J0, pl.row, sc, tw, ant,
@@ -1246,7 +1229,7 @@ extern "C" int mmn_backproject_backward(const mmn_problem *p, const float *grad_
     }
     if (grad_meas && pl.meas_nufft) {
         LocalParams q = lq;
-        pl.meas.set(q);
+        set_local_tiles(q, p, pl.meas);
         q.slots = pl.mslots;
         q.vox = reinterpret_cast<float4 *>(ws + pl.off_nvox);
         NuMeasParams o;
