@@ -16,10 +16,10 @@
 // index.  A thread owns 4 voxels in a row along z, whose lateral distance is one.
 //
 // NN follows from theta = pi F |slope| / c * D, the largest phase excursion of M over the half
-// width (local_nodes).  Up to NN = 12
-// the polynomial is evaluated in monomials by Horner (theta <= 2.6, so the coefficients' sum, and with it the FP32 rounding, stays within a few units); 16 and 24 by Clenshaw in the
-// Chebyshev basis.  An antenna whose theta is larger still (a 2 cm voxel pitch at 4 GHz of
-// bandwidth), or not a number, takes a tap run per voxel.
+// width (local_nodes).  Up to NN = 12 the polynomial is evaluated in monomials by Horner (theta
+// <= 2.6, so the coefficients' sum, and with it the FP32 rounding, stays within a few units).  An
+// antenna whose theta is larger (from a 7 to 11 mm voxel pitch on at 4 GHz of bandwidth), or not a
+// number, takes a tap run per pair (local_chunk).
 //
 // Bound: instruction dispatch (68 instructions a pair, 235 dispatch slots a pair before; packed
 // FP32 and FP64 instructions take about two slots).  Measured on 96^3 voxels x 4096 antennas x
@@ -41,8 +41,9 @@ namespace {
 constexpr int kLocThreads = 128;
 constexpr int kLocRun = 4;      // voxels of a thread, consecutive in z
 constexpr int kLocAnts = 32;    // antennas per chunk
-constexpr int kLocNodes = 24;   // most nodes
-constexpr int kLocHorner = 12;  // most nodes evaluated in monomials
+constexpr int kLocNodes = 24;   // most nodes (measurement pass)
+constexpr int kLocHorner = 12;  // most nodes evaluated, in monomials (forward, position pass)
+constexpr int kLocWide = 99;
 
 // Monomial coefficients of the Chebyshev polynomials T_0 .. T_11.
 __constant__ float kChebMono[kLocHorner][kLocHorner] = {
@@ -61,15 +62,15 @@ __constant__ float kChebMono[kLocHorner][kLocHorner] = {
 };
 
 // Nodes for a phase excursion theta: 2 (theta/2)^NN / NN! < 1.2e-7 at the band's edge, which
-// is about 3e-8 rms over its samples (the error of sample j' goes with |2 j'/F|^NN); 0: too
-// wide.
+// is about 3e-8 rms over its samples (the error of sample j' goes with |2 j'/F|^NN);
+// kLocWide: too wide for any.
 __device__ __forceinline__ int local_nodes(float theta) {
     if (theta <= 0.94f) return 8;
     if (theta <= 1.72f) return 10;
     if (theta <= 2.64f) return 12;
     if (theta <= 4.8f) return 16;
     if (theta <= 9.8f) return 24;
-    return 0;  // NaN lands here too
+    return kLocWide;  // NaN lands here too
 }
 
 // One antenna of a chunk, as the voxel loop reads it.
@@ -77,7 +78,7 @@ struct __align__(16) LocRec {
     double tx[3], rx[3];
     double inv, off;  // x = d * inv + off on [-1, 1]
     float txf[3], rxf[3], u[3];
-    int nn;           // nodes; 0: a tap run per voxel
+    int nn;           // nodes; 0: a tap run per voxel; -1: that, and anchors from FP64 phases
 };
 static_assert(sizeof(LocRec) % 16 == 0, "LocRec rows are read in 16-byte words");
 
@@ -168,28 +169,6 @@ __device__ __forceinline__ void eval_mono(const float2 *cf, const float (&x)[kLo
     }
 }
 
-// The same from Chebyshev coefficients, by Clenshaw's recurrence.
-__device__ __forceinline__ void eval_cheb(const float2 *cf, int nn, const float (&x)[kLocRun],
-                                          float2 (&h)[kLocRun]) {
-    float2 b1[kLocRun], b2[kLocRun];
-#pragma unroll
-    for (int k = 0; k < kLocRun; ++k) b1[k] = b2[k] = make_float2(0.f, 0.f);
-    for (int q = nn - 1; q >= 1; --q) {
-        const float2 c = cf[q];
-#pragma unroll
-        for (int k = 0; k < kLocRun; ++k) {
-            const float2 dd = __fadd2_rn(c, make_float2(-b2[k].x, -b2[k].y));
-            b2[k] = b1[k];
-            b1[k] = __ffma2_rn(make_float2(2.f * x[k], 2.f * x[k]), b1[k], dd);
-        }
-    }
-    const float2 c = cf[0];
-#pragma unroll
-    for (int k = 0; k < kLocRun; ++k)
-        h[k] = __ffma2_rn(make_float2(x[k], x[k]), b1[k],
-                          __fadd2_rn(c, make_float2(-b2[k].x, -b2[k].y)));
-}
-
 // h_k and its derivative g_k in x.
 template <int NN>
 __device__ __forceinline__ void eval_mono_d(const float2 *cf, const float (&x)[kLocRun],
@@ -242,13 +221,23 @@ __device__ __forceinline__ float2 tap_run(const float2 *row, double d, double uq
     return h;
 }
 
-// The whole sum of one (voxel, antenna) pair by a tap run; not inlined, so that the wide-box
-// path stays out of the loops' register allocation.
-__device__ __noinline__ float2 pair_sum(const float2 *row, double d, double uq, double k0c,
-                                        int n) {
-    const float2 h = tap_run(row, d, uq, n);
-    const float2 an = cis_fp64_phase(-d * k0c);
-    return make_float2(fmaf(an.x, h.x, -an.y * h.y), fmaf(an.x, h.y, an.y * h.x));
+// The anchors e^{-2 pi i d t0c} of two ranges: wrapped turns in 2^-32 steps, or, for ranges beyond
+// what those hold (local_chunk), FP64 phases.  (cos, cos, sin, sin)
+__device__ __noinline__ float4 cis_wide_pair(double d0, double d1, double k0c) {
+    const float2 a = cis_fp64_phase(-d0 * k0c), b = cis_fp64_phase(-d1 * k0c);
+    return make_float4(a.x, b.x, a.y, b.y);
+}
+__device__ __forceinline__ void anchor_pair(const LocalParams &q, double d0, double d1, bool wide,
+                                            float2 &c, float2 &s) {
+    const double kM = 6755399441055744.0;  // 1.5 * 2^52
+    if (!wide) {
+        cis_half_pair(__double2loint(fma(d0, q.t0c_fixed, kM)),
+                      __double2loint(fma(d1, q.t0c_fixed, kM)), c, s);
+    } else {
+        const float4 w = cis_wide_pair(d0, d1, q.k0c);
+        c = make_float2(w.x, w.y);
+        s = make_float2(w.z, w.w);
+    }
 }
 
 // 1/sqrt of a sum of squares, subnormals flushed: one MUFU.
@@ -300,14 +289,13 @@ __device__ __forceinline__ void run_ranges(const LocRec &a, float vx, float vy,
 // Shared memory of one CTA.
 struct __align__(16) LocShared {
     LocRec rec[kLocAnts];
-    double2 node_val[kLocAnts][kLocNodes];
-    float2 coef[kLocAnts][kLocNodes];   // monomials, or Chebyshev coefficients
-    float2 deriv[kLocAnts][kLocNodes];  // Chebyshev coefficients of the derivative
+    double2 node_val[kLocAnts][kLocHorner];
+    float2 coef[kLocAnts][kLocHorner];  // monomials
     double centre[kLocAnts], half[kLocAnts];
-    double node[kLocNodes];
-    double table[4 * kLocNodes];
+    double node[kLocHorner];
+    double table[4 * kLocHorner];
     double basis[kLocHorner * kLocHorner];  // monomials from node values
-    int nn;
+    int nn, taps;
 };
 
 // An antenna's positions in the boxes' axis order; t, o: TX and RX in FP32.
@@ -324,21 +312,23 @@ __device__ __forceinline__ void load_antenna(const AntRec *ar, const LocalTiles 
     }
 }
 
-// Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the chunk's node count (0: every
-// antenna takes tap runs).  Called by all threads; barriers inside.
+// Steps 1 to 3 for antennas a0 .. a0 + na - 1.  Returns the node count of those whose boxes take
+// kLocHorner nodes at most (0: none); taps: whether any takes tap runs instead.  Called by all
+// threads; barriers inside.
+// 16 and 24 nodes by Clenshaw's recurrence measured slower than a tap run per pair (64^3 voxels at
+// a 14 mm pitch x 1024 antennas x 128 samples at 4 GHz: forward 2.47 ms and position pass 5.1;
+// tap runs 1.54 and 2.38).
 // Node values and coefficients are formed in FP64: their rounding is shared by all voxels of a
 // box, and in FP32 it put the sums of 256 antennas 2.06e-7 from 64 bits (position gradient
 // 2.27e-7), where tap runs per pair were 1.75e-7 (2.05e-7) and this is 1.78e-7 (1.98e-7).  The
 // products with one basis matrix in place of two transforms pay for it: 96^3 x 4096 x 200 went
 // from 9.17 to 9.02 ms.
-// With DERIV and more than kLocHorner nodes, the derivative's coefficients too.
-template <bool DERIV>
 __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, int a0, int na,
                                            const float (&lo)[3], const float (&hi)[3],
-                                           int &table_nn) {
+                                           int &table_nn, bool &taps) {
     const FwdParams &p = q.f;
     __syncthreads();  // the previous chunk's readers are done
-    if (threadIdx.x == 0) sh.nn = 0;
+    if (threadIdx.x == 0) sh.nn = sh.taps = 0;
     __syncthreads();
     if (threadIdx.x < na) {
         LocRec &r = sh.rec[threadIdx.x];
@@ -348,128 +338,93 @@ __device__ __forceinline__ int local_chunk(const LocalParams &q, LocShared &sh, 
         range_bounds(lo, hi, t, o, c, half, dmax);
         half = fmaxf(half, q.half_min);
         const double centre = (double)c + p.ti;
-        const double inv = 1.0 / (double)half;
         sh.centre[threadIdx.x] = centre;
         sh.half[threadIdx.x] = (double)half;
-        r.inv = inv;
-        r.off = -centre * inv;
         // the anchor's turn count must fit the fixed-point reduction (|turns| < 2^18)
         const bool fits = ((double)dmax + p.ti) * fabs(q.t0c) < 262144.0;
-        r.nn = fits ? local_nodes(q.theta_per_m * half) : 0;
-        atomicMax(&sh.nn, r.nn);
+        const int nodes = local_nodes(q.theta_per_m * half);
+        r.nn = !fits ? -1 : (nodes > kLocHorner ? 0 : nodes);
+        const double inv = r.nn > 0 ? 1.0 / (double)half : 0.0;
+        r.inv = inv;
+        r.off = r.nn > 0 ? -centre * inv : 0.0;
+        if (r.nn > 0) atomicMax(&sh.nn, r.nn);
+        else sh.taps = 1;
     }
     __syncthreads();
     const int nn = sh.nn;
+    taps = sh.taps != 0;
     if (nn == 0) return 0;
     if (nn != table_nn) {
         cheb_tables(nn, sh.table, sh.node);
         table_nn = nn;
         __syncthreads();
-        if (nn <= kLocHorner) {
-            // monomial c of the interpolant: sum_j basis[c][j] M_j
-            for (int i = threadIdx.x; i < nn * nn; i += kLocThreads) {
-                const int c = i / nn, j = i - c * nn;
-                double s = 0.0;
-                for (int m = c; m < nn; m += 2)
-                    s = fma((double)kChebMono[m][c] * (m == 0 ? 1.0 : 2.0),
-                            sh.table[m * (2 * j + 1) % (4 * nn)], s);
-                sh.basis[i] = s / nn;
-            }
-            __syncthreads();
+        // monomial c of the interpolant: sum_j basis[c][j] M_j
+        for (int i = threadIdx.x; i < nn * nn; i += kLocThreads) {
+            const int c = i / nn, j = i - c * nn;
+            double s = 0.0;
+            for (int m = c; m < nn; m += 2)
+                s = fma((double)kChebMono[m][c] * (m == 0 ? 1.0 : 2.0),
+                        sh.table[m * (2 * j + 1) % (4 * nn)], s);
+            sh.basis[i] = s / nn;
         }
+        __syncthreads();
     }
     for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
         const int la = i / nn, j = i - la * nn;
-        const LocRec &r = sh.rec[la];
-        if (r.nn == 0) continue;
+        // (an antenna with tap runs: the zero polynomial, so that the loop over the monomials
+        // needs no test)
+        sh.node_val[la][j] = make_double2(0.0, 0.0);
+        if (sh.rec[la].nn <= 0) continue;
         const double d = fma(sh.node[j], sh.half[la], sh.centre[la]);
         sh.node_val[la][j] = tap_run64(q.rows + (size_t)(a0 + la) * q.row, d, q.uq, q.n);
     }
     __syncthreads();
-    if (nn <= kLocHorner) {
-        for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
-            const int la = i / nn, c = i - la * nn;
-            const double *b = sh.basis + c * nn;
-            double2 s = make_double2(0.0, 0.0);
-            for (int j = 0; j < nn; ++j) {
-                const double2 v = sh.node_val[la][j];
-                s.x = fma(b[j], v.x, s.x);
-                s.y = fma(b[j], v.y, s.y);
-            }
-            sh.coef[la][c] = make_float2((float)s.x, (float)s.y);
-        }
-        __syncthreads();
-        return nn;
-    }
-    // Chebyshev coefficients c_p = (2 - [p = 0]) / NN sum_j M_j cos(pi p (2 j + 1) / (2 NN))
     for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
         const int la = i / nn, c = i - la * nn;
+        const double *b = sh.basis + c * nn;
         double2 s = make_double2(0.0, 0.0);
-        int m = c;
         for (int j = 0; j < nn; ++j) {
-            const double t = sh.table[m];
             const double2 v = sh.node_val[la][j];
-            s.x = fma(t, v.x, s.x);
-            s.y = fma(t, v.y, s.y);
-            m += 2 * c;
-            if (m >= 4 * nn) m -= 4 * nn;
+            s.x = fma(b[j], v.x, s.x);
+            s.y = fma(b[j], v.y, s.y);
         }
-        const double sc = (c == 0 ? 1.0 : 2.0) / nn;
-        sh.coef[la][c] = make_float2((float)(s.x * sc), (float)(s.y * sc));
+        sh.coef[la][c] = make_float2((float)s.x, (float)s.y);
     }
     __syncthreads();
-    if (DERIV) {
-        // d_p = (2 - [p = 0]) sum_{m > p, m - p odd} m c_m
-        for (int i = threadIdx.x; i < na * nn; i += kLocThreads) {
-            const int la = i / nn, c = i - la * nn;
-            float2 s = make_float2(0.f, 0.f);
-            for (int m = c + 1; m < nn; m += 2)
-                s = __ffma2_rn(make_float2((float)m, (float)m), sh.coef[la][m], s);
-            const float f = c == 0 ? 1.f : 2.f;
-            sh.deriv[la][c] = make_float2(f * s.x, f * s.y);
-        }
-        __syncthreads();
-    }
     return nn;
 }
 
-// Step 4 for one chunk.  NN: 8, 10, 12 monomials; 0: Chebyshev with nn coefficients (or tap
-// runs only, nn = 0).
+// Step 4 for one chunk.  NN: 8, 10 or 12, the monomials (zero for the antennas with tap runs); 0:
+// those antennas.
 template <bool MONO, int NN>
 __device__ __forceinline__ void local_forward(const LocalParams &q, const LocShared &sh, int a0,
-                                              int na, int nn, float vx, float vy,
+                                              int na, float vx, float vy,
                                               const float (&vz)[kLocRun],
                                               float2 (&acc)[kLocRun][4]) {
-    const double kM = 6755399441055744.0;  // 1.5 * 2^52
     for (int la = 0; la < na; ++la) {
         const LocRec &a = sh.rec[la];
+        if (NN == 0 && a.nn > 0) continue;
         double d[kLocRun];
         float rf[kLocRun], rb[kLocRun];
         run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d, rf, rb);
         float2 h[kLocRun];
-        if (a.nn > 0) {
+        if (NN > 0) {
             float x[kLocRun];
 #pragma unroll
             for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
-            if (NN > 0)
-                eval_mono<(NN > 0 ? NN : 8)>(sh.coef[la], x, h);
-            else
-                eval_cheb(sh.coef[la], nn, x, h);
-            // times the anchor e^{-2 pi i d t0c}: wrapped turns in 2^-32 steps
-#pragma unroll
-            for (int k = 0; k < kLocRun; k += 2) {
-                float2 c, s;
-                cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
-                              __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), c, s);
-                h[k] = make_float2(fmaf(c.x, h[k].x, -s.x * h[k].y),
-                                   fmaf(c.x, h[k].y, s.x * h[k].x));
-                h[k + 1] = make_float2(fmaf(c.y, h[k + 1].x, -s.y * h[k + 1].y),
-                                       fmaf(c.y, h[k + 1].y, s.y * h[k + 1].x));
-            }
+            eval_mono<(NN > 0 ? NN : 8)>(sh.coef[la], x, h);
         } else {
             const float2 *row = q.rows + (size_t)(a0 + la) * q.row;
 #pragma unroll
-            for (int k = 0; k < kLocRun; ++k) h[k] = pair_sum(row, d[k], q.uq, q.k0c, q.n);
+            for (int k = 0; k < kLocRun; ++k) h[k] = tap_run(row, d[k], q.uq, q.n);
+        }
+#pragma unroll
+        for (int k = 0; k < kLocRun; k += 2) {
+            float2 c, s;
+            anchor_pair(q, d[k], d[k + 1], NN == 0 && a.nn < 0, c, s);
+            h[k] = make_float2(fmaf(c.x, h[k].x, -s.x * h[k].y), fmaf(c.x, h[k].y, s.x * h[k].x));
+            h[k + 1] = make_float2(fmaf(c.y, h[k + 1].x, -s.y * h[k + 1].y),
+                                   fmaf(c.y, h[k + 1].y, s.y * h[k + 1].x));
         }
         // the vote about the run's first voxel: the others' share is (z_0 - z_k) I at the end
         const float ux = a.u[0] - vx, uy = a.u[1] - vy, uz = a.u[2] - vz[0];
@@ -488,10 +443,10 @@ __device__ __forceinline__ void local_forward_nn(const LocalParams &q, const Loc
                                                  int na, int nn, float vx, float vy,
                                                  const float (&vz)[kLocRun],
                                                  float2 (&acc)[kLocRun][4]) {
-    if (nn == 8) local_forward<MONO, 8>(q, sh, a0, na, nn, vx, vy, vz, acc);
-    else if (nn == 10) local_forward<MONO, 10>(q, sh, a0, na, nn, vx, vy, vz, acc);
-    else if (nn == 12) local_forward<MONO, 12>(q, sh, a0, na, nn, vx, vy, vz, acc);
-    else local_forward<MONO, 0>(q, sh, a0, na, nn, vx, vy, vz, acc);
+    if (nn == 8) local_forward<MONO, 8>(q, sh, a0, na, vx, vy, vz, acc);
+    else if (nn == 10) local_forward<MONO, 10>(q, sh, a0, na, vx, vy, vz, acc);
+    else if (nn == 12) local_forward<MONO, 12>(q, sh, a0, na, vx, vy, vz, acc);
+    else local_forward<MONO, 0>(q, sh, a0, na, vx, vy, vz, acc);
 }
 
 }  // namespace
@@ -518,18 +473,24 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
     int table_nn = 0;
     for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
         const int na = min(kLocAnts, a_end - a0);
-        const int nn = local_chunk<false>(q, sh, a0, na, lo, hi, table_nn);
+        bool taps;
+        const int nn = local_chunk(q, sh, a0, na, lo, hi, table_nn, taps);
+        // the antennas with monomials, then those with tap runs
+        for (int pass = nn > 0 ? nn : 0;;) {
 #pragma unroll
-        for (int k = 0; k < kLocRun; ++k)
+            for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[k][c] = make_float2(0.f, 0.f);
-        if (mono) local_forward_nn<true>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, acc);
-        else local_forward_nn<false>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, acc);
+                for (int c = 0; c < 4; ++c) acc[k][c] = make_float2(0.f, 0.f);
+            if (mono) local_forward_nn<true>(q, sh, a0, na, pass, s.vx, s.vy, s.vz, acc);
+            else local_forward_nn<false>(q, sh, a0, na, pass, s.vx, s.vy, s.vz, acc);
 #pragma unroll
-        for (int k = 0; k < kLocRun; ++k)
+            for (int k = 0; k < kLocRun; ++k)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                total[k][c][threadIdx.x] = __fadd2_rn(total[k][c][threadIdx.x], acc[k][c]);
+                for (int c = 0; c < 4; ++c)
+                    total[k][c][threadIdx.x] = __fadd2_rn(total[k][c][threadIdx.x], acc[k][c]);
+            if (pass == 0 || !taps) break;
+            pass = 0;
+        }
     }
     const LocSlot e = local_slot(q, tile, threadIdx.x);  // (again: nothing of it stays in the loop)
     // W's components back in the grid's axis order
@@ -563,7 +524,7 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
 namespace {
 
 // M and dM/dd of a pair by a tap run (wide boxes).
-__device__ __noinline__ float4 tap_run_d(const float2 *row, double d, double uq, int n) {
+__device__ __forceinline__ float4 tap_run_d(const float2 *row, double d, double uq, int n) {
     int ix;
     float w[kNuW], t;
     nufft_taps(d, uq, n, ix, w, &t);
@@ -588,13 +549,6 @@ __device__ __noinline__ float4 tap_run_d(const float2 *row, double d, double uq,
     return make_float4(h.x, h.y, g.x * s, g.y * s);
 }
 
-// The anchors of two pairs from FP64 phases (wide boxes and ranges beyond the fixed-point turns):
-// (cos, cos, sin, sin)
-__device__ __noinline__ float4 cis_wide_pair(double d0, double d1, double k0c) {
-    const float2 a = cis_fp64_phase(-d0 * k0c), b = cis_fp64_phase(-d1 * k0c);
-    return make_float4(a.x, b.x, a.y, b.y);
-}
-
 // Sums of v0, v1, v2 over the warp: in lanes 0-7, 8-15 and 16-23.
 __device__ __forceinline__ float warp_sum3(float v0, float v1, float v2) {
     const int lane = threadIdx.x & 31;
@@ -607,31 +561,28 @@ __device__ __forceinline__ float warp_sum3(float v0, float v1, float v2) {
     return a;
 }
 
+// NN: 8, 10 or 12, the monomials (zero for the antennas with tap runs); 0: those antennas, after
+// the others.
 template <bool VOTE, bool MONO, int NN>
 __device__ __forceinline__ void local_position(const LocalParams &q, const LocShared &sh, int a0,
-                                               int na, int nn, float vx, float vy,
+                                               int na, float vx, float vy,
                                                const float (&vz)[kLocRun],
                                                const float2 (&gi)[kLocRun],
                                                const float2 (&gw)[kLocRun][3], float *wsum) {
-    const double kM = 6755399441055744.0;  // 1.5 * 2^52
     const int lane = threadIdx.x & 31;
     const float k0c = (float)q.k0c;
     for (int la = 0; la < na; ++la) {
         const LocRec &a = sh.rec[la];
+        if (NN == 0 && a.nn > 0) continue;
         double d[kLocRun];
         float rf[kLocRun], rb[kLocRun];
         run_ranges<MONO>(a, vx, vy, vz, q.f.ti, d, rf, rb);
         float2 h[kLocRun], g[kLocRun];  // M, dM/dd
-        if (a.nn > 0) {
+        if (NN > 0) {
             float x[kLocRun];
 #pragma unroll
             for (int k = 0; k < kLocRun; ++k) x[k] = (float)fma(d[k], a.inv, a.off);
-            if (NN > 0) {
-                eval_mono_d<(NN > 0 ? NN : 8)>(sh.coef[la], x, h, g);
-            } else {
-                eval_cheb(sh.coef[la], nn, x, h);
-                eval_cheb(sh.deriv[la], nn, x, g);
-            }
+            eval_mono_d<(NN > 0 ? NN : 8)>(sh.coef[la], x, h, g);
             const float inv = (float)a.inv;
 #pragma unroll
             for (int k = 0; k < kLocRun; ++k) g[k] = __fmul2_rn(g[k], make_float2(inv, inv));
@@ -651,14 +602,7 @@ __device__ __forceinline__ void local_position(const LocalParams &q, const LocSh
 #pragma unroll
         for (int k = 0; k < kLocRun; k += 2) {
             float2 ac, as;
-            if (a.nn > 0) {
-                cis_half_pair(__double2loint(fma(d[k], q.t0c_fixed, kM)),
-                              __double2loint(fma(d[k + 1], q.t0c_fixed, kM)), ac, as);
-            } else {  // the fixed-point turns may not hold the anchor's (local_chunk)
-                const float4 w = cis_wide_pair(d[k], d[k + 1], q.k0c);
-                ac = make_float2(w.x, w.y);
-                as = make_float2(w.z, w.w);
-            }
+            anchor_pair(q, d[k], d[k + 1], NN == 0 && a.nn < 0, ac, as);
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
                 const int j = k + l;
@@ -706,14 +650,15 @@ __device__ __forceinline__ void local_position(const LocalParams &q, const LocSh
 
 template <bool VOTE, bool MONO>
 __device__ __forceinline__ void local_position_nn(const LocalParams &q, const LocShared &sh,
-                                                  int a0, int na, int nn, float vx, float vy,
+                                                  int a0, int na, int nn, bool taps, float vx,
+                                                  float vy,
                                                   const float (&vz)[kLocRun],
                                                   const float2 (&gi)[kLocRun],
                                                   const float2 (&gw)[kLocRun][3], float *wsum) {
-    if (nn == 8) local_position<VOTE, MONO, 8>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
-    else if (nn == 10) local_position<VOTE, MONO, 10>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
-    else if (nn == 12) local_position<VOTE, MONO, 12>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
-    else local_position<VOTE, MONO, 0>(q, sh, a0, na, nn, vx, vy, vz, gi, gw, wsum);
+    if (nn == 8) local_position<VOTE, MONO, 8>(q, sh, a0, na, vx, vy, vz, gi, gw, wsum);
+    else if (nn == 10) local_position<VOTE, MONO, 10>(q, sh, a0, na, vx, vy, vz, gi, gw, wsum);
+    else if (nn == 12) local_position<VOTE, MONO, 12>(q, sh, a0, na, vx, vy, vz, gi, gw, wsum);
+    if (taps) local_position<VOTE, MONO, 0>(q, sh, a0, na, vx, vy, vz, gi, gw, wsum);
 }
 
 }  // namespace
@@ -745,9 +690,12 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_bwd_pos_local_kernel(const 
     int table_nn = 0;
     for (int a0 = a_begin; a0 < a_end; a0 += kLocAnts) {
         const int na = min(kLocAnts, a_end - a0);
-        const int nn = local_chunk<true>(q, sh, a0, na, lo, hi, table_nn);
-        if (mono) local_position_nn<VOTE, true>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, gi, gw, mine);
-        else local_position_nn<VOTE, false>(q, sh, a0, na, nn, s.vx, s.vy, s.vz, gi, gw, mine);
+        bool taps;
+        const int nn = local_chunk(q, sh, a0, na, lo, hi, table_nn, taps);
+        if (mono)
+            local_position_nn<VOTE, true>(q, sh, a0, na, nn, taps, s.vx, s.vy, s.vz, gi, gw, mine);
+        else
+            local_position_nn<VOTE, false>(q, sh, a0, na, nn, taps, s.vx, s.vy, s.vz, gi, gw, mine);
         __syncthreads();
         for (int i = threadIdx.x; i < na * 3; i += kLocThreads) {
             float t = 0.f;
@@ -1093,7 +1041,8 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
         half = fmaxf(half, q.half_min);
         const double centre = (double)c + p.ti;
         const bool fits = ((double)dmax + p.ti) * fabs(q.t0c) < 262144.0;
-        const int nn = fits ? local_nodes(q.theta_per_m * half) : 0;
+        const int nodes = local_nodes(q.theta_per_m * half);
+        const int nn = fits && nodes != kLocWide ? nodes : 0;
         __syncwarp();
         if (lane == 0) {
             const double inv = 1.0 / (double)half;

@@ -72,3 +72,20 @@ def test_few_antennas_with_wide_windows(cuda_dev, oracle, ants, nf, spacing):
     assert oracle.rel_l2(I, Io) < TOL and oracle.rel_l2(W, Wo) < TOL
     runs, (_, gp_o) = _gradients(cuda_dev, oracle, sc, np.zeros((1, 3), np.float32), False, nf)
     assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1e-5
+
+
+@pytest.mark.parametrize("spacing,nf", [(0.004, 50), (0.008, 64), (0.016, 33)])
+@pytest.mark.parametrize("rx", [1, 3])
+def test_chunks_of_narrow_and_wide_boxes(cuda_dev, oracle, spacing, nf, rx):
+    """Columns of voxels seen by antennas from the side, whose range over a box varies little, and
+    from below, where it takes tap runs: both in the same chunks of 32."""
+    sc = _scene((3, 4, 70), 75, nf, spacing, 800 + nf)
+    sc.antenna_locs[::2] += np.array([0.9, 0.2, 0.6], np.float32)
+    rxo = np.array([[0, 0, 0], [0.004, -0.01, 0], [0.02, 0.003, 0.001]], np.float32)[-rx:]
+    I, W = run_ops(cuda_dev, sc, "nufft", rxo=rxo)
+    Io, Wo = oracle.full(sc.voxel_centres(), sc.antenna_locs, rxo, sc.meas, sc.wavelength,
+                         sc.slope)
+    assert oracle.rel_l2(I, Io) < TOL and oracle.rel_l2(W, Wo) < TOL
+    runs, (gm_o, gp_o) = _gradients(cuda_dev, oracle, sc, rxo, False, rx)
+    assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < TOL
+    assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1e-5
