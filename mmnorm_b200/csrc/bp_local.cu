@@ -30,6 +30,7 @@
 // the tap form's.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 
 #include "bp_stage.cuh"
 #include "nufft_taps.cuh"
@@ -82,6 +83,17 @@ struct __align__(16) LocRec {
 };
 static_assert(sizeof(LocRec) % 16 == 0, "LocRec rows are read in 16-byte words");
 
+// Minima and maxima over the warp.
+__device__ __forceinline__ void warp_bounds(float (&lo)[3], float (&hi)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+        }
+}
+
 // Voxel box of a tile, by all threads of the CTA: per-axis minimum and maximum of the
 // coordinates it covers (any order of the coordinate arrays).
 __device__ __forceinline__ void tile_box(const float *locs, int first, int count, int total,
@@ -119,14 +131,26 @@ struct LocSlot {
     int64_t v;                  // flat index of the run's first voxel
     int count;                  // voxels of the run inside the grid; 0: an idle slot
 };
+// COMPACT: 32 consecutive slots are 8 x 4 columns of one layer of runs (measurement pass), not rows
+// of columns of all runs.
+template <bool COMPACT>
 __device__ __forceinline__ LocSlot local_slot(const LocalParams &q, int tile, int slot) {
     const LocalTiles &t = q.t;
     const int tz = tile % t.tiles_z, txy = tile / t.tiles_z;
     const int ty = txy % t.tiles_y, tx = txy / t.tiles_y;
     const int used = t.bx * t.by * t.runs;
     const int s = min(slot, used - 1);
-    const int run = s % t.runs, c = s / t.runs;
-    const int ix = tx * t.bx + c / t.by, iy = ty * t.by + c % t.by;
+    int run = s % t.runs, c = s / t.runs, cx = c / t.by, cy = c - cx * t.by;
+    if (COMPACT) {
+        const int columns = t.bx * t.by, band = min(8, t.by) * t.bx;
+        run = s / columns;
+        c = s - run * columns;
+        const int b = c / band, width = min(8, t.by - 8 * b);  // band of up to 8 columns in y
+        c -= b * band;
+        cx = c / width;
+        cy = 8 * b + c - cx * width;
+    }
+    const int ix = tx * t.bx + cx, iy = ty * t.by + cy;
     const int iz = (tz * t.runs + run) * kLocRun;
     LocSlot o;
     o.vx = __ldg(q.locs[0] + min(ix, t.dim[0] - 1));
@@ -297,6 +321,9 @@ struct __align__(16) LocShared {
     double basis[kLocHorner * kLocHorner];  // monomials from node values
     int nn, taps;
 };
+static_assert(offsetof(LocShared, node_val) % 16 == 0 && offsetof(LocShared, coef) % 16 == 0 &&
+                  sizeof(float2) * kLocHorner % 16 == 0,
+              "node values and monomials are read in 16-byte words");
 
 // An antenna's positions in the boxes' axis order; t, o: TX and RX in FP32.
 __device__ __forceinline__ void load_antenna(const AntRec *ar, const LocalTiles &lt, LocRec &r,
@@ -463,7 +490,7 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
     const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
     float lo[3], hi[3];
     tile_bounds(q, tile, lo, hi);
-    const LocSlot s = local_slot(q, tile, threadIdx.x);
+    const LocSlot s = local_slot<false>(q, tile, threadIdx.x);
     float2 acc[kLocRun][4];
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k)
@@ -492,7 +519,7 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_fwd_local_kernel(const Loca
             pass = 0;
         }
     }
-    const LocSlot e = local_slot(q, tile, threadIdx.x);  // (again: nothing of it stays in the loop)
+    const LocSlot e = local_slot<false>(q, tile, threadIdx.x);  // (again: nothing of it stays in the loop)
     // W's components back in the grid's axis order
     int from[3];
 #pragma unroll
@@ -674,7 +701,7 @@ __global__ void __launch_bounds__(kLocThreads, 4) bp_bwd_pos_local_kernel(const 
     const int a_end = min(p.num_ant, a_begin + p.ant_per_split);
     float lo[3], hi[3];
     tile_bounds(q, tile, lo, hi);
-    const LocSlot s = local_slot(q, tile, threadIdx.x);
+    const LocSlot s = local_slot<false>(q, tile, threadIdx.x);
     float2 gi[kLocRun], gw[kLocRun][3];
 #pragma unroll
     for (int k = 0; k < kLocRun; ++k) {
@@ -756,7 +783,7 @@ __global__ void __launch_bounds__(512) local_vox_kernel(const LocalParams q) {
         r.box[2 * tile] = make_float4(lo[0], lo[1], lo[2], 0.f);
         r.box[2 * tile + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
-    const LocSlot s = local_slot(q, tile, slot);
+    const LocSlot s = local_slot<true>(q, tile, slot);
     const size_t at = (size_t)tile * q.slots + slot;
     r.xy[at] = make_float4(s.vx, s.vy, 0.f, 0.f);
 #pragma unroll
@@ -785,29 +812,36 @@ __device__ __forceinline__ int node_offset(int nn) {  // sum of the smaller coun
     return nn == 8 ? 0 : nn == 10 ? 8 : nn == 12 ? 18 : nn == 16 ? 30 : 46;
 }
 
+constexpr int kNuWin = 16;  // cells of a window (spread_voxels)
+
 // Per-warp scratch of the spread.
 struct __align__(16) LocSpread {
-    float2 w[32][kNuW];
+    union {
+        float2 w[32][kNuW];       // node values: tap weights by lane
+        float2 win[kNuWin][32];   // voxels: a window's cells by lane
+    };
     int ix[32];
-    double mom[2 * kLocNodes];
+    float box[6];             // bounds of a part of a box
+    double centre, half;      // its range interval, and slots a part, kept out of registers
+    int part;
+    alignas(16) double mom[2 * kLocNodes];  // (re, im) pairs
 };
+static_assert(offsetof(LocSpread, mom) % 16 == 0 && sizeof(LocSpread) % 16 == 0,
+              "moments are read in 16-byte words");
 
-// Adds value * (tap weights at range d) of every active lane to the warp's grid row, in lane
-// order per cell.  NODES: node values, whose weights are formed in FP64 (their rounding would be
-// all of the box's voxels').
-template <bool NODES>
+// Adds a node value per active lane times its tap weights at range d to the warp's grid row, in
+// lane order per cell.  The weights are formed in FP64 (their rounding would be all of the box's
+// voxels').
 __device__ __noinline__ void spread_row(LocSpread &sp, float2 *row, int mrow, double d,
                                         float2 value, bool active, double uq, int n) {
     const int lane = threadIdx.x & 31;
     int ix;
     float w[kNuW];
-    if (NODES) {
+    {
         double w64[kNuW];
         nufft_taps64(d, uq, n, ix, w64);
 #pragma unroll
         for (int i = 0; i < kNuW; ++i) w[i] = (float)w64[i];
-    } else {
-        nufft_taps(d, uq, n, ix, w);
     }
 #pragma unroll
     for (int i = 0; i < kNuW; ++i) sp.w[lane][i] = make_float2(value.x * w[i], value.y * w[i]);
@@ -829,6 +863,51 @@ __device__ __noinline__ void spread_row(LocSpread &sp, float2 *row, int mrow, do
         // the next window, 25 cells on or less where the row wraps, reads cells that other lanes
         // wrote here (the ballot orders no memory); it also frees the scratch for the next call
         __syncwarp();
+    }
+}
+
+// The same for a voxel per lane: windows of 16 cells from the least cell left, each lane's products
+// with its weights (FP32) put into its column of the window, 32 components summed over the lanes by
+// a transposing reduction.  (Column entry s of lane l holds component s ^ l, cell by cell: every
+// access of a half-warp falls in 16 different banks.)  A fifth of spread_row's instructions where
+// all 32 lanes have values.
+__device__ __noinline__ void spread_voxels(LocSpread &sp, float2 *row, double d, float2 value,
+                                           double uq, int n) {
+    const int lane = threadIdx.x & 31;
+    int ix;
+    float w[kNuW];
+    nufft_taps(d, uq, n, ix, w);
+    const bool odd = lane & 1;  // odd lanes keep (im, re)
+    const float h0 = odd ? value.y : value.x, h1 = odd ? value.x : value.y;
+    float *rowf = reinterpret_cast<float *>(row);
+    unsigned pending = 0xffffffffu;
+    while (pending) {
+        const bool left = (pending >> lane) & 1u;
+        const int base = __reduce_min_sync(0xffffffffu, left ? ix : 0x7fffffff);
+        const int off = ix - base;
+        const bool mine = left && off <= kNuWin - kNuW;
+        if (mine) {
+#pragma unroll
+            for (int i = 0; i < kNuW; ++i)
+                sp.win[off + i][lane] = make_float2(h0 * w[i], h1 * w[i]);
+        }
+        float v[32];
+#pragma unroll
+        for (int s = 0; s < kNuWin; ++s) {
+            const int cell = s ^ (lane >> 1), i = cell - off;
+            float2 t = make_float2(0.f, 0.f);
+            if (mine && i >= 0 && i < kNuW) t = sp.win[cell][lane];
+            v[2 * s] = t.x;
+            v[2 * s + 1] = t.y;
+        }
+#pragma unroll
+        for (int h = 16; h >= 1; h >>= 1) {
+#pragma unroll
+            for (int i = 0; i < h; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i + h], h);
+        }
+        rowf[2 * (base + (lane >> 1)) + (lane & 1)] += v[0];
+        pending &= ~__ballot_sync(0xffffffffu, mine);
+        __syncwarp();  // the next window reads cells that other lanes wrote here
     }
 }
 
@@ -865,12 +944,37 @@ __device__ __forceinline__ void warp_sums(const float *v, double *out) {
     out[at] = w[0];  // the lanes of a group write the same value
 }
 
-// One box against the warp's antenna: the moments into sp.mom (NN > 0), or every voxel's
+// Bounds of `count` slots (a multiple of 32) of the records xys, zs into box, by the warp.
+__device__ __noinline__ void slot_bounds(const float4 *xys, const float4 *zs, int count,
+                                         float *box) {
+    const float inf = __int_as_float(0x7f800000);
+    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+    for (int i = threadIdx.x & 31; i < count; i += 32) {
+        const float4 xy = __ldg(xys + i), z = __ldg(zs + i);
+        lo[0] = fminf(lo[0], xy.x);
+        hi[0] = fmaxf(hi[0], xy.x);
+        lo[1] = fminf(lo[1], xy.y);
+        hi[1] = fmaxf(hi[1], xy.y);
+        lo[2] = fminf(lo[2], fminf(fminf(z.x, z.y), fminf(z.z, z.w)));
+        hi[2] = fmaxf(hi[2], fmaxf(fmaxf(z.x, z.y), fmaxf(z.z, z.w)));
+    }
+    warp_bounds(lo, hi);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            box[k] = lo[k];
+            box[3 + k] = hi[k];
+        }
+    __syncwarp();
+}
+
+// A part of a box against the warp's antenna: the moments into sp.mom (NN > 0), or every voxel's
 // spread (NN = 0).
 template <bool VOTE, bool MONO, int NN>
 __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &vx, int tile,
-                                            const LocRec &a, LocSpread &sp, float2 *row,
-                                            int mrow) {
+                                            int s0, int s1, const LocRec &a, LocSpread &sp,
+                                            float2 *row, int mrow) {
     const double kM = 6755399441055744.0;  // 1.5 * 2^52
     const int lane = threadIdx.x & 31;
     constexpr int NV = NN > 0 ? NN : 1;
@@ -886,15 +990,11 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
     // The coordinates lead the FP64 chain and come from L2: a run ahead (64^3 voxels x 4096 antennas x
     // 128 samples, forward and backward: 12.56 -> 12.36 ms).
     const float4 *pxy = vx.xy + (size_t)tile * q.slots, *pz = vx.z + (size_t)tile * q.slots;
-    float4 nxy = make_float4(0.f, 0.f, 0.f, 0.f), nz = nxy;
-    if (lane < q.slots) {
-        nxy = __ldg(pxy + lane);
-        nz = __ldg(pz + lane);
-    }
+    float4 nxy = __ldg(pxy + s0 + lane), nz = __ldg(pz + s0 + lane);
 #pragma unroll 1
-    for (int slot = lane; slot < q.slots; slot += 32) {
+    for (int slot = s0 + lane; slot < s1; slot += 32) {
         const float4 xy = nxy, z4 = nz;
-        if (slot + 32 < q.slots) {
+        if (slot + 32 < s1) {
             nxy = __ldg(pxy + slot + 32);
             nz = __ldg(pz + slot + 32);
         }
@@ -956,10 +1056,10 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
 #pragma unroll
                 for (int l = 0; l < L; ++l) {
                     const float2 an = cis_fp64_phase(-d[k + l] * q.k0c);
-                    spread_row<false>(sp, row, mrow, d[k + l],
-                               make_float2(fmaf(t0[l].x, an.x, t0[l].y * an.y),
-                                           fmaf(t0[l].y, an.x, -t0[l].x * an.y)),
-                               true, q.uq, q.n);
+                    spread_voxels(sp, row, d[k + l],
+                                  make_float2(fmaf(t0[l].x, an.x, t0[l].y * an.y),
+                                              fmaf(t0[l].y, an.x, -t0[l].x * an.y)),
+                                  q.uq, q.n);
                 }
             }
         }
@@ -986,15 +1086,15 @@ __device__ __forceinline__ void box_moments(const LocalParams &q, const LocVox &
 
 template <bool VOTE, bool MONO>
 __device__ __forceinline__ void box_moments_nn(const LocalParams &q, const LocVox &vx, int tile,
-                                               const LocRec &a, LocSpread &sp, float2 *row,
+                                               int s0, int s1, const LocRec &a, LocSpread &sp, float2 *row,
                                                int mrow) {
     switch (a.nn) {
-        case 8: box_moments<VOTE, MONO, 8>(q, vx, tile, a, sp, row, mrow); break;
-        case 10: box_moments<VOTE, MONO, 10>(q, vx, tile, a, sp, row, mrow); break;
-        case 12: box_moments<VOTE, MONO, 12>(q, vx, tile, a, sp, row, mrow); break;
-        case 16: box_moments<VOTE, MONO, 16>(q, vx, tile, a, sp, row, mrow); break;
-        case 24: box_moments<VOTE, MONO, 24>(q, vx, tile, a, sp, row, mrow); break;
-        default: box_moments<VOTE, MONO, 0>(q, vx, tile, a, sp, row, mrow);
+        case 8: box_moments<VOTE, MONO, 8>(q, vx, tile, s0, s1, a, sp, row, mrow); break;
+        case 10: box_moments<VOTE, MONO, 10>(q, vx, tile, s0, s1, a, sp, row, mrow); break;
+        case 12: box_moments<VOTE, MONO, 12>(q, vx, tile, s0, s1, a, sp, row, mrow); break;
+        case 16: box_moments<VOTE, MONO, 16>(q, vx, tile, s0, s1, a, sp, row, mrow); break;
+        case 24: box_moments<VOTE, MONO, 24>(q, vx, tile, s0, s1, a, sp, row, mrow); break;
+        default: box_moments<VOTE, MONO, 0>(q, vx, tile, s0, s1, a, sp, row, mrow);
     }
 }
 
@@ -1033,8 +1133,22 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
     const bool mono = *p.mono_flag != 0;
     const LocVox vx = loc_vox(q);
     const int t0 = range * tiles_per_range, t1 = min(p.num_tiles, t0 + tiles_per_range);
-    for (int tile = t0; tile < t1; ++tile) {
-        const float4 l4 = __ldg(vx.box + 2 * tile), h4 = __ldg(vx.box + 2 * tile + 1);
+    // a box too wide for kLocNodes goes in parts, down to 32 slots
+    int tile = t0, s0 = 0;
+    if (lane == 0) sp.part = q.slots;
+    __syncwarp();
+    while (tile < t1) {
+        int s1 = min(s0 + sp.part, q.slots);
+        float4 l4, h4;
+        if (s1 - s0 == q.slots) {
+            l4 = __ldg(vx.box + 2 * tile);
+            h4 = __ldg(vx.box + 2 * tile + 1);
+        } else {
+            const size_t at = (size_t)tile * q.slots + s0;
+            slot_bounds(vx.xy + at, vx.z + at, s1 - s0, sp.box);
+            l4 = make_float4(sp.box[0], sp.box[1], sp.box[2], 0.f);
+            h4 = make_float4(sp.box[3], sp.box[4], sp.box[5], 0.f);
+        }
         const float lo[3] = {l4.x, l4.y, l4.z}, hi[3] = {h4.x, h4.y, h4.z};
         float c, half, dmax;
         range_bounds(lo, hi, t, r, c, half, dmax);
@@ -1042,17 +1156,26 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
         const double centre = (double)c + p.ti;
         const bool fits = ((double)dmax + p.ti) * fabs(q.t0c) < 262144.0;
         const int nodes = local_nodes(q.theta_per_m * half);
+        if (fits && nodes == kLocWide && s1 - s0 > 32) {
+            __syncwarp();
+            if (lane == 0) sp.part = ((s1 - s0) / 2 + 31) / 32 * 32;
+            __syncwarp();
+            continue;
+        }
         const int nn = fits && nodes != kLocWide ? nodes : 0;
+        if (nn == 0) s1 = q.slots;  // the rest of the box by voxels too
         __syncwarp();
         if (lane == 0) {
             const double inv = 1.0 / (double)half;
             rec.inv = inv;
             rec.off = -centre * inv;
             rec.nn = nn;
+            sp.centre = centre;
+            sp.half = (double)half;
         }
         __syncwarp();
-        if (mono) box_moments_nn<VOTE, true>(q, vx, tile, rec, sp, row, mrow);
-        else box_moments_nn<VOTE, false>(q, vx, tile, rec, sp, row, mrow);
+        if (mono) box_moments_nn<VOTE, true>(q, vx, tile, s0, s1, rec, sp, row, mrow);
+        else box_moments_nn<VOTE, false>(q, vx, tile, s0, s1, rec, sp, row, mrow);
         if (nn > 0) {
             // node values: sum_q (2 - [q = 0]) / NN cos(pi q (2 i + 1) / (2 NN)) moment_q
             const int no = node_offset(nn), i = min(lane, nn - 1);
@@ -1068,8 +1191,15 @@ __global__ void __launch_bounds__(kLocMeasWarps * 32, 4)
                 if (m >= 4 * nn) m -= 4 * nn;
             }
             const double sc = 2.0 / nn;
-            spread_row<true>(sp, row, mrow, fma(s_node[no + i], (double)half, centre),
+            spread_row(sp, row, mrow, fma(s_node[no + i], sp.half, sp.centre),
                        make_float2((float)(s.x * sc), (float)(s.y * sc)), lane < nn, q.uq, q.n);
+        }
+        s0 = s1 < q.slots ? s1 : 0;
+        if (s0 == 0) {
+            ++tile;
+            __syncwarp();
+            if (lane == 0) sp.part = min(2 * sp.part, q.slots);
+            __syncwarp();
         }
     }
     __syncwarp();
@@ -1095,7 +1225,7 @@ cudaError_t launch_local_meas(const LocalParams &q, float2 *part, int mrow, int 
     local_vox_kernel<<<q.f.num_tiles, q.slots, 0, stream>>>(q);
     const void *fn = local_meas_kernel_ptr(q.grad_vote != nullptr);
     const size_t smem = local_meas_smem(mrow);
-    if (smem > 32 * 1024)
+    if (smem > 24 * 1024)
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int groups = (q.f.num_ant + kLocMeasWarps - 1) / kLocMeasWarps;
     void *args[] = {const_cast<LocalParams *>(&q), &part, &mrow, &tiles_per_range};

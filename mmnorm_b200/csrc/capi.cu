@@ -854,7 +854,7 @@ int plan_backward(const mmn_problem *p, bool image_only, int form, int meas_form
         pl->mrow = pl->nu_n + 16;
         const size_t msmem = local_meas_smem(pl->mrow);
         const void *mfn = local_meas_kernel_ptr(!image_only);
-        if (msmem > 32 * 1024)
+        if (msmem > 24 * 1024)
             cudaFuncSetAttribute(mfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
         int per_sm = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mfn, local_meas_warps() * 32,

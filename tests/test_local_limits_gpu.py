@@ -89,3 +89,14 @@ def test_chunks_of_narrow_and_wide_boxes(cuda_dev, oracle, spacing, nf, rx):
     runs, (gm_o, gp_o) = _gradients(cuda_dev, oracle, sc, rxo, False, rx)
     assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < TOL
     assert oracle.rel_l2(runs[0][1].astype(np.float64), gp_o) < 1e-5
+
+
+@pytest.mark.parametrize("spacing", [0.006, 0.011, 0.016, 0.021, 0.035])
+def test_measurement_boxes_in_parts(cuda_dev, oracle, spacing):
+    """Boxes of 2048 voxels that are narrow enough, too wide as a whole, in halves, and down to
+    128 voxels, whose parts then go by moments or voxel by voxel."""
+    sc = _scene((48, 50, 54), 75, 16, spacing, 900)
+    sc.f_hi = sc.f_lo + 4e9
+    runs, (gm_o, _) = _gradients(cuda_dev, oracle, sc, np.zeros((1, 3), np.float32), False, 1)
+    assert np.array_equal(runs[0][0], runs[1][0])
+    assert oracle.rel_l2(runs[0][0].astype(np.complex128), gm_o) < TOL

@@ -1,5 +1,5 @@
-"""The measurement gradient's spread onto an antenna's grid row (spread_row, bp_local.cu), run on
-the host by 32 threads: every access to the warp's shared memory is recorded with the number of
+"""The measurement gradient's spreads onto an antenna's grid row (spread_row for node values,
+spread_voxels, bp_local.cu), run on the host by 32 threads: every access to the warp's shared memory is recorded with the number of
 warp barriers its lane has passed, and two lanes that touch one cell between the same two barriers,
 one of them writing, are a race (ballots and reductions order no memory).  The row's sums are
 checked too, against numpy's (FP32 sums of at most 32 terms: 1e-5 relative)."""
@@ -54,7 +54,12 @@ struct Cell {
     operator int() const { touch(this, false); return v; }
     Cell &operator=(int a) { touch(this, true); v = a; return *this; }
 };
-struct LocSpread { float2 w[32][kNuW]; Cell ix[32]; };
+struct Comp {   // a float of the row
+    float v;
+    Comp &operator+=(float a) { touch(this, false); touch(this, true); v += a; return *this; }
+};
+constexpr int kNuWin = 16;
+struct LocSpread { float2 w[32][kNuW]; float2 win[kNuWin][32]; Cell ix[32]; };
 static float2 make_float2(float a, float b) { return float2(a, b); }
 static float2 __fadd2_rn(float2 a, float2 b) { return float2(a.x + b.x, a.y + b.y); }
 static int __ffs(unsigned m) { return __builtin_ffs(m); }
@@ -70,6 +75,12 @@ static int __reduce_min_sync(unsigned, int v) {
     int m = g_vals[0]; for (int i = 1; i < 32; ++i) m = g_vals[i] < m ? g_vals[i] : m;
     g_bar.arrive_and_wait(); return m;
 }
+static float g_fvals[32];
+static float __shfl_xor_sync(unsigned, float v, int m) {
+    g_fvals[threadIdx.x] = v; g_bar.arrive_and_wait();
+    const float r = g_fvals[threadIdx.x ^ m];
+    g_bar.arrive_and_wait(); return r;
+}
 static const int *g_cell;
 static void nufft_taps(double, double, int, int &cell, float (&w)[kNuW]) {
     cell = g_cell[threadIdx.x];
@@ -84,7 +95,7 @@ static void nufft_taps64(double, double, int, int &cell, double (&w)[kNuW]) {
 #define __forceinline__
 @FUNCTION@
 struct Shared { LocSpread sp; float2 row[4096]; };
-extern "C" int spread(const int *cells, const int *active, int calls, int mrow, float *out) {
+extern "C" int spread(const int *cells, const int *active, int calls, int mrow, float *out, int voxels) {
     static Shared sh;
     g_lo = (const char *)&sh; g_hi = (const char *)(&sh + 1);
     g_races = 0; g_use.clear();
@@ -97,8 +108,8 @@ extern "C" int spread(const int *cells, const int *active, int calls, int mrow, 
                 threadIdx.x = l; t_epoch = 1000 * c;
                 const float2 v = make_float2(1.f + l, -2.f * l);
                 const bool on = active[32 * c + l] != 0;
-                if (c & 1) spread_row<false>(sh.sp, sh.row, mrow, 0.0, v, on, 0.0, 0);
-                else spread_row<true>(sh.sp, sh.row, mrow, 0.0, v, on, 0.0, 0);
+                if (voxels) spread_voxels(sh.sp, sh.row, 0.0, v, 0.0, 0);
+                else spread_row(sh.sp, sh.row, mrow, 0.0, v, on, 0.0, 0);
             });
         for (auto &x : t) x.join();
     }
@@ -112,17 +123,22 @@ extern "C" int spread(const int *cells, const int *active, int calls, int mrow, 
 def lib(tmp_path_factory):
     with open(SOURCE) as f:
         text = f.read()
-    body = re.search(r"template [^\n]*\n__device__ [^\n]*void spread_row\(.*?\n}\n", text, re.S)
-    assert body, "spread_row not found"
+    body = ""
+    for name in ("spread_row", "spread_voxels"):
+        m = re.search(r"__device__ [^\n]*void %s\(.*?\n}\n" % name, text, re.S)
+        assert m, name + " not found"
+        body += m.group(0)
+    body = body.replace("float *rowf = reinterpret_cast<float *>", "Comp *rowf = reinterpret_cast<Comp *>")
     d = tmp_path_factory.mktemp("spread")
     src, out = str(d / "spread.cpp"), str(d / "spread.so")
     with open(src, "w") as f:
-        f.write(HARNESS.replace("@FUNCTION@", body.group(0)))
+        f.write(HARNESS.replace("@FUNCTION@", body))
     subprocess.run(["g++", "-std=c++20", "-O1", "-shared", "-fPIC", "-pthread", "-w", "-o", out,
                     src], check=True)
     return ctypes.CDLL(out)
 
 
+@pytest.mark.parametrize("voxels", [False, True])
 @pytest.mark.parametrize("n,lo,hi,active", [
     (256, 40, 60, 32),     # one window
     (256, 40, 60, 8),      # node values of a box: a lane each
@@ -131,8 +147,9 @@ def lib(tmp_path_factory):
     (48, 30, 70, 32),      # a short grid, cells that wrap past its end
     (32, 0, 32, 32),
 ])
-def test_no_lane_reads_what_another_wrote(lib, n, lo, hi, active):
+def test_no_lane_reads_what_another_wrote(lib, n, lo, hi, active, voxels):
     rng = np.random.default_rng(n + hi)
+    active = 32 if voxels else active
     calls, mrow = 3, n + 16
     cells = np.sort(rng.integers(lo, hi, (calls, 32)) % n, axis=1).astype(np.int32)
     rng.shuffle(cells, axis=1)
@@ -140,7 +157,7 @@ def test_no_lane_reads_what_another_wrote(lib, n, lo, hi, active):
     act[:, :active] = 1
     out = np.zeros((mrow, 2), np.float32)
     p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
-    races = lib.spread(p(cells), p(act), calls, mrow, p(out))
+    races = lib.spread(p(cells), p(act), calls, mrow, p(out), int(voxels))
     ref = np.zeros((mrow, 2))
     for c in range(calls):
         for lane in range(active):
