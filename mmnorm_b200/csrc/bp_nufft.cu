@@ -141,29 +141,33 @@ __device__ __forceinline__ void cell_window(const float *box, const AntRec &ar, 
 }
 
 // Forward rows: rows[a][jj] = (G_k.re, G_k.im) for cell k = (jj - (W/2 - 1)) mod N, jj < row.
-// One lane per cell, over the cells of the antenna's window only: a 0.19 m grid at 4 GHz touches
-// about 30 of the 400 cells of 200 samples (592 us for all cells of 4096 antennas).  Cells
-// outside the window are left unwritten and are never read.  blockIdx.y: every gridDim.y-th
-// 32 cells of a window, where few antennas would leave their wide windows to a warp each (4
-// antennas x 1000 samples over a 10 m scene: 0.88 ms for the image, 0.15 so).
+// One block per antenna, one lane per cell, a quarter of the samples per warp (their sums added in
+// order), over the cells of the antenna's window only: a 0.19 m grid at 4 GHz touches about 30 of
+// the 400 cells of 200 samples (592 us for all cells of 4096 antennas).  Cells outside the window
+// are left unwritten and are never read.  blockIdx.y: every gridDim.y-th 32 cells of a window.
+// Both splits are for few antennas, whose windows a warp or two took long over: 4 antennas x 1000
+// samples over a 10 m scene, the whole image 0.88 ms with a warp an antenna, 0.15 with a warp per
+// 32 cells, 0.076 so.
 constexpr int kGridWarps = 4;
 __global__ void __launch_bounds__(kGridWarps * 32)
-    nufft_grid_window_kernel(const float2 *__restrict__ meas, int A, int F, int N, int J0, int row,
+    nufft_grid_window_kernel(const float2 *__restrict__ meas, int F, int N, int J0, int row,
                              const double *__restrict__ sc, const double2 *__restrict__ tw,
                              const AntRec *__restrict__ ant, const float *__restrict__ box,
                              double ti, double uq, float2 *__restrict__ rows) {
-    const int a = blockIdx.x * kGridWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (a >= A) return;
+    __shared__ double2 part[kGridWarps][32];
+    const int a = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int first, count;
     cell_window(box, ant[a], ti, uq, N, first, count);
     const float2 *m = meas + (size_t)a * F;
     float2 *out = rows + (size_t)a * row;
-    for (int c = blockIdx.y * 32 + lane; c < count; c += 32 * gridDim.y) {
-        const int k = (int)((((int64_t)first + c) % N + N) % N);
-        int idx = (int)((((int64_t)(-J0) * k) % N + N) % N);  // (j - J0) k mod N at j = 0
+    const int j0 = (int)((int64_t)F * warp / kGridWarps);
+    const int j1 = (int)((int64_t)F * (warp + 1) / kGridWarps);
+    for (int c0 = blockIdx.y * 32; c0 < count; c0 += 32 * gridDim.y) {
+        const int k = (int)((((int64_t)first + min(c0 + lane, count - 1)) % N + N) % N);
+        int idx = (int)((((int64_t)(j0 - J0) * k) % N + N) % N);  // (j - J0) k mod N at j = j0
         double gr = 0.0, gi = 0.0;
 #pragma unroll 4
-        for (int j = 0; j < F; ++j) {
+        for (int j = j0; j < j1; ++j) {
             const float2 mv = __ldg(m + j);
             const double s = __ldg(sc + j);
             const double2 t = __ldg(tw + idx);
@@ -173,8 +177,18 @@ __global__ void __launch_bounds__(kGridWarps * 32)
             idx += k;
             if (idx >= N) idx -= N;
         }
-        for (int jj = (k + kNuW / 2 - 1) % N; jj < row; jj += N)
-            out[jj] = make_float2((float)gr, (float)gi);
+        part[warp][lane] = make_double2(gr, gi);
+        __syncthreads();
+        if (warp == 0 && c0 + lane < count) {
+#pragma unroll
+            for (int w = 1; w < kGridWarps; ++w) {
+                gr += part[w][lane].x;
+                gi += part[w][lane].y;
+            }
+            for (int jj = (k + kNuW / 2 - 1) % N; jj < row; jj += N)
+                out[jj] = make_float2((float)gr, (float)gi);
+        }
+        __syncthreads();
     }
 }
 
@@ -477,10 +491,9 @@ cudaError_t launch_nufft_grid_window(const float *meas, int A, int F, int N, int
                                      const double *sc, const double2 *tw, const AntRec *ant,
                                      const float *box, double ti, double uq, float2 *rows,
                                      cudaStream_t stream) {
-    const int groups = (A + kGridWarps - 1) / kGridWarps;
-    const int parts = std::max(1, std::min((N + 31) / 32, 148 * 8 / groups));
-    nufft_grid_window_kernel<<<dim3(groups, parts), kGridWarps * 32, 0, stream>>>(
-        reinterpret_cast<const float2 *>(meas), A, F, N, J0, row, sc, tw, ant, box, ti, uq, rows);
+    const int parts = std::max(1, std::min((N + 31) / 32, 148 * 8 / A));
+    nufft_grid_window_kernel<<<dim3(A, parts), kGridWarps * 32, 0, stream>>>(
+        reinterpret_cast<const float2 *>(meas), F, N, J0, row, sc, tw, ant, box, ti, uq, rows);
     return cudaGetLastError();
 }
 
