@@ -375,12 +375,14 @@ struct NuVariant {
 // Variant 0, the default, is the tile-local form (bp_local.cu; its pointers are filled in by
 // bwd_pos_nufft_kernel_ptr).  The others are launch shapes of this file's tap-run kernel: at
 // 64^3 voxels, 4096 antennas, 128 samples (position pass alone; with vote term / image loss
-// only) 9.64/8.16, 11.1/11.8, 10.7/9.85 ms in this order.
+// only) 9.08/8.22, 12.1/11.8, 10.6/9.82 and 8.97/8.21 ms in this order (4.55/3.73 the default).  The
+// last was variant 0 before the local form; it keeps its name, at the end.
 const NuVariant kNuVariants[] = {
     {4, 128, 0, nullptr, nullptr, "interp_local_t4_n128"},
     MMN_NU_VARIANT(2, 256, 24),
     MMN_NU_VARIANT(1, 256, 48),
     MMN_NU_VARIANT(1, 128, 16),
+    MMN_NU_VARIANT(2, 128, 24),
 };
 #undef MMN_NU_VARIANT
 
