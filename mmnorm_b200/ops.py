@@ -22,9 +22,16 @@ def _vp(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
 
 
+# The current stream's handle without a Stream object around it (1 us of a small call); not part of
+# torch's public interface, so a build without it takes the public way.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device):
+    if _raw_stream is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
     index = device.index if device.index is not None else torch.cuda.current_device()
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(index))
+    return ctypes.c_void_p(_raw_stream(index))
 
 
 def _plain(t):
