@@ -447,6 +447,16 @@ int mmn_cuda_sn_est_fast(float *normals_x, float *normals_y, float *normals_z,
 int mmn_fp32_peak_probe(int blocks, int iters, float *out, cudaStream_t stream);
 
 /*
+ * Check of the interpolated mode's exact form (no counterpart in the reference): its short
+ * evaluations against the library functions whose bits they promise, for the floats with bit
+ * patterns first .. first + count - 1 (taken as squared legs and, if wavelength > 0, as paths).
+ * counts (device, 3 words): square roots that differ, phasors that differ, phasors that left the
+ * decision to the library functions.
+ */
+int mmn_interp_exact_probe(uint32_t first, uint64_t count, float wavelength, uint64_t *counts,
+                           cudaStream_t stream);
+
+/*
  * Bounded-wait check (no counterpart in the reference, whose kernels have no waits): one
  * warp waits on an mbarrier with the same bounded wait the copy pipelines use (which give up
  * after one second), here giving up after `limit_us` microseconds (at most 10 s, else

@@ -139,6 +139,7 @@ SIGNATURES = [
                                   _F, _F, _F, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _SZ,
                                   _P]),
     ("mmn_fp32_peak_probe", _I, [_I, _I, _P, _P]),
+    ("mmn_interp_exact_probe", _I, [ctypes.c_uint32, ctypes.c_uint64, _F, _P, _P]),
     ("mmn_wait_timeout_probe", _I, [ctypes.c_uint32, _I, _P, _P]),
     ("mmn_batch_create", _I, [_PROB, _I32, _I32, _P, _P, _I32, ctypes.POINTER(_P),
                               ctypes.POINTER(_SZ)]),

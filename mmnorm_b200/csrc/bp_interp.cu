@@ -869,7 +869,7 @@ unsigned pack_blocks(int64_t count) {
 }  // namespace
 
 // The run kernel where it wastes little: whole columns of the grid are covered, so the slots past
-// a column's end (nz not a multiple of 4) and the parts of the first and last column outside
+// a column's end (nz odd) and the parts of the first and last column outside
 // [start, start + count) are idle.
 static bool image_runs(const InterpParams &p, int64_t *first, int *runs, unsigned *blocks) {
     *first = p.start / p.nz;
@@ -926,3 +926,52 @@ cudaError_t launch_interp_normals_fast(const InterpParams &p, cudaStream_t strea
 }
 
 }  // namespace mmn
+
+namespace mmn {
+namespace {
+
+__device__ __forceinline__ bool same_float(float a, float b) {
+    return __float_as_uint(a) == __float_as_uint(b) || (a != a && b != b);
+}
+
+// Whether the exact form's short evaluations give the library functions' bits, for the floats with
+// bit patterns first .. first + count - 1: counts[0] square roots that differ (either half of
+// sqrt2), counts[1] phasors of a path that differ, counts[2] phasors that took the library.
+__global__ void exact_probe_kernel(uint32_t first, uint64_t count, float wavelength, double ninv,
+                                   unsigned long long *counts) {
+    unsigned long long bad_root = 0, bad_phasor = 0, library = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const float x = __uint_as_float(first + (uint32_t)i);
+        const float2 r = sqrt2(make_float2(x, 2.f)), s = sqrt2(make_float2(2.f, x));
+        const float root = sqrtf(x);
+        if (!same_float(r.x, root) || !same_float(s.y, root)) ++bad_root;
+        if (wavelength > 0.f) {
+            float c, sn;
+            if (!phasor_exact(x, ninv, c, sn)) {
+                ++library;
+            } else {
+                const float2 l = phasor_library(x, wavelength);
+                if (!same_float(c, l.x) || !same_float(sn, l.y)) ++bad_phasor;
+            }
+        }
+    }
+    atomicAdd(counts, bad_root);
+    atomicAdd(counts + 1, bad_phasor);
+    atomicAdd(counts + 2, library);
+}
+
+}  // namespace
+}  // namespace mmn
+
+extern "C" int mmn_interp_exact_probe(uint32_t first, uint64_t count, float wavelength,
+                                      uint64_t *counts, cudaStream_t stream) {
+    if (count < 1 || count > 0x100000000ull) return MMN_ERR_INVALID_ARGUMENT;
+    if (!counts) return MMN_ERR_NULL_POINTER;
+    if (cudaMemsetAsync(counts, 0, 3 * sizeof(uint64_t), stream) != cudaSuccess)
+        return MMN_ERR_CUDA;
+    mmn::exact_probe_kernel<<<148 * 8, 256, 0, stream>>>(
+        first, count, wavelength, -1.0 / (double)wavelength,
+        reinterpret_cast<unsigned long long *>(counts));
+    return cudaGetLastError() == cudaSuccess ? MMN_OK : MMN_ERR_CUDA;
+}
