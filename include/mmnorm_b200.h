@@ -164,7 +164,7 @@ int mmn_get_position_variant(void); /* the selected index */
  * Fused backprojection + vote with the per-(voxel, antenna) sample sum evaluated by
  * interpolation (no counterpart in the reference; not its "interpolated mode", which reads
  * one range bin): each antenna's samples go once onto a 2x oversampled grid, and each
- * (voxel, antenna) evaluates a polynomial of 8-24 terms that its voxel box took from the
+ * (voxel, antenna) evaluates a polynomial of 8-12 terms that its voxel box took from the
  * grid (8 cells a node, exponential-of-semicircle weights) -- a type-2 non-uniform FFT whose
  * cost per pair does not grow with F.  Same outputs and problem fields as
  * mmn_backproject in MMN_MODE_MIXED, ~1e-7 relative from it; F up to ~3000

@@ -29,10 +29,10 @@
 //    antenna pairs in the halves of FFMA2 (the sample duplicated into (re, re, im, im)
 //    or antenna-pair records), or scalar FFMA.
 //
-// Bound of the second-order forms: instruction dispatch, where a packed instruction takes about
-// two slots: per pair of the default variant 8 a step of its two chains, 1/2 a shared load, some
-// 110 for range, rotation and vote and 32 a block (128^3 voxels x 4096 antennas x 256 samples:
-// 1300 of the 1316 slots that pass).  Integer turn counts by one FP64 FMA each and the range's
+// Bound of the second-order forms: the FMA lanes, which a packed instruction holds for two cycles
+// (FP64 runs beside them).  They are 83 % busy at 256 samples and 70-72 % at 100 and 64, where
+// range, rotation, vote and anchor -- half FMA work, half conversions, sines and loads -- are a
+// larger part.  Integer turn counts by one FP64 FMA each and the range's
 // shared Newton factor took 48^3 x 1024 x 64 from 1418 to 1340 us; running a row's last partial
 // block on the same chains instead of a scalar first-order loop took a 75 x 61 x 53 grid x 1236
 // antennas x 100 samples from 6.85 to 5.56 ms.

@@ -449,8 +449,8 @@ __device__ __forceinline__ bool phasor_exact(float path, double ninv, float &c, 
 }
 
 // The reference's FP32 phasors of two paths, bit for bit: about one evaluation in 4000 cannot
-// decide its rounding and takes the library functions.  Bound: instruction dispatch (the FP64
-// and packed instructions take about two slots).  90 x 100 x 70 voxels x 4096 antennas, four
+// decide its rounding and takes the library functions.  Bound: instruction issue (142 a pair,
+// active 79 % of cycles), then the conversions and root seeds (XU 41 %).  90 x 100 x 70 voxels x 4096 antennas, four
 // receivers, TI offset: 20.3 ms with the two library calls per pair, 13.5 ms.
 __device__ __forceinline__ void phasor2_exact(float2 path, float wavelength, double ninv,
                                               float2 &c, float2 &s) {

@@ -1,5 +1,5 @@
 // bp_local.cu -- the interpolation form by tile-local polynomials: the forward kernel of mode
-// "nufft" (mmn_backproject_nufft).
+// "nufft" (mmn_backproject_nufft) and the default kernels of both gradients.
 //
 // One antenna's sample sum is e^{-2pi i d t0c} M(u), u = d slope/c, with M band-limited
 // (bp_nufft.cu).  Over a compact box of voxels u covers a short interval only, on which M is a
@@ -13,7 +13,7 @@
 //      image + vote sums.
 // Per (voxel, antenna) that leaves NN packed FMAs on coefficients that all voxels of the thread
 // share, where a tap run per pair costs 44 FMAs of weights, 8 shared loads and the FP64 cell
-// index.  A thread owns 4 voxels in a row along z, whose lateral distance is one.
+// index.  A thread owns 4 voxels in a row along one axis, whose lateral distance is one.
 //
 // NN follows from theta = pi F |slope| / c * D, the largest phase excursion of M over the half
 // width (local_nodes).  Up to NN = 12 the polynomial is evaluated in monomials by Horner (theta
@@ -21,10 +21,11 @@
 // antenna whose theta is larger (from a 7 to 11 mm voxel pitch on at 4 GHz of bandwidth), or not a
 // number, takes a tap run per pair (local_chunk).
 //
-// Bound: instruction dispatch (68 instructions a pair, 235 dispatch slots a pair before; packed
-// FP32 and FP64 instructions take about two slots).  Measured on 96^3 voxels x 4096 antennas x
-// 200 samples: 23.5 ms for the whole forward with a tap run per pair, 9.2 ms with this kernel;
-// error against 64 bits 1.2e-6 before, 2.4e-7 now (sums over 32 antennas at a time).  96 or 80
+// Bound: no single unit.  64^3 x 4096 x 128: 58 instructions a pair, issue 61 % active, FMA lanes
+// 50 % (a packed instruction holds them two cycles), FP64 23 %, conversions 29 %, with the four
+// warps a scheduler that 128 registers leave waiting out fixed latencies.  Measured on 96^3 voxels
+// x 4096 antennas x 200 samples: 23.5 ms for the whole forward with a tap run per pair, 9.0 ms with
+// this kernel; error against 64 bits 1.1e-6 before, 2.3e-7 now (sums over 32 antennas at a time).  96 or 80
 // registers (5 or 6 CTAs per SM) measured the same or 2 % slower than 128.  The hardware sine
 // and cosine in place of cis_half_pair: 8.1 ms, but 2.2e-7 of error on short sums, more than
 // the tap form's.
@@ -746,13 +747,14 @@ const void *bwd_pos_local_kernel_ptr(bool vote, int *threads) {
 // sum_v h_v T_q(x_v) in registers (two packed instructions each); the transposed interpolation
 // turns the moments into NN node values, and only those are spread onto the antenna's grid row
 // (8 cells each).  A warp owns one antenna and its row and walks a range of boxes, 32 voxel
-// runs at a time; everything is summed in a fixed order.  Boxes too wide for the nodes spread
-// every voxel.
+// runs at a time; everything is summed in a fixed order.  Boxes too wide for the nodes go in parts,
+// and parts of 128 voxels that still are spread every voxel.
 //
-// A box costs some 500 instructions besides its voxels' 85 each (bounds, the warp sums, the
+// A box costs some 700 instructions besides its voxels' 90 each (bounds, the warp sums, the
 // spread), so boxes are larger than the forward's where enough of them remain to fill the GPU:
 // 2048, else 1024, else 512 voxels.  64^3 voxels x 4096 antennas x 128 samples (this pass):
-// 16.3 ms with a spread per voxel, 6.2 / 5.1 / 4.5 ms with boxes of 512 / 1024 / 2048.
+// 16.3 ms with a spread per voxel, 6.2 / 5.1 / 4.5 ms with boxes of 512 / 1024 / 2048.  Bound as
+// the forward: 94 instructions a pair, issue 62 % active, FMA lanes 49 %, conversions 29 %.
 namespace {
 
 constexpr int kLocMeasWarps = 4;

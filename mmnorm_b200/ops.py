@@ -124,7 +124,7 @@ def backproject(x_locs, y_locs, z_locs, antenna_locs, rx_offsets, meas, waveleng
     ``mode``: 'mixed' (FP64 range/wrap + FP32 recurrence), 'plain' (FP32 sincos per
     sample), 'interp' (reference interpolated mode; ``meas`` holds range-FFT bins) or
     'nufft' (the mixed form's sum by polynomials over voxel boxes, taken from each antenna's
-    2x oversampled grid; ~1e-7 from the exact sum, 8-24 terms instead of F per voxel and
+    2x oversampled grid; ~1e-7 from the exact sum, 8-12 terms instead of F per voxel and
     antenna; F <= ~3000).
     """
     meas = _plain(meas)

@@ -16,7 +16,7 @@ and the full matched filter runs the mixed-precision kernel (FP64 range and phas
 wrap, FP32 rotation recurrence) instead of one FP64 sin/cos pair per sample.
 ``precision='plain'`` selects the FP32 sincos-per-sample kernel instead, and
 ``precision='nufft'`` the same sums by local polynomials from per-antenna oversampled
-grids (~2e-6 from the mixed form, faster for F above ~100; F up to ~1500).  In
+grids (~2e-6 from the mixed form, faster for F above ~100; F up to ~3000).  In
 interpolated mode the default is the reference's arithmetic bit for bit, and
 ``precision='fast'`` the fast form: the same range bins, the phasor from the wrapped
 FP32 turn count and the hardware sine/cosine (~5e-7 per term from the reference's).
