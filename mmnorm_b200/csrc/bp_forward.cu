@@ -1056,11 +1056,12 @@ const FwdVariant *fwd_variants(int *count) {
     // mixed_clen_fx2_t4_n128 78.5 -> 77.0 on 128^3 voxels x 1024 antennas x 256 samples;
     // plain_t2_n256 9.88 -> 9.39 s at 16384 antennas); it cost
     // mixed_clen64_fx2_t4_n128 75.0 -> 80.4, mixed_antpair_fx2_t1_n256 86.5 -> 89.2 and
-    // mixed_ffma_t4_n128 105 -> 117.
+    // mixed_ffma_t4_n128 105 -> 117.  The forms with 64-bit block steps have none: 48^3 voxels x
+    // 1024 antennas x 1600 samples takes 29.3 ms without, 32.5 with 2 and 35.2 with 1.
     static const FwdVariant v[] = {
         // default: 64-sample blocks as two second-order chains in z^2 (near the Horner
         // form's accuracy at close to the fastest form's speed)
-        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), 0, fwd_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2, 2>(), pers_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2, 2>()},
+        {2, 256, false, 8, fwd_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), "mixed_clen64eo_fx2_t2_n256", 0, pers_ptr<2, 256, kFormMixedClenEO, kAnchorFixed2, 2>(), 0, fwd_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2>(), pers_ptr<2, 256, kFormMixedClenEOWide, kAnchorFixed2>()},
         {4, 128, false, 8, fwd_ptr<4, 128, kFormMixedClen, kAnchorFixed2, 1>(), "mixed_clen_fx2_t4_n128_s24", 0, pers_ptr<4, 128, kFormMixedClen, kAnchorFixed2>(), 24 * 1024},
         {2, 256, false, 16, fwd_ptr<2, 256, kFormMixedPair, kAnchorFixed>(), "mixed_ffma2_fx_t2_n256", 1, pers_ptr<2, 256, kFormMixedPair, kAnchorFixed>()},
         // each block as two 16-step chains joined by z^16 (kFormMixedPairSplit)
